@@ -213,6 +213,14 @@ int Engine::init(const pbf_domain_configuration* scenes, const uint32_t scene_co
     float* d_radii = arena_.alloc<float>(scene_count, e);
     predicted_ = arena_.alloc<float4>(count_, e);
     packed_ = alloc_packed(arena_, count_, e);
+    bool boundary = false;
+    for (uint32_t s = 0; s < scene_count; ++s) boundary = boundary || scenes[s].boundary_particle_count > 0;
+    if (mode == PBF_EXECUTION_FORWARD && !boundary) {
+        packed_next_ = alloc_packed(arena_, count_, e);
+        packed_velocity_ = alloc_packed(arena_, count_, e);
+        packed_mass_ = arena_.alloc<float>(static_cast<size_t>(count_) + 4u, e);
+        packed_magnitude_ = arena_.alloc<float>(static_cast<size_t>(count_) + 4u, e);
+    }
     arrival_ = arena_.alloc<uint32_t>(count_, e);
     unordered_ = arena_.alloc<uint32_t>(count_, e);
     tile_sums_ = arena_.alloc<uint32_t>(scan_tile_count(cells_ + 1), e);
@@ -357,7 +365,8 @@ int Engine::allocate_record(StepRecord& r) {
         for (auto& p : r.checkpoints) p = r.arena.alloc<float4>(n, e);
     }
     r.lambda.assign(keep ? K : (K ? 1 : 0), nullptr);
-    for (auto& p : r.lambda) p = r.arena.alloc<float>(n, e);
+    // the staged passes read lambda sixteen bytes at a time
+    for (auto& p : r.lambda) p = r.arena.alloc<float>(static_cast<size_t>(n) + 4u, e);
     if (keep) {
         r.density.assign(K, nullptr);
         r.gsum.assign(K, nullptr);
@@ -371,7 +380,7 @@ int Engine::allocate_record(StepRecord& r) {
         for (uint32_t k = 0; k < K; ++k) r.mask[k] = r.arena.alloc<uint8_t>(n, e);
     }
     r.first_density = r.arena.alloc<float>(n, e);
-    r.first_lambda = r.arena.alloc<float>(n, e);
+    r.first_lambda = r.arena.alloc<float>(static_cast<size_t>(n) + 4u, e);
     r.neighbor_count = r.arena.alloc<uint32_t>(n, e);
     r.velocity = r.arena.alloc<float4>(n, e);
     r.vorticity = r.arena.alloc<float4>(n, e);
@@ -387,6 +396,7 @@ int Engine::allocate_record(StepRecord& r) {
         r.list_entries[l] = r.arena.alloc<uint32_t>(padded * r.list_capacity, e);
         r.list_counts[l] = r.arena.alloc<uint32_t>(n, e);
     }
+    if (packed_mass_) r.list_windows = r.arena.alloc<uint32_t>(window_words(n), e);
     if (boundary_count_ > 0) {
         r.boundary_offsets = r.arena.alloc<uint32_t>(cells_ + 1, e);
         r.boundary = r.arena.alloc<float4>(boundary_count_, e);
@@ -541,6 +551,7 @@ int Engine::launch_forward(cudaStream_t stream, const pbf_particle_state* state,
     g.params_b = r.params_b;
     g.input_flags = input_checks_ ? d_input_flags_ : nullptr;
     g.packed = packed_;
+    g.packed_mass = packed_mass_;
     timer_.begin(stream, kPassGrid);
     if (int rc = check(launch_grid_build(stream, g), "grid build")) return rc;
     if (boundary_count_ > 0) {
@@ -550,17 +561,19 @@ int Engine::launch_forward(cudaStream_t stream, const pbf_particle_state* state,
     }
     timer_.end(stream, kPassGrid);
 
+    if (runs_staged(shape_, diff, boundary_count_ > 0, K)) {
+        if (int rc = launch_staged(stream, state, next_state, r)) return rc;
+        return check(launch_advance_step(stream, d_step_), "step counter");
+    }
     const GatherCommon gc = gather_common(r);
     const Field3 previous{state->positions.x, state->positions.y, state->positions.z};
     const MutField3 out_positions{next_state->positions.x, next_state->positions.y, next_state->positions.z};
-    // Forward-mode steps of scenes without boundary particles may store hit-mask lists (launch shape).
-    const int masks = stores_masks(shape_, diff, boundary_count_ > 0) ? 1 : 0;
     for (uint32_t k = 0; k < K; ++k) {
         const float4* xk = r.iterate(k, K, diff);
         float4* xk1 = const_cast<float4*>(r.iterate(k + 1, K, diff));
         float* lam = keep ? r.lambda[k] : (k == 0 ? r.first_lambda : r.lambda[0]);
         const uint32_t l = keep ? k : 0u;
-        const StoredList list{r.list_entries[l], r.list_counts[l], r.list_capacity, masks};
+        const StoredList list{r.list_entries[l], r.list_counts[l], r.list_capacity};
         ListScanArgs scan{gc, xk, list, 1};
         scan.packed = packed_;
         DensityLambdaArgs d{gc, xk, lam, keep ? r.density[k] : (k == 0 ? r.first_density : nullptr),
@@ -596,16 +609,9 @@ int Engine::launch_forward(cudaStream_t stream, const pbf_particle_state* state,
                            "reconstruct"))
             return rc;
     }
-    // next_state.positions are final here.  Under capture the record must be external to become an
-    // event node of the graph; outside a capture it is a plain record.
-    if (positions_ready_) {
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        if (int rc = check(cudaStreamIsCapturing(stream, &capture), "capture status")) return rc;
-        const unsigned flags = capture == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault;
-        if (int rc = check(cudaEventRecordWithFlags(positions_ready_, stream, flags), "positions event")) return rc;
-    }
+    if (int rc = record_positions_ready(stream)) return rc;
     const uint32_t lp = keep ? K : 0u;
-    const StoredList post{r.list_entries[lp], r.list_counts[lp], r.list_capacity, masks};
+    const StoredList post{r.list_entries[lp], r.list_counts[lp], r.list_capacity};
     timer_.begin(stream, kPassListScan);
     ListScanArgs post_scan{gc, xK, post};
     post_scan.packed = packed_;
@@ -629,6 +635,62 @@ int Engine::launch_forward(cudaStream_t stream, const pbf_particle_state* state,
     if (int rc = check(launch_xsph(stream, x, shape_.block), "xsph")) return rc;
     timer_.end(stream, kPassXsph);
     return check(launch_advance_step(stream, d_step_), "step counter");
+}
+
+// next_state.positions are final here.  Under capture the record must be external to become an event
+// node of the graph; outside a capture it is a plain record.
+int Engine::record_positions_ready(cudaStream_t stream) {
+    if (!positions_ready_) return PBF_SUCCESS;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (int rc = check(cudaStreamIsCapturing(stream, &capture), "capture status")) return rc;
+    const unsigned flags = capture == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault;
+    return check(cudaEventRecordWithFlags(positions_ready_, stream, flags), "positions event");
+}
+
+// The Jacobi iterations and the post-loop passes over staged windows (staged.cu): two kernels per
+// iteration, then three.
+int Engine::launch_staged(cudaStream_t stream, const pbf_particle_state* state, pbf_particle_state* next_state, StepRecord& r) {
+    const GatherCommon gc = gather_common(r);
+    // passes that read what their predecessor wrote last start there (it is the part still in L2)
+    GatherCommon gc_reverse = gc;
+    gc_reverse.reverse = 1;
+    const uint32_t K = iterations_;
+    const StagedList list{{r.list_entries[0], r.list_counts[0], r.list_capacity}, r.list_windows};
+    PackedPositions current = packed_, next = packed_next_;
+    for (uint32_t k = 0; k < K; ++k) {
+        const float4* xk = r.iterate(k, K, false);
+        float* lambda = k == 0 ? r.first_lambda : r.lambda[0];
+        const StagedDensityArgs d{gc, list, current, packed_mass_, xk, lambda, k == 0 ? r.first_density : nullptr,
+                                  k == 0 ? r.neighbor_count : nullptr};
+        timer_.begin(stream, kPassScanDensityLambda);
+        if (int rc = check(launch_staged_density(stream, d), "staged scan + density/lambda")) return rc;
+        timer_.end(stream, kPassScanDensityLambda);
+        const StagedCorrectionArgs c{gc_reverse, list, current, packed_mass_, lambda, xk, next,
+                                     const_cast<float4*>(r.iterate(k + 1, K, false)), k + 1 == K ? 1 : 0,
+                                     {state->positions.x, state->positions.y, state->positions.z}, r.sorted_index,
+                                     {next_state->positions.x, next_state->positions.y, next_state->positions.z}, r.velocity,
+                                     packed_velocity_};
+        timer_.begin(stream, kPassCorrection);
+        if (int rc = check(launch_staged_correction(stream, c), "staged correction/project")) return rc;
+        timer_.end(stream, kPassCorrection);
+        std::swap(current, next);
+    }
+    if (int rc = record_positions_ready(stream)) return rc;
+    const float4* xK = r.iterate(K, K, false);
+    const StagedVorticityArgs v{gc_reverse, list, current, packed_velocity_, xK, r.velocity, r.vorticity, packed_magnitude_};
+    timer_.begin(stream, kPassVorticity);
+    if (int rc = check(launch_staged_vorticity(stream, v), "staged scan + vorticity")) return rc;
+    timer_.end(stream, kPassVorticity);
+    const StagedNormalArgs n{gc, list, current, packed_magnitude_, xK, r.velocity, r.vorticity, r.normal, r.confined, next};
+    timer_.begin(stream, kPassNormal);
+    if (int rc = check(launch_staged_normal(stream, n), "staged normal/confinement")) return rc;
+    timer_.end(stream, kPassNormal);
+    const StagedXsphArgs x{gc_reverse, list, current, next, xK, r.confined, r.sorted_index,
+                           {next_state->velocities.x, next_state->velocities.y, next_state->velocities.z}};
+    timer_.begin(stream, kPassXsph);
+    if (int rc = check(launch_staged_xsph(stream, x), "staged xsph")) return rc;
+    timer_.end(stream, kPassXsph);
+    return PBF_SUCCESS;
 }
 
 int Engine::segment_workspace(Segment** out) {
@@ -730,22 +792,25 @@ int Engine::autotune(const pbf_particle_state* state, const pbf_control* control
         timer_.enable(false);
         return rc;
     };
-    const uint32_t scans[5] = {kScanPerLane, kScanCooperative, kScanStaged, kScanFusedDensity, kScanFusedMasks};
+    const uint32_t scans[4] = {kScanPerLane, kScanCooperative, kScanStaged, kScanStaged16};
     const uint32_t blocks[4] = {32u, 64u, 96u, 128u};
     double ms[kPassCount];
     int rc = PBF_SUCCESS;
-    // 1. the list scan: variant x block size, by the time of the scans and the density + lambda
-    //    passes (one kernel in the fused variant)
+    // 1. the list scan: variant x block size, by the time of the scans and the gather passes (the
+    //    variants differ in which passes they fuse).  The staged passes have a block size of their own.
+    const bool staged = runs_staged(LaunchShape{kScanStaged16, 128u, 128u}, differentiable(), boundary_count_ > 0, iterations_);
     LaunchShape best = previous;
     best.block = 128u;
     double best_scan = -1.0;
-    for (int v = 0; v < 5 && !rc; ++v)
+    for (int v = 0; v < 4 && !rc; ++v)
         for (int b = 0; b < 4 && !rc; ++b) {
+            if (staged && scans[v] == kScanStaged16 && b != 3) continue;
             shape_ = best;
             shape_.scan = scans[v];
             shape_.scan_block = blocks[b];
             if ((rc = measure(ms))) break;
-            const double scan_ms = ms[kPassListScan] + ms[kPassDensityLambda] + ms[kPassScanDensityLambda];
+            double scan_ms = ms[kPassListScan] + ms[kPassDensityLambda] + ms[kPassScanDensityLambda];
+            for (const int pass : {kPassCorrection, kPassVorticity, kPassNormal, kPassXsph}) scan_ms += ms[pass];
             if (best_scan < 0.0 || scan_ms < best_scan) {
                 best_scan = scan_ms;
                 best.scan = scans[v];

@@ -16,7 +16,7 @@
 // math (sqrt, divisions) keeps that math convergent across the warp.
 #include <climits>
 
-#include "gather.cuh"
+#include "forward_ops.cuh"
 
 namespace pbf {
 
@@ -76,72 +76,6 @@ struct RangeScan {
     }
 };
 
-// The same test over positions stored as three arrays, two candidates per packed FP32 instruction
-// (__fadd2_rn, __fmul2_rn, __ffma2_rn round each half exactly as the scalar intrinsics do).  The
-// difference is taken as candidate minus particle; it is the exact negation of the scalar form's
-// particle minus candidate, so the squared distance has the same bits.  Groups of four slots are
-// loaded as one aligned float4 per axis: a range is widened down to a multiple of four and the
-// slots outside it are dropped from the mask.
-struct PackedScan {
-    float2 nx, ny, nz;   // the particle's negated coordinates, in both halves
-    float threshold;
-    uint32_t capacity;
-    uint32_t* __restrict__ entries;
-    uint32_t n;
-
-    __device__ __forceinline__ uint32_t hits2(const float2 x, const float2 y, const float2 z) const {
-        const float2 dx = __fadd2_rn(x, nx), dy = __fadd2_rn(y, ny), dz = __fadd2_rn(z, nz);
-        const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dx, dx, __fmul2_rn(dy, dy)));
-        return (r2.x < threshold ? 1u : 0u) | (r2.y < threshold ? 2u : 0u);
-    }
-    __device__ __forceinline__ uint32_t hits4(const float4 x, const float4 y, const float4 z) const {
-        return hits2(make_float2(x.x, x.y), make_float2(y.x, y.y), make_float2(z.x, z.y)) |
-               (hits2(make_float2(x.z, x.w), make_float2(y.z, y.w), make_float2(z.z, z.w)) << 2);
-    }
-    __device__ __forceinline__ void append(uint32_t mask, const uint32_t base) {
-        while (mask) {
-            const uint32_t k = static_cast<uint32_t>(__ffs(mask)) - 1u;
-            if (n < capacity) entries[static_cast<size_t>(n) * 32u] = base + k;
-            ++n;
-            mask &= mask - 1u;
-        }
-    }
-    // Hit mask of the 32-slot block at `base` (4-aligned) of the range [first, end).
-    __device__ __forceinline__ uint32_t block_mask(const PackedPositions p, const uint32_t base, const uint32_t first,
-                                                   const uint32_t end) const {
-        const uint32_t stop = min(end, base + 32u);
-        uint32_t mask = 0u;
-        for (uint32_t k = 0u; base + k < stop; k += 4u) {
-            const uint32_t t = base + k;
-            mask |= hits4(*reinterpret_cast<const float4*>(p.x + t), *reinterpret_cast<const float4*>(p.y + t),
-                          *reinterpret_cast<const float4*>(p.z + t))
-                    << k;
-        }
-        if (base < first) mask &= ~0u << (first - base);
-        if (end - base < 32u) mask &= (1u << (end - base)) - 1u;
-        return mask;
-    }
-    __device__ __forceinline__ void run(const PackedPositions p, const uint32_t first, const uint32_t end) {
-        if (first >= end) return;
-        for (uint32_t base = first & ~3u; base < end; base += 32u) append(block_mask(p, base, first, end), base);
-    }
-    // The same blocks stored as a hit-mask list: one (base, mask) pair per block with a hit, `pairs`
-    // of them so far (at most `pair_capacity` are written), `n` neighbours.
-    __device__ __forceinline__ void run_masks(const PackedPositions p, const uint32_t first, const uint32_t end,
-                                              uint2* __restrict__ row, const uint32_t pair_capacity, uint32_t& pairs) {
-        if (first >= end) return;
-        for (uint32_t base = first & ~3u; base < end; base += 32u) {
-            const uint32_t mask = block_mask(p, base, first, end);
-            if (mask) {
-                if (pairs < pair_capacity) row[static_cast<size_t>(pairs) * 32u] = make_uint2(base, mask);
-                ++pairs;
-                n += static_cast<uint32_t>(__popc(mask));
-            }
-        }
-    }
-};
-
-template <bool Masks>
 __global__ void __launch_bounds__(kBlock, 12) list_walk_kernel(const ListScanArgs a) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= a.g.count) return;
@@ -158,6 +92,14 @@ __global__ void __launch_bounds__(kBlock, 12) list_walk_kernel(const ListScanArg
     scan.entries = a.list.entries + list_row(s, scan.capacity);
     scan.n = 0;
     const uint32_t* __restrict__ offsets = a.g.cell_offsets;
+    PackedScan packed;
+    packed.nx = make_float2(-scan.x.x, -scan.x.x);
+    packed.ny = make_float2(-scan.x.y, -scan.x.y);
+    packed.nz = make_float2(-scan.x.z, -scan.x.z);
+    packed.threshold = scan.threshold;
+    packed.capacity = scan.capacity;
+    packed.entries = scan.entries;
+    packed.n = 0;
     if (a.boundary && a.g.boundary_offsets) {
         // cell by cell: each cell's fluid particles, then its boundary particles (pbf/pbf.cu:111-121)
         const uint32_t* __restrict__ boffsets = a.g.boundary_offsets;
@@ -177,28 +119,6 @@ __global__ void __launch_bounds__(kBlock, 12) list_walk_kernel(const ListScanArg
     } else if (a.packed.x) {
         // At 1M particles the packed test cut a scan from 0.233 to 0.200 ms.  A budget of 40
         // registers (12 blocks of 128 per SM) measured fastest; 45 and 52 were within 1 %.
-        PackedScan packed;
-        packed.nx = make_float2(-scan.x.x, -scan.x.x);
-        packed.ny = make_float2(-scan.x.y, -scan.x.y);
-        packed.nz = make_float2(-scan.x.z, -scan.x.z);
-        packed.threshold = scan.threshold;
-        packed.capacity = scan.capacity;
-        packed.entries = scan.entries;
-        packed.n = 0;
-        if constexpr (Masks) {
-            const uint32_t pair_capacity = scan.capacity / 2u;
-            uint2* row = reinterpret_cast<uint2*>(a.list.entries) + mask_row(s, pair_capacity);
-            uint32_t pairs = 0;
-#pragma unroll 1
-            for (int o = 0; o < 9; ++o) {
-                const int x = c.x + o / 3 - 1, y = c.y + o % 3 - 1;
-                if (x < 0 || x >= cx || y < 0 || y >= cy) continue;
-                packed.run_masks(a.packed, offsets[cell_index(grid, x, y, z_lo)], offsets[cell_index(grid, x, y, z_hi) + 1u],
-                                 row, pair_capacity, pairs);
-            }
-            a.list.counts[s] = pairs <= pair_capacity ? packed.n : kOverflow;
-            return;
-        }
 #pragma unroll 1
         for (int o = 0; o < 9; ++o) {
             const int x = c.x + o / 3 - 1, y = c.y + o % 3 - 1;
@@ -395,69 +315,6 @@ __global__ void __launch_bounds__(kBlock) list_scan_kernel(const ListScanArgs a)
 }
 
 // ------------------------------------------------------------------ density + lambda
-// density (density/density.cu:18-40) and lambda (pbf/pbf.cu:95-127) of one particle in one walk.
-// m_j / rho0_i for a run of neighbours: most neighbours share a mass, so the last quotient is
-// kept and reused while the mass bits repeat (same operands, same correctly rounded quotient).
-struct MassRatio {
-    uint32_t mass_bits;
-    float quotient;
-    __device__ __forceinline__ void reset(const float mass, const float rest_density) {
-        mass_bits = __float_as_uint(mass);
-        quotient = __fdiv_rn(mass, rest_density);
-    }
-    __device__ __forceinline__ float operator()(const float mass, const float rest_density) {
-        const uint32_t bits = __float_as_uint(mass);
-        if (bits != mass_bits) reset(mass, rest_density);
-        return quotient;
-    }
-};
-
-// WithBoundary: the scene has boundary particles (their entries carry kBoundaryBit); the plain
-// instantiation, launched otherwise, carries no boundary test.
-template <bool WithBoundary>
-struct DensityLambdaOp {
-    static constexpr bool kBoundary = WithBoundary;
-    const float4* __restrict__ pos;
-    const float4* __restrict__ boundary;
-    f3 x;
-    uint32_t self;
-    float rest_density;
-    KernelConstants k;
-    float density;
-    f3 gradient_sum;
-    float denominator;
-    uint32_t neighbors;
-    MassRatio ratio;
-
-    __device__ __forceinline__ float4 prefetch(const uint32_t t) const {
-        if constexpr (WithBoundary) return (t & kBoundaryBit) ? boundary[t & ~kBoundaryBit] : pos[t];
-        return pos[t];
-    }
-    __device__ __forceinline__ void apply(const uint32_t t, const float4 q) {
-        const f3 d = sub(x, xyz(q));
-        const float r2 = squared(d);
-        if (WithBoundary && (t & kBoundaryBit)) {
-            // boundary particle b: density += rho0_i V_b W (density/density.cu:34-37),
-            // S += V_b grad W (pbf/pbf.cu:118-121); no denominator term
-            if (r2 < k.h2) density = __fmaf_rn(__fmul_rn(rest_density, q.w), poly6_inside(r2, k), density);
-            const float distance = __fsqrt_rn(r2);
-            if (distance == 0.0F || distance >= k.h) return;
-            gradient_sum = fma3(q.w, spiky_gradient_at(d, distance, k), gradient_sum);
-            return;
-        }
-        if (r2 < k.h2) density = __fmaf_rn(q.w, poly6_inside(r2, k), density);
-        if (t == self) return;
-        if (r2 < k.h2) ++neighbors;
-        const float distance = __fsqrt_rn(r2);
-        if (distance == 0.0F || distance >= k.h) return;
-        const f3 gradient = spiky_gradient_at(d, distance, k);
-        const float coefficient = ratio(q.w, rest_density);
-        gradient_sum = fma3(coefficient, gradient, gradient_sum);
-        denominator = __fmaf_rn(__fmul_rn(coefficient, coefficient), sq_xfirst(gradient), denominator);
-    }
-    __device__ __forceinline__ void process(const uint32_t t) { apply(t, prefetch(t)); }
-};
-
 template <bool WithBoundary>
 __global__ void __launch_bounds__(kBlock) density_lambda_kernel(const DensityLambdaArgs a) {
     const Particle p = locate(a.g);
@@ -504,14 +361,9 @@ __global__ void __launch_bounds__(kBlock) density_lambda_kernel(const DensityLam
 #endif
 constexpr uint32_t kStagedEntries = PBF_FUSED_STAGED_ENTRIES;   // 40: 20 KB of shared memory per 128-thread block
 
-// Masks: the list is stored as a hit-mask list (one (base, mask) pair per block with a hit), the
-// first kStagedEntries / 2 pairs staged in the same shared memory.
-template <bool Masks>
 __global__ void __launch_bounds__(kBlock, PBF_FUSED_MIN_BLOCKS) scan_density_lambda_kernel(const ListScanArgs a,
                                                                                           const DensityLambdaArgs d) {
-    __shared__ __align__(8) uint32_t staged[kStagedEntries * kBlock];
-    constexpr uint32_t kStagedPairs = kStagedEntries / 2u;
-    uint2* const staged_pairs = reinterpret_cast<uint2*>(staged);
+    __shared__ uint32_t staged[kStagedEntries * kBlock];
     const Particle p = locate(a.g);
     if (!p.active) return;
     const uint32_t s = p.s, lane_slot = threadIdx.x;
@@ -521,12 +373,10 @@ __global__ void __launch_bounds__(kBlock, PBF_FUSED_MIN_BLOCKS) scan_density_lam
     const uint32_t z_hi = static_cast<uint32_t>(p.c.z + 1 < cz ? p.c.z + 1 : cz - 1);
     const float4 xi = a.pos[s];
     const uint32_t capacity = a.list.capacity;
-    const uint32_t pair_capacity = capacity / 2u;
     uint32_t* __restrict__ entries = a.list.entries + list_row(s, capacity);
-    uint2* __restrict__ pairs_row = reinterpret_cast<uint2*>(a.list.entries) + mask_row(s, pair_capacity);
     const uint32_t* __restrict__ offsets = a.g.cell_offsets;
     // 1. the per-lane packed scan (PackedScan), appending to the stored list and the stage
-    uint32_t n = 0, pairs = 0;
+    uint32_t n = 0;
     {
         PackedScan scan;
         scan.nx = make_float2(-xi.x, -xi.x);
@@ -543,26 +393,16 @@ __global__ void __launch_bounds__(kBlock, PBF_FUSED_MIN_BLOCKS) scan_density_lam
             if (first >= end) continue;
             for (uint32_t base = first & ~3u; base < end; base += 32u) {
                 uint32_t mask = scan.block_mask(pk, base, first, end);
-                if constexpr (Masks) {
-                    if (mask) {
-                        const uint2 pair = make_uint2(base, mask);
-                        if (pairs < pair_capacity) pairs_row[static_cast<size_t>(pairs) * 32u] = pair;
-                        if (pairs < kStagedPairs) staged_pairs[pairs * kBlock + lane_slot] = pair;
-                        ++pairs;
-                        n += static_cast<uint32_t>(__popc(mask));
-                    }
-                } else {
-                    while (mask) {
-                        const uint32_t k = static_cast<uint32_t>(__ffs(mask)) - 1u;
-                        if (n < capacity) entries[static_cast<size_t>(n) * 32u] = base + k;
-                        if (n < kStagedEntries) staged[n * kBlock + lane_slot] = base + k;
-                        ++n;
-                        mask &= mask - 1u;
-                    }
+                while (mask) {
+                    const uint32_t k = static_cast<uint32_t>(__ffs(mask)) - 1u;
+                    if (n < capacity) entries[static_cast<size_t>(n) * 32u] = base + k;
+                    if (n < kStagedEntries) staged[n * kBlock + lane_slot] = base + k;
+                    ++n;
+                    mask &= mask - 1u;
                 }
             }
         }
-        const bool overflow = Masks ? pairs > pair_capacity : n > capacity;
+        const bool overflow = n > capacity;
         a.list.counts[s] = overflow ? kOverflow : n;
         if (overflow) n = kOverflow;
     }
@@ -583,29 +423,8 @@ __global__ void __launch_bounds__(kBlock, PBF_FUSED_MIN_BLOCKS) scan_density_lam
     if (n == kOverflow) {
         walk(op, p, a.g);
     } else if (n > 0) {
-        uint2 current{}, upcoming{};
-        uint32_t next_pair = 2u;
-        auto pair_at = [&](const uint32_t j) -> uint2 {
-            return j < kStagedPairs ? staged_pairs[j * kBlock + lane_slot] : pairs_row[static_cast<size_t>(j) * 32u];
-        };
-        if constexpr (Masks) {
-            current = pair_at(0);
-            upcoming = pairs > 1u ? pair_at(1) : make_uint2(0u, 0u);
-        }
         auto entry = [&](const uint32_t k) -> uint32_t {
-            if constexpr (Masks) {
-                (void)k;
-                if (current.y == 0u) {
-                    current = upcoming;
-                    upcoming = next_pair < pairs ? pair_at(next_pair) : make_uint2(0u, 0u);
-                    ++next_pair;
-                }
-                const uint32_t bit = static_cast<uint32_t>(__ffs(current.y)) - 1u;
-                current.y &= current.y - 1u;
-                return current.x + bit;
-            } else {
-                return k < kStagedEntries ? staged[k * kBlock + lane_slot] : entries[static_cast<size_t>(k) * 32u];
-            }
+            return k < kStagedEntries ? staged[k * kBlock + lane_slot] : entries[static_cast<size_t>(k) * 32u];
         };
         uint32_t t = entry(0);
         uint32_t tn = n > 1u ? entry(1) : 0u;
@@ -628,61 +447,6 @@ __global__ void __launch_bounds__(kBlock, PBF_FUSED_MIN_BLOCKS) scan_density_lam
 }
 
 // ------------------------------------------------------- correction + project
-// correction (pbf/pbf.cu:254-288) and project (pbf/pbf.cu:417-431); on the last iteration
-// also reconstruct (pbf/pbf.cu:456-460) and the write-back of next_state.positions.
-struct PositionLambda {
-    float4 q;
-    float lambda;
-};
-
-template <bool WithBoundary>
-struct CorrectionOp {
-    static constexpr bool kBoundary = WithBoundary;
-    const float4* __restrict__ pos;
-    const float4* __restrict__ boundary;
-    const float* __restrict__ lambda;
-    f3 x;
-    uint32_t self;
-    float rest_density;
-    float lambda_i;
-    float strength, exponent, reference_weight;
-    bool artificial_full;
-    KernelConstants k;
-    f3 correction;
-    MassRatio ratio;
-
-    __device__ __forceinline__ PositionLambda prefetch(const uint32_t t) const {
-        if (WithBoundary && (t & kBoundaryBit)) return {boundary[t & ~kBoundaryBit], 0.0F};
-        return {pos[t], lambda[t]};
-    }
-    __device__ __forceinline__ void apply(const uint32_t t, const PositionLambda in) {
-        if (t == self) return;
-        const f3 d = sub(x, xyz(in.q));
-        const float r2 = squared(d);
-        const float distance = __fsqrt_rn(r2);
-        if (distance == 0.0F || distance >= k.h) return;
-        // s_corr (pbf/pbf.cu:56-71).  With zero strength it is -strength * ratio^n, i.e. -0 inside
-        // the poly6 support and 0 outside, which the fast branch yields without powf.
-        float artificial;
-        if (artificial_full) {
-            const float weight = r2 >= k.h2 ? 0.0F : poly6_inside(r2, k);
-            artificial = weight == 0.0F ? 0.0F : __fmul_rn(-strength, powf(__fdiv_rn(weight, reference_weight), exponent));
-        } else {
-            artificial = r2 < k.h2 ? -strength : 0.0F;
-        }
-        if (WithBoundary && (t & kBoundaryBit)) {
-            // boundary particle b: V_b (lambda_i + s_corr) grad W (pbf/pbf.cu:278-285)
-            const float factor = __fmul_rn(in.q.w, __fadd_rn(lambda_i, artificial));
-            correction = fma3(factor, spiky_gradient_at(d, distance, k), correction);
-            return;
-        }
-        const float coefficient = ratio(in.q.w, rest_density);
-        const float factor = __fmul_rn(coefficient, __fadd_rn(__fadd_rn(lambda_i, in.lambda), artificial));
-        correction = fma3(factor, spiky_gradient_at(d, distance, k), correction);
-    }
-    __device__ __forceinline__ void process(const uint32_t t) { apply(t, prefetch(t)); }
-};
-
 // Resident 128-thread blocks per SM the register budget of the correction and of the post-loop
 // passes is sized for (compile-time tuning knobs; 0 leaves the register count to the compiler).
 // At 1M particles (substeps 25-28, ms per launch): the correction at 9 (56 registers instead of
@@ -696,7 +460,7 @@ struct CorrectionOp {
 #define PBF_POST_MIN_BLOCKS 10
 #endif
 
-template <bool WithBoundary, bool Masks>
+template <bool WithBoundary>
 __global__ void __launch_bounds__(kBlock, PBF_CORRECTION_MIN_BLOCKS) correction_kernel(const CorrectionArgs a) {
     const Particle p = locate(a.g);
     if (!p.active) return;
@@ -718,7 +482,7 @@ __global__ void __launch_bounds__(kBlock, PBF_CORRECTION_MIN_BLOCKS) correction_
     op.artificial_full = pb.x != 0.0F;
     op.reference_weight = op.artificial_full ? poly6(mk(pb.z, 0.0F, 0.0F), p.k) : 1.0F;
     op.correction = mk(0.0F, 0.0F, 0.0F);
-    replay_list<Masks>(op, p, a.g, a.list);
+    replay<2>(op, p, a.g, a.list);
     const Box& box = p.scene->box;
     const f3 candidate = add(op.x, op.correction);
     uint32_t mask = 0u;
@@ -746,32 +510,6 @@ __global__ void __launch_bounds__(kBlock, PBF_CORRECTION_MIN_BLOCKS) correction_
 }
 
 // ---------------------------------------------------------------- vorticity
-// vorticity (pbf/pbf.cu:476-497) and its magnitude (pbf/pbf.cu:565-569).
-struct PositionVector {
-    float4 q;
-    float4 v;
-};
-
-struct VorticityOp {
-    const float4* __restrict__ pos;
-    const float4* __restrict__ velocity;
-    f3 x, v;
-    uint32_t self;
-    KernelConstants k;
-    f3 vorticity;
-
-    __device__ __forceinline__ PositionVector prefetch(const uint32_t t) const { return {pos[t], velocity[t]}; }
-    __device__ __forceinline__ void apply(const uint32_t t, const PositionVector in) {
-        if (t == self) return;
-        const f3 d = sub(x, xyz(in.q));
-        const float distance = __fsqrt_rn(squared(d));
-        if (distance == 0.0F || distance >= k.h) return;
-        vorticity = add(vorticity, cross_f(sub(xyz(in.v), v), spiky_gradient_at(d, distance, k)));
-    }
-    __device__ __forceinline__ void process(const uint32_t t) { apply(t, prefetch(t)); }
-};
-
-template <bool Masks>
 __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) vorticity_kernel(const VorticityArgs a) {
     const Particle p = locate(a.g);
     if (!p.active) return;
@@ -783,38 +521,11 @@ __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) vorticity_kernel(
     op.x = xyz(a.pos[p.s]);
     op.v = xyz(a.velocity[p.s]);
     op.vorticity = mk(0.0F, 0.0F, 0.0F);
-    replay_list<Masks>(op, p, a.g, a.list);
+    replay<2>(op, p, a.g, a.list);
     a.vorticity[p.s] = make_float4(op.vorticity.x, op.vorticity.y, op.vorticity.z, __fsqrt_rn(sq_xfirst(op.vorticity)));
 }
 
 // ------------------------------------------------------- normal + confinement
-// normal (pbf/pbf.cu:571-593) and confinement (pbf/pbf.cu:674-678).
-struct PositionScalar {
-    float4 q;
-    float w;
-};
-
-struct NormalOp {
-    const float4* __restrict__ pos;
-    const float4* __restrict__ vorticity;
-    f3 x;
-    float magnitude;
-    uint32_t self;
-    KernelConstants k;
-    f3 gradient;
-
-    __device__ __forceinline__ PositionScalar prefetch(const uint32_t t) const { return {pos[t], vorticity[t].w}; }
-    __device__ __forceinline__ void apply(const uint32_t t, const PositionScalar in) {
-        if (t == self) return;
-        const f3 d = sub(x, xyz(in.q));
-        const float distance = __fsqrt_rn(squared(d));
-        if (distance == 0.0F || distance >= k.h) return;
-        gradient = fma3(__fsub_rn(in.w, magnitude), spiky_gradient_at(d, distance, k), gradient);
-    }
-    __device__ __forceinline__ void process(const uint32_t t) { apply(t, prefetch(t)); }
-};
-
-template <bool Masks>
 __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) normal_kernel(const NormalArgs a) {
     const Particle p = locate(a.g);
     if (!p.active) return;
@@ -827,7 +538,7 @@ __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) normal_kernel(con
     op.x = xyz(a.pos[p.s]);
     op.magnitude = wi.w;
     op.gradient = mk(0.0F, 0.0F, 0.0F);
-    replay_list<Masks>(op, p, a.g, a.list);
+    replay<2>(op, p, a.g, a.list);
     const float normalizer = __fsqrt_rn(sq_yfirst(op.gradient));
     const f3 normal = normalizer > 0.0F ? scale(op.gradient, __fdiv_rn(1.0F, normalizer)) : mk(0.0F, 0.0F, 0.0F);
     a.normal[p.s] = make_float4(normal.x, normal.y, normal.z, normalizer);
@@ -838,27 +549,6 @@ __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) normal_kernel(con
 }
 
 // ---------------------------------------------------------------------- XSPH
-// XSPH (pbf/pbf.cu:700-721) and the write-back of next_state.velocities.
-struct XsphOp {
-    const float4* __restrict__ pos;
-    const float4* __restrict__ confined;
-    f3 x, v;
-    uint32_t self;
-    KernelConstants k;
-    f3 smoothing;
-
-    __device__ __forceinline__ PositionVector prefetch(const uint32_t t) const { return {pos[t], confined[t]}; }
-    __device__ __forceinline__ void apply(const uint32_t t, const PositionVector in) {
-        if (t == self) return;
-        const f3 d = sub(x, xyz(in.q));
-        const float r2 = squared(d);
-        if (r2 >= k.h2) return;
-        smoothing = fma3(poly6_inside(r2, k), sub(xyz(in.v), v), smoothing);
-    }
-    __device__ __forceinline__ void process(const uint32_t t) { apply(t, prefetch(t)); }
-};
-
-template <bool Masks>
 __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) xsph_kernel(const XsphArgs a) {
     const Particle p = locate(a.g);
     if (!p.active) return;
@@ -870,7 +560,7 @@ __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) xsph_kernel(const
     op.x = xyz(a.pos[p.s]);
     op.v = xyz(a.confined[p.s]);
     op.smoothing = mk(0.0F, 0.0F, 0.0F);
-    replay_list<Masks>(op, p, a.g, a.list);
+    replay<2>(op, p, a.g, a.list);
     const float viscosity = a.g.params_a[p.s].z;
     const f3 out = fma3(viscosity, op.smoothing, op.v);
     const uint32_t i = a.sorted_index[p.s];
@@ -883,39 +573,7 @@ __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) xsph_kernel(const
 __global__ void constants_kernel(const float* __restrict__ radii, const uint32_t n, KernelConstants* __restrict__ out) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float h = radii[i];
-    const float squared_radius = __fmul_rn(h, h);
-    KernelConstants k;
-    k.h = h;
-    k.h2 = squared_radius;
-    k.poly6_denominator = __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(64.0F * kPi, squared_radius), squared_radius),
-                                                                     squared_radius), h), h), h);
-    k.poly6_grad_denominator = __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(32.0F * kPi, squared_radius), squared_radius),
-                                                                          squared_radius), h), h), h);
-    k.spiky_coefficient = __fdiv_rn(-45.0F, __fmul_rn(kPi, powf(h, 6.0F)));
-    // Smallest float r2 with sqrtf(r2) >= h; sqrtf is monotone, so bisect on the bit pattern.
-    uint32_t lo = 0u, hi = 0x7f800000u;
-    while (hi - lo > 1u) {
-        const uint32_t mid = lo + (hi - lo) / 2u;
-        if (sqrtf(__uint_as_float(mid)) >= h) hi = mid;
-        else lo = mid;
-    }
-    k.spiky_threshold = __uint_as_float(hi);
-    k.union_threshold = fmaxf(k.h2, k.spiky_threshold);
-    // Smallest float r2 with sqrt((double)r2) >= h (the FP64 Hessian's support test).
-    lo = 0u;
-    hi = 0x7f800000u;
-    while (hi - lo > 1u) {
-        const uint32_t mid = lo + (hi - lo) / 2u;
-        if (sqrt(static_cast<double>(__uint_as_float(mid))) >= static_cast<double>(h)) hi = mid;
-        else lo = mid;
-    }
-    k.hessian_threshold = __uint_as_float(hi);
-    k.adjoint_threshold = fmaxf(k.spiky_threshold, k.hessian_threshold);
-    k.list_threshold = fmaxf(k.union_threshold, k.hessian_threshold);
-    k.poly6_radial_coefficient = __fdiv_rn(315.0F, __fmul_rn(64.0F * kPi, powf(h, 9.0F)));
-    k.spiky_coefficient_d = -45.0 / (static_cast<double>(kPi) * pow(static_cast<double>(h), 6.0));
-    out[i] = k;
+    out[i] = kernel_constants(radii[i]);
 }
 
 __global__ void unsort_float4_kernel(const uint32_t count, const uint32_t* __restrict__ sorted_index,
@@ -1001,17 +659,17 @@ cudaError_t launch_constants(cudaStream_t stream, const float* radii, const uint
 bool valid_shape(const LaunchShape& shape) {
     auto ok = [](const uint32_t b) { return b >= 32u && b <= static_cast<uint32_t>(kBlock) && b % 32u == 0u; };
     return (shape.scan == kScanPerLane || shape.scan == kScanCooperative || shape.scan == kScanStaged ||
-            shape.scan == kScanFusedDensity || shape.scan == kScanFusedMasks) &&
+            shape.scan == kScanFusedDensity || shape.scan == kScanStaged16) &&
            ok(shape.scan_block) && ok(shape.block);
 }
 
 bool fuses_density(const LaunchShape& shape, const ListScanArgs& a) {
-    return (shape.scan == kScanFusedDensity || shape.scan == kScanFusedMasks) && a.packed.x && !a.g.boundary &&
+    return (shape.scan == kScanFusedDensity || shape.scan == kScanStaged16) && a.packed.x && !a.g.boundary &&
            !a.g.boundary_offsets;
 }
 
-bool stores_masks(const LaunchShape& shape, const bool differentiable, const bool boundary) {
-    return shape.scan == kScanFusedMasks && !differentiable && !boundary;
+bool runs_staged(const LaunchShape& shape, const bool differentiable, const bool boundary, const uint32_t iterations) {
+    return shape.scan == kScanStaged16 && !differentiable && !boundary && iterations > 0;
 }
 
 namespace {
@@ -1026,15 +684,12 @@ cudaError_t launch_list_scan(cudaStream_t stream, const ListScanArgs& a, const L
     // the cooperative and staged scans list fluid particles only; lists with boundary particles
     // use the per-lane walk
     const bool fluid_only = !(a.boundary && a.g.boundary_offsets);
-    if (a.list.masks) {   // hit-mask lists: the per-lane packed walk, scenes without boundary particles
-        if (!fluid_only || !a.packed.x) return cudaErrorInvalidValue;
-        list_walk_kernel<true><<<grid_of(a.g.count, block), block, 0, stream>>>(a);
-    } else if (shape.scan == kScanCooperative && fluid_only)
+    if (shape.scan == kScanCooperative && fluid_only)
         list_scan_kernel<<<grid_of(a.g.count, block), block, 0, stream>>>(a);
     else if (shape.scan == kScanStaged && fluid_only)
         list_staged_kernel<<<grid_of(a.g.count, block), block, 0, stream>>>(a);
     else
-        list_walk_kernel<false><<<grid_of(a.g.count, block), block, 0, stream>>>(a);
+        list_walk_kernel<<<grid_of(a.g.count, block), block, 0, stream>>>(a);
     count_launch();
     return cudaGetLastError();
 }
@@ -1043,17 +698,13 @@ cudaError_t launch_scan_density_lambda(cudaStream_t stream, const ListScanArgs& 
                                        const LaunchShape& shape) {
     if (a.g.count == 0) return cudaSuccess;
     const unsigned block = block_of(shape.scan_block);
-    if (a.list.masks)
-        scan_density_lambda_kernel<true><<<grid_of(a.g.count, block), block, 0, stream>>>(a, d);
-    else
-        scan_density_lambda_kernel<false><<<grid_of(a.g.count, block), block, 0, stream>>>(a, d);
+    scan_density_lambda_kernel<<<grid_of(a.g.count, block), block, 0, stream>>>(a, d);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_density_lambda(cudaStream_t stream, const DensityLambdaArgs& a, const unsigned block_size) {
     if (a.g.count == 0) return cudaSuccess;
-    if (a.list.masks) return cudaErrorInvalidValue;   // hit-mask lists are read by the fused scan only
     const unsigned block = block_of(block_size);
     if (a.g.boundary)
         density_lambda_kernel<true><<<grid_of(a.g.count, block), block, 0, stream>>>(a);
@@ -1067,12 +718,9 @@ cudaError_t launch_correction(cudaStream_t stream, const CorrectionArgs& a, cons
     if (a.g.count == 0) return cudaSuccess;
     const unsigned block = block_of(block_size);
     if (a.g.boundary) {
-        if (a.list.masks) return cudaErrorInvalidValue;
-        correction_kernel<true, false><<<grid_of(a.g.count, block), block, 0, stream>>>(a);
-    } else if (a.list.masks) {
-        correction_kernel<false, true><<<grid_of(a.g.count, block), block, 0, stream>>>(a);
+        correction_kernel<true><<<grid_of(a.g.count, block), block, 0, stream>>>(a);
     } else {
-        correction_kernel<false, false><<<grid_of(a.g.count, block), block, 0, stream>>>(a);
+        correction_kernel<false><<<grid_of(a.g.count, block), block, 0, stream>>>(a);
     }
     count_launch();
     return cudaGetLastError();
@@ -1081,10 +729,7 @@ cudaError_t launch_correction(cudaStream_t stream, const CorrectionArgs& a, cons
 cudaError_t launch_vorticity(cudaStream_t stream, const VorticityArgs& a, const unsigned block_size) {
     if (a.g.count == 0) return cudaSuccess;
     const unsigned block = block_of(block_size);
-    if (a.list.masks)
-        vorticity_kernel<true><<<grid_of(a.g.count, block), block, 0, stream>>>(a);
-    else
-        vorticity_kernel<false><<<grid_of(a.g.count, block), block, 0, stream>>>(a);
+    vorticity_kernel<<<grid_of(a.g.count, block), block, 0, stream>>>(a);
     count_launch();
     return cudaGetLastError();
 }
@@ -1092,10 +737,7 @@ cudaError_t launch_vorticity(cudaStream_t stream, const VorticityArgs& a, const 
 cudaError_t launch_normal(cudaStream_t stream, const NormalArgs& a, const unsigned block_size) {
     if (a.g.count == 0) return cudaSuccess;
     const unsigned block = block_of(block_size);
-    if (a.list.masks)
-        normal_kernel<true><<<grid_of(a.g.count, block), block, 0, stream>>>(a);
-    else
-        normal_kernel<false><<<grid_of(a.g.count, block), block, 0, stream>>>(a);
+    normal_kernel<<<grid_of(a.g.count, block), block, 0, stream>>>(a);
     count_launch();
     return cudaGetLastError();
 }
@@ -1103,10 +745,7 @@ cudaError_t launch_normal(cudaStream_t stream, const NormalArgs& a, const unsign
 cudaError_t launch_xsph(cudaStream_t stream, const XsphArgs& a, const unsigned block_size) {
     if (a.g.count == 0) return cudaSuccess;
     const unsigned block = block_of(block_size);
-    if (a.list.masks)
-        xsph_kernel<true><<<grid_of(a.g.count, block), block, 0, stream>>>(a);
-    else
-        xsph_kernel<false><<<grid_of(a.g.count, block), block, 0, stream>>>(a);
+    xsph_kernel<<<grid_of(a.g.count, block), block, 0, stream>>>(a);
     count_launch();
     return cudaGetLastError();
 }

@@ -197,7 +197,7 @@ __global__ void reorder_kernel(const uint32_t count, const SceneDesc* __restrict
                                uint32_t* __restrict__ sorted_index, uint32_t* __restrict__ slot_of,
                                int4* __restrict__ cell, float4* __restrict__ topology, float4* __restrict__ params_a,
                                float4* __restrict__ params_b, const Field3 velocities, float4* __restrict__ sorted_velocity,
-                               const PackedPositions packed) {
+                               const PackedPositions packed, float* __restrict__ packed_mass) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= count) return;
     const uint32_t i = unordered[t];
@@ -214,6 +214,7 @@ __global__ void reorder_kernel(const uint32_t count, const SceneDesc* __restrict
         packed.x[s] = xs.x;
         packed.y[s] = xs.y;
         packed.z[s] = xs.z;
+        if (packed_mass) packed_mass[s] = xs.w;
     }
     const uint32_t scene = scene_of ? scene_of[i] : 0u;
     const Grid& g = scenes[scene].grid;
@@ -371,7 +372,8 @@ cudaError_t launch_grid_build(cudaStream_t stream, const GridBuildArgs& a) {
         scatter_kernel<<<blocks_for(a.count, tpb), tpb, 0, stream>>>(a.count, a.keys, a.arrival, a.cell_offsets, a.unordered);
         reorder_kernel<<<blocks_for(a.count, tpb), tpb, 0, stream>>>(
             a.count, a.scenes, a.scene_of, a.keys, a.cell_offsets, a.unordered, a.predicted, a.params, a.sorted_index,
-            a.slot_of, a.cell, a.topology, a.params_a, a.params_b, a.velocities, a.sorted_velocity, a.packed);
+            a.slot_of, a.cell, a.topology, a.params_a, a.params_b, a.velocities, a.sorted_velocity, a.packed,
+            a.packed_mass);
         count_launch(2);
     }
     return cudaGetLastError();

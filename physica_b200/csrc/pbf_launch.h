@@ -42,6 +42,7 @@ struct GridBuildArgs {
     int key_current = 0;               // key the input positions instead of the predicted ones (SPH)
     float4* sorted_velocity = nullptr; // optional (v, 0) in sorted order
     PackedPositions packed{};          // optional x* as three arrays in sorted order
+    float* packed_mass = nullptr;      // optional, with `packed`: the masses in sorted order
 };
 
 size_t scan_tile_count(uint64_t n);
@@ -55,18 +56,13 @@ cudaError_t launch_reference_order(cudaStream_t stream, uint32_t count, const Sc
                                    const uint32_t* sorted_index, const uint32_t* keys, const uint32_t* cell_offsets,
                                    const uint32_t* reference_offsets, uint32_t* out_index, unsigned long long* out_keys);
 
-// A stored neighbour list (warp-interleaved entries + per-particle counts).  Two formats share the
-// buffer of `capacity` 32-bit words per particle:
-// - index lists (masks = 0): one sorted slot per in-support neighbour, counts = entries;
-// - hit-mask lists (masks = 1): one (slot of bit 0, 32-bit hit mask) pair per 32-slot block of a
-//   stencil column that holds a neighbour, capacity / 2 pairs per particle, counts = neighbours.
-// Either lists the same neighbours in the same order; kOverflow marks a particle whose list did not
-// fit (it walks its stencil instead).
+// A stored neighbour list: `capacity` 32-bit words per particle, warp-interleaved, one sorted slot per
+// in-support neighbour, and the entries' count; kOverflow marks a particle whose list did not fit (it
+// walks its stencil instead).  The staged passes pack two entries in a word (StagedList).
 struct StoredList {
     uint32_t* entries;
     uint32_t* counts;
     uint32_t capacity;
-    int masks = 0;
 };
 
 // Common inputs of every neighbour-gather pass.
@@ -176,11 +172,11 @@ enum ListScanVariant : uint32_t {
     kScanStaged = 2,        // a warp stages its column group's candidates in shared memory
     kScanFusedDensity = 3,  // per lane, and the Jacobi iterations' scans also run density + lambda
                             // in the same kernel (scenes without boundary particles)
-    kScanFusedMasks = 4,    // as 3, and forward-mode steps store hit-mask lists (scenes without
-                            // boundary particles; differentiable steps store index lists)
+    kScanStaged16 = 4,      // as 3, and forward-mode steps of scenes without boundary particles run
+                            // every pass over windows staged in shared memory (staged.cu)
 };
 struct LaunchShape {
-    uint32_t scan = kScanPerLane;
+    uint32_t scan = kScanStaged16;   // fastest at every size measured (5k to 1M particles)
     uint32_t scan_block = 128;   // threads per block of the list scan: 32, 64, 96 or 128
     uint32_t block = 128;        // threads per block of the gather passes: 32, 64, 96 or 128
 };
@@ -189,8 +185,8 @@ bool valid_shape(const LaunchShape& shape);
 cudaError_t launch_list_scan(cudaStream_t stream, const ListScanArgs& a, const LaunchShape& shape = LaunchShape{});
 // Whether `shape` runs the scan of `a` fused with density + lambda (launch_scan_density_lambda).
 bool fuses_density(const LaunchShape& shape, const ListScanArgs& a);
-// Whether a forward-mode step with `shape` stores hit-mask lists (no boundary particles).
-bool stores_masks(const LaunchShape& shape, bool differentiable, bool boundary);
+// Whether a step with `shape` runs the staged passes.
+bool runs_staged(const LaunchShape& shape, bool differentiable, bool boundary, uint32_t iterations);
 // The list scan of a Jacobi iteration and its density + lambda pass in one kernel (same list and
 // results as launch_list_scan followed by launch_density_lambda).
 cudaError_t launch_scan_density_lambda(cudaStream_t stream, const ListScanArgs& a, const DensityLambdaArgs& d,
@@ -210,6 +206,77 @@ cudaError_t launch_xsph(cudaStream_t stream, const XsphArgs& a, unsigned block);
 cudaError_t launch_reconstruct(cudaStream_t stream, uint32_t count, const SceneDesc* scenes, const int4* cell,
                                const float4* positions, Field3 previous_positions, const uint32_t* sorted_index,
                                MutField3 out_positions, float4* velocity);
+
+// ---- forward passes over windows staged in shared memory (staged.cu): forward mode, no boundary
+// particles.  A list is a StoredList whose entries are pairs of 16-bit staged positions (or, for the
+// blocks that do not fit the stage, sorted slots as elsewhere), and its blocks' windows.
+constexpr uint32_t kWindowWords = 32;          // words of one block's record
+size_t window_words(uint32_t count);           // words of the records of `count` particles
+struct StagedList {
+    StoredList list;
+    uint32_t* windows;
+};
+struct StagedDensityArgs {
+    GatherCommon g;
+    StagedList list;           // written
+    PackedPositions positions;
+    const float* mass;
+    const float4* pos;         // the same positions and masses, for blocks that work on global memory
+    float* lambda;
+    float* density;            // optional record
+    uint32_t* neighbor_count;  // optional record
+};
+struct StagedCorrectionArgs {
+    GatherCommon g;
+    StagedList list;
+    PackedPositions positions;
+    const float* mass;
+    const float* lambda;
+    const float4* pos;
+    PackedPositions positions_next;
+    float4* pos_next;
+    int last;                  // last iteration: reconstruct velocities and write positions out
+    Field3 previous_positions;
+    const uint32_t* sorted_index;
+    MutField3 out_positions;
+    float4* velocity;
+    PackedPositions velocities;
+};
+struct StagedVorticityArgs {
+    GatherCommon g;
+    StagedList list;           // written: the post-loop list
+    PackedPositions positions, velocities;
+    const float4* pos;
+    const float4* velocity;
+    float4* vorticity;
+    float* magnitude;
+};
+struct StagedNormalArgs {
+    GatherCommon g;
+    StagedList list;
+    PackedPositions positions;
+    const float* magnitude;
+    const float4* pos;
+    const float4* velocity;
+    const float4* vorticity;
+    float4* normal;
+    float4* confined;
+    PackedPositions confined_soa;
+};
+struct StagedXsphArgs {
+    GatherCommon g;
+    StagedList list;
+    PackedPositions positions, confined_soa;
+    const float4* pos;
+    const float4* confined;
+    const uint32_t* sorted_index;
+    MutField3 out_velocities;
+};
+cudaError_t launch_staged_density(cudaStream_t stream, const StagedDensityArgs& a);
+cudaError_t launch_staged_correction(cudaStream_t stream, const StagedCorrectionArgs& a);
+cudaError_t launch_staged_vorticity(cudaStream_t stream, const StagedVorticityArgs& a);
+cudaError_t launch_staged_normal(cudaStream_t stream, const StagedNormalArgs& a);
+cudaError_t launch_staged_xsph(cudaStream_t stream, const StagedXsphArgs& a);
 
 // FP64 dst[f][i] += src[f][i] for up to six fields.
 cudaError_t launch_accumulate(cudaStream_t stream, size_t count, const double* const* src, double* const* dst, int fields);

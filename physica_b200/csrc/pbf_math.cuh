@@ -101,7 +101,57 @@ struct KernelConstants {
     float list_threshold;      // max of all: every kernel term of every pass is zero at r2 >= this
     float poly6_radial_coefficient; // 315 / (64 pi powf(h, 9))  (pbf/pbf.cu:22)
     double spiky_coefficient_d;    // -45 / (pi pow(h, 6)) in FP64 (pbf/pbf.cu:52)
+    float poly6_reciprocal;    // 1 / poly6_denominator, correctly rounded
+    float poly6_grad_reciprocal;   // 1 / poly6_grad_denominator, correctly rounded
+    float fast_min;            // smallest and largest non-zero r2 of the two-pair arithmetic below
+    float fast_max;            // (largest < smallest where h is outside its range)
 };
+
+// The constants of support radius h.
+__device__ inline KernelConstants kernel_constants(const float h) {
+    const float squared_radius = __fmul_rn(h, h);
+    KernelConstants k;
+    k.h = h;
+    k.h2 = squared_radius;
+    k.poly6_denominator = __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(64.0F * kPi, squared_radius), squared_radius),
+                                                                     squared_radius), h), h), h);
+    k.poly6_grad_denominator = __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(32.0F * kPi, squared_radius), squared_radius),
+                                                                          squared_radius), h), h), h);
+    k.spiky_coefficient = __fdiv_rn(-45.0F, __fmul_rn(kPi, powf(h, 6.0F)));
+    // Smallest float r2 with sqrtf(r2) >= h; sqrtf is monotone, so bisect on the bit pattern.
+    uint32_t lo = 0u, hi = 0x7f800000u;
+    while (hi - lo > 1u) {
+        const uint32_t mid = lo + (hi - lo) / 2u;
+        if (sqrtf(__uint_as_float(mid)) >= h) hi = mid;
+        else lo = mid;
+    }
+    k.spiky_threshold = __uint_as_float(hi);
+    k.union_threshold = fmaxf(k.h2, k.spiky_threshold);
+    // Smallest float r2 with sqrt((double)r2) >= h (the FP64 Hessian's support test).
+    lo = 0u;
+    hi = 0x7f800000u;
+    while (hi - lo > 1u) {
+        const uint32_t mid = lo + (hi - lo) / 2u;
+        if (sqrt(static_cast<double>(__uint_as_float(mid))) >= static_cast<double>(h)) hi = mid;
+        else lo = mid;
+    }
+    k.hessian_threshold = __uint_as_float(hi);
+    k.adjoint_threshold = fmaxf(k.spiky_threshold, k.hessian_threshold);
+    k.list_threshold = fmaxf(k.union_threshold, k.hessian_threshold);
+    k.poly6_radial_coefficient = __fdiv_rn(315.0F, __fmul_rn(64.0F * kPi, powf(h, 9.0F)));
+    k.spiky_coefficient_d = -45.0 / (static_cast<double>(kPi) * pow(static_cast<double>(h), 6.0));
+    k.poly6_reciprocal = __frcp_rn(k.poly6_denominator);
+    k.poly6_grad_reciprocal = __frcp_rn(k.poly6_grad_denominator);
+    // fast_pair's range.  At its ends every intermediate of the packed arithmetic, and every last bit of
+    // its residuals, is a normal float: r >= 2^-30 h, and a poly6 numerator 315 (h2 - r2)^3 >= 2^-100.
+    k.fast_min = __fmul_rn(squared_radius, 0x1p-60F);
+    k.fast_max = -1.0F;
+    if (h >= 0x1p-10F && h <= 0x1p10F) {
+        const float below = __uint_as_float(__float_as_uint(fminf(squared_radius, k.spiky_threshold)) - 1u);
+        k.fast_max = fminf(below, __fsub_rn(squared_radius, 0x1p-36F));
+    }
+    return k;
+}
 
 // ------------------------------------------------------------ FP32 kernel functions
 // Squared distance of a displacement, with the reference's rounding.
@@ -133,15 +183,171 @@ __device__ __forceinline__ f3 spiky_gradient_at(const f3 d, const float distance
     return scale(d, __fdiv_rn(__fmul_rn(__fmul_rn(k.spiky_coefficient, difference), difference), distance));
 }
 
+// The same values out of line, for the pairs outside the range of the packed arithmetic below: a rare
+// path, whose inlined root and divisions would cost the replay loops registers.
+static __device__ __noinline__ float poly6_call(const float r2, const float h2, const float denominator) {
+    const float difference = __fsub_rn(h2, r2);
+    return __fdiv_rn(__fmul_rn(__fmul_rn(__fmul_rn(315.0F, difference), difference), difference), denominator);
+}
+static __device__ __noinline__ float sqrt_call(const float v) { return __fsqrt_rn(v); }
+static __device__ __noinline__ float spiky_scale_call(const float distance, const float h, const float coefficient) {
+    const float difference = __fsub_rn(h, distance);
+    return __fdiv_rn(__fmul_rn(__fmul_rn(coefficient, difference), difference), distance);
+}
+
 __device__ __forceinline__ f3 spiky_gradient(const f3 d, const KernelConstants& k) {
     const float distance = __fsqrt_rn(squared(d));
     if (distance == 0.0F || distance >= k.h) return {0.0F, 0.0F, 0.0F};
     return spiky_gradient_at(d, distance, k);
 }
 
+// ------------------------------------------------- two pairs at a time, packed FP32
+// The replay passes were bound by instruction issue, and most of a pair's instructions were its IEEE
+// square root and divisions, each with range tests and a branch around a slow path.  Inside a
+// range of r2 where nothing can overflow or turn subnormal (fast_pair) the same correctly rounded
+// values follow from one reciprocal square root and fused residual corrections, without a branch,
+// so two pairs share every instruction (packed FP32, each half rounded as the scalar intrinsic):
+//   sqrt:  s0 = r2 y, s = s0 + (r2 - s0^2) y / 2 with y ~ 1 / sqrt(r2).  Equal to __fsqrt_rn for
+//          every r2 of the range (all floats checked by tests/test_gpu_pair_math.py).
+//   a / b: q0 = a R, q = q0 + (a - b q0) R with R = RN(1 / b), which is RN(a / b)
+//          (P. Markstein, IBM J. Res. Dev. 34(1), 1990; M. Cornea, J. Harrison, P. Tang, Scientific
+//          Computing on Itanium, 2002).  For b = s, R = y + y (e + 2^-44)
+//          with e = 1 - s y: a Newton step that rounds up (|e| < 2^-22.2, so e^2 < 2^-44).  Without
+//          the 2^-44, R is an ulp low for s = 2 - 2^-23 and 1 / s comes out wrong.  The same test
+//          checks, for every s, the quotients that lie nearest a rounding boundary.
+__device__ __forceinline__ float2 both(const float v) { return make_float2(v, v); }
+
+// Whether r2 is in the range of the packed arithmetic (0 is: the weight there needs no root).
+__device__ __forceinline__ bool fast_pair(const float r2, const KernelConstants& k) {
+    return r2 <= k.fast_max && (r2 >= k.fast_min || r2 == 0.0F);
+}
+
+// The negated squared distance, -squared(d), of displacement d.
+__device__ __forceinline__ float negated_squared(const f3 d) {
+    return __fmaf_rn(-d.z, d.z, __fmaf_rn(-d.x, d.x, -__fmul_rn(d.y, d.y)));
+}
+
+__device__ __forceinline__ float approximate_rsqrt(const float v) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(v));
+    return y;
+}
+
+// a / b of two pairs, given -b and the correctly rounded 1 / b.
+__device__ __forceinline__ float2 quotient_pair(const float2 a, const float2 negated_b, const float2 reciprocal) {
+    const float2 q = __fmul2_rn(a, reciprocal);
+    return __ffma2_rn(__ffma2_rn(negated_b, q, a), reciprocal, q);
+}
+
+// -sqrt(r2) of two pairs from -r2, and the correctly rounded 1 / sqrt(r2) of that root.
+__device__ __forceinline__ float2 negated_root_pair(const float2 nr2, float2& reciprocal) {
+    const float2 y = make_float2(approximate_rsqrt(-nr2.x), approximate_rsqrt(-nr2.y));
+    const float2 ns0 = __fmul2_rn(nr2, y);
+    const float2 ns = __ffma2_rn(__ffma2_rn(ns0, ns0, nr2), __fmul2_rn(y, both(0.5F)), ns0);
+    const float2 e = __ffma2_rn(ns, y, both(1.0F));
+    reciprocal = __ffma2_rn(__fadd2_rn(e, both(0x1p-44F)), y, y);
+    return ns;
+}
+
+// poly6_inside of two pairs from their negated squared distances.
+__device__ __forceinline__ float2 poly6_pair(const float2 nr2, const KernelConstants& k) {
+    const float2 difference = __fadd2_rn(both(k.h2), nr2);
+    const float2 a = __fmul2_rn(__fmul2_rn(__fmul2_rn(both(315.0F), difference), difference), difference);
+    return quotient_pair(a, both(-k.poly6_denominator), both(k.poly6_reciprocal));
+}
+
+// The scale of spiky_gradient_at, grad W = d * scale, of two pairs (undefined at r2 = 0).
+__device__ __forceinline__ float2 spiky_scale_pair(const float2 nr2, const KernelConstants& k) {
+    float2 reciprocal;
+    const float2 ns = negated_root_pair(nr2, reciprocal);
+    const float2 difference = __fadd2_rn(both(k.h), ns);
+    const float2 a = __fmul2_rn(__fmul2_rn(both(k.spiky_coefficient), difference), difference);
+    return quotient_pair(a, ns, reciprocal);
+}
+
 // ------------------------------------------------------------------ FP64 helpers of the adjoint
 __device__ __forceinline__ d3 ld3(const double4 v) { return {v.x, v.y, v.z}; }
 __device__ __forceinline__ double4 st3(const d3 v) { return make_double4(v.x, v.y, v.z, 0.0); }
+
+// FP64 1 / sqrt(v) and 1 / v of a float: the FP32 approximation and one third-order step (relative
+// error of the start e: 5/16 e^3 and e^3, below 2^-65), where rsqrt() and a division test their range
+// and take two steps.
+__device__ __forceinline__ double wide_rsqrt(const float v, const float approximation) {
+    const double y = approximation;
+    const double e = fma(-(static_cast<double>(v) * y), y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+__device__ __forceinline__ double wide_rsqrt(const float v) {
+    if (v >= 0x1p-100F && v <= 0x1p100F) return wide_rsqrt(v, approximate_rsqrt(v));
+    return rsqrt(static_cast<double>(v));
+}
+__device__ __forceinline__ double wide_reciprocal(const float v) {
+    if (!(v >= 0x1p-100F && v <= 0x1p100F)) return 1.0 / static_cast<double>(v);
+    float approximation;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(approximation) : "f"(v));
+    const double y = approximation;
+    const double e = fma(-static_cast<double>(v), y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+
+// One pair's kernel derivatives for the FP64 reverse passes: grad W = d * scale, rounded as
+// spiky_gradient, and the Hessian as H(d) v = along v + across (d . v) d in FP64.  H is linear and
+// H(-d) = H(d), so a pair's two directions need one product, of the difference of their vectors:
+// half the FP64 work of a product each, and no unit direction is formed.  The FP64 reciprocal root
+// starts from the FP32 one that the gradient needs anyway.
+struct PairDerivatives {
+    float scale;
+    double along, across;
+};
+__device__ __forceinline__ PairDerivatives pair_derivatives(const float r2, const KernelConstants& k) {   // 0 < r2
+    PairDerivatives p;
+    const double r2d = r2;
+    double inverse;
+    if (r2 >= k.fast_min && r2 <= k.fast_max) {
+        const float y = approximate_rsqrt(r2);
+        const float s0 = r2 * y;
+        const float s = __fmaf_rn(__fmaf_rn(-s0, s0, r2), 0.5F * y, s0);
+        const float reciprocal = __fmaf_rn(__fadd_rn(__fmaf_rn(-s, y, 1.0F), 0x1p-44F), y, y);
+        const float difference = __fsub_rn(k.h, s);
+        const float a = __fmul_rn(__fmul_rn(k.spiky_coefficient, difference), difference);
+        const float q = __fmul_rn(a, reciprocal);
+        p.scale = __fmaf_rn(__fmaf_rn(-s, q, a), reciprocal, q);
+        inverse = wide_rsqrt(r2, y);
+    } else {
+        p.scale = r2 < k.spiky_threshold ? spiky_scale_call(sqrt_call(r2), k.h, k.spiky_coefficient) : 0.0F;
+        inverse = rsqrt(r2d);
+    }
+    const double difference = k.h - r2d * inverse;
+    const double slope = k.spiky_coefficient_d * difference;
+    p.along = slope * difference * inverse;
+    p.across = -(slope + slope + p.along) * (inverse * inverse);
+    if (r2 >= k.hessian_threshold) p.along = p.across = 0.0;   // sqrt((double)r2) >= h
+    return p;
+}
+// H(d) v
+__device__ __forceinline__ d3 hessian_product(const PairDerivatives& p, const d3 d, const d3 v) {
+    const double across = p.across * (d.x * v.x + d.y * v.y + d.z * v.z);
+    return {fma(across, d.x, p.along * v.x), fma(across, d.y, p.along * v.y), fma(across, d.z, p.along * v.z)};
+}
+__device__ __forceinline__ d3 wide(const f3 v) { return {v.x, v.y, v.z}; }
+
+// The poly6 weight of poly6_inside without its division's range tests (r2 inside fast_pair's range).
+__device__ __forceinline__ float poly6_weight(const float r2, const KernelConstants& k) {
+    if (r2 > k.fast_max) return r2 >= k.h2 ? 0.0F : poly6_call(r2, k.h2, k.poly6_denominator);
+    const float difference = __fsub_rn(k.h2, r2);
+    const float a = __fmul_rn(__fmul_rn(__fmul_rn(315.0F, difference), difference), difference);
+    const float q = __fmul_rn(a, k.poly6_reciprocal);
+    return __fmaf_rn(__fmaf_rn(-k.poly6_denominator, q, a), k.poly6_reciprocal, q);
+}
+
+// The scale of poly6_gradient, grad W = d * scale, likewise (r2 < h2).
+__device__ __forceinline__ float poly6_gradient_scale(const float r2, const KernelConstants& k) {
+    const float difference = __fsub_rn(k.h2, r2);
+    const float a = __fmul_rn(__fmul_rn(-945.0F, difference), difference);
+    if (r2 > k.fast_max) return __fdiv_rn(a, k.poly6_grad_denominator);
+    const float q = __fmul_rn(a, k.poly6_grad_reciprocal);
+    return __fmaf_rn(__fmaf_rn(-k.poly6_grad_denominator, q, a), k.poly6_grad_reciprocal, q);
+}
 
 // Spiky Hessian applied to a vector, in FP64 (pbf/pbf.cu:45-54 evaluation order).
 // The adjoint is held to FP64 rounding against the reference, so the distance and its reciprocal

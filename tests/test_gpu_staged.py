@@ -1,0 +1,108 @@
+"""The staged forward passes (launch-shape variant 4, physica_b200/csrc/staged.cu) against the per-lane
+passes (variant 0), bit for bit: the same sums in the same order, so any difference is a fault."""
+import dataclasses
+
+import numpy as np
+import pytest
+import torch
+
+from physica_b200 import pbf, scenes
+
+pytestmark = pytest.mark.gpu
+
+PER_LANE, STAGED = pbf.LaunchShape(0, 128, 128), pbf.LaunchShape(4, 128, 128)
+
+
+def run(scene, shape, steps):
+    solver, state, control, params = pbf.solver_for_scene(scene)
+    solver.launch_shape = shape
+    cache, following = solver.allocate_step_cache(), solver.allocate_state()
+    out = []
+    for _ in range(steps):
+        solver.forward_step(state, control, params, following, cache)
+        out += [following.positions.clone(), following.velocities.clone()]
+        for field in (pbf.CacheField.FIRST_DENSITIES, pbf.CacheField.FIRST_LAMBDAS, pbf.CacheField.NEIGHBOR_COUNTS,
+                      pbf.CacheField.VORTICITY_MAGNITUDES, pbf.CacheField.VORTICITY_NORMALS, pbf.CacheField.CONFINED_VELOCITIES,
+                      pbf.CacheField.CORRECTED_POSITIONS, pbf.CacheField.RECONSTRUCTED_VELOCITIES):
+            out.append(cache.read(field))
+        state, following = following, state
+    solver.synchronize()
+    return [t.cpu().numpy() for t in out]
+
+
+def check(scene, steps=3):
+    for a, b in zip(run(scene, PER_LANE, steps), run(scene, STAGED, steps)):
+        np.testing.assert_array_equal(a.view(np.int32), b.view(np.int32))
+
+
+def block(count, seed=1, iterations=3, **options):
+    """`count` particles of a lattice block in motion."""
+    n = int(np.ceil(count ** (1 / 3)))
+    s = scenes.dam_break((n, n, n), (0.0, 0.0, 0.0), (2.5 * n * 0.0125 + 0.05,) * 3, seed, iterations, velocity_sigma=0.5, **options)
+    keep = {f.name: getattr(s, f.name)[..., :count] for f in dataclasses.fields(s)
+            if isinstance(getattr(s, f.name), np.ndarray)}
+    return dataclasses.replace(s, **{k: np.ascontiguousarray(v) for k, v in keep.items()})
+
+
+@pytest.mark.parametrize("count", [1, 2, 31, 33, 127, 128, 129, 255, 257, 1000, 4097])
+def test_counts_around_the_block(count):
+    check(block(count))
+
+
+def test_spray_whose_windows_exceed_the_stage():
+    """Thin spray beside and above a dense block: its blocks' windows cover the block's columns."""
+    s = block(8000)
+    rng = np.random.default_rng(3)
+    fly = rng.permutation(8000)[:900]
+    s.positions[:, fly] = (rng.random((3, 900)) * np.asarray(s.box_max)[:, None]).astype(np.float32)
+    check(s)
+
+
+def test_crowded_lists_overflow():
+    s = block(3000)
+    s.positions[:] = (0.2 + 0.06 * np.random.default_rng(4).random((3, 3000))).astype(np.float32)
+    check(s, steps=2)
+
+
+@pytest.mark.parametrize("strength", [0.0, 1e-5])
+def test_mixed_masses_and_coincident_particles(strength):
+    s = block(2000, seed=5)
+    rng = np.random.default_rng(6)
+    s.masses[:] *= rng.choice([0.5, 1.0, 1.5], 2000).astype(np.float32)
+    s.rest_densities[:] *= rng.choice([0.8, 1.0], 2000).astype(np.float32)
+    s.artificial_pressure_strength[:] = strength
+    s.positions[:, 100:110] = s.positions[:, 110:120]
+    s.velocities[:, 100:110] = s.velocities[:, 110:120]
+    s.positions[:, 200:210] = s.positions[:, 210:220] + np.float32(1e-12)
+    check(s)
+
+
+@pytest.mark.parametrize("h", [0.0008, 0.003, 1.0, 3000.0])
+def test_support_radii_inside_and_outside_the_packed_range(h):
+    """The packed pair arithmetic covers radii from 2^-10 to 2^10; others take the scalar path."""
+    n, spacing = 9, 0.5 * h
+    s = scenes.dam_break((n, n, n), (0.0, 0.0, 0.0), (12 * spacing,) * 3, 7, 3, h=h, velocity_sigma=0.2 * h)
+    check(s, steps=2)
+
+
+def test_moving_box():
+    """The sort cells and the gather cells of a moving box round differently."""
+    s = dataclasses.replace(block(4000, seed=8), box_velocity=(0.37, -0.11, 0.23))
+    check(s, steps=6)
+
+
+def test_batch_blocks_span_scenes():
+    parts = [scenes.batched_scene(c, 40 + k, 3, velocity_sigma=0.3) for k, c in enumerate((65, 700, 3, 1, 2049, 130))]
+    results = []
+    for shape in (PER_LANE, STAGED):
+        batch, state, control, params = pbf.batch_for_scenes(parts)
+        batch.launch_shape = shape
+        batch.reserve_caches(1)
+        following = batch.allocate_state()
+        for _ in range(3):
+            batch.forward_step(state, control, params, following, 0)
+            state, following = following, state
+        torch.cuda.synchronize()
+        results.append((state.positions.cpu().numpy(), state.velocities.cpu().numpy()))
+    for a, b in zip(*results):
+        np.testing.assert_array_equal(a.view(np.int32), b.view(np.int32))
