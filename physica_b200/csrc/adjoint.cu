@@ -191,22 +191,18 @@ struct XsphVjpOp {
     __device__ __forceinline__ void process(const uint32_t t) {
         if (t == self) return;
         const f3 d = sub(x, xyz(pos[t]));
-        if (squared(d) >= k.h2) return;
-        const f3 vj = xyz(confined[t]);
-        const f3 difference = vj - v;
-        const float weight = poly6(d, k);
-        const f3 gradient = poly6_gradient(d, k);
-        vc = vc + times(ob, -viscosity * weight);
-        pc = pc + times(gradient, viscosity * dot(ob, difference));
-        cc += weight * dot(ob, difference);
+        const float r2 = squared(d);
+        if (r2 >= k.h2) return;
+        const d3 difference = wide(xyz(confined[t]) - v);
+        const float weight = poly6_weight(r2, k);   // W(-d) = W(d), grad W(-d) = -grad W(d), exactly
+        const f3 gradient = scale(d, poly6_gradient_scale(r2, k));
         const d3 rob = ld3(output_velocity[t]);
-        const f3 rdiff = v - vj;
-        // W(-d) = W(d) and grad W(-d) = -grad W(d), exactly (the same squared distance; every
-        // component is a product whose sign alone flips)
-        const float rweight = weight;
         const float rviscosity = params_a[t].z;
-        vc = vc + times(rob, rviscosity * rweight);
-        pc = pc + times(scale(gradient, -1.0F), -rviscosity * dot(rob, rdiff));
+        const double own = viscosity * weight, reverse = rviscosity * weight;
+        vc = vc + (times(rob, reverse) - times(ob, own));
+        const double change = dot(ob, difference);
+        pc = pc + times(gradient, viscosity * change - rviscosity * dot(rob, difference));
+        cc += weight * change;
     }
 };
 
@@ -290,18 +286,11 @@ struct NormalVjpOp {
         const f3 d = sub(x, xyz(pos[t]));
         const float r2 = squared(d);
         if (r2 == 0.0F || r2 >= k.adjoint_threshold) return;
-        const f3 gradient = spiky_gradient(d, k);
-        const float magnitude_j = vorticity[t].w;
-        const float difference = magnitude_j - magnitude;
-        const f3 rg = scale(gradient, -1.0F);   // spiky_gradient(-d), exactly
-        const d3 reb = ld3(eta[t]);
-        const float rdiff = magnitude - magnitude_j;
-        d3 hessian, reverse_hessian;   // H(d) applied to both sides' adjoints; H(-d) = H(d)
-        spiky_hessian_products(d, times(eb, difference), times(reb, rdiff), k, hessian, reverse_hessian);
-        pc = pc + hessian;
-        mc -= dot(eb, gradient);
-        pc = pc + times(reverse_hessian, -1.0);
-        mc += dot(reb, rg);
+        // the reverse term has -d, -grad W and -difference, exactly: both terms in one, of the sum
+        const PairDerivatives w = pair_derivatives(r2, k);
+        const d3 both_eta = eb + ld3(eta[t]);
+        mc -= dot(both_eta, scale(d, w.scale));
+        pc = pc + hessian_product(w, wide(d), times(both_eta, static_cast<double>(vorticity[t].w - magnitude)));
     }
 };
 
@@ -358,18 +347,11 @@ struct VorticityVjpOp {
         const f3 d = sub(x, xyz(pos[t]));
         const float r2 = squared(d);
         if (r2 == 0.0F || r2 >= k.adjoint_threshold) return;
-        const f3 gradient = spiky_gradient(d, k);
-        const f3 vj = xyz(velocity[t]);
-        const f3 difference = vj - v;
-        const d3 rwb = ld3(vorticity_adjoint[t]);
-        const f3 rg = scale(gradient, -1.0F);   // spiky_gradient(-d), exactly
-        const f3 rdiff = v - vj;
-        d3 hessian, reverse_hessian;   // H(d) applied to both sides' adjoints; H(-d) = H(d)
-        spiky_hessian_products(d, cross(wb, difference), cross(rwb, rdiff), k, hessian, reverse_hessian);
-        vc = vc + cross(wb, gradient);
-        pc = pc + hessian;
-        vc = vc + cross(rg, rwb);
-        pc = pc + times(reverse_hessian, -1.0);
+        // the reverse term has -d, -grad W and -difference, exactly: both terms in one, of the sum
+        const PairDerivatives w = pair_derivatives(r2, k);
+        const d3 both_adjoints = wb + ld3(vorticity_adjoint[t]);
+        vc = vc + cross(both_adjoints, wide(scale(d, w.scale)));
+        pc = pc + hessian_product(w, wide(d), cross(both_adjoints, wide(xyz(velocity[t]) - v)));
     }
 };
 
@@ -479,9 +461,9 @@ struct CorrectionVjpOp {
         const f3 d = sub(x, xyz(q));
         const float r2 = squared(d);
         if (r2 == 0.0F || r2 >= k.adjoint_threshold) return;
-        const f3 gradient = spiky_gradient(d, k);
-        const f3 rg = scale(gradient, -1.0F);   // spiky_gradient(-d), exactly
-        const float weight = r2 >= k.h2 ? 0.0F : poly6_inside(r2, k);   // W(d) = W(-d)
+        const PairDerivatives w = pair_derivatives(r2, k);
+        const f3 gradient = scale(d, w.scale);      // grad W(-d) = -grad W(d), exactly
+        const float weight = poly6_weight(r2, k);   // W(d) = W(-d)
         const ArtificialPressure ap = zero_strength_i ? zero_strength_pressure(weight, reference_i, strength, exponent, true)
                                                       : artificial_pressure(d, k, strength, exponent, radius);
         const float4 rv = reverse[t];   // (rho0_j, strength_j, exponent_j, zero-strength flag)
@@ -490,27 +472,27 @@ struct CorrectionVjpOp {
         const float coefficient = own_ratio(q.w, rest_density);
         const float lambda_j = lambda[t];
         const float multiplier = lambda_i + lambda_j + ap.value;
-        const double scalar_adjoint = coefficient * dot(ob, gradient);
+        const d3 wide_gradient = wide(gradient);
+        const double scalar_adjoint = coefficient * dot(ob, wide_gradient);
         const float rrest = rv.x;
         reverse_ratio.update(mass, rrest);
         const float rcoefficient = reverse_ratio.value;
         const float rmultiplier = lambda_j + lambda_i + rap.value;
         const d3 rob = ld3(correction[t]);
-        const double rscalar = rcoefficient * dot(rob, rg);
-        d3 hessian, reverse_hessian;   // H(d) applied to both sides' adjoints; H(-d) = H(d)
-        spiky_hessian_products(d, times(ob, coefficient * multiplier), times(rob, rcoefficient * rmultiplier), k, hessian,
-                               reverse_hessian);
-        pc = pc + hessian;
-        pc = pc + times(ap.gradient, scalar_adjoint);
-        lc += scalar_adjoint;
-        rc += dot(ob, times(gradient, coefficient * multiplier));   // divided by -rho0_i once, at the end
+        const double rscalar = -(rcoefficient * dot(rob, wide_gradient));
+        const float factor = coefficient * multiplier;
+        const double own = factor, reverse = rcoefficient * rmultiplier;
+        pc = pc + hessian_product(w, wide(d), times(ob, own) - times(rob, reverse));
+        lc += scalar_adjoint + rscalar;
+        rc += dot(ob, times(gradient, factor));   // divided by -rho0_i once, at the end
         sc += scalar_adjoint * ap.d_strength;
-        ec += scalar_adjoint * ap.d_exponent;
-        qc += scalar_adjoint * ap.d_radius;
-        pc = pc + times(reverse_hessian, -1.0);
-        pc = pc + times(rap.gradient, -rscalar);
-        lc += rscalar;
-        mc += dot(rob, times(rg, rmultiplier / rrest));
+        if (!zero_strength_i) {   // otherwise all zeros
+            pc = pc + times(ap.gradient, scalar_adjoint);
+            ec += scalar_adjoint * ap.d_exponent;
+            qc += scalar_adjoint * ap.d_radius;
+        }
+        if (rv.w == 0.0F) pc = pc + times(rap.gradient, -rscalar);
+        mc -= dot(rob, times(gradient, rmultiplier / rrest));
     }
     // boundary particle (position at the step's time, volume): pbf.cu:390-405
     __device__ __forceinline__ void boundary_term(const float4 q) {
@@ -642,28 +624,24 @@ struct LambdaVjpOp {
         const f3 d = sub(x, xyz(q));
         const float r2 = squared(d);
         if (r2 == 0.0F || r2 >= k.adjoint_threshold) return;
-        const f3 gradient = spiky_gradient(d, k);
+        const PairDerivatives w = pair_derivatives(r2, k);
+        const f3 gradient = scale(d, w.scale);   // grad W(-d) = -grad W(d), exactly
         const float coefficient = own_ratio(q.w, rest_density);
         const f3 neighbor_gradient = times(gradient, -coefficient);
         const d3 neighbor_gradient_adjoint = times(neighbor_gradient, 2.0 * db);
-        const d3 gradient_adjoint = times(sb - neighbor_gradient_adjoint, coefficient);
+        const d3 gradient_adjoint = times(sb - neighbor_gradient_adjoint, static_cast<double>(coefficient));
         self_gradient = fma3(coefficient, gradient, self_gradient);
         rc_pairs += dot(neighbor_gradient_adjoint, neighbor_gradient);   // divided by -rho0_i once, at the end
         const float4 gj = gradient_sum_rest[t];   // (S_j, rho0_j)
         const float rrest = gj.w;
         const double rdb = constraint_weight[t];   // the neighbour's db, as its own lambda VJP forms it
         const d3 rsb = times(xyz(gj), 2.0 * rdb);
-        const f3 rg = scale(gradient, -1.0F);   // spiky_gradient(-d), exactly
         reverse_ratio.update(mass, rrest);
         const float rcoefficient = reverse_ratio.value;
-        const f3 rneighbor_gradient = times(rg, -rcoefficient);
-        const d3 rneighbor_gradient_adjoint = times(rneighbor_gradient, 2.0 * rdb);
-        const d3 rgradient_adjoint = times(rsb - rneighbor_gradient_adjoint, rcoefficient);
-        d3 hessian, reverse_hessian;   // H(d) applied to both sides' adjoints; H(-d) = H(d)
-        spiky_hessian_products(d, gradient_adjoint, rgradient_adjoint, k, hessian, reverse_hessian);
-        pc = pc + hessian;
-        pc = pc + times(reverse_hessian, -1.0);
-        mc += dot(rsb - rneighbor_gradient_adjoint, rg) * reverse_ratio.reciprocal;
+        const f3 rneighbor_gradient = times(gradient, rcoefficient);
+        const d3 reverse_adjoint = rsb - times(rneighbor_gradient, 2.0 * rdb);
+        pc = pc + hessian_product(w, wide(d), gradient_adjoint - times(reverse_adjoint, static_cast<double>(rcoefficient)));
+        mc -= dot(reverse_adjoint, gradient) * reverse_ratio.reciprocal;
     }
 };
 
@@ -749,11 +727,12 @@ struct DensityVjpOp {
         }
         const float4 q = pos[t];
         const f3 d = sub(x, xyz(q));
-        if (squared(d) >= k.h2) return;
-        const f3 gradient = poly6_gradient(d, k);
+        const float r2 = squared(d);
+        if (r2 >= k.h2) return;
+        const f3 gradient = scale(d, poly6_gradient_scale(r2, k));
         const double rb = density_adjoint[t];
         pc = pc + times(gradient, ob * q.w + rb * mass);
-        mc += rb * poly6(d, k);
+        mc += rb * poly6_weight(r2, k);
     }
 };
 
