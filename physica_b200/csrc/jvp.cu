@@ -76,15 +76,14 @@ __device__ __forceinline__ f3 spiky_gradient_tangent(const f3 d, const f3 dd, co
 // and divisions pair by pair.
 __device__ __forceinline__ void spiky_pair(const f3 d, const f3 dd, const float r2, const KernelConstants& k, f3& gradient,
                                            f3& gradient_dot) {
+    // grad W = along d and its derivative along dd + across (d . dd) d
     const float inverse = rsqrtf(r2);
-    const float distance = r2 * inverse;
-    const f3 direction = times(d, inverse);
-    const float difference = k.h - distance;
-    const float radial = dot(direction, dd);
-    gradient = times(direction, k.spiky_coefficient * difference * difference);
-    const f3 direction_tangent = times(dd + times(direction, -radial), inverse);
-    gradient_dot = times(times(direction, -2.0F * difference * radial) + times(direction_tangent, difference * difference),
-                         k.spiky_coefficient);
+    const float difference = k.h - r2 * inverse;
+    const float slope = k.spiky_coefficient * difference;
+    const float along = slope * difference * inverse;
+    const float across = -(slope + slope + along) * (inverse * inverse) * dot(d, dd);
+    gradient = times(d, along);
+    gradient_dot = times(dd, along) + times(d, across);
 }
 
 // ------------------------------------------------------------------- seed
@@ -100,7 +99,8 @@ __global__ void tangent_seed_kernel(const uint32_t count, const uint32_t* __rest
     const f3 vd = mk(v_dot.x[i], v_dot.y[i], v_dot.z[i]);
     const f3 ad = mk(a_dot.x[i], a_dot.y[i], a_dot.z[i]);
     const f3 predicted = xd + times(vd + times(ad, dt), dt);
-    x0[s] = make_float4(predicted.x, predicted.y, predicted.z, 0.0F);
+    // the passes read a neighbour's position and mass tangents in one load
+    x0[s] = make_float4(predicted.x, predicted.y, predicted.z, or_zero(pt.masses, i));
     x_state[s] = make_float4(xd.x, xd.y, xd.z, 0.0F);
     params_a[s] = make_float4(or_zero(pt.masses, i), or_zero(pt.rest_densities, i), or_zero(pt.relaxation, i), or_zero(pt.xsph, i));
     params_b[s] = make_float4(or_zero(pt.strength, i), or_zero(pt.exponent, i), or_zero(pt.radius, i), or_zero(pt.vorticity, i));
@@ -108,8 +108,7 @@ __global__ void tangent_seed_kernel(const uint32_t count, const uint32_t* __rest
 
 struct Pair {
     float4 q;    // neighbour position and mass
-    float4 qd;   // neighbour position tangent
-    float4 aux;  // pass-specific neighbour data
+    float4 qd;   // their tangents
 };
 
 // ------------------------------------------------------ density + lambda
@@ -129,7 +128,6 @@ struct DensityLambdaJvpOp {
     const float4* __restrict__ pos;
     const float4* __restrict__ boundary;
     const float4* __restrict__ x_dot;
-    const float4* __restrict__ params_a_dot;
     f3 x, xd;
     uint32_t self;
     float rest, rest_dot, inverse_rest;
@@ -138,8 +136,8 @@ struct DensityLambdaJvpOp {
     f3 gsum_dot;
 
     __device__ __forceinline__ Pair prefetch(const uint32_t t) const {
-        if (t & kBoundaryBit) return {boundary[t & ~kBoundaryBit], make_float4(0, 0, 0, 0), make_float4(0, 0, 0, 0)};
-        return {pos[t], x_dot[t], params_a_dot[t]};
+        if (t & kBoundaryBit) return {boundary[t & ~kBoundaryBit], make_float4(0, 0, 0, 0)};
+        return {pos[t], x_dot[t]};
     }
     __device__ __forceinline__ void apply(const uint32_t t, const Pair& in) {
         const f3 d = x - xyz(in.q);
@@ -155,8 +153,8 @@ struct DensityLambdaJvpOp {
             gsum_dot = gsum_dot + times(spiky_gradient_tangent(d, xd, distance, k), volume);
             return;
         }
-        const float mass_dot = in.aux.x;
-        if (r2 < k.h2) density_dot += mass_dot * poly6_inside(r2, k) + in.q.w * dot(poly6_gradient(d, k), dd);
+        const float mass_dot = in.qd.w;
+        if (r2 < k.h2) density_dot += mass_dot * poly6_weight(r2, k) + in.q.w * dot(scale(d, poly6_gradient_scale(r2, k)), dd);
         if (t == self) return;
         // one reciprocal square root per pair and the reciprocal rest density instead of IEEE
         // divisions (the 1M tangent step: 10.65 -> 9.65 ms; 1.6e-7 relative to the reference
@@ -188,7 +186,6 @@ __global__ void __launch_bounds__(kBlock, PBF_JVP_MIN_BLOCKS) density_lambda_jvp
     op.pos = a.pos;
     op.boundary = a.g.boundary;
     op.x_dot = a.x_dot;
-    op.params_a_dot = a.params_a_dot;
     op.self = p.s;
     op.k = p.k;
     op.x = xyz(a.pos[p.s]);
@@ -231,7 +228,7 @@ struct CorrectionJvpArgs {
 
 struct CorrectionPair {
     float4 q, qd;
-    float lambda, lambda_dot, mass_dot;
+    float lambda, lambda_dot;
 };
 
 struct CorrectionJvpOp {
@@ -241,7 +238,6 @@ struct CorrectionJvpOp {
     const float4* __restrict__ x_dot;
     const float* __restrict__ lambda;
     const float* __restrict__ lambda_dot;
-    const float4* __restrict__ params_a_dot;
     f3 x, xd;
     uint32_t self;
     float rest, rest_dot, inverse_rest, lambda_i, lambda_dot_i;
@@ -251,8 +247,8 @@ struct CorrectionJvpOp {
     f3 result;
 
     __device__ __forceinline__ CorrectionPair prefetch(const uint32_t t) const {
-        if (t & kBoundaryBit) return {boundary[t & ~kBoundaryBit], make_float4(0, 0, 0, 0), 0.0F, 0.0F, 0.0F};
-        return {pos[t], x_dot[t], lambda[t], lambda_dot[t], params_a_dot[t].x};
+        if (t & kBoundaryBit) return {boundary[t & ~kBoundaryBit], make_float4(0, 0, 0, 0), 0.0F, 0.0F};
+        return {pos[t], x_dot[t], lambda[t], lambda_dot[t]};
     }
     __device__ __forceinline__ void apply(const uint32_t t, const CorrectionPair& in) {
         if (t == self) return;
@@ -278,7 +274,7 @@ struct CorrectionJvpOp {
         f3 gradient, gradient_dot;
         spiky_pair(d, dd, r2, k, gradient, gradient_dot);
         const float coefficient = in.q.w * inverse_rest;
-        const float coefficient_dot = (in.mass_dot - in.q.w * rest_dot * inverse_rest) * inverse_rest;
+        const float coefficient_dot = (in.qd.w - in.q.w * rest_dot * inverse_rest) * inverse_rest;
         const float multiplier = lambda_i + in.lambda + art;
         const float multiplier_dot = lambda_dot_i + in.lambda_dot + art_dot;
         result = result + times(gradient, coefficient_dot * multiplier + coefficient * multiplier_dot) +
@@ -299,7 +295,6 @@ __global__ void __launch_bounds__(kBlock, 7) correction_jvp_kernel(const Correct
     op.x_dot = a.x_dot;
     op.lambda = a.lambda;
     op.lambda_dot = a.lambda_dot;
-    op.params_a_dot = a.params_a_dot;
     op.self = p.s;
     op.k = p.k;
     op.x = xyz(a.pos[p.s]);
@@ -322,7 +317,7 @@ __global__ void __launch_bounds__(kBlock, 7) correction_jvp_kernel(const Correct
     op.result = mk(0.0F, 0.0F, 0.0F);
     replay(op, p, a.g, a.list);
     const f3 next = masked(op.xd + op.result, a.mask[p.s]);
-    a.x_dot_next[p.s] = make_float4(next.x, next.y, next.z, 0.0F);
+    a.x_dot_next[p.s] = make_float4(next.x, next.y, next.z, pad.x);
     if (!a.last) return;
     const uint32_t i = a.sorted_index[p.s];
     a.out_positions.x[i] = next.x;
@@ -519,8 +514,8 @@ struct XsphJvpOp {
         const float r2 = squared(d);
         if (r2 >= k.h2) return;
         const f3 dd = xd - xyz(in.qd);
-        const float weight = poly6_inside(r2, k);
-        const float weight_dot = dot(poly6_gradient(d, k), dd);
+        const float weight = poly6_weight(r2, k);
+        const float weight_dot = dot(scale(d, poly6_gradient_scale(r2, k)), dd);
         const f3 difference = xyz(in.w) - v;
         const f3 difference_dot = xyz(in.wd) - vd;
         smoothing = smoothing + times(difference, weight);
