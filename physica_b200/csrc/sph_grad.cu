@@ -302,16 +302,16 @@ struct ForceVjpOp {
         v_speed += vc.second_speed;
         // pressure (sph/common.cu:263-277)
         const f3 gradient = cubic_gradient_value(disp, k);
-        const double second_term = static_cast<double>(d.p) / (d.aux.x * d.aux.x);
+        const double second_term = d.p * wide_reciprocal(d.aux.x * d.aux.x);
         const double sum = first_term + second_term;
         const double local_factor = -mj * sum;
         const double local_factor_adjoint = dot(adjoint, gradient);
         first_term_adjoint -= mj * local_factor_adjoint;
-        p_position = p_position + hessian_times(H, disp, times(adjoint, local_factor));
         const double cross_projection = dot(cross, gradient);
         p_mass += sum * cross_projection;
         first_term_adjoint += mass * cross_projection;
-        p_position = p_position + hessian_times(H, disp, times(cross, mass * sum));
+        // both directions' Hessian products in one: H is linear and H(-d) = H(d)
+        p_position = p_position + hessian_times(H, disp, times(adjoint, local_factor) + times(cross, mass * sum));
     }
     __device__ __forceinline__ void process(const uint32_t t) { apply(t, prefetch(t)); }
 };
@@ -587,17 +587,17 @@ struct PressureVjpOp {
         }
         if (t == self) return;
         const float mj = d.q.w;
-        const double second_term = static_cast<double>(d.p) / (d.rho * d.rho);
+        const double second_term = d.p * wide_reciprocal(d.rho * d.rho);
         const double sum = first_term + second_term;
         const double local_factor = -mj * sum;
         const double local_factor_adjoint = dot(adjoint, gradient);
         first_term_adjoint -= mj * local_factor_adjoint;
-        position = position + hessian_times(H, disp, times(adjoint, local_factor));
         const d3 cross = ld(d.adjoint);
         const double cross_projection = dot(cross, gradient);
         mass_sum += sum * cross_projection;
         first_term_adjoint += mass * cross_projection;
-        position = position + hessian_times(H, disp, times(cross, mass * sum));
+        // both directions' Hessian products in one: H is linear and H(-d) = H(d)
+        position = position + hessian_times(H, disp, times(adjoint, local_factor) + times(cross, mass * sum));
     }
     __device__ __forceinline__ void process(const uint32_t t) { apply(t, prefetch(t)); }
 };
@@ -686,6 +686,7 @@ struct NonPressureVjpOp {
     uint32_t self;
     f3 x, v;
     float mass, density, viscosity;
+    double inverse_density, inverse_density_squared;   // 1 / rho_i and 1 / (rho_i rho_i), the product in float
     d3 adjoint;
     SphConstants k;
     d3 position, velocity;
@@ -717,17 +718,17 @@ struct NonPressureVjpOp {
         const float weight = __fdiv_rn(__fmul_rn(__fmul_rn(mu, mj), laplacian), rho_j);
         const double weight_adjoint = dot(adjoint, difference);
         velocity = velocity + times(adjoint, -weight);
-        const double viscosity_adjoint = weight_adjoint * mj * laplacian / rho_j;
-        viscosity_sum += 0.5 * viscosity_adjoint;
-        position = position + laplacian_gradient(disp, k, weight_adjoint * mu * mj / rho_j);
+        const double inverse_rho = wide_reciprocal(rho_j);
+        const double own = weight_adjoint * mj * inverse_rho;
         const d3 cross = ld(d.adjoint);
         const float cross_weight = __fdiv_rn(__fmul_rn(__fmul_rn(mu, mass), laplacian), density);
         const double cross_weight_adjoint = dot(cross, scale(difference, -1.0F));
         velocity = velocity + times(cross, cross_weight);
-        mass_sum += cross_weight_adjoint * mu * laplacian / density;
-        density_sum -= cross_weight_adjoint * mu * mass * laplacian / (density * density);
-        viscosity_sum += 0.5 * cross_weight_adjoint * mass * laplacian / density;
-        position = position + laplacian_gradient(disp, k, cross_weight_adjoint * mu * mass / density);
+        const double reverse = cross_weight_adjoint * inverse_density;
+        mass_sum += reverse * mu * laplacian;
+        density_sum -= cross_weight_adjoint * mu * mass * laplacian * inverse_density_squared;
+        viscosity_sum += 0.5 * laplacian * (own + reverse * mass);
+        position = position + laplacian_gradient(disp, k, mu * (own + reverse * mass));
     }
     __device__ __forceinline__ void process(const uint32_t t) { apply(t, prefetch(t)); }
 };
@@ -750,6 +751,8 @@ __global__ void __launch_bounds__(kBlock, PBF_SPH_NON_PRESSURE_VJP_MIN_BLOCKS) n
     op.v = xyz(st.velocity[s]);
     op.mass = o.mass;
     op.density = st.aux[s].x;
+    op.inverse_density = 1.0 / static_cast<double>(op.density);
+    op.inverse_density_squared = 1.0 / static_cast<double>(op.density * op.density);
     op.viscosity = o.pa.y;
     op.adjoint = ld(a.adjoint[s]);
     op.k = *o.k;

@@ -165,7 +165,8 @@ struct CubicHessian {
 
 __device__ __forceinline__ CubicHessian cubic_hessian(const f3 d, const SphConstants& k) {
     CubicHessian H{};
-    const double r2 = static_cast<double>(sq_xfirst(d));
+    const float r2f = sq_xfirst(d);
+    const double r2 = static_cast<double>(r2f);
     const double c = k.cubic_coefficient_d;
     if (r2 == 0.0) {
         H.kind = 1;
@@ -173,7 +174,7 @@ __device__ __forceinline__ CubicHessian cubic_hessian(const f3 d, const SphConst
         return H;
     }
     if (r2 >= k.support_squared_d) return H;
-    const double inverse_r = rsqrt(r2);
+    const double inverse_r = wide_rsqrt(r2f);
     const double q = r2 * inverse_r * k.inverse_h_d;
     const double first = q <= 0.5 ? 18.0 * q * q - 12.0 * q : -6.0 * (1.0 - q) * (1.0 - q);
     const double second = q <= 0.5 ? 36.0 * q - 12.0 : 12.0 * (1.0 - q);
@@ -194,9 +195,9 @@ __device__ __forceinline__ d3 hessian_times(const CubicHessian& H, const f3 d, c
 // Gradient of the viscosity Laplacian times `scalar`, in FP64 (density/device.cuh:84-88); -45 / (pi h^6)
 // is the per-scene constant SphConstants::laplacian_scale_d, and the support test is the exact one above.
 __device__ __forceinline__ d3 laplacian_gradient(const f3 d, const SphConstants& k, const double scalar) {
-    const double r2 = static_cast<double>(sq_xfirst(d));
-    if (r2 == 0.0 || r2 >= k.support_squared_d) return {0.0, 0.0, 0.0};
-    return times(d, k.laplacian_scale_d * scalar * rsqrt(r2));
+    const float r2 = sq_xfirst(d);
+    if (r2 == 0.0F || static_cast<double>(r2) >= k.support_squared_d) return {0.0, 0.0, 0.0};
+    return times(d, k.laplacian_scale_d * scalar * wide_rsqrt(r2));
 }
 
 // The unclamped prediction's collision mask (sph/pcisph.cu:20-24, 69-71).
