@@ -109,6 +109,13 @@ __global__ void __launch_bounds__(kBlock, 12) list_walk_kernel(const ListScanArg
             for (int dy = -1; dy <= 1; ++dy) {
                 const int y = c.y + dy;
                 if (y < 0 || y >= cy) continue;
+                const uint32_t low = cell_index(grid, x, y, z_lo), high = cell_index(grid, x, y, z_hi) + 1u;
+                if (a.packed.x && boffsets[low] == boffsets[high]) {   // no boundary particle in the column: one range
+                    packed.n = scan.n;
+                    packed.run(a.packed, offsets[low], offsets[high]);
+                    scan.n = packed.n;
+                    continue;
+                }
                 for (uint32_t z = z_lo; z <= z_hi; ++z) {
                     const uint32_t cell = cell_index(grid, x, y, z);
                     scan.run(a.pos, offsets[cell], offsets[cell + 1u]);
