@@ -138,6 +138,14 @@ Engine::~Engine() {
 
 static bool finite_positive(const float v) { return std::isfinite(v) && v > 0.0F; }
 
+namespace {
+// A differentiable step over staged windows also stores the lists of sorted slots that the reverse and
+// tangent sweeps replay.  That costs as much as the windows save up to about 400k particles and pays above:
+// tangent step at 262k 1.54 ms against 1.55 with the fused per-lane scan, 590k 2.96 / 3.04, 1M 4.78 / 5.20;
+// gradient step at 64k 1.14 / 1.07, 262k 3.06 / 3.05, 590k 6.30 / 6.38.
+constexpr uint32_t kStagedDifferentiable = 1u << 19;
+}  // namespace
+
 int Engine::init(const pbf_domain_configuration* scenes, const uint32_t scene_count, const pbf_configuration* configuration,
                  const pbf_execution_mode mode, cudaStream_t stream) {
     if (!scenes || scene_count == 0 || !configuration) {
@@ -215,11 +223,16 @@ int Engine::init(const pbf_domain_configuration* scenes, const uint32_t scene_co
     packed_ = alloc_packed(arena_, count_, e);
     bool boundary = false;
     for (uint32_t s = 0; s < scene_count; ++s) boundary = boundary || scenes[s].boundary_particle_count > 0;
-    if (mode == PBF_EXECUTION_FORWARD && !boundary) {
+    if (!boundary && (mode == PBF_EXECUTION_FORWARD || count_ >= kStagedDifferentiable)) {
         packed_next_ = alloc_packed(arena_, count_, e);
         packed_velocity_ = alloc_packed(arena_, count_, e);
         packed_mass_ = arena_.alloc<float>(static_cast<size_t>(count_) + 4u, e);
         packed_magnitude_ = arena_.alloc<float>(static_cast<size_t>(count_) + 4u, e);
+        staged_list_.windows = arena_.alloc<uint32_t>(window_words(count_), e);
+        if (mode == PBF_EXECUTION_DIFFERENTIABLE) {
+            const size_t padded = (static_cast<size_t>(count_) + 31u) / 32u * 32u;
+            staged_list_.list = {arena_.alloc<uint32_t>(padded * kListCapacity, e), arena_.alloc<uint32_t>(count_, e), kListCapacity};
+        }
     }
     arrival_ = arena_.alloc<uint32_t>(count_, e);
     unordered_ = arena_.alloc<uint32_t>(count_, e);
@@ -396,7 +409,6 @@ int Engine::allocate_record(StepRecord& r) {
         r.list_entries[l] = r.arena.alloc<uint32_t>(padded * r.list_capacity, e);
         r.list_counts[l] = r.arena.alloc<uint32_t>(n, e);
     }
-    if (packed_mass_) r.list_windows = r.arena.alloc<uint32_t>(window_words(n), e);
     if (boundary_count_ > 0) {
         r.boundary_offsets = r.arena.alloc<uint32_t>(cells_ + 1, e);
         r.boundary = r.arena.alloc<float4>(boundary_count_, e);
@@ -561,7 +573,7 @@ int Engine::launch_forward(cudaStream_t stream, const pbf_particle_state* state,
     }
     timer_.end(stream, kPassGrid);
 
-    if (runs_staged(shape_, diff, boundary_count_ > 0, K)) {
+    if (runs_staged_passes(shape_)) {
         if (int rc = launch_staged(stream, state, next_state, r)) return rc;
         return check(launch_advance_step(stream, d_step_), "step counter");
     }
@@ -647,26 +659,42 @@ int Engine::record_positions_ready(cudaStream_t stream) {
     return check(cudaEventRecordWithFlags(positions_ready_, stream, flags), "positions event");
 }
 
-// The Jacobi iterations and the post-loop passes over staged windows (staged.cu): two kernels per
-// iteration, then three.
+bool Engine::runs_staged_passes(const LaunchShape& shape) const {
+    return runs_staged(shape, boundary_count_ > 0, iterations_) && (!differentiable() || count_ >= kStagedDifferentiable);
+}
+
+// The Jacobi iterations and the post-loop passes over staged windows (staged.cu): two
+// kernels per iteration, then three.
 int Engine::launch_staged(cudaStream_t stream, const pbf_particle_state* state, pbf_particle_state* next_state, StepRecord& r) {
     const GatherCommon gc = gather_common(r);
     // passes that read what their predecessor wrote last start there (it is the part still in L2)
     GatherCommon gc_reverse = gc;
     gc_reverse.reverse = 1;
+    const bool diff = differentiable();
+    const bool keep = r.keeps_all(diff);
     const uint32_t K = iterations_;
-    const StagedList list{{r.list_entries[0], r.list_counts[0], r.list_capacity}, r.list_windows};
+    StagedList list = staged_list_;
+    if (!diff) list.list = {r.list_entries[0], r.list_counts[0], r.list_capacity};
+    // the lists of sorted slots that the reverse and tangent sweeps replay: every iterate's where all
+    // are kept, and the post-loop one
+    auto slots = [&](const uint32_t k) {
+        if (!diff || (k < K && !keep)) return StoredList{};
+        const uint32_t l = keep ? k : 0u;
+        return StoredList{r.list_entries[l], r.list_counts[l], r.list_capacity};
+    };
     PackedPositions current = packed_, next = packed_next_;
     for (uint32_t k = 0; k < K; ++k) {
-        const float4* xk = r.iterate(k, K, false);
-        float* lambda = k == 0 ? r.first_lambda : r.lambda[0];
-        const StagedDensityArgs d{gc, list, current, packed_mass_, xk, lambda, k == 0 ? r.first_density : nullptr,
+        const float4* xk = r.iterate(k, K, diff);
+        float* lambda = keep ? r.lambda[k] : (k == 0 ? r.first_lambda : r.lambda[0]);
+        const StagedDensityArgs d{gc, list, slots(k), current, packed_mass_, xk, lambda,
+                                  keep ? r.density[k] : (k == 0 ? r.first_density : nullptr), keep ? r.gsum[k] : nullptr,
                                   k == 0 ? r.neighbor_count : nullptr};
         timer_.begin(stream, kPassScanDensityLambda);
         if (int rc = check(launch_staged_density(stream, d), "staged scan + density/lambda")) return rc;
         timer_.end(stream, kPassScanDensityLambda);
         const StagedCorrectionArgs c{gc_reverse, list, current, packed_mass_, lambda, xk, next,
-                                     const_cast<float4*>(r.iterate(k + 1, K, false)), k + 1 == K ? 1 : 0,
+                                     const_cast<float4*>(r.iterate(k + 1, K, diff)), diff ? r.mask[k] : nullptr,
+                                     k + 1 == K ? 1 : 0,
                                      {state->positions.x, state->positions.y, state->positions.z}, r.sorted_index,
                                      {next_state->positions.x, next_state->positions.y, next_state->positions.z}, r.velocity,
                                      packed_velocity_};
@@ -676,8 +704,8 @@ int Engine::launch_staged(cudaStream_t stream, const pbf_particle_state* state, 
         std::swap(current, next);
     }
     if (int rc = record_positions_ready(stream)) return rc;
-    const float4* xK = r.iterate(K, K, false);
-    const StagedVorticityArgs v{gc_reverse, list, current, packed_velocity_, xK, r.velocity, r.vorticity, packed_magnitude_};
+    const float4* xK = r.iterate(K, K, diff);
+    const StagedVorticityArgs v{gc_reverse, list, slots(K), current, packed_velocity_, xK, r.velocity, r.vorticity, packed_magnitude_};
     timer_.begin(stream, kPassVorticity);
     if (int rc = check(launch_staged_vorticity(stream, v), "staged scan + vorticity")) return rc;
     timer_.end(stream, kPassVorticity);
@@ -798,7 +826,7 @@ int Engine::autotune(const pbf_particle_state* state, const pbf_control* control
     int rc = PBF_SUCCESS;
     // 1. the list scan: variant x block size, by the time of the scans and the gather passes (the
     //    variants differ in which passes they fuse).  The staged passes have a block size of their own.
-    const bool staged = runs_staged(LaunchShape{kScanStaged16, 128u, 128u}, differentiable(), boundary_count_ > 0, iterations_);
+    const bool staged = runs_staged_passes(LaunchShape{kScanStaged16, 128u, 128u});
     LaunchShape best = previous;
     best.block = 128u;
     double best_scan = -1.0;

@@ -102,7 +102,6 @@ struct StepRecord {
     std::vector<uint32_t*> list_entries;
     std::vector<uint32_t*> list_counts;
     uint32_t list_capacity = 0;
-    uint32_t* list_windows = nullptr;   // staged passes: the lists' windows (forward mode)
     // Boundary particles of the step (only when the scenes have some).
     uint32_t* boundary_offsets = nullptr;   // cells + 1
     float4* boundary = nullptr;             // (position at the step's time, volume), cell-sorted
@@ -294,12 +293,15 @@ private:
     // The current iterate as three arrays in sorted order (x, y, z), written by the grid build and
     // every correction, read by the per-lane list scan.
     PackedPositions packed_{};
-    // Forward mode without boundary particles: the staged passes' fields in sorted order.  Iterates
-    // alternate between packed_ and packed_next_; the confined velocities reuse the free one.
+    // Scenes without boundary particles: the staged passes' fields in sorted order.  Iterates alternate
+    // between packed_ and packed_next_; the confined velocities reuse the free one.  Differentiable
+    // steps, whose records hold lists of sorted slots, keep the staged list here.
     PackedPositions packed_next_{}, packed_velocity_{};
     float* packed_mass_ = nullptr;
     float* packed_magnitude_ = nullptr;
+    StagedList staged_list_{};
     int record_positions_ready(cudaStream_t stream);
+    bool runs_staged_passes(const LaunchShape& shape) const;
     int launch_staged(cudaStream_t stream, const pbf_particle_state* state, pbf_particle_state* next_state, StepRecord& r);
     uint32_t* arrival_ = nullptr;
     uint32_t* unordered_ = nullptr;

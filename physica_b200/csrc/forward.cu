@@ -675,8 +675,8 @@ bool fuses_density(const LaunchShape& shape, const ListScanArgs& a) {
            !a.g.boundary_offsets;
 }
 
-bool runs_staged(const LaunchShape& shape, const bool differentiable, const bool boundary, const uint32_t iterations) {
-    return shape.scan == kScanStaged16 && !differentiable && !boundary && iterations > 0;
+bool runs_staged(const LaunchShape& shape, const bool boundary, const uint32_t iterations) {
+    return shape.scan == kScanStaged16 && !boundary && iterations > 0;
 }
 
 namespace {

@@ -60,9 +60,9 @@ cudaError_t launch_reference_order(cudaStream_t stream, uint32_t count, const Sc
 // in-support neighbour, and the entries' count; kOverflow marks a particle whose list did not fit (it
 // walks its stencil instead).  The staged passes pack two entries in a word (StagedList).
 struct StoredList {
-    uint32_t* entries;
-    uint32_t* counts;
-    uint32_t capacity;
+    uint32_t* entries = nullptr;
+    uint32_t* counts = nullptr;
+    uint32_t capacity = 0;
 };
 
 // Common inputs of every neighbour-gather pass.
@@ -172,8 +172,8 @@ enum ListScanVariant : uint32_t {
     kScanStaged = 2,        // a warp stages its column group's candidates in shared memory
     kScanFusedDensity = 3,  // per lane, and the Jacobi iterations' scans also run density + lambda
                             // in the same kernel (scenes without boundary particles)
-    kScanStaged16 = 4,      // as 3, and forward-mode steps of scenes without boundary particles run
-                            // every pass over windows staged in shared memory (staged.cu)
+    kScanStaged16 = 4,      // every forward pass of scenes without boundary particles over windows staged in
+                            // shared memory (staged.cu; differentiable steps of large scenes only); otherwise as 3
 };
 struct LaunchShape {
     uint32_t scan = kScanStaged16;   // fastest at every size measured (5k to 1M particles)
@@ -186,7 +186,7 @@ cudaError_t launch_list_scan(cudaStream_t stream, const ListScanArgs& a, const L
 // Whether `shape` runs the scan of `a` fused with density + lambda (launch_scan_density_lambda).
 bool fuses_density(const LaunchShape& shape, const ListScanArgs& a);
 // Whether a step with `shape` runs the staged passes.
-bool runs_staged(const LaunchShape& shape, bool differentiable, bool boundary, uint32_t iterations);
+bool runs_staged(const LaunchShape& shape, bool boundary, uint32_t iterations);
 // The list scan of a Jacobi iteration and its density + lambda pass in one kernel (same list and
 // results as launch_list_scan followed by launch_density_lambda).
 cudaError_t launch_scan_density_lambda(cudaStream_t stream, const ListScanArgs& a, const DensityLambdaArgs& d,
@@ -207,23 +207,25 @@ cudaError_t launch_reconstruct(cudaStream_t stream, uint32_t count, const SceneD
                                const float4* positions, Field3 previous_positions, const uint32_t* sorted_index,
                                MutField3 out_positions, float4* velocity);
 
-// ---- forward passes over windows staged in shared memory (staged.cu): forward mode, no boundary
+// ---- forward passes over windows staged in shared memory (staged.cu): scenes without boundary
 // particles.  A list is a StoredList whose entries are pairs of 16-bit staged positions (or, for the
-// blocks that do not fit the stage, sorted slots as elsewhere), and its blocks' windows.
+// particles that do not fit, hit masks over sorted slots), and its blocks' windows.
 constexpr uint32_t kWindowWords = 32;          // words of one block's record
-size_t window_words(uint32_t count);           // words of the records of `count` particles
+size_t window_words(uint32_t count);           // words of the records of `count` particles, in blocks of any size
 struct StagedList {
-    StoredList list;
-    uint32_t* windows;
+    StoredList list{};
+    uint32_t* windows = nullptr;
 };
 struct StagedDensityArgs {
     GatherCommon g;
     StagedList list;           // written
+    StoredList slots;          // also written (entries null: not): the list of sorted slots
     PackedPositions positions;
     const float* mass;
     const float4* pos;         // the same positions and masses, for blocks that work on global memory
     float* lambda;
     float* density;            // optional record
+    float4* gsum_denom;        // optional record
     uint32_t* neighbor_count;  // optional record
 };
 struct StagedCorrectionArgs {
@@ -235,6 +237,7 @@ struct StagedCorrectionArgs {
     const float4* pos;
     PackedPositions positions_next;
     float4* pos_next;
+    uint8_t* mask;             // optional record of the collision mask
     int last;                  // last iteration: reconstruct velocities and write positions out
     Field3 previous_positions;
     const uint32_t* sorted_index;
@@ -245,6 +248,7 @@ struct StagedCorrectionArgs {
 struct StagedVorticityArgs {
     GatherCommon g;
     StagedList list;           // written: the post-loop list
+    StoredList slots;          // also written (entries null: not)
     PackedPositions positions, velocities;
     const float4* pos;
     const float4* velocity;

@@ -44,32 +44,36 @@ def block(count, seed=1, iterations=3, **options):
     return dataclasses.replace(s, **{k: np.ascontiguousarray(v) for k, v in keep.items()})
 
 
-@pytest.mark.parametrize("count", [1, 2, 31, 33, 127, 128, 129, 255, 257, 1000, 4097])
+# four lanes per particle up to 20480 particles, blocks of 32; one lane above, blocks of 128
+@pytest.mark.parametrize("count", [1, 2, 31, 33, 127, 128, 129, 255, 257, 1000, 4097, 20480, 20481])
 def test_counts_around_the_block(count):
     check(block(count))
 
 
-def test_spray_whose_windows_exceed_the_stage():
+@pytest.mark.parametrize("count", [8000, 40000])
+def test_spray_whose_windows_exceed_the_stage(count):
     """Thin spray beside and above a dense block: its blocks' windows cover the block's columns."""
-    s = block(8000)
+    s = block(count)
     rng = np.random.default_rng(3)
-    fly = rng.permutation(8000)[:900]
-    s.positions[:, fly] = (rng.random((3, 900)) * np.asarray(s.box_max)[:, None]).astype(np.float32)
+    fly = rng.permutation(count)[:count // 9]
+    s.positions[:, fly] = (rng.random((3, count // 9)) * np.asarray(s.box_max)[:, None]).astype(np.float32)
     check(s)
 
 
-def test_crowded_lists_overflow():
-    s = block(3000)
-    s.positions[:] = (0.2 + 0.06 * np.random.default_rng(4).random((3, 3000))).astype(np.float32)
+@pytest.mark.parametrize("count", [3000, 24000])
+def test_crowded_lists_overflow(count):
+    s = block(count)
+    s.positions[:, :3000] = (0.2 + 0.06 * np.random.default_rng(4).random((3, 3000))).astype(np.float32)
     check(s, steps=2)
 
 
+@pytest.mark.parametrize("count", [2000, 21000])
 @pytest.mark.parametrize("strength", [0.0, 1e-5])
-def test_mixed_masses_and_coincident_particles(strength):
-    s = block(2000, seed=5)
+def test_mixed_masses_and_coincident_particles(strength, count):
+    s = block(count, seed=5)
     rng = np.random.default_rng(6)
-    s.masses[:] *= rng.choice([0.5, 1.0, 1.5], 2000).astype(np.float32)
-    s.rest_densities[:] *= rng.choice([0.8, 1.0], 2000).astype(np.float32)
+    s.masses[:] *= rng.choice([0.5, 1.0, 1.5], count).astype(np.float32)
+    s.rest_densities[:] *= rng.choice([0.8, 1.0], count).astype(np.float32)
     s.artificial_pressure_strength[:] = strength
     s.positions[:, 100:110] = s.positions[:, 110:120]
     s.velocities[:, 100:110] = s.velocities[:, 110:120]
@@ -77,18 +81,55 @@ def test_mixed_masses_and_coincident_particles(strength):
     check(s)
 
 
+@pytest.mark.parametrize("n", [9, 28])
 @pytest.mark.parametrize("h", [0.0008, 0.003, 1.0, 3000.0])
-def test_support_radii_inside_and_outside_the_packed_range(h):
+def test_support_radii_inside_and_outside_the_packed_range(h, n):
     """The packed pair arithmetic covers radii from 2^-10 to 2^10; others take the scalar path."""
-    n, spacing = 9, 0.5 * h
-    s = scenes.dam_break((n, n, n), (0.0, 0.0, 0.0), (12 * spacing,) * 3, 7, 3, h=h, velocity_sigma=0.2 * h)
+    spacing = 0.5 * h
+    s = scenes.dam_break((n, n, n), (0.0, 0.0, 0.0), ((n + 3) * spacing,) * 3, 7, 3, h=h, velocity_sigma=0.2 * h)
     check(s, steps=2)
 
 
-def test_moving_box():
+@pytest.mark.parametrize("count", [4000, 21000])
+def test_moving_box(count):
     """The sort cells and the gather cells of a moving box round differently."""
-    s = dataclasses.replace(block(4000, seed=8), box_velocity=(0.37, -0.11, 0.23))
+    s = dataclasses.replace(block(count, seed=8), box_velocity=(0.37, -0.11, 0.23))
     check(s, steps=6)
+
+
+@pytest.mark.parametrize("recompute", [False, True])
+@pytest.mark.parametrize("kind", ["block", "spray", "crowded"])
+def test_differentiable_steps_record_the_same_lists(kind, recompute):
+    """Adjoint and tangent over the lists of sorted slots that the staged passes store (differentiable
+    steps use the staged passes from 2^19 particles on)."""
+    n = (1 << 19) + 77
+    s = block(n, seed=9, iterations=2)
+    rng = np.random.default_rng(10)
+    if kind == "spray":
+        fly = rng.permutation(n)[:20000]
+        s.positions[:, fly] = (rng.random((3, 20000)) * np.asarray(s.box_max)[:, None]).astype(np.float32)
+    if kind == "crowded":
+        s.positions[:, :3000] = (0.2 + 0.06 * rng.random((3, 3000))).astype(np.float32)
+    out = []
+    for shape in (PER_LANE, STAGED):
+        solver, state, control, params = pbf.solver_for_scene(s, mode=pbf.ExecutionMode.differentiable)
+        solver.launch_shape = shape
+        solver.set_checkpoint_recompute(recompute)
+        cache, following = solver.allocate_step_cache(), solver.allocate_state()
+        solver.forward_step(state, control, params, following, cache)
+        g = torch.Generator(device="cuda").manual_seed(11)
+        rand = lambda dtype: torch.randn((3, s.count), generator=g, device="cuda", dtype=dtype)
+        pa, ca, qa = solver.allocate_state_adjoint(), solver.allocate_control_adjoint(), solver.allocate_parameter_adjoint()
+        solver.vjp_step(state, control, params, following, cache, pbf.StateAdjoint(rand(torch.float64), rand(torch.float64)), pa,
+                        ca, qa)
+        tangent = solver.allocate_state_tangent()
+        solver.jvp_step(state, control, params, following, cache, pbf.StateTangent(rand(torch.float32), rand(torch.float32)),
+                        pbf.Control(rand(torch.float32)), solver.allocate_parameter_tangent(), tangent)
+        solver.synchronize()
+        out.append([following.positions, following.velocities, pa.positions, pa.velocities, ca.external_accelerations,
+                    tangent.positions, tangent.velocities, *qa.tensors.values()])
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a.cpu().numpy(), b.cpu().numpy())
 
 
 def test_batch_blocks_span_scenes():
