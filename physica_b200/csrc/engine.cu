@@ -144,6 +144,10 @@ namespace {
 // tangent step at 262k 1.54 ms against 1.55 with the fused per-lane scan, 590k 2.96 / 3.04, 1M 4.78 / 5.20;
 // gradient step at 64k 1.14 / 1.07, 262k 3.06 / 3.05, 590k 6.30 / 6.38.
 constexpr uint32_t kStagedDifferentiable = 1u << 19;
+// Up to this many particles one lane each leaves most of the GPU idle (a wave of the one-lane passes is
+// about 100k particles) and four are faster: a forward step at 5k particles 0.164 ms against 0.240, at 14k
+// 0.228 / 0.253, at 32k 0.31 / 0.285.  Two lanes never were the fastest (0.176, 0.253, 0.297).
+constexpr uint32_t kGroupedParticles = 20480;
 }  // namespace
 
 int Engine::init(const pbf_domain_configuration* scenes, const uint32_t scene_count, const pbf_configuration* configuration,
@@ -663,7 +667,7 @@ bool Engine::runs_staged_passes(const LaunchShape& shape) const {
     return runs_staged(shape, boundary_count_ > 0, iterations_) && (!differentiable() || count_ >= kStagedDifferentiable);
 }
 
-// The Jacobi iterations and the post-loop passes over staged windows (staged.cu): two
+// The Jacobi iterations and the post-loop passes over staged windows (staged.cu, staged_group.cu): two
 // kernels per iteration, then three.
 int Engine::launch_staged(cudaStream_t stream, const pbf_particle_state* state, pbf_particle_state* next_state, StepRecord& r) {
     const GatherCommon gc = gather_common(r);
@@ -672,6 +676,7 @@ int Engine::launch_staged(cudaStream_t stream, const pbf_particle_state* state, 
     gc_reverse.reverse = 1;
     const bool diff = differentiable();
     const bool keep = r.keeps_all(diff);
+    const bool grouped = !diff && count_ <= kGroupedParticles;
     const uint32_t K = iterations_;
     StagedList list = staged_list_;
     if (!diff) list.list = {r.list_entries[0], r.list_counts[0], r.list_capacity};
@@ -690,7 +695,7 @@ int Engine::launch_staged(cudaStream_t stream, const pbf_particle_state* state, 
                                   keep ? r.density[k] : (k == 0 ? r.first_density : nullptr), keep ? r.gsum[k] : nullptr,
                                   k == 0 ? r.neighbor_count : nullptr};
         timer_.begin(stream, kPassScanDensityLambda);
-        if (int rc = check(launch_staged_density(stream, d), "staged scan + density/lambda")) return rc;
+        if (int rc = check(grouped ? launch_group_density(stream, d) : launch_staged_density(stream, d), "staged scan + density/lambda")) return rc;
         timer_.end(stream, kPassScanDensityLambda);
         const StagedCorrectionArgs c{gc_reverse, list, current, packed_mass_, lambda, xk, next,
                                      const_cast<float4*>(r.iterate(k + 1, K, diff)), diff ? r.mask[k] : nullptr,
@@ -699,7 +704,7 @@ int Engine::launch_staged(cudaStream_t stream, const pbf_particle_state* state, 
                                      {next_state->positions.x, next_state->positions.y, next_state->positions.z}, r.velocity,
                                      packed_velocity_};
         timer_.begin(stream, kPassCorrection);
-        if (int rc = check(launch_staged_correction(stream, c), "staged correction/project")) return rc;
+        if (int rc = check(grouped ? launch_group_correction(stream, c) : launch_staged_correction(stream, c), "staged correction/project")) return rc;
         timer_.end(stream, kPassCorrection);
         std::swap(current, next);
     }
@@ -707,16 +712,16 @@ int Engine::launch_staged(cudaStream_t stream, const pbf_particle_state* state, 
     const float4* xK = r.iterate(K, K, diff);
     const StagedVorticityArgs v{gc_reverse, list, slots(K), current, packed_velocity_, xK, r.velocity, r.vorticity, packed_magnitude_};
     timer_.begin(stream, kPassVorticity);
-    if (int rc = check(launch_staged_vorticity(stream, v), "staged scan + vorticity")) return rc;
+    if (int rc = check(grouped ? launch_group_vorticity(stream, v) : launch_staged_vorticity(stream, v), "staged scan + vorticity")) return rc;
     timer_.end(stream, kPassVorticity);
     const StagedNormalArgs n{gc, list, current, packed_magnitude_, xK, r.velocity, r.vorticity, r.normal, r.confined, next};
     timer_.begin(stream, kPassNormal);
-    if (int rc = check(launch_staged_normal(stream, n), "staged normal/confinement")) return rc;
+    if (int rc = check(grouped ? launch_group_normal(stream, n) : launch_staged_normal(stream, n), "staged normal/confinement")) return rc;
     timer_.end(stream, kPassNormal);
     const StagedXsphArgs x{gc_reverse, list, current, next, xK, r.confined, r.sorted_index,
                            {next_state->velocities.x, next_state->velocities.y, next_state->velocities.z}};
     timer_.begin(stream, kPassXsph);
-    if (int rc = check(launch_staged_xsph(stream, x), "staged xsph")) return rc;
+    if (int rc = check(grouped ? launch_group_xsph(stream, x) : launch_staged_xsph(stream, x), "staged xsph")) return rc;
     timer_.end(stream, kPassXsph);
     return PBF_SUCCESS;
 }

@@ -281,6 +281,13 @@ cudaError_t launch_staged_correction(cudaStream_t stream, const StagedCorrection
 cudaError_t launch_staged_vorticity(cudaStream_t stream, const StagedVorticityArgs& a);
 cudaError_t launch_staged_normal(cudaStream_t stream, const StagedNormalArgs& a);
 cudaError_t launch_staged_xsph(cudaStream_t stream, const StagedXsphArgs& a);
+// The same with four lanes per particle (staged_group.cu), for small scenes; no lists of slots and no
+// gradient-sum records (forward mode).
+cudaError_t launch_group_density(cudaStream_t stream, const StagedDensityArgs& a);
+cudaError_t launch_group_correction(cudaStream_t stream, const StagedCorrectionArgs& a);
+cudaError_t launch_group_vorticity(cudaStream_t stream, const StagedVorticityArgs& a);
+cudaError_t launch_group_normal(cudaStream_t stream, const StagedNormalArgs& a);
+cudaError_t launch_group_xsph(cudaStream_t stream, const StagedXsphArgs& a);
 
 // FP64 dst[f][i] += src[f][i] for up to six fields.
 cudaError_t launch_accumulate(cudaStream_t stream, size_t count, const double* const* src, double* const* dst, int fields);
