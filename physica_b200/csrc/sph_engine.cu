@@ -139,6 +139,8 @@ private:
     uint64_t host_step_ = ~0ull;
     float4* scratch_ = nullptr;      // grid build: (x, m) in original order
     PackedPositions packed_{};       // the sorted positions again as x, y, z arrays (packed list scan)
+    float* packed_mass_ = nullptr;   // staged passes (no boundary particles): the sorted masses, and the
+    StagedList staged_list_{};       // list of the step in progress
     uint32_t* arrival_ = nullptr;
     uint32_t* unordered_ = nullptr;
     uint32_t* tile_sums_ = nullptr;
@@ -242,6 +244,14 @@ int SphEngine::init(const pbf_domain_configuration* domain, const sph_configurat
     SphSceneInput* d_input = arena_.alloc<SphSceneInput>(1, e);
     scratch_ = arena_.alloc<float4>(count_, e);
     packed_ = alloc_packed(arena_, count_, e);
+    if (domain->boundary_particle_count == 0) {
+        packed_mass_ = arena_.alloc<float>(static_cast<size_t>(count_) + 4u, e);
+        staged_list_.windows = arena_.alloc<uint32_t>(window_words(count_), e);
+        if (config_.method != SPH_METHOD_WCSPH) {
+            const size_t padded = (static_cast<size_t>(count_) + 31u) / 32u * 32u;
+            staged_list_.list = {arena_.alloc<uint32_t>(padded * kListCapacity, e), arena_.alloc<uint32_t>(count_, e), kListCapacity};
+        }
+    }
     arrival_ = arena_.alloc<uint32_t>(count_, e);
     unordered_ = arena_.alloc<uint32_t>(count_, e);
     tile_sums_ = arena_.alloc<uint32_t>(scan_tile_count(cells_ + 1), e);
@@ -336,7 +346,7 @@ int SphEngine::allocate(SphRecord& r) {
     if (config_.method == SPH_METHOD_WCSPH) {
         Phase& ph = r.phase[0];
         ph.pressure.push_back(r.arena.alloc<float>(n, e));
-        ph.pressure_term = r.arena.alloc<float>(n, e);
+        ph.pressure_term = r.arena.alloc<float>(static_cast<size_t>(n) + 4u, e);   // staged sixteen bytes at a time
         r.viscosity_acceleration = r.arena.alloc<float4>(n, e);
         r.surface_acceleration = r.arena.alloc<float4>(n, e);
         if (differentiable_) r.total_acceleration = r.arena.alloc<float4>(n, e);
@@ -356,7 +366,7 @@ int SphEngine::allocate(SphRecord& r) {
             for (uint32_t k = 0; k < copies; ++k) ph.predicted_density.push_back(r.arena.alloc<float>(n, e));
             if (differentiable_)
                 for (uint32_t k = 0; k <= K; ++k) ph.acceleration.push_back(r.arena.alloc<float4>(n, e));
-            ph.pressure_term = r.arena.alloc<float>(n, e);
+            ph.pressure_term = r.arena.alloc<float>(static_cast<size_t>(n) + 4u, e);   // staged sixteen bytes at a time
         }
         if (dfsph && !differentiable_) r.divergence_acceleration = r.arena.alloc<float4>(n, e);
     }
@@ -457,6 +467,7 @@ int SphEngine::launch(cudaStream_t s, const pbf_particle_state* state, const sph
     g.key_current = 1;
     g.sorted_velocity = r.velocity;
     g.packed = packed_;
+    g.packed_mass = packed_mass_;
     if (int rc = check(launch_grid_build(s, g), "grid build")) return rc;
     if (boundary_count_ > 0) {
         BoundaryBuildArgs b{boundary_count_, cells_, d_scenes_, nullptr, boundary_rest_, boundary_velocity_, boundary_keys_,
@@ -470,9 +481,12 @@ int SphEngine::launch(cudaStream_t s, const pbf_particle_state* state, const sph
         gc.boundary = r.boundary;
     }
     const StoredList list{r.list_entries, r.list_counts, r.list_capacity};
-    ListScanArgs scan{gc, r.topology, list, 1};
-    scan.packed = packed_;
-    if (int rc = check(launch_list_scan(s, scan, shape), "neighbour list scan")) return rc;
+    const bool staged = runs_staged(shape, boundary_count_ > 0, 1u);
+    if (!staged) {
+        ListScanArgs scan{gc, r.topology, list, 1};
+        scan.packed = packed_;
+        if (int rc = check(launch_list_scan(s, scan, shape), "neighbour list scan")) return rc;
+    }
     SphStep st{gc,
                d_constants_,
                r.topology,
@@ -491,8 +505,10 @@ int SphEngine::launch(cudaStream_t s, const pbf_particle_state* state, const sph
     const bool warm = method == SPH_METHOD_DFSPH && config_.pressure_warm_start != 0;
     const bool diff = differentiable_;
     Phase& p0 = r.phase[0];
-    if (int rc = check(launch_density(s, st, method, r.density, p0.P(0), p0.pressure_term,
-                                      warm ? method_state->warm_divergence_pressure : nullptr, block),
+    const float* first_warm = warm ? method_state->warm_divergence_pressure : nullptr;
+    if (int rc = check(staged ? launch_staged_sph_density(s, st, SphStaged{staged_list_, packed_, packed_mass_}, method, r.density,
+                                                          p0.P(0), p0.pressure_term, first_warm)
+                              : launch_density(s, st, method, r.density, p0.P(0), p0.pressure_term, first_warm, block),
                        "density"))
         return rc;
     if (method == SPH_METHOD_WCSPH) {
@@ -514,7 +530,9 @@ int SphEngine::launch(cudaStream_t s, const pbf_particle_state* state, const sph
         }
         SphStep sk = st;
         sk.predicted = ph.X(k);
-        return check(launch_predicted_density(s, sk, update, ph.P(k), ph.pressure_term, ph.R(k), block), "predicted density");
+        return check(staged ? launch_staged_predicted_density(s, sk, staged_list_, update, ph.P(k), ph.pressure_term, ph.R(k))
+                            : launch_predicted_density(s, sk, update, ph.P(k), ph.pressure_term, ph.R(k), block),
+                     "predicted density");
     };
     auto pressure_pass = [&](Phase& ph, const uint32_t k, PressurePassArgs a) -> int {
         SphStep sk = st;
@@ -525,7 +543,8 @@ int SphEngine::launch(cudaStream_t s, const pbf_particle_state* state, const sph
         a.out_velocities = out_v;
         a.displacement_slot = ph.first_slot + k;
         if (diff) a.store_acceleration = ph.A(k);
-        return check(launch_pressure(s, sk, a, block), "pressure acceleration");
+        return check(staged ? launch_staged_pressure(s, sk, staged_list_, a) : launch_pressure(s, sk, a, block),
+                     "pressure acceleration");
     };
     if (method == SPH_METHOD_PCISPH || method == SPH_METHOD_IISPH) {
         const uint32_t K = p0.iterations;

@@ -36,6 +36,11 @@ struct SphConstants {
     double inverse_hh_d;            // 1 / (h h), h h rounded to float as in density/device.cuh:59-70
     double cubic_coefficient_d;     // 8 / (pi h h h) in FP64                (density/device.cuh:59-70)
     double laplacian_scale_d;       // -45 / (pi pow(h, 6)) in FP64          (density/device.cuh:84-88)
+    // Last: the force pass reads the fields above in wide loads, which other offsets break up (0.25 against
+    // 0.34 ms at 1M particles).
+    float inverse_h;                // 1 / h, correctly rounded
+    float fast_min, fast_max;       // range of non-zero r2 of the packed pair arithmetic (sph_math.cuh), up to
+                                    // 2 h h (largest < smallest where h is outside its range)
 };
 
 // Sorted per-particle parameters of an SPH step, packed by the grid build:
@@ -66,6 +71,17 @@ struct SphStep {
 // pressures in original order, or null (pressure 0).
 cudaError_t launch_density(cudaStream_t stream, const SphStep& st, uint32_t method, float* density_record, float* pressure,
                            float* pressure_term, const float* warm, unsigned block);
+
+// The same passes over windows staged in shared memory (sph_staged.cu; scenes without boundary
+// particles).  The density pass also scans: it writes st.list (sorted slots) and, for the iterative
+// methods, the staged list that the predicted-density and pressure passes replay.
+struct SphStaged {
+    StagedList list;             // WCSPH: only its windows are used
+    PackedPositions positions;   // the sorted positions
+    const float* mass;
+};
+cudaError_t launch_staged_sph_density(cudaStream_t stream, const SphStep& st, const SphStaged& staged, uint32_t method,
+                                      float* density_record, float* pressure, float* pressure_term, const float* warm);
 
 // WCSPH forces (pressure, artificial viscosity, surface), external acceleration and integration
 // (sph/sph.cpp:214-225) in one pass; writes the next state in original order.
@@ -114,6 +130,9 @@ struct PressurePassArgs {
     uint32_t displacement_slot;   // where the prediction's max displacement goes (when not last)
 };
 cudaError_t launch_pressure(cudaStream_t stream, const SphStep& st, const PressurePassArgs& a, unsigned block);
+cudaError_t launch_staged_predicted_density(cudaStream_t stream, const SphStep& st, const StagedList& list, PressureUpdate update,
+                                            float* pressure, float* pressure_term, float* predicted_density_record);
+cudaError_t launch_staged_pressure(cudaStream_t stream, const SphStep& st, const StagedList& list, const PressurePassArgs& a);
 
 // Constants of every scene (host inputs: support radius, particle radius, box velocity, no-slip
 // flag and the reference gradient norm per scene).

@@ -2,7 +2,7 @@
 // Built and called by tests/test_gpu_pair_math.py; every entry returns the number of mismatches.
 #include <cstdint>
 
-#include "pbf_math.cuh"
+#include "sph_math.cuh"
 
 namespace {
 
@@ -81,6 +81,12 @@ __global__ void constant_quotient_kernel(const int limit, unsigned long long* ba
     const float R = __frcp_rn(b);
     auto check = [&](const float a) { count(bad, differs(quotient_pair(both(a), both(-b), both(R)).x, __fdiv_rn(a, b))); };
     nearest_boundaries(i | 0x800000u, limit, check);
+    // a reciprocal that rounds up where 1 / b lies within 2^-18 ulp below the next rounding boundary
+    const double above = 1.0 / static_cast<double>(b) * (1.0 + 0x1p-41);
+    const float U = static_cast<float>(above);
+    if (U != R) nearest_boundaries(i | 0x800000u, limit, [&](const float a) {
+        count(bad, differs(quotient_pair(both(a), both(-b), both(U)).x, __fdiv_rn(a, b)));
+    });
     for (uint32_t t = 0; t < 32u; ++t) check(__uint_as_float(0x3f800000u | (mix(i * 32u + t) >> 9)));
 }
 
@@ -118,6 +124,32 @@ __global__ void kernels_kernel(const float h, const uint32_t n, unsigned long lo
     // the distance's rounding (2^-52 h) moves the gap h - r, the other factors a few 2^-53
     const double bound = 0x1p-48 + 0x1p-50 * k.h / gap;
     count(bad, !(fabs(w.along - along) <= bound * fabs(along)) || !(fabs(w.across - across) <= bound * fabs(across)));
+}
+
+// the cubic spline's values likewise, to beyond the support
+__global__ void cubic_kernel(const float h, const uint32_t n, unsigned long long* bad, unsigned long long* tested) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    sph::SphConstants k{};
+    k.h = h;
+    k.cubic_coefficient = __fdiv_rn(8.0F, __fmul_rn(__fmul_rn(__fmul_rn(kPi, h), h), h));
+    k.cubic_coefficient_2 = __fmul_rn(k.cubic_coefficient, 2.0F);
+    k.support_threshold = kernel_constants(h).spiky_threshold;
+    k.inverse_h = __frcp_rn(h);
+    k.fast_min = __fmul_rn(__fmul_rn(h, h), 0x1p-60F);
+    k.fast_max = __fmul_rn(__fmul_rn(h, h), 2.0F);
+    float r2 = h * h * 1.3F * (static_cast<float>(mix(i) >> 8) * 0x1p-24F);
+    if (i % 4u == 1u) r2 = __uint_as_float(__float_as_uint(k.support_threshold) + 64u - (mix(i) & 0xffffu));
+    if (i % 4u == 2u) r2 = ldexpf(r2, -static_cast<int>(mix(~i) % 60u));
+    const float2 nr2 = make_float2(-r2, -r2);
+    if (!sph::detail::in_range(nr2, k)) return;
+    atomicAdd(tested, 1ull);
+    const float distance = __fsqrt_rn(r2);
+    const float weight = distance < h ? sph::detail::cubic_inside(distance, k) : 0.0F;
+    const float slope = distance < h ? sph::detail::cubic_gradient_scale(distance, k) : 0.0F;
+    count(bad, differs(sph::detail::cubic_pair(nr2, k).y, weight) || differs(sph::detail::any_cubic(r2, &k), weight));
+    const float packed = sph::detail::cubic_gradient_pair(nr2, k).y;   // a zero's sign may differ
+    count(bad, packed != slope || differs(sph::detail::any_cubic_gradient(r2, &k), slope));
 }
 
 unsigned long long* counter() {
@@ -158,6 +190,15 @@ extern "C" long long check_constant_quotients(const int limit) {
 extern "C" long long check_kernels(const float h, const uint32_t n, long long* tested) {
     unsigned long long* bad = counter();
     kernels_kernel<<<(n + 255u) / 256u, 256>>>(h, n, bad, bad + 1);
+    cudaDeviceSynchronize();
+    *tested = static_cast<long long>(bad[1]);
+    return finish(bad);
+}
+
+// The same for the cubic spline.
+extern "C" long long check_cubic(const float h, const uint32_t n, long long* tested) {
+    unsigned long long* bad = counter();
+    cubic_kernel<<<(n + 255u) / 256u, 256>>>(h, n, bad, bad + 1);
     cudaDeviceSynchronize();
     *tested = static_cast<long long>(bad[1]);
     return finish(bad);

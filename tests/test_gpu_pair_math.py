@@ -18,10 +18,11 @@ def check(tmp_path_factory):
     subprocess.run([build.nvcc(), *build.ARCH, *build.FLAGS, "-w", "-shared", "-cudart=static", "-Xcompiler",
                     "-fvisibility=default", "-o", str(out), str(ROOT / "tests" / "cpp" / "pair_math_check.cu")], check=True)
     lib = ctypes.CDLL(str(out))
-    for name in ("check_roots", "check_root_quotients", "check_constant_quotients", "check_kernels"):
+    for name in ("check_roots", "check_root_quotients", "check_constant_quotients", "check_kernels", "check_cubic"):
         getattr(lib, name).restype = ctypes.c_longlong
     lib.check_roots.argtypes = [ctypes.c_uint32, ctypes.c_uint32]
-    lib.check_kernels.argtypes = [ctypes.c_float, ctypes.c_uint32, ctypes.POINTER(ctypes.c_longlong)]
+    for name in ("check_kernels", "check_cubic"):
+        getattr(lib, name).argtypes = [ctypes.c_float, ctypes.c_uint32, ctypes.POINTER(ctypes.c_longlong)]
     return lib
 
 
@@ -43,8 +44,9 @@ def test_quotients_nearest_a_rounding_boundary(check):
 @pytest.mark.parametrize("h", [2.0 ** -10, 0.00123, 0.0125, 0.025, 0.05, 0.1, 1.0 / 3.0, 1.0, 7.7, 333.0, 1024.0])
 def test_kernel_values(check, h):
     tested = ctypes.c_longlong()
-    assert check.check_kernels(h, 1 << 22, ctypes.byref(tested)) == 0
-    assert tested.value > 1 << 21
+    for entry in (check.check_kernels, check.check_cubic):
+        assert entry(h, 1 << 22, ctypes.byref(tested)) == 0
+        assert tested.value > 1 << 21
 
 
 @pytest.mark.parametrize("h", [2.0 ** -11, 2048.0])
