@@ -16,6 +16,7 @@
 // Buffers that the reference clears before accumulating into them are written as
 // 0.0 + contribution, which reproduces its values including the sign of zero.
 #include "engine.h"
+#include "dependent_launch.cuh"
 #include "gather.cuh"
 
 namespace pbf {
@@ -135,6 +136,7 @@ __device__ __forceinline__ void finish(const Tail& t, const uint32_t s, const ui
 __global__ void seed_kernel(const GatherCommon g, const uint32_t* __restrict__ sorted_index, const ConstAdjField3 next_x,
                             const ConstAdjField3 next_v, double4* __restrict__ x, double4* __restrict__ out_v,
                             float2* __restrict__ s_corr, float4* __restrict__ reverse) {
+    after_predecessor();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= g.count) return;
     const uint32_t i = sorted_index[s];
@@ -218,6 +220,7 @@ struct XsphVjpOp {
 #define PBF_DENSITY_VJP_MIN_BLOCKS 0
 #endif
 __global__ void __launch_bounds__(kBlock, PBF_POST_VJP_MIN_BLOCKS) xsph_vjp_kernel(const XsphVjpArgs a) {
+    after_predecessor();
     uint32_t half;
     const Particle p = locate_pair(a.g, half);
     XsphVjpOp op;
@@ -295,6 +298,7 @@ struct NormalVjpOp {
 };
 
 __global__ void __launch_bounds__(kBlock, PBF_POST_VJP_MIN_BLOCKS) normal_vjp_kernel(const NormalVjpArgs a) {
+    after_predecessor();
     uint32_t half;
     const Particle p = locate_pair(a.g, half);
     NormalVjpOp op;
@@ -356,6 +360,7 @@ struct VorticityVjpOp {
 };
 
 __global__ void __launch_bounds__(kBlock, PBF_POST_VJP_MIN_BLOCKS) vorticity_vjp_kernel(const VorticityVjpArgs a) {
+    after_predecessor();
     uint32_t half;
     const Particle p = locate_pair(a.g, half);
     VorticityVjpOp op;
@@ -519,6 +524,7 @@ struct CorrectionVjpOp {
 #define PBF_CORRECTION_VJP_MIN_BLOCKS 4
 #endif
 __global__ void __launch_bounds__(kBlock, PBF_CORRECTION_VJP_MIN_BLOCKS) correction_vjp_kernel(const CorrectionVjpArgs a) {
+    after_predecessor();
     uint32_t half;
     const Particle p = locate_pair(a.g, half);
     CorrectionVjpOp op;
@@ -649,6 +655,7 @@ struct LambdaVjpOp {
 #define PBF_LAMBDA_VJP_MIN_BLOCKS 4
 #endif
 __global__ void __launch_bounds__(kBlock, PBF_LAMBDA_VJP_MIN_BLOCKS) lambda_vjp_kernel(const LambdaVjpArgs a) {
+    after_predecessor();
     const Particle p = locate(a.g);
     LambdaVjpOp op;
     op.pos = a.pos;
@@ -737,6 +744,7 @@ struct DensityVjpOp {
 };
 
 __global__ void __launch_bounds__(kBlock, PBF_DENSITY_VJP_MIN_BLOCKS) density_vjp_kernel(const DensityVjpArgs a) {
+    after_predecessor();
     uint32_t half;
     const Particle p = locate_pair(a.g, half);
     DensityVjpOp op;
@@ -768,6 +776,7 @@ inline unsigned grid_of(const uint32_t n, const unsigned block) { return (n + bl
 
 __global__ void accumulate6_kernel(const size_t count, const ConstAdjField3 s0, const ConstAdjField3 s1, const AdjField3 d0,
                                    const AdjField3 d1, const int fields) {
+    after_predecessor();
     const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= count) return;
     const double* src[6] = {s0.x, s0.y, s0.z, s1.x, s1.y, s1.z};
@@ -797,6 +806,7 @@ __device__ __forceinline__ Compensated combine(Compensated a, const Compensated 
 
 __global__ void segment_sum_kernel(const double* __restrict__ values, const uint32_t* __restrict__ first,
                                    const uint32_t* __restrict__ count, const uint32_t single_count, double* __restrict__ out) {
+    after_predecessor();
     __shared__ double sums[256];
     __shared__ double carries[256];
     const uint32_t seg = blockIdx.x;
@@ -824,7 +834,7 @@ __global__ void segment_sum_kernel(const double* __restrict__ values, const uint
 cudaError_t launch_segment_sums(cudaStream_t stream, const double* values, const uint32_t* first, const uint32_t* count,
                                 const uint32_t segments, const uint32_t single_count, double* out) {
     if (segments == 0) return cudaSuccess;
-    segment_sum_kernel<<<segments, 256, 0, stream>>>(values, first, count, single_count, out);
+    launch_after(stream, segment_sum_kernel, segments, 256, values, first, count, single_count, out);
     count_launch();
     return cudaGetLastError();
 }
@@ -837,8 +847,8 @@ cudaError_t launch_accumulate(cudaStream_t stream, const size_t count, const dou
     const ConstAdjField3 s1{fields > 3 ? src[3] : nullptr, fields > 4 ? src[4] : nullptr, fields > 5 ? src[5] : nullptr};
     const AdjField3 d0{dst[0], fields > 1 ? dst[1] : nullptr, fields > 2 ? dst[2] : nullptr};
     const AdjField3 d1{fields > 3 ? dst[3] : nullptr, fields > 4 ? dst[4] : nullptr, fields > 5 ? dst[5] : nullptr};
-    accumulate6_kernel<<<static_cast<unsigned>((count + 255) / 256), 256, 0, stream>>>(count, s0, s1, d0, d1,
-                                                                                     fields < 6 ? fields : 6);
+    launch_after(stream, accumulate6_kernel, static_cast<unsigned>((count + 255) / 256), 256, count, s0, s1, d0, d1,
+                 fields < 6 ? fields : 6);
     count_launch();
     return cudaGetLastError();
 }
@@ -918,24 +928,24 @@ int Engine::reverse(const pbf_particle_state* state, const pbf_control* control,
     const StoredList post_list{r.list_entries[keep ? K : 0u], r.list_counts[keep ? K : 0u], r.list_capacity};
 
     timer_.begin(stream_, kPassSeed);
-    seed_kernel<<<grid_of(n, 256), 256, 0, stream_>>>(
-        gc, r.sorted_index, {next_adjoint->positions.x, next_adjoint->positions.y, next_adjoint->positions.z},
-        {next_adjoint->velocities.x, next_adjoint->velocities.y, next_adjoint->velocities.z}, ws->x[0], ws->output_velocity,
-        ws->s_corr, ws->reverse);
+    launch_after(stream_, seed_kernel, grid_of(n, 256), 256, gc, r.sorted_index,
+                 {next_adjoint->positions.x, next_adjoint->positions.y, next_adjoint->positions.z},
+                 {next_adjoint->velocities.x, next_adjoint->velocities.y, next_adjoint->velocities.z}, ws->x[0],
+                 ws->output_velocity, ws->s_corr, ws->reverse);
     timer_.end(stream_, kPassSeed);
     XsphVjpArgs xa{gc, post_list, r.sorted_index, xK, r.confined, r.vorticity, r.normal, ws->output_velocity, ws->x[0], ws->velocity,
                    ws->vorticity, ws->eta, pa};
     timer_.begin(stream_, kPassXsphVjp);
-    xsph_vjp_kernel<<<pair_blocks, kBlock, 0, stream_>>>(xa);
+    launch_after(stream_, xsph_vjp_kernel, pair_blocks, kBlock, xa);
     timer_.end(stream_, kPassXsphVjp);
     NormalVjpArgs na{gc_reverse, post_list, xK, r.vorticity, ws->eta, ws->x[0], ws->vorticity};
     timer_.begin(stream_, kPassNormalVjp);
-    normal_vjp_kernel<<<pair_blocks, kBlock, 0, stream_>>>(na);
+    launch_after(stream_, normal_vjp_kernel, pair_blocks, kBlock, na);
     timer_.end(stream_, kPassNormalVjp);
     Tail tail{K ? r.mask[K - 1] : nullptr, ws->x[1], ws->correction, prev_x, prev_v, ctrl};
     VorticityVjpArgs va{gc, post_list, r.sorted_index, xK, r.velocity, ws->vorticity, ws->x[0], ws->velocity, tail};
     timer_.begin(stream_, kPassVorticityVjp);
-    vorticity_vjp_kernel<<<pair_blocks, kBlock, 0, stream_>>>(va);
+    launch_after(stream_, vorticity_vjp_kernel, pair_blocks, kBlock, va);
     timer_.end(stream_, kPassVorticityVjp);
     count_launch(4);
     // Checkpoint recomputation (pbf/pbf.cpp:232-245): before the iterations of a segment between two
@@ -970,17 +980,17 @@ int Engine::reverse(const pbf_particle_state* state, const pbf_control* control,
         CorrectionVjpArgs ca{gc, it_list, r.sorted_index, xk, ws->s_corr, ws->reverse, lambda_k, ws->correction, acc,
                              ws->lambda, pa, density_k, gsum_k, ws->constraint_weight, ws->gradient_sum_rest};
         timer_.begin(stream_, kPassCorrectionVjp);
-        correction_vjp_kernel<<<pair_blocks, kBlock, 0, stream_>>>(ca);
+        launch_after(stream_, correction_vjp_kernel, pair_blocks, kBlock, ca);
         timer_.end(stream_, kPassCorrectionVjp);
         LambdaVjpArgs la{gc_reverse, it_list, r.sorted_index, xk, density_k, gsum_k, ws->lambda, ws->constraint_weight,
                          ws->gradient_sum_rest, acc, ws->density, pa};
         timer_.begin(stream_, kPassLambdaVjp);
-        lambda_vjp_kernel<<<blocks, kBlock, 0, stream_>>>(la);
+        launch_after(stream_, lambda_vjp_kernel, blocks, kBlock, la);
         timer_.end(stream_, kPassLambdaVjp);
         Tail t{k ? r.mask[k - 1] : nullptr, other, ws->correction, prev_x, prev_v, ctrl};
         DensityVjpArgs da{gc, it_list, r.sorted_index, xk, ws->density, acc, pa, t};
         timer_.begin(stream_, kPassDensityVjp);
-        density_vjp_kernel<<<pair_blocks, kBlock, 0, stream_>>>(da);
+        launch_after(stream_, density_vjp_kernel, pair_blocks, kBlock, da);
         timer_.end(stream_, kPassDensityVjp);
         count_launch(3);
     }

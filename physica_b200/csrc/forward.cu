@@ -16,6 +16,7 @@
 // math (sqrt, divisions) keeps that math convergent across the warp.
 #include <climits>
 
+#include "dependent_launch.cuh"
 #include "forward_ops.cuh"
 
 namespace pbf {
@@ -77,6 +78,7 @@ struct RangeScan {
 };
 
 __global__ void __launch_bounds__(kBlock, 12) list_walk_kernel(const ListScanArgs a) {
+    after_predecessor();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= a.g.count) return;
     const int4 c = a.g.cell[s];
@@ -152,6 +154,7 @@ __global__ void __launch_bounds__(kBlock, 12) list_walk_kernel(const ListScanArg
 constexpr uint32_t kStageCapacity = 704;   // float4 per warp (44 KB per 128-thread block)
 
 __global__ void __launch_bounds__(kBlock) list_staged_kernel(const ListScanArgs a) {
+    after_predecessor();
     __shared__ float4 stage[kWarpsPerBlock][kStageCapacity];
     __shared__ uint32_t column_first[kWarpsPerBlock][9];
     __shared__ uint32_t column_base[kWarpsPerBlock][9];
@@ -243,6 +246,7 @@ __global__ void __launch_bounds__(kBlock) list_staged_kernel(const ListScanArgs 
 }
 
 __global__ void __launch_bounds__(kBlock) list_scan_kernel(const ListScanArgs a) {
+    after_predecessor();
     __shared__ float4 home_s[kWarpsPerBlock][32];
     __shared__ uint32_t first_s[kWarpsPerBlock][32];
     __shared__ uint32_t base_s[kWarpsPerBlock][32];
@@ -324,6 +328,7 @@ __global__ void __launch_bounds__(kBlock) list_scan_kernel(const ListScanArgs a)
 // ------------------------------------------------------------------ density + lambda
 template <bool WithBoundary>
 __global__ void __launch_bounds__(kBlock) density_lambda_kernel(const DensityLambdaArgs a) {
+    after_predecessor();
     const Particle p = locate(a.g);
     if (!p.active) return;
     DensityLambdaOp<WithBoundary> op;
@@ -370,6 +375,7 @@ constexpr uint32_t kStagedEntries = PBF_FUSED_STAGED_ENTRIES;   // 40: 20 KB of 
 
 __global__ void __launch_bounds__(kBlock, PBF_FUSED_MIN_BLOCKS) scan_density_lambda_kernel(const ListScanArgs a,
                                                                                           const DensityLambdaArgs d) {
+    after_predecessor();
     __shared__ uint32_t staged[kStagedEntries * kBlock];
     const Particle p = locate(a.g);
     if (!p.active) return;
@@ -469,6 +475,7 @@ __global__ void __launch_bounds__(kBlock, PBF_FUSED_MIN_BLOCKS) scan_density_lam
 
 template <bool WithBoundary>
 __global__ void __launch_bounds__(kBlock, PBF_CORRECTION_MIN_BLOCKS) correction_kernel(const CorrectionArgs a) {
+    after_predecessor();
     const Particle p = locate(a.g);
     if (!p.active) return;
     CorrectionOp<WithBoundary> op;
@@ -518,6 +525,7 @@ __global__ void __launch_bounds__(kBlock, PBF_CORRECTION_MIN_BLOCKS) correction_
 
 // ---------------------------------------------------------------- vorticity
 __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) vorticity_kernel(const VorticityArgs a) {
+    after_predecessor();
     const Particle p = locate(a.g);
     if (!p.active) return;
     VorticityOp op;
@@ -534,6 +542,7 @@ __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) vorticity_kernel(
 
 // ------------------------------------------------------- normal + confinement
 __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) normal_kernel(const NormalArgs a) {
+    after_predecessor();
     const Particle p = locate(a.g);
     if (!p.active) return;
     NormalOp op;
@@ -557,6 +566,7 @@ __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) normal_kernel(con
 
 // ---------------------------------------------------------------------- XSPH
 __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) xsph_kernel(const XsphArgs a) {
+    after_predecessor();
     const Particle p = locate(a.g);
     if (!p.active) return;
     XsphOp op;
@@ -578,6 +588,7 @@ __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) xsph_kernel(const
 
 // ------------------------------------------------------------------ constants
 __global__ void constants_kernel(const float* __restrict__ radii, const uint32_t n, KernelConstants* __restrict__ out) {
+    after_predecessor();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     out[i] = kernel_constants(radii[i]);
@@ -586,6 +597,7 @@ __global__ void constants_kernel(const float* __restrict__ radii, const uint32_t
 __global__ void unsort_float4_kernel(const uint32_t count, const uint32_t* __restrict__ sorted_index,
                                      const float4* __restrict__ in, const int components, float* out_x, float* out_y,
                                      float* out_z, float* out_w) {
+    after_predecessor();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= count) return;
     const uint32_t i = sorted_index[s];
@@ -598,6 +610,7 @@ __global__ void unsort_float4_kernel(const uint32_t count, const uint32_t* __res
 
 __global__ void unsort_mask_kernel(const uint32_t count, const uint32_t* __restrict__ sorted_index,
                                    const uint8_t* __restrict__ in, uint32_t* __restrict__ out) {
+    after_predecessor();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= count) return;
     out[sorted_index[s]] = in[s];
@@ -605,6 +618,7 @@ __global__ void unsort_mask_kernel(const uint32_t count, const uint32_t* __restr
 
 __global__ void unsort_scalar_kernel(const uint32_t count, const uint32_t* __restrict__ sorted_index, const uint8_t* in,
                                      const uint32_t bytes, uint8_t* out) {
+    after_predecessor();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= count) return;
     const uint32_t i = sorted_index[s];
@@ -614,6 +628,7 @@ __global__ void unsort_scalar_kernel(const uint32_t count, const uint32_t* __res
 __global__ void reconstruct_kernel(const uint32_t count, const SceneDesc* __restrict__ scenes, const int4* __restrict__ cell,
                                    const float4* __restrict__ positions, const Field3 previous,
                                    const uint32_t* __restrict__ sorted_index, const MutField3 out, float4* __restrict__ velocity) {
+    after_predecessor();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= count) return;
     const SceneDesc& sc = scenes[cell[s].w];
@@ -634,6 +649,7 @@ __global__ void export_frame_kernel(const uint32_t count, const Field3 positions
                                     const uint32_t* __restrict__ slot_of, const float4* __restrict__ vorticity,
                                     float* __restrict__ out_positions, float* __restrict__ out_velocities,
                                     float* __restrict__ out_vorticity) {
+    after_predecessor();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     out_positions[3u * i] = positions.x[i];
@@ -651,14 +667,14 @@ cudaError_t launch_export_frame(cudaStream_t stream, const uint32_t count, const
                                 const uint32_t* slot_of, const float4* vorticity, float* out_positions, float* out_velocities,
                                 float* out_vorticity) {
     if (count == 0) return cudaSuccess;
-    export_frame_kernel<<<grid_of(count, 256), 256, 0, stream>>>(count, positions, velocities, slot_of, vorticity, out_positions,
-                                                                  out_velocities, out_vorticity);
+    launch_after(stream, export_frame_kernel, grid_of(count, 256), 256, count, positions, velocities, slot_of, vorticity,
+                 out_positions, out_velocities, out_vorticity);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_constants(cudaStream_t stream, const float* radii, const uint32_t n, KernelConstants* out) {
-    constants_kernel<<<grid_of(n, 64), 64, 0, stream>>>(radii, n, out);
+    launch_after(stream, constants_kernel, grid_of(n, 64), 64, radii, n, out);
     count_launch();
     return cudaGetLastError();
 }
@@ -692,11 +708,11 @@ cudaError_t launch_list_scan(cudaStream_t stream, const ListScanArgs& a, const L
     // use the per-lane walk
     const bool fluid_only = !(a.boundary && a.g.boundary_offsets);
     if (shape.scan == kScanCooperative && fluid_only)
-        list_scan_kernel<<<grid_of(a.g.count, block), block, 0, stream>>>(a);
+        launch_after(stream, list_scan_kernel, grid_of(a.g.count, block), block, a);
     else if (shape.scan == kScanStaged && fluid_only)
-        list_staged_kernel<<<grid_of(a.g.count, block), block, 0, stream>>>(a);
+        launch_after(stream, list_staged_kernel, grid_of(a.g.count, block), block, a);
     else
-        list_walk_kernel<<<grid_of(a.g.count, block), block, 0, stream>>>(a);
+        launch_after(stream, list_walk_kernel, grid_of(a.g.count, block), block, a);
     count_launch();
     return cudaGetLastError();
 }
@@ -705,7 +721,7 @@ cudaError_t launch_scan_density_lambda(cudaStream_t stream, const ListScanArgs& 
                                        const LaunchShape& shape) {
     if (a.g.count == 0) return cudaSuccess;
     const unsigned block = block_of(shape.scan_block);
-    scan_density_lambda_kernel<<<grid_of(a.g.count, block), block, 0, stream>>>(a, d);
+    launch_after(stream, scan_density_lambda_kernel, grid_of(a.g.count, block), block, a, d);
     count_launch();
     return cudaGetLastError();
 }
@@ -714,9 +730,9 @@ cudaError_t launch_density_lambda(cudaStream_t stream, const DensityLambdaArgs& 
     if (a.g.count == 0) return cudaSuccess;
     const unsigned block = block_of(block_size);
     if (a.g.boundary)
-        density_lambda_kernel<true><<<grid_of(a.g.count, block), block, 0, stream>>>(a);
+        launch_after(stream, density_lambda_kernel<true>, grid_of(a.g.count, block), block, a);
     else
-        density_lambda_kernel<false><<<grid_of(a.g.count, block), block, 0, stream>>>(a);
+        launch_after(stream, density_lambda_kernel<false>, grid_of(a.g.count, block), block, a);
     count_launch();
     return cudaGetLastError();
 }
@@ -725,9 +741,9 @@ cudaError_t launch_correction(cudaStream_t stream, const CorrectionArgs& a, cons
     if (a.g.count == 0) return cudaSuccess;
     const unsigned block = block_of(block_size);
     if (a.g.boundary) {
-        correction_kernel<true><<<grid_of(a.g.count, block), block, 0, stream>>>(a);
+        launch_after(stream, correction_kernel<true>, grid_of(a.g.count, block), block, a);
     } else {
-        correction_kernel<false><<<grid_of(a.g.count, block), block, 0, stream>>>(a);
+        launch_after(stream, correction_kernel<false>, grid_of(a.g.count, block), block, a);
     }
     count_launch();
     return cudaGetLastError();
@@ -736,7 +752,7 @@ cudaError_t launch_correction(cudaStream_t stream, const CorrectionArgs& a, cons
 cudaError_t launch_vorticity(cudaStream_t stream, const VorticityArgs& a, const unsigned block_size) {
     if (a.g.count == 0) return cudaSuccess;
     const unsigned block = block_of(block_size);
-    vorticity_kernel<<<grid_of(a.g.count, block), block, 0, stream>>>(a);
+    launch_after(stream, vorticity_kernel, grid_of(a.g.count, block), block, a);
     count_launch();
     return cudaGetLastError();
 }
@@ -744,7 +760,7 @@ cudaError_t launch_vorticity(cudaStream_t stream, const VorticityArgs& a, const 
 cudaError_t launch_normal(cudaStream_t stream, const NormalArgs& a, const unsigned block_size) {
     if (a.g.count == 0) return cudaSuccess;
     const unsigned block = block_of(block_size);
-    normal_kernel<<<grid_of(a.g.count, block), block, 0, stream>>>(a);
+    launch_after(stream, normal_kernel, grid_of(a.g.count, block), block, a);
     count_launch();
     return cudaGetLastError();
 }
@@ -752,7 +768,7 @@ cudaError_t launch_normal(cudaStream_t stream, const NormalArgs& a, const unsign
 cudaError_t launch_xsph(cudaStream_t stream, const XsphArgs& a, const unsigned block_size) {
     if (a.g.count == 0) return cudaSuccess;
     const unsigned block = block_of(block_size);
-    xsph_kernel<<<grid_of(a.g.count, block), block, 0, stream>>>(a);
+    launch_after(stream, xsph_kernel, grid_of(a.g.count, block), block, a);
     count_launch();
     return cudaGetLastError();
 }
@@ -761,8 +777,8 @@ cudaError_t launch_reconstruct(cudaStream_t stream, const uint32_t count, const 
                                const float4* positions, const Field3 previous_positions, const uint32_t* sorted_index,
                                const MutField3 out_positions, float4* velocity) {
     if (count == 0) return cudaSuccess;
-    reconstruct_kernel<<<grid_of(count, 256), 256, 0, stream>>>(count, scenes, cell, positions, previous_positions, sorted_index,
-                                                               out_positions, velocity);
+    launch_after(stream, reconstruct_kernel, grid_of(count, 256), 256, count, scenes, cell, positions, previous_positions,
+                 sorted_index, out_positions, velocity);
     count_launch();
     return cudaGetLastError();
 }
@@ -770,7 +786,8 @@ cudaError_t launch_reconstruct(cudaStream_t stream, const uint32_t count, const 
 cudaError_t launch_unsort_float4(cudaStream_t stream, const uint32_t count, const uint32_t* sorted_index, const float4* in,
                                  const int components, float* out_x, float* out_y, float* out_z, float* out_w) {
     if (count == 0) return cudaSuccess;
-    unsort_float4_kernel<<<grid_of(count, 256), 256, 0, stream>>>(count, sorted_index, in, components, out_x, out_y, out_z, out_w);
+    launch_after(stream, unsort_float4_kernel, grid_of(count, 256), 256, count, sorted_index, in, components, out_x, out_y,
+                 out_z, out_w);
     count_launch();
     return cudaGetLastError();
 }
@@ -778,7 +795,7 @@ cudaError_t launch_unsort_float4(cudaStream_t stream, const uint32_t count, cons
 cudaError_t launch_unsort_mask(cudaStream_t stream, const uint32_t count, const uint32_t* sorted_index, const uint8_t* in,
                                uint32_t* out) {
     if (count == 0) return cudaSuccess;
-    unsort_mask_kernel<<<grid_of(count, 256), 256, 0, stream>>>(count, sorted_index, in, out);
+    launch_after(stream, unsort_mask_kernel, grid_of(count, 256), 256, count, sorted_index, in, out);
     count_launch();
     return cudaGetLastError();
 }
@@ -786,8 +803,8 @@ cudaError_t launch_unsort_mask(cudaStream_t stream, const uint32_t count, const 
 cudaError_t launch_unsort_scalar(cudaStream_t stream, const uint32_t count, const uint32_t* sorted_index, const void* in,
                                  const uint32_t bytes, void* out) {
     if (count == 0) return cudaSuccess;
-    unsort_scalar_kernel<<<grid_of(count, 256), 256, 0, stream>>>(count, sorted_index, static_cast<const uint8_t*>(in), bytes,
-                                                                 static_cast<uint8_t*>(out));
+    launch_after(stream, unsort_scalar_kernel, grid_of(count, 256), 256, count, sorted_index, static_cast<const uint8_t*>(in),
+                 bytes, static_cast<uint8_t*>(out));
     count_launch();
     return cudaGetLastError();
 }

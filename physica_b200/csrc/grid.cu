@@ -12,6 +12,7 @@
 // ordered), so one sort serves one scene or many.
 #include "pbf_internal.h"
 #include "../../include/physica_pbf.h"
+#include "dependent_launch.cuh"
 #include "pbf_launch.h"
 
 namespace pbf {
@@ -30,6 +31,7 @@ __global__ void predict_key_kernel(const uint32_t count, const SceneDesc* __rest
                                    uint32_t* __restrict__ keys, uint32_t* __restrict__ arrival,
                                    uint32_t* __restrict__ histogram, uint32_t* __restrict__ input_flags,
                                    const int key_current) {
+    after_predecessor();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     const SceneDesc& sc = scenes[scene_of ? scene_of[i] : 0u];
@@ -75,6 +77,7 @@ __device__ __forceinline__ uint32_t warp_inclusive(uint32_t v) {
 }
 
 __global__ void scan_reduce_kernel(const uint32_t* __restrict__ data, const uint64_t n, uint32_t* __restrict__ tile_sums) {
+    after_predecessor();
     const uint64_t base = static_cast<uint64_t>(blockIdx.x) * kScanTile;
     uint32_t s = 0;
 #pragma unroll
@@ -96,6 +99,7 @@ __global__ void scan_reduce_kernel(const uint32_t* __restrict__ data, const uint
 
 // Exclusive scan of the tile sums by one block, in chunks.
 __global__ void scan_tiles_kernel(uint32_t* __restrict__ tile_sums, const uint32_t tiles) {
+    after_predecessor();
     __shared__ uint32_t carry_s;
     __shared__ uint32_t warp_tot[kScanThreads / 32];
     if (threadIdx.x == 0) carry_s = 0;
@@ -122,6 +126,7 @@ __global__ void scan_tiles_kernel(uint32_t* __restrict__ tile_sums, const uint32
 
 // In-place exclusive scan of each tile plus its tile prefix: histogram -> cell offsets.
 __global__ void scan_apply_kernel(uint32_t* __restrict__ data, const uint64_t n, const uint32_t* __restrict__ tile_sums) {
+    after_predecessor();
     const uint64_t base = static_cast<uint64_t>(blockIdx.x) * kScanTile;
     // each thread owns kScanItems consecutive elements
     uint32_t vals[kScanItems];
@@ -184,6 +189,7 @@ __global__ void scan_apply_kernel(uint32_t* __restrict__ data, const uint64_t n,
 
 __global__ void scatter_kernel(const uint32_t count, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ arrival,
                                const uint32_t* __restrict__ cell_offsets, uint32_t* __restrict__ unordered) {
+    after_predecessor();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     unordered[cell_offsets[keys[i]] + arrival[i]] = i;
@@ -198,6 +204,7 @@ __global__ void reorder_kernel(const uint32_t count, const SceneDesc* __restrict
                                int4* __restrict__ cell, float4* __restrict__ topology, float4* __restrict__ params_a,
                                float4* __restrict__ params_b, const Field3 velocities, float4* __restrict__ sorted_velocity,
                                const PackedPositions packed, float* __restrict__ packed_mass) {
+    after_predecessor();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= count) return;
     const uint32_t i = unordered[t];
@@ -235,6 +242,7 @@ __global__ void boundary_key_kernel(const uint32_t count, const SceneDesc* __res
                                     const uint32_t* __restrict__ scene_of, const float4* __restrict__ rest,
                                     const float4* __restrict__ velocity, uint32_t* __restrict__ keys,
                                     uint32_t* __restrict__ arrival, uint32_t* __restrict__ histogram) {
+    after_predecessor();
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= count) return;
     const Grid& g = scenes[scene_of ? scene_of[b] : 0u].grid;
@@ -254,6 +262,7 @@ __global__ void boundary_reorder_kernel(const uint32_t count, const SceneDesc* _
                                         const uint32_t* __restrict__ cell_offsets, const uint32_t* __restrict__ unordered,
                                         const float4* __restrict__ rest, const float4* __restrict__ velocity,
                                         float4* __restrict__ sorted, float4* __restrict__ sorted_velocity) {
+    after_predecessor();
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= count) return;
     const uint32_t key = keys[b];
@@ -270,6 +279,7 @@ __global__ void boundary_reorder_kernel(const uint32_t count, const SceneDesc* _
 // ---- export in the reference's grid layout (cell index x fastest) ----
 // Particle count of every cell of one scene, stored at the cell's reference index.
 __global__ void reference_counts_kernel(const Grid g, const uint32_t* __restrict__ cell_offsets, uint32_t* __restrict__ out) {
+    after_predecessor();
     const uint32_t local = blockIdx.x * blockDim.x + threadIdx.x;
     if (local >= g.cells_x * g.cells_y * g.cells_z) return;
     const uint32_t z = local % g.cells_z, y = (local / g.cells_z) % g.cells_y, x = local / (g.cells_z * g.cells_y);
@@ -283,6 +293,7 @@ __global__ void reference_order_kernel(const uint32_t count, const SceneDesc* __
                                        const uint32_t* __restrict__ sorted_index, const uint32_t* __restrict__ keys,
                                        const uint32_t* __restrict__ cell_offsets, const uint32_t* __restrict__ reference_offsets,
                                        uint32_t* __restrict__ out_index, unsigned long long* __restrict__ out_keys) {
+    after_predecessor();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= count) return;
     const uint32_t i = sorted_index[s];
@@ -296,8 +307,14 @@ __global__ void reference_order_kernel(const uint32_t count, const SceneDesc* __
     if (out_keys) out_keys[slot] = reference;
 }
 
-__global__ void set_step_kernel(unsigned long long* step, const unsigned long long value) { *step = value; }
-__global__ void advance_step_kernel(unsigned long long* step) { *step += 1ull; }
+__global__ void set_step_kernel(unsigned long long* step, const unsigned long long value) {
+    after_predecessor();
+    *step = value;
+}
+__global__ void advance_step_kernel(unsigned long long* step) {
+    after_predecessor();
+    *step += 1ull;
+}
 
 // Per-step scene fields from the device step counter (the step advances state `step` to `step + 1`):
 // time = float(step + 1) * dt (pbf/pbf.cpp:18, neighborhood/neighborhood.cu:55), or float(step) * dt
@@ -306,6 +323,7 @@ __global__ void advance_step_kernel(unsigned long long* step) { *step += 1ull; }
 // float operation order of the reference's host code.
 __global__ void scene_time_kernel(const SceneStatic* __restrict__ statics, SceneDesc* __restrict__ scenes,
                                   const unsigned long long* __restrict__ step, const uint32_t count) {
+    after_predecessor();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= count) return;
     const SceneStatic st = statics[s];
@@ -331,20 +349,20 @@ inline unsigned blocks_for(const uint64_t n, const unsigned threads) { return st
 }  // namespace
 
 cudaError_t launch_set_step(cudaStream_t stream, unsigned long long* step, const uint64_t value) {
-    set_step_kernel<<<1, 1, 0, stream>>>(step, value);
+    launch_after(stream, set_step_kernel, 1, 1, step, value);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_advance_step(cudaStream_t stream, unsigned long long* step) {
-    advance_step_kernel<<<1, 1, 0, stream>>>(step);
+    launch_after(stream, advance_step_kernel, 1, 1, step);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_scene_time(cudaStream_t stream, const SceneStatic* statics, SceneDesc* scenes, const unsigned long long* step,
                               const uint32_t count) {
-    scene_time_kernel<<<blocks_for(count, 128), 128, 0, stream>>>(statics, scenes, step, count);
+    launch_after(stream, scene_time_kernel, blocks_for(count, 128), 128, statics, scenes, step, count);
     count_launch();
     return cudaGetLastError();
 }
@@ -356,24 +374,23 @@ cudaError_t launch_grid_build(cudaStream_t stream, const GridBuildArgs& a) {
     cudaError_t e = cudaMemsetAsync(a.cell_offsets, 0, (a.cells + 1) * sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
     if (a.count > 0) {
-        predict_key_kernel<<<blocks_for(a.count, tpb), tpb, 0, stream>>>(a.count, a.scenes, a.scene_of, a.positions,
-                                                                         a.velocities, a.controls, a.params.masses,
-                                                                         a.predicted, a.keys, a.arrival, a.cell_offsets,
-                                                                         a.input_flags, a.key_current);
+        launch_after(stream, predict_key_kernel, blocks_for(a.count, tpb), tpb, a.count, a.scenes, a.scene_of, a.positions,
+                     a.velocities, a.controls, a.params.masses, a.predicted, a.keys, a.arrival, a.cell_offsets, a.input_flags,
+                     a.key_current);
         count_launch();
     }
     const uint64_t n = a.cells + 1;
     const unsigned tiles = static_cast<unsigned>(scan_tile_count(n));
-    scan_reduce_kernel<<<tiles, kScanThreads, 0, stream>>>(a.cell_offsets, n, a.tile_sums);
-    scan_tiles_kernel<<<1, kScanThreads, 0, stream>>>(a.tile_sums, tiles);
-    scan_apply_kernel<<<tiles, kScanThreads, 0, stream>>>(a.cell_offsets, n, a.tile_sums);
+    launch_after(stream, scan_reduce_kernel, tiles, kScanThreads, a.cell_offsets, n, a.tile_sums);
+    launch_after(stream, scan_tiles_kernel, 1, kScanThreads, a.tile_sums, tiles);
+    launch_after(stream, scan_apply_kernel, tiles, kScanThreads, a.cell_offsets, n, a.tile_sums);
     count_launch(3);
     if (a.count > 0) {
-        scatter_kernel<<<blocks_for(a.count, tpb), tpb, 0, stream>>>(a.count, a.keys, a.arrival, a.cell_offsets, a.unordered);
-        reorder_kernel<<<blocks_for(a.count, tpb), tpb, 0, stream>>>(
-            a.count, a.scenes, a.scene_of, a.keys, a.cell_offsets, a.unordered, a.predicted, a.params, a.sorted_index,
-            a.slot_of, a.cell, a.topology, a.params_a, a.params_b, a.velocities, a.sorted_velocity, a.packed,
-            a.packed_mass);
+        launch_after(stream, scatter_kernel, blocks_for(a.count, tpb), tpb, a.count, a.keys, a.arrival, a.cell_offsets,
+                     a.unordered);
+        launch_after(stream, reorder_kernel, blocks_for(a.count, tpb), tpb, a.count, a.scenes, a.scene_of, a.keys,
+                     a.cell_offsets, a.unordered, a.predicted, a.params, a.sorted_index, a.slot_of, a.cell, a.topology,
+                     a.params_a, a.params_b, a.velocities, a.sorted_velocity, a.packed, a.packed_mass);
         count_launch(2);
     }
     return cudaGetLastError();
@@ -383,23 +400,23 @@ cudaError_t launch_boundary_build(cudaStream_t stream, const BoundaryBuildArgs& 
     cudaError_t e = cudaMemsetAsync(a.cell_offsets, 0, (a.cells + 1) * sizeof(uint32_t), stream);
     if (e != cudaSuccess || a.count == 0) return e;
     const unsigned tpb = 256;
-    boundary_key_kernel<<<blocks_for(a.count, tpb), tpb, 0, stream>>>(a.count, a.scenes, a.scene_of, a.rest, a.velocity, a.keys,
-                                                                      a.arrival, a.cell_offsets);
+    launch_after(stream, boundary_key_kernel, blocks_for(a.count, tpb), tpb, a.count, a.scenes, a.scene_of, a.rest,
+                 a.velocity, a.keys, a.arrival, a.cell_offsets);
     count_launch();
     if ((e = launch_exclusive_scan(stream, a.cell_offsets, a.cells + 1, a.tile_sums)) != cudaSuccess) return e;
-    scatter_kernel<<<blocks_for(a.count, tpb), tpb, 0, stream>>>(a.count, a.keys, a.arrival, a.cell_offsets, a.unordered);
-    boundary_reorder_kernel<<<blocks_for(a.count, tpb), tpb, 0, stream>>>(a.count, a.scenes, a.scene_of, a.keys, a.cell_offsets,
-                                                                          a.unordered, a.rest, a.velocity, a.sorted,
-                                                                          a.sorted_velocity);
+    launch_after(stream, scatter_kernel, blocks_for(a.count, tpb), tpb, a.count, a.keys, a.arrival, a.cell_offsets,
+                 a.unordered);
+    launch_after(stream, boundary_reorder_kernel, blocks_for(a.count, tpb), tpb, a.count, a.scenes, a.scene_of, a.keys,
+                 a.cell_offsets, a.unordered, a.rest, a.velocity, a.sorted, a.sorted_velocity);
     count_launch(2);
     return cudaGetLastError();
 }
 
 cudaError_t launch_exclusive_scan(cudaStream_t stream, uint32_t* data, const uint64_t n, uint32_t* tile_sums) {
     const unsigned tiles = static_cast<unsigned>(scan_tile_count(n));
-    scan_reduce_kernel<<<tiles, kScanThreads, 0, stream>>>(data, n, tile_sums);
-    scan_tiles_kernel<<<1, kScanThreads, 0, stream>>>(tile_sums, tiles);
-    scan_apply_kernel<<<tiles, kScanThreads, 0, stream>>>(data, n, tile_sums);
+    launch_after(stream, scan_reduce_kernel, tiles, kScanThreads, data, n, tile_sums);
+    launch_after(stream, scan_tiles_kernel, 1, kScanThreads, tile_sums, tiles);
+    launch_after(stream, scan_apply_kernel, tiles, kScanThreads, data, n, tile_sums);
     count_launch(3);
     return cudaGetLastError();
 }
@@ -411,7 +428,7 @@ cudaError_t launch_reference_offsets(cudaStream_t stream, const SceneDesc* host_
     for (uint32_t s = 0; s < scene_count && e == cudaSuccess; ++s) {
         const Grid& g = host_scenes[s].grid;
         const uint32_t n = g.cells_x * g.cells_y * g.cells_z;
-        reference_counts_kernel<<<blocks_for(n, 256), 256, 0, stream>>>(g, cell_offsets, reference_offsets);
+        launch_after(stream, reference_counts_kernel, blocks_for(n, 256), 256, g, cell_offsets, reference_offsets);
         count_launch();
         e = cudaGetLastError();
     }
@@ -423,8 +440,8 @@ cudaError_t launch_reference_order(cudaStream_t stream, const uint32_t count, co
                                    const uint32_t* sorted_index, const uint32_t* keys, const uint32_t* cell_offsets,
                                    const uint32_t* reference_offsets, uint32_t* out_index, unsigned long long* out_keys) {
     if (count == 0) return cudaSuccess;
-    reference_order_kernel<<<blocks_for(count, 256), 256, 0, stream>>>(count, scenes, cell, sorted_index, keys, cell_offsets,
-                                                                       reference_offsets, out_index, out_keys);
+    launch_after(stream, reference_order_kernel, blocks_for(count, 256), 256, count, scenes, cell, sorted_index, keys,
+                 cell_offsets, reference_offsets, out_index, out_keys);
     count_launch();
     return cudaGetLastError();
 }

@@ -15,6 +15,7 @@
 // Tangents are FP32, as in the reference.  Every pair outside a term's support contributes an
 // exact zero there, so the in-support lists give the same sums up to FP32 rounding.
 #include "engine.h"
+#include "dependent_launch.cuh"
 #include "gather.cuh"
 
 namespace pbf {
@@ -91,6 +92,7 @@ __global__ void tangent_seed_kernel(const uint32_t count, const uint32_t* __rest
                                     const SceneDesc* __restrict__ scenes, const Field3 x_dot, const Field3 v_dot,
                                     const Field3 a_dot, const ParamTangent pt, float4* __restrict__ x0,
                                     float4* __restrict__ x_state, float4* __restrict__ params_a, float4* __restrict__ params_b) {
+    after_predecessor();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= count) return;
     const uint32_t i = sorted_index[s];
@@ -180,6 +182,7 @@ struct DensityLambdaJvpOp {
 #define PBF_JVP_MIN_BLOCKS 0
 #endif
 __global__ void __launch_bounds__(kBlock, PBF_JVP_MIN_BLOCKS) density_lambda_jvp_kernel(const DensityLambdaJvpArgs a) {
+    after_predecessor();
     const Particle p = locate(a.g);
     if (!p.active) return;
     DensityLambdaJvpOp op;
@@ -287,6 +290,7 @@ struct CorrectionJvpOp {
 // blocks unbounded: the pass waits on its neighbours' loads, and the extra warps hide more of that
 // (the 1M tangent step fell from 11.54 to 10.64 ms; 80 and 64 registers were slower).
 __global__ void __launch_bounds__(kBlock, 7) correction_jvp_kernel(const CorrectionJvpArgs a) {
+    after_predecessor();
     const Particle p = locate(a.g);
     if (!p.active) return;
     CorrectionJvpOp op;
@@ -332,6 +336,7 @@ __global__ void tangent_reconstruct_kernel(const uint32_t count, const int4* __r
                                            const uint32_t* __restrict__ sorted_index, const float4* __restrict__ x_dot,
                                            const float4* __restrict__ x_state, float4* __restrict__ velocity_dot,
                                            const MutField3 out_positions) {
+    after_predecessor();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= count) return;
     const f3 xd = xyz(x_dot[s]);
@@ -385,6 +390,7 @@ struct VorticityJvpOp {
 };
 
 __global__ void __launch_bounds__(kBlock, PBF_JVP_MIN_BLOCKS) vorticity_jvp_kernel(const VorticityJvpArgs a) {
+    after_predecessor();
     const Particle p = locate(a.g);
     if (!p.active) return;
     VorticityJvpOp op;
@@ -451,6 +457,7 @@ struct NormalJvpOp {
 };
 
 __global__ void __launch_bounds__(kBlock, PBF_JVP_MIN_BLOCKS) normal_jvp_kernel(const NormalJvpArgs a) {
+    after_predecessor();
     const Particle p = locate(a.g);
     if (!p.active) return;
     NormalJvpOp op;
@@ -525,6 +532,7 @@ struct XsphJvpOp {
 };
 
 __global__ void __launch_bounds__(kBlock, PBF_JVP_MIN_BLOCKS) xsph_jvp_kernel(const XsphJvpArgs a) {
+    after_predecessor();
     const Particle p = locate(a.g);
     if (!p.active) return;
     XsphJvpOp op;
@@ -613,13 +621,11 @@ int Engine::tangent(const pbf_particle_state* state, const StepRecord& r, const 
     const MutField3 out_v{next_state_tangent->velocities.x, next_state_tangent->velocities.y, next_state_tangent->velocities.z};
 
     timer_.begin(stream_, kPassTangentSeed);
-    tangent_seed_kernel<<<blocks_of(n, 256), 256, 0, stream_>>>(
-        n, r.sorted_index, r.cell, d_scenes_,
-        {state_tangent->positions.x, state_tangent->positions.y, state_tangent->positions.z},
-        {state_tangent->velocities.x, state_tangent->velocities.y, state_tangent->velocities.z},
-        {control_tangent->external_accelerations.x, control_tangent->external_accelerations.y,
-         control_tangent->external_accelerations.z},
-        pt, ws->x[0], ws->x_state, ws->params_a, ws->params_b);
+    launch_after(stream_, tangent_seed_kernel, blocks_of(n, 256), 256, n, r.sorted_index, r.cell, d_scenes_,
+                 {state_tangent->positions.x, state_tangent->positions.y, state_tangent->positions.z},
+                 {state_tangent->velocities.x, state_tangent->velocities.y, state_tangent->velocities.z},
+                 {control_tangent->external_accelerations.x, control_tangent->external_accelerations.y, control_tangent->external_accelerations.z},
+                 pt, ws->x[0], ws->x_state, ws->params_a, ws->params_b);
     timer_.end(stream_, kPassTangentSeed);
     count_launch();
     const bool keep = r.keeps_all(true);
@@ -660,7 +666,7 @@ int Engine::tangent(const pbf_particle_state* state, const StepRecord& r, const 
         }
         DensityLambdaJvpArgs dl{gc, list, xk, ws->x[k & 1u], ws->params_a, density_k, gsum_k, ws->lambda};
         timer_.begin(stream_, kPassDensityLambdaJvp);
-        density_lambda_jvp_kernel<<<blocks, block, 0, stream_>>>(dl);
+        launch_after(stream_, density_lambda_jvp_kernel, blocks, block, dl);
         timer_.end(stream_, kPassDensityLambdaJvp);
         if (!keep && k + 1u < K) {   // the next primal iterate (the last one, x_K, is kept)
             CorrectionArgs c{gc, xk, sg->lambda[0], sg->positions[k & 1u], nullptr, 0, Field3{}, r.sorted_index, MutField3{},
@@ -671,29 +677,29 @@ int Engine::tangent(const pbf_particle_state* state, const StepRecord& r, const 
         CorrectionJvpArgs ca{gc_reverse, list, xk, ws->x[k & 1u], lambda_k, ws->lambda, ws->params_a, ws->params_b, r.mask[k],
                              ws->x[(k + 1u) & 1u], k + 1u == K ? 1 : 0, r.sorted_index, ws->x_state, ws->velocity, out_x};
         timer_.begin(stream_, kPassCorrectionJvp);
-        correction_jvp_kernel<<<blocks, block, 0, stream_>>>(ca);
+        launch_after(stream_, correction_jvp_kernel, blocks, block, ca);
         timer_.end(stream_, kPassCorrectionJvp);
         count_launch(2);
     }
     const float4* x_dot_K = ws->x[K & 1u];
     if (K == 0) {
-        tangent_reconstruct_kernel<<<blocks_of(n, 256), 256, 0, stream_>>>(n, r.cell, d_scenes_, r.sorted_index, x_dot_K,
-                                                                           ws->x_state, ws->velocity, out_x);
+        launch_after(stream_, tangent_reconstruct_kernel, blocks_of(n, 256), 256, n, r.cell, d_scenes_, r.sorted_index,
+                     x_dot_K, ws->x_state, ws->velocity, out_x);
         count_launch();
     }
     const float4* xK = r.iterate(K, K, true);
     const StoredList post{r.list_entries[keep ? K : 0u], r.list_counts[keep ? K : 0u], r.list_capacity};
     VorticityJvpArgs va{gc, post, xK, x_dot_K, r.velocity, ws->velocity, r.vorticity, ws->vorticity};
     timer_.begin(stream_, kPassVorticityJvp);
-    vorticity_jvp_kernel<<<blocks, block, 0, stream_>>>(va);
+    launch_after(stream_, vorticity_jvp_kernel, blocks, block, va);
     timer_.end(stream_, kPassVorticityJvp);
     NormalJvpArgs na{gc_reverse, post, xK, x_dot_K, r.vorticity, ws->vorticity, r.normal, ws->velocity, ws->params_b, ws->confined};
     timer_.begin(stream_, kPassNormalJvp);
-    normal_jvp_kernel<<<blocks, block, 0, stream_>>>(na);
+    launch_after(stream_, normal_jvp_kernel, blocks, block, na);
     timer_.end(stream_, kPassNormalJvp);
     XsphJvpArgs xa{gc, post, xK, x_dot_K, r.confined, ws->confined, ws->params_a, r.sorted_index, out_v};
     timer_.begin(stream_, kPassXsphJvp);
-    xsph_jvp_kernel<<<blocks, block, 0, stream_>>>(xa);
+    launch_after(stream_, xsph_jvp_kernel, blocks, block, xa);
     timer_.end(stream_, kPassXsphJvp);
     count_launch(3);
     return check(cudaGetLastError(), "jvp_step");

@@ -21,6 +21,7 @@
 // so that pass walks the full stencil of the input positions, as the reference does.
 #include <cmath>
 
+#include "dependent_launch.cuh"
 #include "sph_ops.cuh"
 
 namespace pbf {
@@ -57,6 +58,7 @@ using namespace detail;
 template <bool WithBoundary>
 __global__ void __launch_bounds__(kBlock, PBF_SPH_DENSITY_MIN_BLOCKS) sph_density_kernel(const SphStep st, const uint32_t method, float* density_record,
                                                              float* pressure, float* pressure_term, const float* warm) {
+    after_predecessor();
     const Own o = own(st);
     if (!o.p.active) return;
     DensityOp<WithBoundary> op;
@@ -84,6 +86,7 @@ struct WcsphForceArgs {
 
 template <bool WithBoundary>
 __global__ void __launch_bounds__(kBlock, PBF_WCSPH_FORCE_MIN_BLOCKS) wcsph_force_kernel(const WcsphForceArgs a) {
+    after_predecessor();
     const SphStep& st = a.st;
     const Own o = own(st);
     if (!o.p.active) return;
@@ -188,6 +191,7 @@ struct NonPressureOp {
 template <bool WithBoundary>
 __global__ void __launch_bounds__(kBlock, PBF_SPH_NON_PRESSURE_MIN_BLOCKS) non_pressure_kernel(const SphStep st, const int mode, const MutField3 out_positions,
                                                               const MutField3 out_velocities, const uint32_t displacement_slot) {
+    after_predecessor();
     const Own o = own(st);
     if (!o.p.active) return;
     const uint32_t s = o.p.s;
@@ -229,6 +233,7 @@ __global__ void __launch_bounds__(kBlock, PBF_SPH_NON_PRESSURE_MIN_BLOCKS) non_p
 template <bool WithBoundary>
 __global__ void __launch_bounds__(kBlock, PBF_SPH_DENSITY_MIN_BLOCKS) predicted_density_kernel(const SphStep st, const PressureUpdate update,
                                                                    float* pressure, float* pressure_term, float* record) {
+    after_predecessor();
     const Own o = own(st);
     if (!o.p.active) return;
     const uint32_t s = o.p.s;
@@ -255,6 +260,7 @@ struct PressureKernelArgs {
 
 template <bool WithBoundary>
 __global__ void __launch_bounds__(kBlock, PBF_SPH_PRESSURE_MIN_BLOCKS) pressure_kernel(const PressureKernelArgs a) {
+    after_predecessor();
     const SphStep& st = a.st;
     const Own o = own(st);
     if (!o.p.active) return;
@@ -276,6 +282,7 @@ __global__ void __launch_bounds__(kBlock, PBF_SPH_PRESSURE_MIN_BLOCKS) pressure_
 // ------------------------------------------------------------------ constants
 __global__ void sph_constants_kernel(const SphSceneInput* __restrict__ inputs, const uint32_t n, SphConstants* __restrict__ out,
                                      KernelConstants* __restrict__ list_constants) {
+    after_predecessor();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const SphSceneInput in = inputs[i];
@@ -341,7 +348,7 @@ unsigned block_of(const unsigned block) {
 
 cudaError_t launch_sph_constants(cudaStream_t stream, const SphSceneInput* inputs, const uint32_t n, SphConstants* out,
                                  KernelConstants* list_constants) {
-    sph_constants_kernel<<<grid_of(n, 64), 64, 0, stream>>>(inputs, n, out, list_constants);
+    launch_after(stream, sph_constants_kernel, grid_of(n, 64), 64, inputs, n, out, list_constants);
     count_launch();
     return cudaGetLastError();
 }
@@ -351,9 +358,11 @@ cudaError_t launch_density(cudaStream_t stream, const SphStep& st, const uint32_
     if (st.g.count == 0) return cudaSuccess;
     const unsigned b = block_of(block);
     if (st.g.boundary)
-        sph_density_kernel<true><<<grid_of(st.g.count, b), b, 0, stream>>>(st, method, density_record, pressure, pressure_term, warm);
+        launch_after(stream, sph_density_kernel<true>, grid_of(st.g.count, b), b, st, method, density_record, pressure,
+                     pressure_term, warm);
     else
-        sph_density_kernel<false><<<grid_of(st.g.count, b), b, 0, stream>>>(st, method, density_record, pressure, pressure_term, warm);
+        launch_after(stream, sph_density_kernel<false>, grid_of(st.g.count, b), b, st, method, density_record, pressure,
+                     pressure_term, warm);
     count_launch();
     return cudaGetLastError();
 }
@@ -365,8 +374,8 @@ cudaError_t launch_wcsph_forces(cudaStream_t stream, const SphStep& st, const fl
     const unsigned b = block_of(block);
     const WcsphForceArgs a{st, pressure_term, out_positions, out_velocities, record_pressure, record_viscosity, record_surface,
                            record_total};
-    if (st.g.boundary) wcsph_force_kernel<true><<<grid_of(st.g.count, b), b, 0, stream>>>(a);
-    else wcsph_force_kernel<false><<<grid_of(st.g.count, b), b, 0, stream>>>(a);
+    if (st.g.boundary) launch_after(stream, wcsph_force_kernel<true>, grid_of(st.g.count, b), b, a);
+    else launch_after(stream, wcsph_force_kernel<false>, grid_of(st.g.count, b), b, a);
     count_launch();
     return cudaGetLastError();
 }
@@ -376,11 +385,11 @@ cudaError_t launch_non_pressure(cudaStream_t stream, const SphStep& st, const in
     if (st.g.count == 0) return cudaSuccess;
     const unsigned b = block_of(block);
     if (st.g.boundary)
-        non_pressure_kernel<true><<<grid_of(st.g.count, b), b, 0, stream>>>(st, mode, out_positions, out_velocities,
-                                                                           displacement_slot);
+        launch_after(stream, non_pressure_kernel<true>, grid_of(st.g.count, b), b, st, mode, out_positions, out_velocities,
+                     displacement_slot);
     else
-        non_pressure_kernel<false><<<grid_of(st.g.count, b), b, 0, stream>>>(st, mode, out_positions, out_velocities,
-                                                                            displacement_slot);
+        launch_after(stream, non_pressure_kernel<false>, grid_of(st.g.count, b), b, st, mode, out_positions, out_velocities,
+                     displacement_slot);
     count_launch();
     return cudaGetLastError();
 }
@@ -390,9 +399,11 @@ cudaError_t launch_predicted_density(cudaStream_t stream, const SphStep& st, con
     if (st.g.count == 0) return cudaSuccess;
     const unsigned b = block_of(block);
     if (st.g.boundary)
-        predicted_density_kernel<true><<<grid_of(st.g.count, b), b, 0, stream>>>(st, update, pressure, pressure_term, record);
+        launch_after(stream, predicted_density_kernel<true>, grid_of(st.g.count, b), b, st, update, pressure, pressure_term,
+                     record);
     else
-        predicted_density_kernel<false><<<grid_of(st.g.count, b), b, 0, stream>>>(st, update, pressure, pressure_term, record);
+        launch_after(stream, predicted_density_kernel<false>, grid_of(st.g.count, b), b, st, update, pressure, pressure_term,
+                     record);
     count_launch();
     return cudaGetLastError();
 }
@@ -401,8 +412,8 @@ cudaError_t launch_pressure(cudaStream_t stream, const SphStep& st, const Pressu
     if (st.g.count == 0) return cudaSuccess;
     const unsigned b = block_of(block);
     const PressureKernelArgs a{st, p};
-    if (st.g.boundary) pressure_kernel<true><<<grid_of(st.g.count, b), b, 0, stream>>>(a);
-    else pressure_kernel<false><<<grid_of(st.g.count, b), b, 0, stream>>>(a);
+    if (st.g.boundary) launch_after(stream, pressure_kernel<true>, grid_of(st.g.count, b), b, a);
+    else launch_after(stream, pressure_kernel<false>, grid_of(st.g.count, b), b, a);
     count_launch();
     return cudaGetLastError();
 }

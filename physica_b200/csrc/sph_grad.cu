@@ -15,6 +15,7 @@
 //   PCISPH / IISPH / DFSPH
 //           final prediction -> per iteration, newest first: pressure + pressure update, then
 //           predicted density + the prediction that produced it -> non-pressure -> density
+#include "dependent_launch.cuh"
 #include "sph_math.cuh"
 
 // Resident 128-thread blocks per SM the register budgets of the reverse and tangent list-replay
@@ -148,6 +149,7 @@ struct IntegrateVjpArgs {
 
 // integrate_vjp (sph/common.cu:344-366) and the control adjoint (sph/sph.cpp:244).
 __global__ void integrate_vjp_kernel(const IntegrateVjpArgs a) {
+    after_predecessor();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= a.st.g.count) return;
     const uint32_t i = a.st.sorted_index[s];
@@ -317,6 +319,7 @@ struct ForceVjpOp {
 };
 
 __global__ void __launch_bounds__(kBlock, PBF_WCSPH_FORCE_VJP_MIN_BLOCKS) wcsph_force_vjp_kernel(const ForceVjpArgs a) {
+    after_predecessor();
     const SphStep& st = a.st;
     const Own o = own(st);
     if (!o.p.active) return;
@@ -433,6 +436,7 @@ struct DensityVjpOp {
 };
 
 __global__ void __launch_bounds__(kBlock, PBF_SPH_DENSITY_VJP_MIN_BLOCKS) density_vjp_kernel(const DensityVjpArgs a) {
+    after_predecessor();
     const SphStep& st = a.st;
     const Own o = own(st);
     if (!o.p.active) return;
@@ -495,6 +499,7 @@ struct PredictVjpArgs {
 };
 
 __global__ void predict_vjp_kernel(const PredictVjpArgs a) {
+    after_predecessor();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= a.st.g.count) return;
     const uint32_t i = a.st.sorted_index[s];
@@ -603,6 +608,7 @@ struct PressureVjpOp {
 };
 
 __global__ void __launch_bounds__(kBlock, PBF_SPH_PRESSURE_VJP_MIN_BLOCKS) pressure_vjp_kernel(const PressureVjpArgs a) {
+    after_predecessor();
     const SphStep& st = a.st;
     const Own o = own(st);
     if (!o.p.active) return;
@@ -734,6 +740,7 @@ struct NonPressureVjpOp {
 };
 
 __global__ void __launch_bounds__(kBlock, PBF_SPH_NON_PRESSURE_VJP_MIN_BLOCKS) non_pressure_vjp_kernel(const NonPressureVjpArgs a) {
+    after_predecessor();
     const SphStep& st = a.st;
     const Own o = own(st);
     if (!o.p.active) return;
@@ -770,6 +777,7 @@ __global__ void __launch_bounds__(kBlock, PBF_SPH_NON_PRESSURE_VJP_MIN_BLOCKS) n
 __global__ void phase_seed_kernel(const uint32_t count, const uint32_t* __restrict__ sorted_index, const double4* __restrict__ from,
                                   double4* __restrict__ acceleration_adjoint, const double* __restrict__ next_warm,
                                   double* __restrict__ pressure_adjoint) {
+    after_predecessor();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= count) return;
     acceleration_adjoint[s] = from[s];
@@ -787,8 +795,8 @@ unsigned block_of(const unsigned block) {
 cudaError_t launch_integrate_vjp(cudaStream_t stream, const SphStep& st, const float4* total, ConstAdjField3 next_x,
                                  ConstAdjField3 next_v, AdjField3 x, AdjField3 v, AdjField3 control, double4* acceleration) {
     if (st.g.count == 0) return cudaSuccess;
-    integrate_vjp_kernel<<<grid_of(st.g.count, 256), 256, 0, stream>>>(
-        IntegrateVjpArgs{st, total, next_x, next_v, x, v, control, acceleration});
+    launch_after(stream, integrate_vjp_kernel, grid_of(st.g.count, 256), 256,
+                 IntegrateVjpArgs{st, total, next_x, next_v, x, v, control, acceleration});
     count_launch();
     return cudaGetLastError();
 }
@@ -799,7 +807,8 @@ cudaError_t launch_wcsph_force_vjp(cudaStream_t stream, const SphStep& st, const
     if (st.g.count == 0) return cudaSuccess;
     const unsigned b = block_of(block);
     const ParameterAdjoints p{pa.masses, pa.rest_densities, pa.viscosities, pa.surface_tensions, pa.method0, pa.method1, pa.method2};
-    wcsph_force_vjp_kernel<<<grid_of(st.g.count, b), b, 0, stream>>>(ForceVjpArgs{st, pressure, acceleration, x, v, p, density_adjoint});
+    launch_after(stream, wcsph_force_vjp_kernel, grid_of(st.g.count, b), b,
+                 ForceVjpArgs{st, pressure, acceleration, x, v, p, density_adjoint});
     count_launch();
     return cudaGetLastError();
 }
@@ -822,7 +831,7 @@ cudaError_t launch_density_vjp(cudaStream_t stream, const DensityVjpLaunch& d, c
                            d.non_pressure_adjoint,
                            d.acceleration_adjoint,
                            d.base_adjoint};
-    density_vjp_kernel<<<grid_of(d.st.g.count, b), b, 0, stream>>>(a);
+    launch_after(stream, density_vjp_kernel, grid_of(d.st.g.count, b), b, a);
     count_launch();
     return cudaGetLastError();
 }
@@ -832,9 +841,8 @@ cudaError_t launch_predict_vjp(cudaStream_t stream, const SphStep& st, const flo
                                double4* acceleration_adjoint, double4* base_adjoint, const double* next_warm,
                                double* pressure_adjoint) {
     if (st.g.count == 0) return cudaSuccess;
-    predict_vjp_kernel<<<grid_of(st.g.count, 256), 256, 0, stream>>>(PredictVjpArgs{
-        st, acceleration, base, next_x, next_v, x, v, non_pressure_adjoint, acceleration_adjoint, base_adjoint, next_warm,
-        pressure_adjoint});
+    launch_after(stream, predict_vjp_kernel, grid_of(st.g.count, 256), 256,
+                 PredictVjpArgs{ st, acceleration, base, next_x, next_v, x, v, non_pressure_adjoint, acceleration_adjoint, base_adjoint, next_warm, pressure_adjoint});
     count_launch();
     return cudaGetLastError();
 }
@@ -859,7 +867,7 @@ cudaError_t launch_pressure_vjp(cudaStream_t stream, const PressureVjpLaunch& d,
                             d.predicted_density_adjoint,
                             d.relaxation_adjoint,
                             d.warm_adjoint};
-    pressure_vjp_kernel<<<grid_of(d.st.g.count, b), b, 0, stream>>>(a);
+    launch_after(stream, pressure_vjp_kernel, grid_of(d.st.g.count, b), b, a);
     count_launch();
     return cudaGetLastError();
 }
@@ -870,7 +878,8 @@ cudaError_t launch_non_pressure_vjp(cudaStream_t stream, const SphStep& st, cons
     if (st.g.count == 0) return cudaSuccess;
     const unsigned b = block_of(block);
     const ParameterAdjoints p{pa.masses, pa.rest_densities, pa.viscosities, pa.surface_tensions, pa.method0, pa.method1, pa.method2};
-    non_pressure_vjp_kernel<<<grid_of(st.g.count, b), b, 0, stream>>>(NonPressureVjpArgs{st, adjoint, x, v, control, density_adjoint, p});
+    launch_after(stream, non_pressure_vjp_kernel, grid_of(st.g.count, b), b,
+                 NonPressureVjpArgs{st, adjoint, x, v, control, density_adjoint, p});
     count_launch();
     return cudaGetLastError();
 }
@@ -878,8 +887,8 @@ cudaError_t launch_non_pressure_vjp(cudaStream_t stream, const SphStep& st, cons
 cudaError_t launch_phase_seed(cudaStream_t stream, const uint32_t count, const uint32_t* sorted_index, const double4* from,
                               double4* acceleration_adjoint, const double* next_warm, double* pressure_adjoint) {
     if (count == 0) return cudaSuccess;
-    phase_seed_kernel<<<grid_of(count, 256), 256, 0, stream>>>(count, sorted_index, from, acceleration_adjoint, next_warm,
-                                                                pressure_adjoint);
+    launch_after(stream, phase_seed_kernel, grid_of(count, 256), 256, count, sorted_index, from, acceleration_adjoint,
+                 next_warm, pressure_adjoint);
     count_launch();
     return cudaGetLastError();
 }
@@ -899,6 +908,7 @@ using namespace detail;
 // Sorted tangents of the inputs: positions and masses, velocities, and the parameters packed as
 // params_a / params_b.
 __global__ void tangent_seed_kernel(const SphTangentStep t, const Field3 x, const Field3 v, const SphParameterTangents pt) {
+    after_predecessor();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= t.st.g.count) return;
     const uint32_t i = t.st.sorted_index[s];
@@ -944,6 +954,7 @@ struct DensityJvpOp {
 // The density tangent at the step's positions (+ WCSPH's equation of state, sph/wcsph.cu:102-117;
 // DFSPH: the divergence phase's warm-start pressure tangent).
 __global__ void __launch_bounds__(kBlock, PBF_SPH_DENSITY_JVP_MIN_BLOCKS) density_jvp_kernel(const SphTangentStep t, const uint32_t method, const float* warm) {
+    after_predecessor();
     const SphStep& st = t.st;
     const Own o = own(st);
     if (!o.p.active) return;
@@ -1110,6 +1121,7 @@ __device__ __forceinline__ void predict_tangent(const f3 x, const f3 v, const f3
 __global__ void __launch_bounds__(kBlock, PBF_WCSPH_FORCE_JVP_MIN_BLOCKS) wcsph_force_jvp_kernel(const SphTangentStep t, const float* pressure,
                                                                  const float4* total, const Field3 control_tangent,
                                                                  const MutField3 out_x, const MutField3 out_v) {
+    after_predecessor();
     const SphStep& st = t.st;
     const Own o = own(st);
     if (!o.p.active) return;
@@ -1222,6 +1234,7 @@ struct NonPressureJvpOp {
 
 __global__ void __launch_bounds__(kBlock, PBF_SPH_NON_PRESSURE_JVP_MIN_BLOCKS) non_pressure_jvp_kernel(const SphTangentStep t, const Field3 control_tangent,
                                                                   const int mode, const MutField3 out_x, const MutField3 out_v) {
+    after_predecessor();
     const SphStep& st = t.st;
     const Own o = own(st);
     if (!o.p.active) return;
@@ -1294,6 +1307,7 @@ struct PredictedDensityJvpOp {
 };
 
 __global__ void __launch_bounds__(kBlock, PBF_SPH_DENSITY_JVP_MIN_BLOCKS) predicted_density_jvp_kernel(const SphTangentStep t, const PredictedJvp u) {
+    after_predecessor();
     const SphStep& st = t.st;
     const Own o = own(st);
     if (!o.p.active) return;
@@ -1371,6 +1385,7 @@ struct PressureJvpOp {
 };
 
 __global__ void __launch_bounds__(kBlock, PBF_SPH_PRESSURE_JVP_MIN_BLOCKS) pressure_jvp_kernel(const SphTangentStep t, const PressureJvp u) {
+    after_predecessor();
     const SphStep& st = t.st;
     const Own o = own(st);
     if (!o.p.active) return;
@@ -1425,7 +1440,7 @@ __global__ void __launch_bounds__(kBlock, PBF_SPH_PRESSURE_JVP_MIN_BLOCKS) press
 cudaError_t launch_tangent_seed(cudaStream_t stream, const SphTangentStep& t, const Field3 x, const Field3 v,
                                 const SphParameterTangents& pt) {
     if (t.st.g.count == 0) return cudaSuccess;
-    tangent_seed_kernel<<<grid_of(t.st.g.count, 256), 256, 0, stream>>>(t, x, v, pt);
+    launch_after(stream, tangent_seed_kernel, grid_of(t.st.g.count, 256), 256, t, x, v, pt);
     count_launch();
     return cudaGetLastError();
 }
@@ -1434,7 +1449,7 @@ cudaError_t launch_density_jvp(cudaStream_t stream, const SphTangentStep& t, con
                                const unsigned block) {
     if (t.st.g.count == 0) return cudaSuccess;
     const unsigned b = block_of(block);
-    density_jvp_kernel<<<grid_of(t.st.g.count, b), b, 0, stream>>>(t, method, warm);
+    launch_after(stream, density_jvp_kernel, grid_of(t.st.g.count, b), b, t, method, warm);
     count_launch();
     return cudaGetLastError();
 }
@@ -1443,7 +1458,8 @@ cudaError_t launch_wcsph_force_jvp(cudaStream_t stream, const SphTangentStep& t,
                                    const Field3 control_tangent, const MutField3 out_x, const MutField3 out_v, const unsigned block) {
     if (t.st.g.count == 0) return cudaSuccess;
     const unsigned b = block_of(block);
-    wcsph_force_jvp_kernel<<<grid_of(t.st.g.count, b), b, 0, stream>>>(t, pressure, total, control_tangent, out_x, out_v);
+    launch_after(stream, wcsph_force_jvp_kernel, grid_of(t.st.g.count, b), b, t, pressure, total, control_tangent, out_x,
+                 out_v);
     count_launch();
     return cudaGetLastError();
 }
@@ -1452,7 +1468,7 @@ cudaError_t launch_non_pressure_jvp(cudaStream_t stream, const SphTangentStep& t
                                     const MutField3 out_x, const MutField3 out_v, const unsigned block) {
     if (t.st.g.count == 0) return cudaSuccess;
     const unsigned b = block_of(block);
-    non_pressure_jvp_kernel<<<grid_of(t.st.g.count, b), b, 0, stream>>>(t, control_tangent, mode, out_x, out_v);
+    launch_after(stream, non_pressure_jvp_kernel, grid_of(t.st.g.count, b), b, t, control_tangent, mode, out_x, out_v);
     count_launch();
     return cudaGetLastError();
 }
@@ -1460,7 +1476,7 @@ cudaError_t launch_non_pressure_jvp(cudaStream_t stream, const SphTangentStep& t
 cudaError_t launch_predicted_density_jvp(cudaStream_t stream, const SphTangentStep& t, const PredictedJvp& u, const unsigned block) {
     if (t.st.g.count == 0) return cudaSuccess;
     const unsigned b = block_of(block);
-    predicted_density_jvp_kernel<<<grid_of(t.st.g.count, b), b, 0, stream>>>(t, u);
+    launch_after(stream, predicted_density_jvp_kernel, grid_of(t.st.g.count, b), b, t, u);
     count_launch();
     return cudaGetLastError();
 }
@@ -1468,7 +1484,7 @@ cudaError_t launch_predicted_density_jvp(cudaStream_t stream, const SphTangentSt
 cudaError_t launch_pressure_jvp(cudaStream_t stream, const SphTangentStep& t, const PressureJvp& u, const unsigned block) {
     if (t.st.g.count == 0) return cudaSuccess;
     const unsigned b = block_of(block);
-    pressure_jvp_kernel<<<grid_of(t.st.g.count, b), b, 0, stream>>>(t, u);
+    launch_after(stream, pressure_jvp_kernel, grid_of(t.st.g.count, b), b, t, u);
     count_launch();
     return cudaGetLastError();
 }

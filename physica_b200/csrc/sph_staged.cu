@@ -7,6 +7,7 @@
 // divisions, one pair at a time; from shared memory they take two pairs at a time with the packed
 // arithmetic of sph_math.cuh.  Lists carry a skin (sph.cu), so the packed values include the zeros
 // beyond the support.  Every sum keeps the reference's order and rounding.
+#include "dependent_launch.cuh"
 #include "sph_ops.cuh"
 #include "staged.cuh"
 
@@ -36,6 +37,7 @@ struct DensityPassArgs {
 
 template <bool Words>
 __global__ void __launch_bounds__(kBlockParticles, 6) staged_sph_density_kernel(const DensityPassArgs a) {
+    after_predecessor();
     __shared__ Windows w;
     __shared__ __align__(16) float field[4][kStage];
     __shared__ ColumnHits columns[9][kBlockParticles];
@@ -95,6 +97,7 @@ struct PredictedPassArgs {
 };
 
 __global__ void __launch_bounds__(kBlockParticles, 8) staged_predicted_density_kernel(const PredictedPassArgs a) {
+    after_predecessor();
     __shared__ Windows w;
     __shared__ __align__(16) float4 positions[kStage];
     const SphStep& st = a.st;
@@ -156,6 +159,7 @@ struct PressurePass {
 };
 
 __global__ void __launch_bounds__(kBlockParticles, 7) staged_pressure_kernel(const PressurePass a) {
+    after_predecessor();
     __shared__ Windows w;
     __shared__ __align__(16) float4 positions[kStage];
     __shared__ __align__(16) float term[1][kStage];
@@ -205,7 +209,7 @@ __global__ void __launch_bounds__(kBlockParticles, 7) staged_pressure_kernel(con
 template <class Args>
 cudaError_t launch(void (*kernel)(Args), cudaStream_t stream, const Args& a) {
     if (a.g.count == 0) return cudaSuccess;
-    kernel<<<(a.g.count + kBlockParticles - 1u) / kBlockParticles, kBlockParticles, 0, stream>>>(a);
+    launch_after(stream, kernel, (a.g.count + kBlockParticles - 1u) / kBlockParticles, kBlockParticles, a);
     count_launch();
     return cudaGetLastError();
 }

@@ -28,6 +28,7 @@
 //
 // Every sum keeps the reference's order and rounding (gather.cuh): the lists hold the same neighbours
 // in the same order, without the particle itself, whose only term is its own density.
+#include "dependent_launch.cuh"
 #include "staged_ops.cuh"
 
 namespace pbf {
@@ -40,6 +41,7 @@ using namespace staged_detail;
 // Slots: also store the list of sorted slots that the reverse and tangent passes read.
 template <bool Slots>
 __global__ void __launch_bounds__(kBlockParticles, 6) staged_density_kernel(const StagedDensityArgs a) {
+    after_predecessor();
     __shared__ Windows w;
     __shared__ __align__(16) float field[4][kStage];
     __shared__ ColumnHits columns[9][kBlockParticles];
@@ -120,6 +122,7 @@ __global__ void __launch_bounds__(kBlockParticles, 6) staged_density_kernel(cons
 
 // ----------------------------------------------------------------- correction + project
 __global__ void __launch_bounds__(kBlockParticles, 7) staged_correction_kernel(const StagedCorrectionArgs a) {
+    after_predecessor();
     __shared__ Windows w;
     __shared__ __align__(16) float field[5][kStage];
     const Particle p = locate(a.g);
@@ -153,6 +156,7 @@ __global__ void __launch_bounds__(kBlockParticles, 7) staged_correction_kernel(c
 // ----------------------------------------------------------- post-loop scan + vorticity
 template <bool Slots>
 __global__ void __launch_bounds__(kBlockParticles, 4) staged_vorticity_kernel(const StagedVorticityArgs a) {
+    after_predecessor();
     __shared__ Windows w;
     __shared__ __align__(16) float field[6][kStage];
     __shared__ ColumnHits columns[9][kBlockParticles];
@@ -197,6 +201,7 @@ __global__ void __launch_bounds__(kBlockParticles, 4) staged_vorticity_kernel(co
 
 // ------------------------------------------------------------------ normal + confinement
 __global__ void __launch_bounds__(kBlockParticles, 8) staged_normal_kernel(const StagedNormalArgs a) {
+    after_predecessor();
     __shared__ Windows w;
     __shared__ __align__(16) float field[4][kStage];
     const Particle p = locate(a.g);
@@ -227,6 +232,7 @@ __global__ void __launch_bounds__(kBlockParticles, 8) staged_normal_kernel(const
 
 // -------------------------------------------------------------------------------- XSPH
 __global__ void __launch_bounds__(kBlockParticles, 5) staged_xsph_kernel(const StagedXsphArgs a) {
+    after_predecessor();
     __shared__ Windows w;
     __shared__ __align__(16) float field[6][kStage];
     const Particle p = locate(a.g);
@@ -262,7 +268,7 @@ inline unsigned blocks_of(const uint32_t n) { return (n + kBlockParticles - 1u) 
 template <class Args>
 cudaError_t launch(void (*kernel)(Args), cudaStream_t stream, const Args& a) {
     if (a.g.count == 0) return cudaSuccess;
-    kernel<<<blocks_of(a.g.count), kBlockParticles, 0, stream>>>(a);
+    launch_after(stream, kernel, blocks_of(a.g.count), kBlockParticles, a);
     count_launch();
     return cudaGetLastError();
 }

@@ -7,6 +7,7 @@
 // list order.  The sums are the same sums in the same order, so the results are those of the other passes
 // bit for bit.  A forward step of 5k particles, four iterations, in a graph: 0.240 ms with one lane, 0.164
 // with four; of those the two passes of an iteration take 23 us in place of 39.
+#include "dependent_launch.cuh"
 #include "staged_ops.cuh"
 
 namespace pbf {
@@ -158,6 +159,7 @@ __device__ __forceinline__ StoredWords stored_words(const StoredList& list, cons
 
 // ------------------------------------------------------------------- density + lambda
 __global__ void __launch_bounds__(kThreads) group_density_kernel(const StagedDensityArgs a) {
+    after_predecessor();
     __shared__ Windows w;
     __shared__ __align__(16) float field[4][kGroupStage];
     __shared__ __align__(16) uint16_t entries[kParticles][kGroupList];
@@ -251,6 +253,7 @@ __global__ void __launch_bounds__(kThreads) group_density_kernel(const StagedDen
 
 // ----------------------------------------------------------------- correction + project
 __global__ void __launch_bounds__(kThreads) group_correction_kernel(const StagedCorrectionArgs a) {
+    after_predecessor();
     __shared__ Windows w;
     __shared__ __align__(16) float field[5][kGroupStage];
     __shared__ __align__(16) Exchange<3> exchange[kParticles];
@@ -291,6 +294,7 @@ __global__ void __launch_bounds__(kThreads) group_correction_kernel(const Staged
 
 // ----------------------------------------------------------- post-loop scan + vorticity
 __global__ void __launch_bounds__(kThreads) group_vorticity_kernel(const StagedVorticityArgs a) {
+    after_predecessor();
     __shared__ Windows w;
     __shared__ __align__(16) float field[6][kGroupStage];
     __shared__ __align__(16) uint16_t entries[kParticles][kGroupList];
@@ -347,6 +351,7 @@ __global__ void __launch_bounds__(kThreads) group_vorticity_kernel(const StagedV
 
 // ------------------------------------------------------------------ normal + confinement
 __global__ void __launch_bounds__(kThreads) group_normal_kernel(const StagedNormalArgs a) {
+    after_predecessor();
     __shared__ Windows w;
     __shared__ __align__(16) float field[4][kGroupStage];
     __shared__ __align__(16) Exchange<3> exchange[kParticles];
@@ -386,6 +391,7 @@ __global__ void __launch_bounds__(kThreads) group_normal_kernel(const StagedNorm
 
 // -------------------------------------------------------------------------------- XSPH
 __global__ void __launch_bounds__(kThreads) group_xsph_kernel(const StagedXsphArgs a) {
+    after_predecessor();
     __shared__ Windows w;
     __shared__ __align__(16) float field[6][kGroupStage];
     __shared__ __align__(16) Exchange<3> exchange[kParticles];
@@ -427,7 +433,7 @@ __global__ void __launch_bounds__(kThreads) group_xsph_kernel(const StagedXsphAr
 template <class Args>
 cudaError_t launch(void (*kernel)(Args), cudaStream_t stream, const Args& a) {
     if (a.g.count == 0) return cudaSuccess;
-    kernel<<<(a.g.count + kParticles - 1u) / kParticles, kThreads, 0, stream>>>(a);
+    launch_after(stream, kernel, (a.g.count + kParticles - 1u) / kParticles, kThreads, a);
     count_launch();
     return cudaGetLastError();
 }

@@ -40,6 +40,7 @@
 #include "../../include/physica_pbf.h"
 #include "engine.h"
 #include "pbf_internal.h"
+#include "dependent_launch.cuh"
 #include "pbf_launch.h"
 
 namespace pbf {
@@ -191,6 +192,7 @@ __global__ void scene_tables_kernel(const SceneDesc desc, const SceneStatic stat
                                     const unsigned long long step, SceneDesc* __restrict__ desc_out,
                                     SceneStatic* __restrict__ statics_out, float* __restrict__ radius_out,
                                     unsigned long long* __restrict__ step_out) {
+    after_predecessor();
     *desc_out = desc;
     *statics_out = statics;
     *radius_out = radius;
@@ -284,7 +286,7 @@ int forward_preallocated(const pbf_domain_configuration* domain, const pbf_confi
     auto* constants = static_cast<KernelConstants*>(at(L.constants));
     auto* radius = static_cast<float*>(at(L.radius));
     auto* step = static_cast<unsigned long long*>(at(L.step));
-    scene_tables_kernel<<<1, 1, 0, stream>>>(d, st, c.support_radius, state->step_index, scenes, statics, radius, step);
+    launch_after(stream, scene_tables_kernel, 1, 1, d, st, c.support_radius, state->step_index, scenes, statics, radius, step);
     count_launch();
     if (int rc = cuda(cudaGetLastError(), "scene table")) return rc;
     if (int rc = cuda(launch_constants(stream, radius, 1, constants), "kernel constants")) return rc;
