@@ -446,8 +446,8 @@ int Engine::forward(const pbf_particle_state* state, const pbf_control* control,
     // The device step counter holds the index of the state being advanced.
     if (host_step_ != state->step_index) {
         if (int rc = check(launch_set_step(stream_, d_step_, state->step_index), "step counter")) return rc;
-        host_step_ = state->step_index;
     }
+    host_step_ = ~0ull;   // unknown again if the step fails halfway
     int rc = PBF_SUCCESS;
     if (graphs_ && !timer_.enabled()) {
         GraphKey key{};
@@ -536,7 +536,8 @@ GatherCommon Engine::gather_common(const StepRecord& r) const {
 
 int Engine::launch_forward(cudaStream_t stream, const pbf_particle_state* state, const pbf_control* control,
                            const pbf_parameters* parameters, pbf_particle_state* next_state, StepRecord& r) {
-    if (int rc = check(launch_scene_time(stream, d_static_, d_scenes_, d_step_, static_cast<uint32_t>(scenes_.size())),
+    if (int rc = check(launch_scene_time(stream, d_static_, d_scenes_, d_step_, static_cast<uint32_t>(scenes_.size()),
+                                         r.cell_offsets, cells_ + 1),
                        "scene table"))
         return rc;
     const bool diff = differentiable();
@@ -569,6 +570,8 @@ int Engine::launch_forward(cudaStream_t stream, const pbf_particle_state* state,
     g.packed = packed_;
     g.packed_mass = packed_mass_;
     timer_.begin(stream, kPassGrid);
+    g.cleared = 1;
+    g.step = d_step_;
     if (int rc = check(launch_grid_build(stream, g), "grid build")) return rc;
     if (boundary_count_ > 0) {
         BoundaryBuildArgs b{boundary_count_, cells_, d_scenes_, boundary_scene_, boundary_rest_, boundary_velocity_,
@@ -578,8 +581,7 @@ int Engine::launch_forward(cudaStream_t stream, const pbf_particle_state* state,
     timer_.end(stream, kPassGrid);
 
     if (runs_staged_passes(shape_)) {
-        if (int rc = launch_staged(stream, state, next_state, r)) return rc;
-        return check(launch_advance_step(stream, d_step_), "step counter");
+        return launch_staged(stream, state, next_state, r);
     }
     const GatherCommon gc = gather_common(r);
     const Field3 previous{state->positions.x, state->positions.y, state->positions.z};
@@ -650,7 +652,7 @@ int Engine::launch_forward(cudaStream_t stream, const pbf_particle_state* state,
     timer_.begin(stream, kPassXsph);
     if (int rc = check(launch_xsph(stream, x, shape_.block), "xsph")) return rc;
     timer_.end(stream, kPassXsph);
-    return check(launch_advance_step(stream, d_step_), "step counter");
+    return PBF_SUCCESS;
 }
 
 // next_state.positions are final here.  Under capture the record must be external to become an event

@@ -10,6 +10,8 @@
 // the stable order, so sorted_index / cell_offsets equal the reference's bit for bit.
 // Keys are global across the scenes of a batch (scene cell ranges are disjoint and
 // ordered), so one sort serves one scene or many.
+#include <algorithm>
+
 #include "pbf_internal.h"
 #include "../../include/physica_pbf.h"
 #include "dependent_launch.cuh"
@@ -30,10 +32,11 @@ __global__ void predict_key_kernel(const uint32_t count, const SceneDesc* __rest
                                    const float* __restrict__ masses, float4* __restrict__ predicted,
                                    uint32_t* __restrict__ keys, uint32_t* __restrict__ arrival,
                                    uint32_t* __restrict__ histogram, uint32_t* __restrict__ input_flags,
-                                   const int key_current) {
+                                   const int key_current, unsigned long long* __restrict__ step) {
     after_predecessor();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
+    if (i == 0u && step) *step += 1ull;   // its reader, scene_time_kernel, has run
     const SceneDesc& sc = scenes[scene_of ? scene_of[i] : 0u];
     const f3 gravity = mk(sc.gravity_x, sc.gravity_y, sc.gravity_z);
     const f3 v = mk(velocities.x[i], velocities.y[i], velocities.z[i]);
@@ -65,6 +68,9 @@ __global__ void predict_key_kernel(const uint32_t count, const SceneDesc* __rest
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;
 constexpr int kScanTile = kScanThreads * kScanItems;
+// Up to this many tiles (4M cells) each block adds up the sums of the tiles before its own, at most four
+// loads a thread, which is cheaper than a launch between the two that scans them.
+constexpr unsigned kSummedTiles = 1024;
 
 __device__ __forceinline__ uint32_t warp_inclusive(uint32_t v) {
     const int lane = threadIdx.x & 31;
@@ -124,7 +130,9 @@ __global__ void scan_tiles_kernel(uint32_t* __restrict__ tile_sums, const uint32
     }
 }
 
-// In-place exclusive scan of each tile plus its tile prefix: histogram -> cell offsets.
+// In-place exclusive scan of each tile plus its tile prefix: histogram -> cell offsets.  tile_sums holds the
+// tiles' sums (Sum: the block adds up those before its own) or their exclusive scan.
+template <bool Sum>
 __global__ void scan_apply_kernel(uint32_t* __restrict__ data, const uint64_t n, const uint32_t* __restrict__ tile_sums) {
     after_predecessor();
     const uint64_t base = static_cast<uint64_t>(blockIdx.x) * kScanTile;
@@ -154,14 +162,22 @@ __global__ void scan_apply_kernel(uint32_t* __restrict__ data, const uint64_t n,
     }
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) local += vals[k];
-    __shared__ uint32_t warp_tot[kScanThreads / 32];
+    __shared__ uint32_t warp_tot[kScanThreads / 32], warp_before[kScanThreads / 32];
     const uint32_t inc = warp_inclusive(local);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 31) warp_tot[warp] = inc;
+    if constexpr (Sum) {
+        uint32_t before = 0;
+        for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kScanThreads) before += tile_sums[t];
+        before = __reduce_add_sync(0xffffffffu, before);
+        if (lane == 0) warp_before[warp] = before;
+    }
     __syncthreads();
-    uint32_t warp_prefix = 0;
-    for (int w = 0; w < warp; ++w) warp_prefix += warp_tot[w];
-    uint32_t running = tile_sums[blockIdx.x] + warp_prefix + inc - local;
+    uint32_t prefix = Sum ? 0u : tile_sums[blockIdx.x];
+    if constexpr (Sum)
+        for (int w = 0; w < kScanThreads / 32; ++w) prefix += warp_before[w];
+    for (int w = 0; w < warp; ++w) prefix += warp_tot[w];
+    uint32_t running = prefix + inc - local;
     if (vector) {
         uint4* const dst = reinterpret_cast<uint4*>(data + first);
 #pragma unroll
@@ -322,9 +338,11 @@ __global__ void advance_step_kernel(unsigned long long* step) {
 // (neighborhood/neighborhood.cpp:83-88) and the collision box (pbf/pbf.cpp:17-31), each with the
 // float operation order of the reference's host code.
 __global__ void scene_time_kernel(const SceneStatic* __restrict__ statics, SceneDesc* __restrict__ scenes,
-                                  const unsigned long long* __restrict__ step, const uint32_t count) {
+                                  const unsigned long long* __restrict__ step, const uint32_t count,
+                                  uint32_t* __restrict__ clear, const uint64_t words) {
     after_predecessor();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint64_t w = s; w < words; w += static_cast<uint64_t>(gridDim.x) * blockDim.x) clear[w] = 0u;
     if (s >= count) return;
     const SceneStatic st = statics[s];
     SceneDesc& d = scenes[s];
@@ -361,8 +379,11 @@ cudaError_t launch_advance_step(cudaStream_t stream, unsigned long long* step) {
 }
 
 cudaError_t launch_scene_time(cudaStream_t stream, const SceneStatic* statics, SceneDesc* scenes, const unsigned long long* step,
-                              const uint32_t count) {
-    launch_after(stream, scene_time_kernel, blocks_for(count, 128), 128, statics, scenes, step, count);
+                              const uint32_t count, uint32_t* clear, const uint64_t words) {
+    // four blocks an SM at most, or as many as the scenes need
+    const unsigned blocks = std::max(blocks_for(count, 128), std::min(blocks_for(words, 128), 592u));
+    if (blocks == 0) return cudaSuccess;
+    launch_after(stream, scene_time_kernel, blocks, 128, statics, scenes, step, count, clear, words);
     count_launch();
     return cudaGetLastError();
 }
@@ -371,20 +392,18 @@ size_t scan_tile_count(const uint64_t n) { return static_cast<size_t>((n + kScan
 
 cudaError_t launch_grid_build(cudaStream_t stream, const GridBuildArgs& a) {
     const unsigned tpb = 256;
-    cudaError_t e = cudaMemsetAsync(a.cell_offsets, 0, (a.cells + 1) * sizeof(uint32_t), stream);
+    cudaError_t e = cudaSuccess;
+    if (!a.cleared) e = cudaMemsetAsync(a.cell_offsets, 0, (a.cells + 1) * sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
     if (a.count > 0) {
         launch_after(stream, predict_key_kernel, blocks_for(a.count, tpb), tpb, a.count, a.scenes, a.scene_of, a.positions,
                      a.velocities, a.controls, a.params.masses, a.predicted, a.keys, a.arrival, a.cell_offsets, a.input_flags,
-                     a.key_current);
+                     a.key_current, a.step);
         count_launch();
+    } else if (a.step) {
+        if ((e = launch_advance_step(stream, a.step)) != cudaSuccess) return e;
     }
-    const uint64_t n = a.cells + 1;
-    const unsigned tiles = static_cast<unsigned>(scan_tile_count(n));
-    launch_after(stream, scan_reduce_kernel, tiles, kScanThreads, a.cell_offsets, n, a.tile_sums);
-    launch_after(stream, scan_tiles_kernel, 1, kScanThreads, a.tile_sums, tiles);
-    launch_after(stream, scan_apply_kernel, tiles, kScanThreads, a.cell_offsets, n, a.tile_sums);
-    count_launch(3);
+    if ((e = launch_exclusive_scan(stream, a.cell_offsets, a.cells + 1, a.tile_sums)) != cudaSuccess) return e;
     if (a.count > 0) {
         launch_after(stream, scatter_kernel, blocks_for(a.count, tpb), tpb, a.count, a.keys, a.arrival, a.cell_offsets,
                      a.unordered);
@@ -415,9 +434,14 @@ cudaError_t launch_boundary_build(cudaStream_t stream, const BoundaryBuildArgs& 
 cudaError_t launch_exclusive_scan(cudaStream_t stream, uint32_t* data, const uint64_t n, uint32_t* tile_sums) {
     const unsigned tiles = static_cast<unsigned>(scan_tile_count(n));
     launch_after(stream, scan_reduce_kernel, tiles, kScanThreads, data, n, tile_sums);
-    launch_after(stream, scan_tiles_kernel, 1, kScanThreads, tile_sums, tiles);
-    launch_after(stream, scan_apply_kernel, tiles, kScanThreads, data, n, tile_sums);
-    count_launch(3);
+    if (tiles <= kSummedTiles) {
+        launch_after(stream, scan_apply_kernel<true>, tiles, kScanThreads, data, n, tile_sums);
+        count_launch(2);
+    } else {
+        launch_after(stream, scan_tiles_kernel, 1, kScanThreads, tile_sums, tiles);
+        launch_after(stream, scan_apply_kernel<false>, tiles, kScanThreads, data, n, tile_sums);
+        count_launch(3);
+    }
     return cudaGetLastError();
 }
 

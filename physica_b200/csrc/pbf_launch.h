@@ -43,6 +43,8 @@ struct GridBuildArgs {
     float4* sorted_velocity = nullptr; // optional (v, 0) in sorted order
     PackedPositions packed{};          // optional x* as three arrays in sorted order
     float* packed_mass = nullptr;      // optional, with `packed`: the masses in sorted order
+    int cleared = 0;                   // cell_offsets is zero already
+    unsigned long long* step = nullptr; // optional device step counter to advance; launch_scene_time() of the step has run
 };
 
 size_t scan_tile_count(uint64_t n);
@@ -195,7 +197,7 @@ cudaError_t launch_scan_density_lambda(cudaStream_t stream, const ListScanArgs& 
 cudaError_t launch_set_step(cudaStream_t stream, unsigned long long* step, uint64_t value);
 cudaError_t launch_advance_step(cudaStream_t stream, unsigned long long* step);
 cudaError_t launch_scene_time(cudaStream_t stream, const SceneStatic* statics, SceneDesc* scenes, const unsigned long long* step,
-                              uint32_t count);
+                              uint32_t count, uint32_t* clear = nullptr, uint64_t words = 0);   // also zeroes `words` words
 cudaError_t launch_constants(cudaStream_t stream, const float* support_radii, uint32_t n, KernelConstants* out);
 cudaError_t launch_density_lambda(cudaStream_t stream, const DensityLambdaArgs& a, unsigned block);
 cudaError_t launch_correction(cudaStream_t stream, const CorrectionArgs& a, unsigned block);

@@ -416,11 +416,10 @@ int SphEngine::forward(const pbf_particle_state* state, const sph_method_state* 
     }
     if (host_step_ != state->step_index) {
         if (int rc = check(launch_set_step(stream_, d_step_, state->step_index), "step counter")) return rc;
-        host_step_ = state->step_index;
     }
+    host_step_ = ~0ull;   // unknown again if the step fails halfway
     if (int rc = launch(stream_, state, method_state, control, parameters, next_state, next_method_state, r)) return rc;
     // the device counter then holds the index of the next state, as the host counter does
-    if (int rc = check(launch_advance_step(stream_, d_step_), "step counter")) return rc;
     host_step_ = state->step_index + 1u;
     next_state->step_index = state->step_index + 1u;
     r.valid = true;
@@ -431,7 +430,7 @@ int SphEngine::forward(const pbf_particle_state* state, const sph_method_state* 
 int SphEngine::launch(cudaStream_t s, const pbf_particle_state* state, const sph_method_state* method_state,
                       const pbf_control* control, const sph_parameters* parameters, pbf_particle_state* next_state,
                       sph_method_state* next_method_state, SphRecord& r) {
-    if (int rc = check(launch_scene_time(s, d_static_, d_scenes_, d_step_, 1), "scene table")) return rc;
+    if (int rc = check(launch_scene_time(s, d_static_, d_scenes_, d_step_, 1, r.cell_offsets, cells_ + 1), "scene table")) return rc;
     const sph_parameters& p = *parameters;
     const uint32_t method = config_.method;
     // params_a = (rest density, viscosity, surface tension, method 0), params_b = (method 1, method 2, 0)
@@ -468,6 +467,8 @@ int SphEngine::launch(cudaStream_t s, const pbf_particle_state* state, const sph
     g.sorted_velocity = r.velocity;
     g.packed = packed_;
     g.packed_mass = packed_mass_;
+    g.cleared = 1;
+    g.step = d_step_;
     if (int rc = check(launch_grid_build(s, g), "grid build")) return rc;
     if (boundary_count_ > 0) {
         BoundaryBuildArgs b{boundary_count_, cells_, d_scenes_, nullptr, boundary_rest_, boundary_velocity_, boundary_keys_,
