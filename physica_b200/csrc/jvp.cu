@@ -25,9 +25,9 @@ struct TangentWorkspace {
     float4* x[2] = {nullptr, nullptr};   // iterate position tangents (ping-pong), sorted
     float4* x_state = nullptr;           // position tangent of the input state, sorted
     float* lambda = nullptr;             // lambda tangent of the current iteration
-    float4* velocity = nullptr;          // reconstructed-velocity tangent
+    float4* records = nullptr;           // three a particle: PairRecord of the post-loop passes
+    float4* magnitudes = nullptr;        // two a particle: (position, |vorticity|), and their tangents
     float4* vorticity = nullptr;         // (vorticity tangent, magnitude tangent)
-    float4* confined = nullptr;          // confined-velocity tangent
     float4* params_a = nullptr;          // tangents of (mass, rest density, relaxation, xsph viscosity)
     float4* params_b = nullptr;          // tangents of (s_corr strength, exponent, radius, vorticity confinement)
 };
@@ -37,6 +37,30 @@ void destroy_tangent_workspace(void* workspace) { delete static_cast<TangentWork
 namespace {
 
 using namespace gather_detail;
+
+// A position and a velocity with their tangents, twelve floats in three 16-byte loads.  The post-loop
+// passes gather 30 neighbours a particle and are bound by the L1's load wavefronts (87-91 % of its peak
+// with a float4 array per field, four loads a neighbour; |vorticity| and its tangent beside position and
+// position tangent took four as well and now take two).  At 1M particles, ms before and now: vorticity
+// 0.269 -> 0.208, normal 0.227 -> 0.175, XSPH 0.261 -> 0.201.  The kernels before them write the records
+// with what else they write.
+struct PairRecord {
+    float4 a, b, c;
+    __device__ __forceinline__ f3 x() const { return mk(a.x, a.y, a.z); }
+    __device__ __forceinline__ f3 x_dot() const { return mk(a.w, b.x, b.y); }
+    __device__ __forceinline__ f3 v() const { return mk(b.z, b.w, c.x); }
+    __device__ __forceinline__ f3 v_dot() const { return mk(c.y, c.z, c.w); }
+};
+__device__ __forceinline__ PairRecord load_record(const float4* records, const uint32_t s) {
+    const float4* r = records + 3u * static_cast<size_t>(s);
+    return {r[0], r[1], r[2]};
+}
+__device__ __forceinline__ void store_record(float4* records, const uint32_t s, const f3 x, const f3 xd, const f3 v, const f3 vd) {
+    float4* r = records + 3u * static_cast<size_t>(s);
+    r[0] = make_float4(x.x, x.y, x.z, xd.x);
+    r[1] = make_float4(xd.y, xd.z, v.x, v.y);
+    r[2] = make_float4(v.z, vd.x, vd.y, vd.z);
+}
 
 inline unsigned blocks_of(const uint32_t n, const unsigned block) { return (n + block - 1) / block; }
 
@@ -225,7 +249,9 @@ struct CorrectionJvpArgs {
     int last;
     const uint32_t* sorted_index;
     const float4* x_state;
-    float4* velocity_dot;      // reconstructed-velocity tangent (last iteration)
+    const float4* final_pos;   // x_K and the reconstructed velocity (last iteration)
+    const float4* velocity;
+    float4* records;           // written in the last iteration
     MutField3 out_positions;   // next-state position tangent (last iteration)
 };
 
@@ -328,13 +354,14 @@ __global__ void __launch_bounds__(kBlock, 7) correction_jvp_kernel(const Correct
     a.out_positions.y[i] = next.y;
     a.out_positions.z[i] = next.z;
     const f3 v = times(next - xyz(a.x_state[p.s]), p.scene->inverse_time_step);
-    a.velocity_dot[p.s] = make_float4(v.x, v.y, v.z, 0.0F);
+    store_record(a.records, p.s, xyz(a.final_pos[p.s]), next, xyz(a.velocity[p.s]), v);
 }
 
 // Reconstruct JVP when no Jacobi iteration runs (K = 0).
 __global__ void tangent_reconstruct_kernel(const uint32_t count, const int4* __restrict__ cell, const SceneDesc* __restrict__ scenes,
                                            const uint32_t* __restrict__ sorted_index, const float4* __restrict__ x_dot,
-                                           const float4* __restrict__ x_state, float4* __restrict__ velocity_dot,
+                                           const float4* __restrict__ x_state, const float4* __restrict__ final_pos,
+                                           const float4* __restrict__ velocity, float4* __restrict__ records,
                                            const MutField3 out_positions) {
     after_predecessor();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -345,45 +372,37 @@ __global__ void tangent_reconstruct_kernel(const uint32_t count, const int4* __r
     out_positions.y[i] = xd.y;
     out_positions.z[i] = xd.z;
     const f3 v = times(xd - xyz(x_state[s]), scenes[cell[s].w].inverse_time_step);
-    velocity_dot[s] = make_float4(v.x, v.y, v.z, 0.0F);
+    store_record(records, s, xyz(final_pos[s]), xd, xyz(velocity[s]), v);
 }
 
 // -------------------------------------------------------------- vorticity
 struct VorticityJvpArgs {
     GatherCommon g;
     StoredList list;
-    const float4* pos;
-    const float4* x_dot;
-    const float4* velocity;
-    const float4* velocity_dot;
+    const float4* records;
     const float4* vorticity;
     float4* vorticity_dot;
+    float4* magnitudes;
 };
 
 struct VorticityJvpOp {
-    const float4* __restrict__ pos;
-    const float4* __restrict__ x_dot;
-    const float4* __restrict__ velocity;
-    const float4* __restrict__ velocity_dot;
+    const float4* __restrict__ records;
     f3 x, xd, v, vd;
     uint32_t self;
     KernelConstants k;
     f3 result;
 
-    struct Data {
-        float4 q, qd, w, wd;
-    };
-    __device__ __forceinline__ Data prefetch(const uint32_t t) const { return {pos[t], x_dot[t], velocity[t], velocity_dot[t]}; }
-    __device__ __forceinline__ void apply(const uint32_t t, const Data& in) {
+    __device__ __forceinline__ PairRecord prefetch(const uint32_t t) const { return load_record(records, t); }
+    __device__ __forceinline__ void apply(const uint32_t t, const PairRecord& in) {
         if (t == self) return;
-        const f3 d = x - xyz(in.q);
-        const f3 dd = xd - xyz(in.qd);
+        const f3 d = x - in.x();
+        const f3 dd = xd - in.x_dot();
         const float r2 = squared(d);
         if (r2 == 0.0F || r2 >= k.spiky_threshold) return;   // sqrtf(r2) == 0 or >= h
         f3 gradient, gradient_dot;
         spiky_pair(d, dd, r2, k, gradient, gradient_dot);
-        const f3 difference = xyz(in.w) - v;
-        const f3 difference_dot = xyz(in.wd) - vd;
+        const f3 difference = in.v() - v;
+        const f3 difference_dot = in.v_dot() - vd;
         result = result + cross(difference_dot, gradient) + cross(difference, gradient_dot);
     }
     __device__ __forceinline__ void process(const uint32_t t) { apply(t, prefetch(t)); }
@@ -394,42 +413,38 @@ __global__ void __launch_bounds__(kBlock, PBF_JVP_MIN_BLOCKS) vorticity_jvp_kern
     const Particle p = locate(a.g);
     if (!p.active) return;
     VorticityJvpOp op;
-    op.pos = a.pos;
-    op.x_dot = a.x_dot;
-    op.velocity = a.velocity;
-    op.velocity_dot = a.velocity_dot;
+    const PairRecord own = load_record(a.records, p.s);
+    op.records = a.records;
     op.self = p.s;
     op.k = p.k;
-    op.x = xyz(a.pos[p.s]);
-    op.xd = xyz(a.x_dot[p.s]);
-    op.v = xyz(a.velocity[p.s]);
-    op.vd = xyz(a.velocity_dot[p.s]);
+    op.x = own.x();
+    op.xd = own.x_dot();
+    op.v = own.v();
+    op.vd = own.v_dot();
     op.result = mk(0.0F, 0.0F, 0.0F);
     replay(op, p, a.g, a.list);
     const float4 w = a.vorticity[p.s];   // (omega, |omega|)
     const float magnitude_dot = w.w > 0.0F ? dot(xyz(w), op.result) / w.w : 0.0F;
     a.vorticity_dot[p.s] = make_float4(op.result.x, op.result.y, op.result.z, magnitude_dot);
+    a.magnitudes[2u * static_cast<size_t>(p.s)] = make_float4(op.x.x, op.x.y, op.x.z, w.w);
+    a.magnitudes[2u * static_cast<size_t>(p.s) + 1u] = make_float4(op.xd.x, op.xd.y, op.xd.z, magnitude_dot);
 }
 
 // ------------------------------------------------------ normal + confinement
 struct NormalJvpArgs {
     GatherCommon g;
     StoredList list;
-    const float4* pos;
-    const float4* x_dot;
+    const float4* magnitudes;
     const float4* vorticity;       // (omega, |omega|)
     const float4* vorticity_dot;   // (omega dot, |omega| dot)
     const float4* normal;          // (N, |eta|)
-    const float4* velocity_dot;
+    const float4* confined;
     const float4* params_b_dot;
-    float4* confined_dot;
+    float4* records;               // own record in: reconstructed velocity and tangent; out: confined ones
 };
 
 struct NormalJvpOp {
-    const float4* __restrict__ pos;
-    const float4* __restrict__ x_dot;
-    const float4* __restrict__ vorticity;
-    const float4* __restrict__ vorticity_dot;
+    const float4* __restrict__ magnitudes;
     f3 x, xd;
     float magnitude, magnitude_dot;
     uint32_t self;
@@ -437,11 +452,11 @@ struct NormalJvpOp {
     f3 result;
 
     struct Data {
-        float4 q, qd;
-        float m, md;
+        float4 q, qd;   // (position, |omega|) and their tangents
     };
     __device__ __forceinline__ Data prefetch(const uint32_t t) const {
-        return {pos[t], x_dot[t], vorticity[t].w, vorticity_dot[t].w};
+        const float4* m = magnitudes + 2u * static_cast<size_t>(t);
+        return {m[0], m[1]};
     }
     __device__ __forceinline__ void apply(const uint32_t t, const Data& in) {
         if (t == self) return;
@@ -451,7 +466,7 @@ struct NormalJvpOp {
         if (r2 == 0.0F || r2 >= k.spiky_threshold) return;   // sqrtf(r2) == 0 or >= h
         f3 gradient, gradient_dot;
         spiky_pair(d, dd, r2, k, gradient, gradient_dot);
-        result = result + times(gradient, in.md - magnitude_dot) + times(gradient_dot, in.m - magnitude);
+        result = result + times(gradient, in.qd.w - magnitude_dot) + times(gradient_dot, in.q.w - magnitude);
     }
     __device__ __forceinline__ void process(const uint32_t t) { apply(t, prefetch(t)); }
 };
@@ -461,14 +476,12 @@ __global__ void __launch_bounds__(kBlock, PBF_JVP_MIN_BLOCKS) normal_jvp_kernel(
     const Particle p = locate(a.g);
     if (!p.active) return;
     NormalJvpOp op;
-    op.pos = a.pos;
-    op.x_dot = a.x_dot;
-    op.vorticity = a.vorticity;
-    op.vorticity_dot = a.vorticity_dot;
+    const PairRecord own = load_record(a.records, p.s);
+    op.magnitudes = a.magnitudes;
     op.self = p.s;
     op.k = p.k;
-    op.x = xyz(a.pos[p.s]);
-    op.xd = xyz(a.x_dot[p.s]);
+    op.x = own.x();
+    op.xd = own.x_dot();
     const float4 w = a.vorticity[p.s], wd = a.vorticity_dot[p.s];
     op.magnitude = w.w;
     op.magnitude_dot = wd.w;
@@ -484,47 +497,38 @@ __global__ void __launch_bounds__(kBlock, PBF_JVP_MIN_BLOCKS) normal_jvp_kernel(
     const f3 force_dot = cross(normal_dot, omega) + cross(normal, omega_dot);
     const float dt = p.scene->time_step;
     const float eps = a.g.params_a[p.s].w, eps_dot = a.params_b_dot[p.s].w;
-    const f3 vc = xyz(a.velocity_dot[p.s]) + times(times(force, eps_dot) + times(force_dot, eps), dt);
-    a.confined_dot[p.s] = make_float4(vc.x, vc.y, vc.z, 0.0F);
+    const f3 vc = own.v_dot() + times(times(force, eps_dot) + times(force_dot, eps), dt);
+    store_record(a.records, p.s, op.x, op.xd, xyz(a.confined[p.s]), vc);
 }
 
 // ------------------------------------------------------------------- XSPH
 struct XsphJvpArgs {
     GatherCommon g;
     StoredList list;
-    const float4* pos;
-    const float4* x_dot;
-    const float4* confined;
-    const float4* confined_dot;
+    const float4* records;
     const float4* params_a_dot;
     const uint32_t* sorted_index;
     MutField3 out_velocities;
 };
 
 struct XsphJvpOp {
-    const float4* __restrict__ pos;
-    const float4* __restrict__ x_dot;
-    const float4* __restrict__ confined;
-    const float4* __restrict__ confined_dot;
+    const float4* __restrict__ records;
     f3 x, xd, v, vd;
     uint32_t self;
     KernelConstants k;
     f3 smoothing, smoothing_dot;
 
-    struct Data {
-        float4 q, qd, w, wd;
-    };
-    __device__ __forceinline__ Data prefetch(const uint32_t t) const { return {pos[t], x_dot[t], confined[t], confined_dot[t]}; }
-    __device__ __forceinline__ void apply(const uint32_t t, const Data& in) {
+    __device__ __forceinline__ PairRecord prefetch(const uint32_t t) const { return load_record(records, t); }
+    __device__ __forceinline__ void apply(const uint32_t t, const PairRecord& in) {
         if (t == self) return;
-        const f3 d = x - xyz(in.q);
+        const f3 d = x - in.x();
         const float r2 = squared(d);
         if (r2 >= k.h2) return;
-        const f3 dd = xd - xyz(in.qd);
+        const f3 dd = xd - in.x_dot();
         const float weight = poly6_weight(r2, k);
         const float weight_dot = dot(scale(d, poly6_gradient_scale(r2, k)), dd);
-        const f3 difference = xyz(in.w) - v;
-        const f3 difference_dot = xyz(in.wd) - vd;
+        const f3 difference = in.v() - v;
+        const f3 difference_dot = in.v_dot() - vd;
         smoothing = smoothing + times(difference, weight);
         smoothing_dot = smoothing_dot + times(difference_dot, weight) + times(difference, weight_dot);
     }
@@ -536,16 +540,14 @@ __global__ void __launch_bounds__(kBlock, PBF_JVP_MIN_BLOCKS) xsph_jvp_kernel(co
     const Particle p = locate(a.g);
     if (!p.active) return;
     XsphJvpOp op;
-    op.pos = a.pos;
-    op.x_dot = a.x_dot;
-    op.confined = a.confined;
-    op.confined_dot = a.confined_dot;
+    const PairRecord own = load_record(a.records, p.s);
+    op.records = a.records;
     op.self = p.s;
     op.k = p.k;
-    op.x = xyz(a.pos[p.s]);
-    op.xd = xyz(a.x_dot[p.s]);
-    op.v = xyz(a.confined[p.s]);
-    op.vd = xyz(a.confined_dot[p.s]);
+    op.x = own.x();
+    op.xd = own.x_dot();
+    op.v = own.v();
+    op.vd = own.v_dot();
     op.smoothing = mk(0.0F, 0.0F, 0.0F);
     op.smoothing_dot = mk(0.0F, 0.0F, 0.0F);
     replay(op, p, a.g, a.list);
@@ -592,9 +594,9 @@ int Engine::tangent(const pbf_particle_state* state, const StepRecord& r, const 
         ws->x[1] = ws->arena.alloc<float4>(n, e);
         ws->x_state = ws->arena.alloc<float4>(n, e);
         ws->lambda = ws->arena.alloc<float>(n, e);
-        ws->velocity = ws->arena.alloc<float4>(n, e);
+        ws->records = ws->arena.alloc<float4>(3u * static_cast<size_t>(n), e);
+        ws->magnitudes = ws->arena.alloc<float4>(2u * static_cast<size_t>(n), e);
         ws->vorticity = ws->arena.alloc<float4>(n, e);
-        ws->confined = ws->arena.alloc<float4>(n, e);
         ws->params_a = ws->arena.alloc<float4>(n, e);
         ws->params_b = ws->arena.alloc<float4>(n, e);
         if (e != cudaSuccess) {
@@ -624,7 +626,8 @@ int Engine::tangent(const pbf_particle_state* state, const StepRecord& r, const 
     launch_after(stream_, tangent_seed_kernel, blocks_of(n, 256), 256, n, r.sorted_index, r.cell, d_scenes_,
                  {state_tangent->positions.x, state_tangent->positions.y, state_tangent->positions.z},
                  {state_tangent->velocities.x, state_tangent->velocities.y, state_tangent->velocities.z},
-                 {control_tangent->external_accelerations.x, control_tangent->external_accelerations.y, control_tangent->external_accelerations.z},
+                 {control_tangent->external_accelerations.x, control_tangent->external_accelerations.y,
+                  control_tangent->external_accelerations.z},
                  pt, ws->x[0], ws->x_state, ws->params_a, ws->params_b);
     timer_.end(stream_, kPassTangentSeed);
     count_launch();
@@ -675,7 +678,8 @@ int Engine::tangent(const pbf_particle_state* state, const StepRecord& r, const 
             if (int rc = check(launch_correction(stream_, c, shape_.block), "recompute: correction/project")) return rc;
         }
         CorrectionJvpArgs ca{gc_reverse, list, xk, ws->x[k & 1u], lambda_k, ws->lambda, ws->params_a, ws->params_b, r.mask[k],
-                             ws->x[(k + 1u) & 1u], k + 1u == K ? 1 : 0, r.sorted_index, ws->x_state, ws->velocity, out_x};
+                             ws->x[(k + 1u) & 1u], k + 1u == K ? 1 : 0, r.sorted_index, ws->x_state,
+                             r.iterate(K, K, true), r.velocity, ws->records, out_x};
         timer_.begin(stream_, kPassCorrectionJvp);
         launch_after(stream_, correction_jvp_kernel, blocks, block, ca);
         timer_.end(stream_, kPassCorrectionJvp);
@@ -684,20 +688,19 @@ int Engine::tangent(const pbf_particle_state* state, const StepRecord& r, const 
     const float4* x_dot_K = ws->x[K & 1u];
     if (K == 0) {
         launch_after(stream_, tangent_reconstruct_kernel, blocks_of(n, 256), 256, n, r.cell, d_scenes_, r.sorted_index,
-                     x_dot_K, ws->x_state, ws->velocity, out_x);
+                     x_dot_K, ws->x_state, r.iterate(K, K, true), r.velocity, ws->records, out_x);
         count_launch();
     }
-    const float4* xK = r.iterate(K, K, true);
     const StoredList post{r.list_entries[keep ? K : 0u], r.list_counts[keep ? K : 0u], r.list_capacity};
-    VorticityJvpArgs va{gc, post, xK, x_dot_K, r.velocity, ws->velocity, r.vorticity, ws->vorticity};
+    VorticityJvpArgs va{gc, post, ws->records, r.vorticity, ws->vorticity, ws->magnitudes};
     timer_.begin(stream_, kPassVorticityJvp);
     launch_after(stream_, vorticity_jvp_kernel, blocks, block, va);
     timer_.end(stream_, kPassVorticityJvp);
-    NormalJvpArgs na{gc_reverse, post, xK, x_dot_K, r.vorticity, ws->vorticity, r.normal, ws->velocity, ws->params_b, ws->confined};
+    NormalJvpArgs na{gc_reverse, post, ws->magnitudes, r.vorticity, ws->vorticity, r.normal, r.confined, ws->params_b, ws->records};
     timer_.begin(stream_, kPassNormalJvp);
     launch_after(stream_, normal_jvp_kernel, blocks, block, na);
     timer_.end(stream_, kPassNormalJvp);
-    XsphJvpArgs xa{gc, post, xK, x_dot_K, r.confined, ws->confined, ws->params_a, r.sorted_index, out_v};
+    XsphJvpArgs xa{gc, post, ws->records, ws->params_a, r.sorted_index, out_v};
     timer_.begin(stream_, kPassXsphJvp);
     launch_after(stream_, xsph_jvp_kernel, blocks, block, xa);
     timer_.end(stream_, kPassXsphJvp);
