@@ -154,8 +154,8 @@ typedef struct pbf_batch pbf_batch;            /* many independent scenes in one
 typedef struct pbf_launch_shape {
     uint32_t list_scan;         /* 0: per-lane walk, 1: warp-cooperative scan, 2: shared-memory staged walk,
                                    3: per-lane walk with density + lambda in the same kernel,
-                                   4 (the default): as 3, and forward-mode steps without boundary
-                                   particles run over windows staged in shared memory */
+                                   4 (the default): as 3, and steps without boundary particles run over windows
+                                   staged in shared memory at the sizes where that is faster */
     uint32_t scan_block_size;   /* threads per block of the list scan: 32, 64, 96 or 128 */
     uint32_t block_size;        /* threads per block of the gather passes: 32, 64, 96 or 128 */
 } pbf_launch_shape;
@@ -341,8 +341,8 @@ int pbf_forward_step_preallocated(const pbf_domain_configuration* domain, const 
  *      candidates once, 2 = each lane walks its stencil in a shared-memory copy of its warp's
  *      stencil columns, 3 = as 0, and each Jacobi iteration's scan also computes density and lambda
  *      in the same kernel, replaying the list from shared memory (scenes with boundary particles run
- *      3 as 0), 4 = as 3, and every pass of a forward-mode step without boundary particles reads its
- *      neighbours from windows of the sorted particles staged in shared memory (the default);
+ *      3 as 0), 4 = as 3, and every pass of a step without boundary particles (of up to 20,480 or more than 170,496
+ *      particles; in differentiable mode of at least 2^19) reads its neighbours from windows of the sorted particles staged in shared memory (the default);
  *      scan_block_size and block_size: 32, 64, 96 or 128 threads (the staged passes have their own).
  *      pbf_autotune times the list-scan shapes 0, 1, 2 and 4 by their scans and gather passes, then the
  *      gather block sizes, on `repeats` forward steps from `state` (writing `scratch_state` and

@@ -144,10 +144,16 @@ namespace {
 // tangent step at 262k 1.54 ms against 1.55 with the fused per-lane scan, 590k 2.96 / 3.04, 1M 4.78 / 5.20;
 // gradient step at 64k 1.14 / 1.07, 262k 3.06 / 3.05, 590k 6.30 / 6.38.
 constexpr uint32_t kStagedDifferentiable = 1u << 19;
-// Up to this many particles one lane each leaves most of the GPU idle (a wave of the one-lane passes is
-// about 100k particles) and four are faster: a forward step at 5k particles 0.164 ms against 0.240, at 14k
-// 0.228 / 0.253, at 32k 0.31 / 0.285.  Two lanes never were the fastest (0.176, 0.253, 0.297).
+// Up to this many particles one lane each leaves most of the GPU idle, and the staged passes with four
+// lanes are the fastest: a forward step at 5k particles 0.164 ms against 0.240 with one lane, at 14k
+// 0.228 / 0.253.  Two lanes never were (0.176, 0.253).
 constexpr uint32_t kGroupedParticles = 20480;
+// Up to here all blocks of the per-lane passes are resident at once (nine of 128 threads on each of 148 SMs),
+// and loads they wait for overlap better than a block's staging, scan and replay, which all its blocks go
+// through at the same time, four to eight to an SM.  Above, the per-lane passes need a second wave.
+// Per lane / staged, ms a step: 22k particles 0.263 / 0.274, 64k 0.305 / 0.321, 110k 0.363 / 0.403, 169k
+// 0.488 / 0.530, 198k 0.634 / 0.548, 246k 0.715 / 0.649, 295k 0.803 / 0.725.
+constexpr uint32_t kOneWave = 9u * 148u * 128u;
 }  // namespace
 
 int Engine::init(const pbf_domain_configuration* scenes, const uint32_t scene_count, const pbf_configuration* configuration,
@@ -666,7 +672,8 @@ int Engine::record_positions_ready(cudaStream_t stream) {
 }
 
 bool Engine::runs_staged_passes(const LaunchShape& shape) const {
-    return runs_staged(shape, boundary_count_ > 0, iterations_) && (!differentiable() || count_ >= kStagedDifferentiable);
+    if (!runs_staged(shape, boundary_count_ > 0, iterations_)) return false;
+    return differentiable() ? count_ >= kStagedDifferentiable : count_ <= kGroupedParticles || count_ > kOneWave;
 }
 
 // The Jacobi iterations and the post-loop passes over staged windows (staged.cu, staged_group.cu): two

@@ -175,7 +175,7 @@ enum ListScanVariant : uint32_t {
     kScanFusedDensity = 3,  // per lane, and the Jacobi iterations' scans also run density + lambda
                             // in the same kernel (scenes without boundary particles)
     kScanStaged16 = 4,      // every forward pass of scenes without boundary particles over windows staged in
-                            // shared memory (staged.cu; differentiable steps of large scenes only); otherwise as 3
+                            // shared memory (staged.cu) at the sizes where that is faster; otherwise as 3
 };
 struct LaunchShape {
     uint32_t scan = kScanStaged16;   // fastest at every size measured (5k to 1M particles)

@@ -7,6 +7,10 @@
 // divisions, one pair at a time; from shared memory they take two pairs at a time with the packed
 // arithmetic of sph_math.cuh.  Lists carry a skin (sph.cu), so the packed values include the zeros
 // beyond the support.  Every sum keeps the reference's order and rounding.
+//
+// A DFSPH substep at 270k particles (ten pressure iterations) went from 1.378 to 1.104 ms, a WCSPH substep at
+// 1M, which uses the scan alone, from 0.665 to 0.634.  The force and non-pressure passes stay per lane: they
+// run once a substep.  What bounds the replays is the shared-memory pipe, as in the PBF passes.
 #include "dependent_launch.cuh"
 #include "sph_ops.cuh"
 #include "staged.cuh"

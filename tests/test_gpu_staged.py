@@ -44,13 +44,14 @@ def block(count, seed=1, iterations=3, **options):
     return dataclasses.replace(s, **{k: np.ascontiguousarray(v) for k, v in keep.items()})
 
 
-# four lanes per particle up to 20480 particles, blocks of 32; one lane above, blocks of 128
-@pytest.mark.parametrize("count", [1, 2, 31, 33, 127, 128, 129, 255, 257, 1000, 4097, 20480, 20481])
+# staged with four lanes per particle up to 20480 particles, blocks of 32; with one lane above 170496,
+# blocks of 128; the per-lane passes between
+@pytest.mark.parametrize("count", [1, 2, 31, 33, 127, 128, 129, 255, 257, 1000, 4097, 20480, 20481, 170496, 170497, 170625])
 def test_counts_around_the_block(count):
     check(block(count))
 
 
-@pytest.mark.parametrize("count", [8000, 40000])
+@pytest.mark.parametrize("count", [8000, 180000])
 def test_spray_whose_windows_exceed_the_stage(count):
     """Thin spray beside and above a dense block: its blocks' windows cover the block's columns."""
     s = block(count)
@@ -60,14 +61,14 @@ def test_spray_whose_windows_exceed_the_stage(count):
     check(s)
 
 
-@pytest.mark.parametrize("count", [3000, 24000])
+@pytest.mark.parametrize("count", [3000, 180000])
 def test_crowded_lists_overflow(count):
     s = block(count)
     s.positions[:, :3000] = (0.2 + 0.06 * np.random.default_rng(4).random((3, 3000))).astype(np.float32)
     check(s, steps=2)
 
 
-@pytest.mark.parametrize("count", [2000, 21000])
+@pytest.mark.parametrize("count", [2000, 180000])
 @pytest.mark.parametrize("strength", [0.0, 1e-5])
 def test_mixed_masses_and_coincident_particles(strength, count):
     s = block(count, seed=5)
@@ -81,7 +82,7 @@ def test_mixed_masses_and_coincident_particles(strength, count):
     check(s)
 
 
-@pytest.mark.parametrize("n", [9, 28])
+@pytest.mark.parametrize("n", [9, 56])
 @pytest.mark.parametrize("h", [0.0008, 0.003, 1.0, 3000.0])
 def test_support_radii_inside_and_outside_the_packed_range(h, n):
     """The packed pair arithmetic covers radii from 2^-10 to 2^10; others take the scalar path."""
@@ -90,7 +91,7 @@ def test_support_radii_inside_and_outside_the_packed_range(h, n):
     check(s, steps=2)
 
 
-@pytest.mark.parametrize("count", [4000, 21000])
+@pytest.mark.parametrize("count", [4000, 180000])
 def test_moving_box(count):
     """The sort cells and the gather cells of a moving box round differently."""
     s = dataclasses.replace(block(count, seed=8), box_velocity=(0.37, -0.11, 0.23))
@@ -132,8 +133,9 @@ def test_differentiable_steps_record_the_same_lists(kind, recompute):
         np.testing.assert_array_equal(a.cpu().numpy(), b.cpu().numpy())
 
 
-def test_batch_blocks_span_scenes():
-    parts = [scenes.batched_scene(c, 40 + k, 3, velocity_sigma=0.3) for k, c in enumerate((65, 700, 3, 1, 2049, 130))]
+@pytest.mark.parametrize("counts", [(65, 700, 3, 1, 2049, 130), (65, 90001, 3, 1, 2049, 80000)])
+def test_batch_blocks_span_scenes(counts):
+    parts = [scenes.batched_scene(c, 40 + k, 3, velocity_sigma=0.3) for k, c in enumerate(counts)]
     results = []
     for shape in (PER_LANE, STAGED):
         batch, state, control, params = pbf.batch_for_scenes(parts)
