@@ -151,6 +151,43 @@ def test_batched_jvp_equals_per_scene_jvp():
         assert np.array_equal(out.velocities[:, sl].cpu().numpy(), mv), s
 
 
+@pytest.mark.parametrize("moves", [False, True])
+@pytest.mark.parametrize("h", [1e-4, 1e-3])
+def test_tangents_of_close_pairs(h, moves):
+    """Isolated pairs a few 1e-6 h apart.  The tangent of a spiky gradient grows as 1 / (h^4 r), and a product with
+    one more power of 1 / r on the way would leave FP32.  The adjoint identity as above, its 1e-4 relative to
+    the sum of the terms' magnitudes.  `moves`: the first correction parts the pairs; otherwise a large
+    relaxation moves them by about 1e-6 h only, and the post-loop passes meet them too."""
+    sc = scenes.dam_break((2, 2, 4), (0, 0, 0), (6 * h, 6 * h, 6 * h), 46, 2, h=h, gravity=(0.0, 0.0, 0.0))
+    rng = np.random.default_rng(47)
+    centre = np.stack(np.meshgrid([1.4 * h, 4.6 * h], [1.3 * h, 4.5 * h], [1.5 * h, 4.4 * h], indexing="ij")).reshape(3, 8)
+    offset = rng.normal(size=(3, 8))
+    offset *= 2.5e-6 * h / np.linalg.norm(offset, axis=0)
+    sc.positions[:, :8], sc.positions[:, 8:] = centre.astype(np.float32), (centre + offset).astype(np.float32)
+    apart = np.linalg.norm(sc.positions[:, 8:].astype(np.float64) - sc.positions[:, :8], axis=0)
+    assert apart.min() > 1e-6 * h and apart.max() < 1e-5 * h
+    sc.rest_densities[:] = 100.0
+    sc.relaxation[:] = 1000.0 if moves else 1e8 / h ** 2
+    t, pt = _tangents(sc, 4)
+    t["positions"] *= h / 0.025
+    mx, mv = my_jvp(sc, t, pt)
+    assert np.isfinite(mx).all() and np.isfinite(mv).all()
+    wx, wv = rng.normal(size=(3, sc.count)), rng.normal(size=(3, sc.count))
+    solver, state, control, params = pbf.solver_for_scene(sc, mode=pbf.ExecutionMode.differentiable)
+    cache, nxt = solver.allocate_step_cache(), solver.allocate_state()
+    solver.forward_step(state, control, params, nxt, cache)
+    pa, ca, qa = solver.allocate_state_adjoint(), solver.allocate_control_adjoint(), solver.allocate_parameter_adjoint()
+    solver.vjp_step(state, control, params, nxt, cache, pbf.StateAdjoint(torch.from_numpy(wx).cuda(), torch.from_numpy(wv).cuda()),
+                    pa, ca, qa)
+    torch.cuda.synchronize()
+    left = np.concatenate([(wx * mx).ravel(), (wv * mv).ravel()])
+    right = [pa.positions.cpu().numpy() * t["positions"], pa.velocities.cpu().numpy() * t["velocities"],
+             ca.external_accelerations.cpu().numpy() * t["control"], *[qa.tensors[k].cpu().numpy() * pt[k] for k in NAMES]]
+    right = np.concatenate([r.ravel() for r in right])
+    scale = max(np.abs(left).sum(), np.abs(right).sum())
+    assert abs(left.sum() - right.sum()) <= 1e-4 * scale, (left.sum(), right.sum(), scale)
+
+
 def test_jvp_needs_a_differentiable_solver():
     sc = _scene((4, 4, 4), 44)
     solver, state, control, params = pbf.solver_for_scene(sc)
