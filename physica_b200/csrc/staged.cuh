@@ -160,7 +160,9 @@ __device__ __forceinline__ Hits scan(const Windows& w, const Particle& p, const 
         const uint32_t a = start + (first - base), b = start + (end - base);
         const uint32_t begin = a & ~3u;
         hits.covered = hits.covered && b - begin <= kColumn;
-        uint32_t self = o == 4 ? start + (p.s - base) - begin : ~0u;   // the particle's place in its own column
+        // the particle's place, in the column that holds its slot: its sort cell's, which is not always its
+        // gather cell's column (the two cell formulas round differently)
+        uint32_t self = p.s - first < end - first ? start + (p.s - base) - begin : ~0u;
         auto test_block = [&](const uint32_t block, const uint32_t stop, const uint32_t valid) -> uint32_t {
             uint32_t mask = 0u, k = block;
             for (; k < stop; k += 4u) {

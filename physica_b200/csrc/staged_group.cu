@@ -112,8 +112,7 @@ __device__ __forceinline__ uint32_t group_scan(Windows& w, const StagedList& lis
                                                float (*shared)[kGroupStage], const f3 xi, ColumnHits (*columns)[kThreads],
                                                uint16_t (*entries)[kGroupList], uint32_t& before) {
     Hits hits{0u, 0u, ~0u, true, true};
-    // Columns 0..2, 3..4, 5..6, 7..8; lane 1 has the particle's own (4).
-    constexpr int own = 1;
+    // Columns 0..2, 3..4, 5..6, 7..8.
     const int from = m.lane == 0u ? 0 : 2 * static_cast<int>(m.lane) + 1;
     const int to = 2 * static_cast<int>(m.lane) + 3;
     if (w.staged) {
@@ -131,7 +130,7 @@ __device__ __forceinline__ uint32_t group_scan(Windows& w, const StagedList& lis
     }
     const uint32_t first = end - hits.count;
     const uint32_t n = __shfl_sync(kFull, end, L - 1u, L);
-    before = __shfl_sync(kFull, hits.before == ~0u ? ~0u : first + hits.before, own, L);
+    before = __reduce_min_sync(group_mask(), hits.before == ~0u ? ~0u : first + hits.before);   // one lane found it
     const bool fits = __reduce_min_sync(group_mask(), hits.covered ? 1u : 0u) != 0u && n < kGroupList;
     if (fits && hits.count > 0u) {
         HitCursor cursor(w, columns);

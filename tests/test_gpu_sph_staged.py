@@ -7,6 +7,7 @@ import pytest
 import torch
 
 from physica_b200 import pbf, scenes, sph
+from test_gpu_staged import straddled
 
 pytestmark = pytest.mark.gpu
 
@@ -25,8 +26,9 @@ def block(count, method, seed=1, h_scale=1.0, sigma=0.3):
     return s
 
 
-def run(scene, method, scan, steps, mode=pbf.ExecutionMode.forward):
+def run(scene, method, scan, steps, mode=pbf.ExecutionMode.forward, first_step=0):
     solver, state, control, params = sph.solver_for_scene(scene, sph.Method[method], mode=mode)
+    state.step_index = first_step
     solver.launch_shape = pbf.LaunchShape(scan, 128, 128)
     cache, following = solver.allocate_step_cache(), solver.allocate_state()
     out = []
@@ -93,3 +95,14 @@ def test_support_radii_outside_the_packed_range(h_scale):
 @pytest.mark.parametrize("method", METHODS)
 def test_differentiable_steps(method):
     check(block(2500, method, seed=8), method, steps=2, mode=pbf.ExecutionMode.differentiable)
+
+
+@pytest.mark.parametrize("method", METHODS)
+def test_sort_cell_and_gather_cell_differ(method):
+    """As in test_gpu_staged.py: particles of a moving box that are sorted into another column than their own."""
+    low = (37.0, -21.0, 0.0)
+    s = scenes.dam_break((36, 36, 4), low, (low[0] + 6.0, low[1] + 6.0, 0.06), 8, 0, dt=scenes.SPH_DT)
+    s = dataclasses.replace(s, box_velocity=(0.37, -0.11, 0.0))
+    assert straddled(s, 41, s.count // 8, 9) > s.count // 100
+    s.sph = scenes.sph_parameter_arrays(s, method=method)
+    check(s, method, steps=1, first_step=41)

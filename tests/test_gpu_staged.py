@@ -98,6 +98,46 @@ def test_moving_box(count):
     check(s, steps=6)
 
 
+def fma32(a, b, c):
+    """float32 fma(a, b, c): the product is exact in float64."""
+    return np.float32(np.float64(a) * np.float64(b) + np.float64(c))
+
+
+def straddled(s, step, per_axis, seed):
+    """Moves `per_axis` particles of the resting scene `s` an axis in x and y onto the floats beside their nearest cell
+    boundary at the time of `step`, and counts, as grid.cu evaluates them, those whose sort cell and gather cell
+    there differ."""
+    rng = np.random.default_rng(seed)
+    h, time = np.float32(s.support_radius), np.float32(np.float32(step) * np.float32(s.time_step))
+    differ = 0
+    for axis in (0, 1):
+        low, speed = np.float32(s.box_min[axis]), np.float32(s.box_velocity[axis])
+        origin = fma32(time, speed, low)
+        x = s.positions[axis]
+        move = rng.permutation(s.count)[:per_axis]
+        k = np.rint((x[move].astype(np.float64) - origin) / h)
+        y = (np.float64(origin) + k * np.float64(h)).astype(np.float32)
+        side = rng.integers(-1, 2, per_axis)
+        y = np.where(side < 0, np.nextafter(y, np.float32(-1e9)), np.where(side > 0, np.nextafter(y, np.float32(1e9)), y))
+        x[move] = y
+        sort_cell = np.floor(fma32(-time, speed, (y - low).astype(np.float32)).astype(np.float32) / h)
+        gather_cell = np.floor((y - origin).astype(np.float32) / h)
+        differ += int((sort_cell != gather_cell).sum())
+    return differ
+
+
+@pytest.mark.parametrize("lattice,box_z", [((36, 36, 4), 0.06), ((210, 210, 4), 0.06), ((36, 36, 14), 0.2)])
+def test_sort_cell_and_gather_cell_differ(lattice, box_z):
+    """In a moving box the two cell formulas round differently; a particle on a cell boundary is then sorted into another
+    stencil column than its own.  The grid has few cells in z, so that a block's windows still cover that column:
+    the particle must find itself there (neighbour counts leave it out)."""
+    low = (37.0, -21.0, 0.0)
+    s = scenes.dam_break(lattice, low, (low[0] + 6.0, low[1] + 6.0, box_z), 8, 2, gravity=(0.0, 0.0, 0.0))
+    s = dataclasses.replace(s, box_velocity=(0.37, -0.11, 0.0))
+    assert straddled(s, 1, s.count // 8, 9) > s.count // 100
+    check(s, steps=1)
+
+
 @pytest.mark.parametrize("recompute", [False, True])
 @pytest.mark.parametrize("kind", ["block", "spray", "crowded"])
 def test_differentiable_steps_record_the_same_lists(kind, recompute):
