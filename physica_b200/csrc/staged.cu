@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kBlockParticles, 6) staged_density_kernel(cons
         const float ratio = __fdiv_rn(mass, pa.x);
         replay_hits<true, Slots>(w, list, a.slots, s, hits, columns,
                                  [&](const uint32_t i0, const uint32_t i1, const bool second, const uint32_t k) {
-            const float m0 = field[3][i0], m1 = field[3][i1];
+            float m0 = field[3][i0], m1 = field[3][i1];
             const TwoPairs t = two_pairs(xi, mk(field[0][i0], field[1][i0], field[2][i0]),
                                          mk(field[0][i1], field[1][i1], field[2][i1]));
             float2 weight = poly6_pair(t.nr2, p.k), spiky = spiky_scale_pair(t.nr2, p.k);
@@ -76,6 +76,11 @@ __global__ void __launch_bounds__(kBlockParticles, 6) staged_density_kernel(cons
                 if (!in_range(t.nr2, p.k)) {
                     weight = any_poly6s(t.nr2, p.k);
                     spiky = any_spiky_scales(t.nr2, p.k);
+                    // no kernel: no term, whatever the factors are
+                    if (spiky.x == 0.0F) c0 = 0.0F;
+                    if (spiky.y == 0.0F) c1 = 0.0F;
+                    if (-t.nr2.x >= p.k.h2) m0 = 0.0F;
+                    if (-t.nr2.y >= p.k.h2) m1 = 0.0F;
                     neighbors -= -t.nr2.x >= p.k.h2 ? 1u : 0u;
                     neighbors -= second && -t.nr2.y >= p.k.h2 ? 1u : 0u;
                 }
@@ -175,11 +180,15 @@ __global__ void __launch_bounds__(kBlockParticles, 4) staged_vorticity_kernel(co
                                  [&](const uint32_t i0, const uint32_t i1, const bool second, uint32_t) {
             const TwoPairs t = two_pairs(xi, mk(field[0][i0], field[1][i0], field[2][i0]),
                                          mk(field[0][i1], field[1][i1], field[2][i1]));
-            const f3 v0 = mk(field[3][i0], field[4][i0], field[5][i0]), v1 = mk(field[3][i1], field[4][i1], field[5][i1]);
+            f3 v0 = sub(mk(field[3][i0], field[4][i0], field[5][i0]), vi);
+            f3 v1 = sub(mk(field[3][i1], field[4][i1], field[5][i1]), vi);
             float2 spiky = spiky_scale_pair(t.nr2, p.k);
-            if (!in_range(t.nr2, p.k)) spiky = any_spiky_scales(t.nr2, p.k);
-            vorticity = add(vorticity, cross_f(sub(v0, vi), scale(t.d0, spiky.x)));
-            if (second) vorticity = add(vorticity, cross_f(sub(v1, vi), scale(t.d1, spiky.y)));
+            if (!in_range(t.nr2, p.k)) {
+                spiky = any_spiky_scales(t.nr2, p.k);
+                only_inside(spiky, v0, v1);
+            }
+            vorticity = add(vorticity, cross_f(v0, scale(t.d0, spiky.x)));
+            if (second) vorticity = add(vorticity, cross_f(v1, scale(t.d1, spiky.y)));
         });
     } else {
         VorticityOp op;
@@ -219,10 +228,14 @@ __global__ void __launch_bounds__(kBlockParticles, 8) staged_normal_kernel(const
         replay_words(list, s, entries_of(n), [&](const uint32_t i0, const uint32_t i1, const bool second) {
             const TwoPairs t = two_pairs(xi, mk(field[0][i0], field[1][i0], field[2][i0]),
                                          mk(field[0][i1], field[1][i1], field[2][i1]));
+            float f0 = __fsub_rn(field[3][i0], wi.w), f1 = __fsub_rn(field[3][i1], wi.w);
             float2 spiky = spiky_scale_pair(t.nr2, p.k);
-            if (!in_range(t.nr2, p.k)) spiky = any_spiky_scales(t.nr2, p.k);
-            gradient = fma3(__fsub_rn(field[3][i0], wi.w), scale(t.d0, spiky.x), gradient);
-            if (second) gradient = fma3(__fsub_rn(field[3][i1], wi.w), scale(t.d1, spiky.y), gradient);
+            if (!in_range(t.nr2, p.k)) {
+                spiky = any_spiky_scales(t.nr2, p.k);
+                only_inside(spiky, f0, f1);
+            }
+            gradient = fma3(f0, scale(t.d0, spiky.x), gradient);
+            if (second) gradient = fma3(f1, scale(t.d1, spiky.y), gradient);
         });
     } else {
         gradient = normal_alone(a, p, xi, wi.w);
@@ -251,11 +264,15 @@ __global__ void __launch_bounds__(kBlockParticles, 5) staged_xsph_kernel(const S
         replay_words(list, s, entries_of(n), [&](const uint32_t i0, const uint32_t i1, const bool second) {
             const TwoPairs t = two_pairs(xi, mk(field[0][i0], field[1][i0], field[2][i0]),
                                          mk(field[0][i1], field[1][i1], field[2][i1]));
-            const f3 v0 = mk(field[3][i0], field[4][i0], field[5][i0]), v1 = mk(field[3][i1], field[4][i1], field[5][i1]);
+            f3 v0 = sub(mk(field[3][i0], field[4][i0], field[5][i0]), vi);
+            f3 v1 = sub(mk(field[3][i1], field[4][i1], field[5][i1]), vi);
             float2 weight = poly6_pair(t.nr2, p.k);
-            if (!in_range(t.nr2, p.k)) weight = any_poly6s(t.nr2, p.k);
-            smoothing = fma3(weight.x, sub(v0, vi), smoothing);
-            if (second) smoothing = fma3(weight.y, sub(v1, vi), smoothing);
+            if (!in_range(t.nr2, p.k)) {
+                weight = any_poly6s(t.nr2, p.k);
+                only_inside(weight, v0, v1);
+            }
+            smoothing = fma3(weight.x, v0, smoothing);
+            if (second) smoothing = fma3(weight.y, v1, smoothing);
         });
     } else {
         smoothing = xsph_alone(a, p, xi, vi);

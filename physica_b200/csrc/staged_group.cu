@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kThreads) group_density_kernel(const StagedDen
     group_replay<5>(scratch.exchange[m.local], m.lane, n, sums,
         [&](const uint32_t j) { return reinterpret_cast<const uint32_t*>(entries[m.local])[j]; },
         [&](const uint32_t i0, const uint32_t i1, float2 (&t0)[5], float2 (&t1)[5]) {
-            const float m0 = field[3][i0], m1 = field[3][i1];
+            float m0 = field[3][i0], m1 = field[3][i1];
             const TwoPairs t = two_pairs(xi, mk(field[0][i0], field[1][i0], field[2][i0]),
                                          mk(field[0][i1], field[1][i1], field[2][i1]));
             float2 weight = poly6_pair(t.nr2, p.k), spiky = spiky_scale_pair(t.nr2, p.k);
@@ -197,6 +197,11 @@ __global__ void __launch_bounds__(kThreads) group_density_kernel(const StagedDen
                 if (!in_range(t.nr2, p.k)) {
                     weight = any_poly6s(t.nr2, p.k);
                     spiky = any_spiky_scales(t.nr2, p.k);
+                    // no kernel: no term, whatever the factors are
+                    if (spiky.x == 0.0F) c0 = 0.0F;
+                    if (spiky.y == 0.0F) c1 = 0.0F;
+                    if (-t.nr2.x >= p.k.h2) m0 = 0.0F;
+                    if (-t.nr2.y >= p.k.h2) m1 = 0.0F;
                     misses += -t.nr2.x >= p.k.h2 ? 1u : 0u;
                     misses += i1 != i0 && -t.nr2.y >= p.k.h2 ? 1u : 0u;   // i1 = i0: a last odd entry repeated
                 }
@@ -316,10 +321,15 @@ __global__ void __launch_bounds__(kThreads) group_vorticity_kernel(const StagedV
         [&](const uint32_t i0, const uint32_t i1, float2 (&t0)[3], float2 (&t1)[3]) {
             const TwoPairs t = two_pairs(xi, mk(field[0][i0], field[1][i0], field[2][i0]),
                                          mk(field[0][i1], field[1][i1], field[2][i1]));
+            f3 v0 = sub(mk(field[3][i0], field[4][i0], field[5][i0]), vi);
+            f3 v1 = sub(mk(field[3][i1], field[4][i1], field[5][i1]), vi);
             float2 spiky = spiky_scale_pair(t.nr2, p.k);
-            if (!in_range(t.nr2, p.k)) spiky = any_spiky_scales(t.nr2, p.k);
-            const f3 c0 = cross_f(sub(mk(field[3][i0], field[4][i0], field[5][i0]), vi), scale(t.d0, spiky.x));
-            const f3 c1 = cross_f(sub(mk(field[3][i1], field[4][i1], field[5][i1]), vi), scale(t.d1, spiky.y));
+            if (!in_range(t.nr2, p.k)) {
+                spiky = any_spiky_scales(t.nr2, p.k);
+                only_inside(spiky, v0, v1);
+            }
+            const f3 c0 = cross_f(v0, scale(t.d0, spiky.x));
+            const f3 c1 = cross_f(v1, scale(t.d1, spiky.y));
             t0[0] = make_float2(0.0F, c0.x);
             t0[1] = make_float2(0.0F, c0.y);
             t0[2] = make_float2(0.0F, c0.z);
@@ -370,9 +380,12 @@ __global__ void __launch_bounds__(kThreads) group_normal_kernel(const StagedNorm
         [&](const uint32_t i0, const uint32_t i1, float2 (&t0)[3], float2 (&t1)[3]) {
             const TwoPairs t = two_pairs(xi, mk(field[0][i0], field[1][i0], field[2][i0]),
                                          mk(field[0][i1], field[1][i1], field[2][i1]));
+            float f0 = __fsub_rn(field[3][i0], wi.w), f1 = __fsub_rn(field[3][i1], wi.w);
             float2 spiky = spiky_scale_pair(t.nr2, p.k);
-            if (!in_range(t.nr2, p.k)) spiky = any_spiky_scales(t.nr2, p.k);
-            const float f0 = __fsub_rn(field[3][i0], wi.w), f1 = __fsub_rn(field[3][i1], wi.w);
+            if (!in_range(t.nr2, p.k)) {
+                spiky = any_spiky_scales(t.nr2, p.k);
+                only_inside(spiky, f0, f1);
+            }
             const f3 g0 = scale(t.d0, spiky.x), g1 = scale(t.d1, spiky.y);
             t0[0] = make_float2(f0, g0.x);
             t0[1] = make_float2(f0, g0.y);
@@ -411,10 +424,13 @@ __global__ void __launch_bounds__(kThreads) group_xsph_kernel(const StagedXsphAr
         [&](const uint32_t i0, const uint32_t i1, float2 (&t0)[3], float2 (&t1)[3]) {
             const TwoPairs t = two_pairs(xi, mk(field[0][i0], field[1][i0], field[2][i0]),
                                          mk(field[0][i1], field[1][i1], field[2][i1]));
+            f3 v0 = sub(mk(field[3][i0], field[4][i0], field[5][i0]), vi);
+            f3 v1 = sub(mk(field[3][i1], field[4][i1], field[5][i1]), vi);
             float2 weight = poly6_pair(t.nr2, p.k);
-            if (!in_range(t.nr2, p.k)) weight = any_poly6s(t.nr2, p.k);
-            const f3 v0 = sub(mk(field[3][i0], field[4][i0], field[5][i0]), vi);
-            const f3 v1 = sub(mk(field[3][i1], field[4][i1], field[5][i1]), vi);
+            if (!in_range(t.nr2, p.k)) {
+                weight = any_poly6s(t.nr2, p.k);
+                only_inside(weight, v0, v1);
+            }
             t0[0] = make_float2(weight.x, v0.x);
             t0[1] = make_float2(weight.x, v0.y);
             t0[2] = make_float2(weight.x, v0.z);

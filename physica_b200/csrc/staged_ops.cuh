@@ -41,6 +41,16 @@ __device__ __forceinline__ float2 any_poly6s(const float2 nr2, const KernelConst
     return make_float2(any_poly6(-nr2.x, k.h2, k.poly6_denominator), any_poly6(-nr2.y, k.h2, k.poly6_denominator));
 }
 
+// A pair whose kernel value is zero adds nothing, whatever its other factor is (it may be infinite).
+__device__ __forceinline__ void only_inside(const float2 kernel, float& f0, float& f1) {
+    if (kernel.x == 0.0F) f0 = 0.0F;
+    if (kernel.y == 0.0F) f1 = 0.0F;
+}
+__device__ __forceinline__ void only_inside(const float2 kernel, f3& f0, f3& f1) {
+    if (kernel.x == 0.0F) f0 = mk(0.0F, 0.0F, 0.0F);
+    if (kernel.y == 0.0F) f1 = mk(0.0F, 0.0F, 0.0F);
+}
+
 // The factors of two correction terms and the scales of their gradients.
 struct PairFactors {
     TwoPairs t;
@@ -75,8 +85,8 @@ __device__ __forceinline__ PairFactors correction_factors(const KernelConstants&
                 a0 = -t.nr2.x < k.h2 ? a0 : 0.0F;
                 a1 = -t.nr2.y < k.h2 ? a1 : 0.0F;
             }
-            if (spiky.x == 0.0F) s0 = a0 = 0.0F;   // no gradient: no term, whatever lambda is
-            if (spiky.y == 0.0F) s1 = a1 = 0.0F;
+            if (spiky.x == 0.0F) c0 = s0 = a0 = 0.0F;   // no gradient: no term, whatever the factors are
+            if (spiky.y == 0.0F) c1 = s1 = a1 = 0.0F;
         }
     }
     const float f0 = __fmul_rn(c0, __fadd_rn(s0, a0));

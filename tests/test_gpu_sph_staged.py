@@ -26,9 +26,12 @@ def block(count, method, seed=1, h_scale=1.0, sigma=0.3):
     return s
 
 
-def run(scene, method, scan, steps, mode=pbf.ExecutionMode.forward, first_step=0):
+def run(scene, method, scan, steps, mode=pbf.ExecutionMode.forward, first_step=0, warm=None):
     solver, state, control, params = sph.solver_for_scene(scene, sph.Method[method], mode=mode)
     state.step_index = first_step
+    if warm is not None:
+        state.warm_divergence_pressure.copy_(torch.from_numpy(warm))
+        state.warm_density_pressure.copy_(torch.from_numpy(warm))
     solver.launch_shape = pbf.LaunchShape(scan, 128, 128)
     cache, following = solver.allocate_step_cache(), solver.allocate_state()
     out = []
@@ -106,3 +109,13 @@ def test_sort_cell_and_gather_cell_differ(method):
     assert straddled(s, 41, s.count // 8, 9) > s.count // 100
     s.sph = scenes.sph_parameter_arrays(s, method=method)
     check(s, method, steps=1, first_step=41)
+
+
+@pytest.mark.parametrize("method", METHODS)
+def test_values_that_are_not_finite(method):
+    """Pairs in the lists' skin, beyond the support, add nothing: neither an infinite mass nor an infinite pressure."""
+    s = block(4000, method, seed=9)
+    s.sph["masses"][[500, 1500]] = np.inf
+    warm = np.full(4000, 10.0, np.float32)
+    warm[[2500, 3500]] = np.inf, np.nan
+    check(s, method, steps=1, **({"warm": warm} if method == "dfsph" else {}))

@@ -138,6 +138,20 @@ def test_sort_cell_and_gather_cell_differ(lattice, box_z):
     check(s, steps=1)
 
 
+@pytest.mark.parametrize("count", [40, 4000, 180000])
+def test_values_that_are_not_finite(count):
+    """Pairs without a kernel term (coincident particles here) add nothing, whatever else they hold: an infinite mass,
+    the infinite velocity of a particle that came from infinity."""
+    s = block(count, seed=12)
+    for i in (10, 20):
+        s.positions[:, i + 1], s.velocities[:, i + 1] = s.positions[:, i], s.velocities[:, i]
+    s.masses[10] = np.inf
+    s.positions[1, 30:32], s.velocities[:, 30:32] = np.inf, 0.0      # clamped to the top of the box
+    s.positions[::2, 31] = s.positions[::2, 30]
+    for a, b in zip(run(s, PER_LANE, 1), run(s, STAGED, 1)):
+        np.testing.assert_array_equal(a, b)
+
+
 @pytest.mark.parametrize("recompute", [False, True])
 @pytest.mark.parametrize("kind", ["block", "spray", "crowded"])
 def test_differentiable_steps_record_the_same_lists(kind, recompute):
