@@ -233,12 +233,16 @@ int Engine::init(const pbf_domain_configuration* scenes, const uint32_t scene_co
     packed_ = alloc_packed(arena_, count_, e);
     bool boundary = false;
     for (uint32_t s = 0; s < scene_count; ++s) boundary = boundary || scenes[s].boundary_particle_count > 0;
-    if (!boundary && (mode == PBF_EXECUTION_FORWARD || count_ >= kStagedDifferentiable)) {
+    if (!boundary && may_run_staged(LaunchShape{})) {
         packed_next_ = alloc_packed(arena_, count_, e);
         packed_velocity_ = alloc_packed(arena_, count_, e);
         packed_mass_ = arena_.alloc<float>(static_cast<size_t>(count_) + 4u, e);
         packed_magnitude_ = arena_.alloc<float>(static_cast<size_t>(count_) + 4u, e);
         staged_list_.windows = arena_.alloc<uint32_t>(window_words(count_), e);
+        if (e == cudaSuccess)
+            e = fit_.init(arena_, stream_,
+                          mode == PBF_EXECUTION_DIFFERENTIABLE ? StagedFit::kDifferentiable
+                                                               : count_ <= kGroupedParticles ? StagedFit::kGrouped : StagedFit::kForward);
         if (mode == PBF_EXECUTION_DIFFERENTIABLE) {
             const size_t padded = (static_cast<size_t>(count_) + 31u) / 32u * 32u;
             staged_list_.list = {arena_.alloc<uint32_t>(padded * kListCapacity, e), arena_.alloc<uint32_t>(count_, e), kListCapacity};
@@ -342,7 +346,7 @@ int Engine::init(const pbf_domain_configuration* scenes, const uint32_t scene_co
 }
 
 bool Engine::GraphKey::operator==(const GraphKey& o) const {
-    if (record != o.record || positions_ready != o.positions_ready) return false;
+    if (record != o.record || positions_ready != o.positions_ready || staged != o.staged) return false;
     for (int k = 0; k < 16; ++k)
         if (p[k] != o.p[k]) return false;
     return true;
@@ -455,8 +459,10 @@ int Engine::forward(const pbf_particle_state* state, const pbf_control* control,
     }
     host_step_ = ~0ull;   // unknown again if the step fails halfway
     int rc = PBF_SUCCESS;
+    staged_step_ = may_run_staged(shape_) && fit_.pays();
     if (graphs_ && !timer_.enabled()) {
         GraphKey key{};
+        key.staged = staged_step_;
         const void* ptrs[16] = {state->positions.x, state->positions.y, state->positions.z, state->velocities.x,
                                 state->velocities.y, state->velocities.z, control->external_accelerations.x,
                                 control->external_accelerations.y, control->external_accelerations.z, parameters->masses,
@@ -518,7 +524,7 @@ int Engine::forward(const pbf_particle_state* state, const pbf_control* control,
     next_state->step_index = state->step_index + 1u;
     r.valid = true;
     r.step_index = state->step_index;
-    return PBF_SUCCESS;
+    return may_run_staged(shape_) ? check(fit_.measure(stream_, gather_common(r)), "staged fit") : PBF_SUCCESS;
 }
 
 int Engine::read_input_checks(uint32_t* flags) {
@@ -586,9 +592,7 @@ int Engine::launch_forward(cudaStream_t stream, const pbf_particle_state* state,
     }
     timer_.end(stream, kPassGrid);
 
-    if (runs_staged_passes(shape_)) {
-        return launch_staged(stream, state, next_state, r);
-    }
+    if (staged_step_) return launch_staged(stream, state, next_state, r);
     const GatherCommon gc = gather_common(r);
     const Field3 previous{state->positions.x, state->positions.y, state->positions.z};
     const MutField3 out_positions{next_state->positions.x, next_state->positions.y, next_state->positions.z};
@@ -671,9 +675,10 @@ int Engine::record_positions_ready(cudaStream_t stream) {
     return check(cudaEventRecordWithFlags(positions_ready_, stream, flags), "positions event");
 }
 
-bool Engine::runs_staged_passes(const LaunchShape& shape) const {
+bool Engine::may_run_staged(const LaunchShape& shape) const {
     if (!runs_staged(shape, boundary_count_ > 0, iterations_)) return false;
-    return differentiable() ? count_ >= kStagedDifferentiable : count_ <= kGroupedParticles || count_ > kOneWave;
+    if (differentiable()) return count_ >= kStagedDifferentiable;
+    return count_ <= kGroupedParticles || count_ > kOneWave;
 }
 
 // The Jacobi iterations and the post-loop passes over staged windows (staged.cu, staged_group.cu): two
@@ -840,7 +845,7 @@ int Engine::autotune(const pbf_particle_state* state, const pbf_control* control
     int rc = PBF_SUCCESS;
     // 1. the list scan: variant x block size, by the time of the scans and the gather passes (the
     //    variants differ in which passes they fuse).  The staged passes have a block size of their own.
-    const bool staged = runs_staged_passes(LaunchShape{kScanStaged16, 128u, 128u});
+    const bool staged = may_run_staged(LaunchShape{kScanStaged16, 128u, 128u});
     LaunchShape best = previous;
     best.block = 128u;
     double best_scan = -1.0;

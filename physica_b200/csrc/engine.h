@@ -12,6 +12,7 @@
 #include "../../include/physica_pbf.h"
 #include "pbf_internal.h"
 #include "pbf_launch.h"
+#include "staged_fit.h"
 
 namespace pbf {
 
@@ -239,6 +240,7 @@ private:
         const void* p[16];
         const StepRecord* record;
         cudaEvent_t positions_ready;
+        bool staged;
         bool operator==(const GraphKey& o) const;
     };
     struct GraphEntry {
@@ -301,7 +303,11 @@ private:
     float* packed_magnitude_ = nullptr;
     StagedList staged_list_{};
     int record_positions_ready(cudaStream_t stream);
-    bool runs_staged_passes(const LaunchShape& shape) const;
+    // Whether steps with `shape` may run the staged passes, by their size; whether they do
+    // also depends on how dense the particles are (staged_fit.h).
+    bool may_run_staged(const LaunchShape& shape) const;
+    StagedFit fit_;
+    bool staged_step_ = false;   // the step being launched does
     int launch_staged(cudaStream_t stream, const pbf_particle_state* state, pbf_particle_state* next_state, StepRecord& r);
     uint32_t* arrival_ = nullptr;
     uint32_t* unordered_ = nullptr;

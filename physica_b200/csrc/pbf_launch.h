@@ -187,7 +187,7 @@ bool valid_shape(const LaunchShape& shape);
 cudaError_t launch_list_scan(cudaStream_t stream, const ListScanArgs& a, const LaunchShape& shape = LaunchShape{});
 // Whether `shape` runs the scan of `a` fused with density + lambda (launch_scan_density_lambda).
 bool fuses_density(const LaunchShape& shape, const ListScanArgs& a);
-// Whether a step with `shape` runs the staged passes.
+// Whether `shape` asks for the staged passes and the scene has what they need.
 bool runs_staged(const LaunchShape& shape, bool boundary, uint32_t iterations);
 // The list scan of a Jacobi iteration and its density + lambda pass in one kernel (same list and
 // results as launch_list_scan followed by launch_density_lambda).

@@ -141,6 +141,8 @@ private:
     PackedPositions packed_{};       // the sorted positions again as x, y, z arrays (packed list scan)
     float* packed_mass_ = nullptr;   // staged passes (no boundary particles): the sorted masses, and the
     StagedList staged_list_{};       // list of the step in progress
+    StagedFit fit_;
+    bool may_run_staged(const LaunchShape& shape) const;
     uint32_t* arrival_ = nullptr;
     uint32_t* unordered_ = nullptr;
     uint32_t* tile_sums_ = nullptr;
@@ -244,9 +246,10 @@ int SphEngine::init(const pbf_domain_configuration* domain, const sph_configurat
     SphSceneInput* d_input = arena_.alloc<SphSceneInput>(1, e);
     scratch_ = arena_.alloc<float4>(count_, e);
     packed_ = alloc_packed(arena_, count_, e);
-    if (domain->boundary_particle_count == 0) {
+    if (domain->boundary_particle_count == 0 && may_run_staged(LaunchShape{})) {
         packed_mass_ = arena_.alloc<float>(static_cast<size_t>(count_) + 4u, e);
         staged_list_.windows = arena_.alloc<uint32_t>(window_words(count_), e);
+        if (e == cudaSuccess) e = fit_.init(arena_, stream_, StagedFit::kSph);
         if (config_.method != SPH_METHOD_WCSPH) {
             const size_t padded = (static_cast<size_t>(count_) + 31u) / 32u * 32u;
             staged_list_.list = {arena_.alloc<uint32_t>(padded * kListCapacity, e), arena_.alloc<uint32_t>(count_, e), kListCapacity};
@@ -424,7 +427,11 @@ int SphEngine::forward(const pbf_particle_state* state, const sph_method_state* 
     next_state->step_index = state->step_index + 1u;
     r.valid = true;
     r.step_index = state->step_index;
-    return PBF_SUCCESS;
+    return may_run_staged(shape) ? check(fit_.measure(stream_, step_of(r).g), "staged fit") : PBF_SUCCESS;
+}
+
+bool SphEngine::may_run_staged(const LaunchShape& shape) const {
+    return runs_staged(shape, boundary_count_ > 0, 1u);
 }
 
 int SphEngine::launch(cudaStream_t s, const pbf_particle_state* state, const sph_method_state* method_state,
@@ -482,7 +489,7 @@ int SphEngine::launch(cudaStream_t s, const pbf_particle_state* state, const sph
         gc.boundary = r.boundary;
     }
     const StoredList list{r.list_entries, r.list_counts, r.list_capacity};
-    const bool staged = runs_staged(shape, boundary_count_ > 0, 1u);
+    const bool staged = may_run_staged(shape) && fit_.pays();
     if (!staged) {
         ListScanArgs scan{gc, r.topology, list, 1};
         scan.packed = packed_;

@@ -13,6 +13,10 @@ constexpr uint32_t kBlockParticles = 128;   // and threads
 // Staged slots: 2 % of the blocks of a 1M-particle dam break need more.  Six fields and the hit masks
 // then fit 48 KB.
 constexpr uint32_t kStage = 1600;
+// The same with four lanes per particle (staged_group.cu): 0.6 % of the blocks of a dam break of 5k to 20k
+// particles have more in their windows.
+constexpr uint32_t kGroupParticles = 32;
+constexpr uint32_t kGroupStage = 704;
 // Candidates of one stencil column that its hit record covers (26 on average in a dam break at its
 // densest, 24 at rest).
 constexpr uint32_t kColumn = 48;

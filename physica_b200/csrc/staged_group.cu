@@ -19,8 +19,7 @@ using namespace staged_detail;
 constexpr uint32_t kThreads = kBlockParticles;
 constexpr int L = 4;   // lanes per particle
 constexpr uint32_t kParticles = kThreads / L;
-// Staged slots: 0.6 % of the blocks of a dam break of 5k to 20k particles have more in their windows.
-constexpr uint32_t kGroupStage = 704;
+static_assert(kParticles == kGroupParticles, "a block's windows");
 // A longer list walks the stencil.
 constexpr uint32_t kGroupList = 96;
 
