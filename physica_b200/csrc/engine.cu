@@ -232,7 +232,10 @@ int Engine::init(const pbf_domain_configuration* scenes, const uint32_t scene_co
     predicted_ = arena_.alloc<float4>(count_, e);
     packed_ = alloc_packed(arena_, count_, e);
     bool boundary = false;
-    for (uint32_t s = 0; s < scene_count; ++s) boundary = boundary || scenes[s].boundary_particle_count > 0;
+    for (uint32_t s = 0; s < scene_count; ++s) {
+        boundary = boundary || scenes[s].boundary_particle_count > 0;
+        packed_radii_ = packed_radii_ && packed_radius(scenes[s].support_radius);
+    }
     if (!boundary && may_run_staged(LaunchShape{})) {
         packed_next_ = alloc_packed(arena_, count_, e);
         packed_velocity_ = alloc_packed(arena_, count_, e);
@@ -677,8 +680,8 @@ int Engine::record_positions_ready(cudaStream_t stream) {
 
 bool Engine::may_run_staged(const LaunchShape& shape) const {
     if (!runs_staged(shape, boundary_count_ > 0, iterations_)) return false;
-    if (differentiable()) return count_ >= kStagedDifferentiable;
-    return count_ <= kGroupedParticles || count_ > kOneWave;
+    if (differentiable()) return count_ >= kStagedDifferentiable && packed_radii_;
+    return count_ <= kGroupedParticles || (count_ > kOneWave && packed_radii_);
 }
 
 // The Jacobi iterations and the post-loop passes over staged windows (staged.cu, staged_group.cu): two

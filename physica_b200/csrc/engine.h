@@ -303,11 +303,12 @@ private:
     float* packed_magnitude_ = nullptr;
     StagedList staged_list_{};
     int record_positions_ready(cudaStream_t stream);
-    // Whether steps with `shape` may run the staged passes, by their size; whether they do
+    // Whether steps with `shape` may run the staged passes, by their size and support radii; whether they do
     // also depends on how dense the particles are (staged_fit.h).
     bool may_run_staged(const LaunchShape& shape) const;
     StagedFit fit_;
     bool staged_step_ = false;   // the step being launched does
+    bool packed_radii_ = true;   // every support radius is in the packed arithmetic's range
     int launch_staged(cudaStream_t stream, const pbf_particle_state* state, pbf_particle_state* next_state, StepRecord& r);
     uint32_t* arrival_ = nullptr;
     uint32_t* unordered_ = nullptr;

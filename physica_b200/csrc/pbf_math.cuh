@@ -86,6 +86,11 @@ __device__ __forceinline__ d3 cross(const d3 a, const d3 b) {
 // The float value of pi used by the reference kernels (density/device.cuh:8).
 constexpr float kPi = 3.14159265358979323846F;
 
+// Whether the packed pair arithmetic below covers support radius h.  Other radii evaluate every pair
+// twice: at 262k particles a step of PBF / PCISPH / WCSPH takes 0.600 / 0.869 / 0.194 ms staged and 0.563 / 0.766 / 0.186 per
+// lane.  With four lanes a particle the staged passes stay ahead: 0.148 against 0.197 ms at 5k.
+__host__ __device__ __forceinline__ bool packed_radius(const float h) { return h >= 0x1p-10F && h <= 0x1p10F; }
+
 // Per-scene constants, derived on the device once so they come from the same
 // device powf / division the reference evaluates inline.
 struct KernelConstants {
@@ -142,11 +147,11 @@ __device__ inline KernelConstants kernel_constants(const float h) {
     k.spiky_coefficient_d = -45.0 / (static_cast<double>(kPi) * pow(static_cast<double>(h), 6.0));
     k.poly6_reciprocal = __frcp_rn(k.poly6_denominator);
     k.poly6_grad_reciprocal = __frcp_rn(k.poly6_grad_denominator);
-    // fast_pair's range.  At its ends every intermediate of the packed arithmetic, and every last bit of
+    // The range of the packed arithmetic.  At its ends every intermediate of the packed arithmetic, and every last bit of
     // its residuals, is a normal float: r >= 2^-30 h, and a poly6 numerator 315 (h2 - r2)^3 >= 2^-100.
     k.fast_min = __fmul_rn(squared_radius, 0x1p-60F);
     k.fast_max = -1.0F;
-    if (h >= 0x1p-10F && h <= 0x1p10F) {
+    if (packed_radius(h)) {
         const float below = __uint_as_float(__float_as_uint(fminf(squared_radius, k.spiky_threshold)) - 1u);
         k.fast_max = fminf(below, __fsub_rn(squared_radius, 0x1p-36F));
     }
@@ -204,7 +209,7 @@ __device__ __forceinline__ f3 spiky_gradient(const f3 d, const KernelConstants& 
 // ------------------------------------------------- two pairs at a time, packed FP32
 // The replay passes were bound by instruction issue, and most of a pair's instructions were its IEEE
 // square root and divisions, each with range tests and a branch around a slow path.  Inside a
-// range of r2 where nothing can overflow or turn subnormal (fast_pair) the same correctly rounded
+// range of r2 where nothing can overflow or turn subnormal (fast_min to fast_max) the same correctly rounded
 // values follow from one reciprocal square root and fused residual corrections, without a branch,
 // so two pairs share every instruction (packed FP32, each half rounded as the scalar intrinsic):
 //   sqrt:  s0 = r2 y, s = s0 + (r2 - s0^2) y / 2 with y ~ 1 / sqrt(r2).  Equal to __fsqrt_rn for
@@ -216,11 +221,6 @@ __device__ __forceinline__ f3 spiky_gradient(const f3 d, const KernelConstants& 
 //          the 2^-44, R is an ulp low for s = 2 - 2^-23 and 1 / s comes out wrong.  The same test
 //          checks, for every s, the quotients that lie nearest a rounding boundary.
 __device__ __forceinline__ float2 both(const float v) { return make_float2(v, v); }
-
-// Whether r2 is in the range of the packed arithmetic (0 is: the weight there needs no root).
-__device__ __forceinline__ bool fast_pair(const float r2, const KernelConstants& k) {
-    return r2 <= k.fast_max && (r2 >= k.fast_min || r2 == 0.0F);
-}
 
 // The negated squared distance, -squared(d), of displacement d.
 __device__ __forceinline__ float negated_squared(const f3 d) {
@@ -331,7 +331,7 @@ __device__ __forceinline__ d3 hessian_product(const PairDerivatives& p, const d3
 }
 __device__ __forceinline__ d3 wide(const f3 v) { return {v.x, v.y, v.z}; }
 
-// The poly6 weight of poly6_inside without its division's range tests (r2 inside fast_pair's range).
+// The poly6 weight of poly6_inside without its division's range tests (r2 up to fast_max).
 __device__ __forceinline__ float poly6_weight(const float r2, const KernelConstants& k) {
     if (r2 > k.fast_max) return r2 >= k.h2 ? 0.0F : poly6_call(r2, k.h2, k.poly6_denominator);
     const float difference = __fsub_rn(k.h2, r2);

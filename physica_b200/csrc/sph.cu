@@ -303,7 +303,7 @@ __global__ void sph_constants_kernel(const SphSceneInput* __restrict__ inputs, c
     // residuals, is a normal float.
     k.inverse_h = __frcp_rn(h);
     k.fast_min = __fmul_rn(__fmul_rn(h, h), 0x1p-60F);
-    k.fast_max = h >= 0x1p-10F && h <= 0x1p10F ? __fmul_rn(__fmul_rn(h, h), 2.0F) : -1.0F;
+    k.fast_max = packed_radius(h) ? __fmul_rn(__fmul_rn(h, h), 2.0F) : -1.0F;
     k.laplacian_denominator = __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(kPi, h), h), h), h), h), h);
     k.laplacian_denominator_d = static_cast<double>(kPi) * pow(static_cast<double>(h), 6.0);
     k.support_squared_d = static_cast<double>(h) * static_cast<double>(h);

@@ -431,7 +431,8 @@ int SphEngine::forward(const pbf_particle_state* state, const sph_method_state* 
 }
 
 bool SphEngine::may_run_staged(const LaunchShape& shape) const {
-    return runs_staged(shape, boundary_count_ > 0, 1u);
+    if (!runs_staged(shape, boundary_count_ > 0, 1u) || !packed_radius(domain_.support_radius)) return false;
+    return true;
 }
 
 int SphEngine::launch(cudaStream_t s, const pbf_particle_state* state, const sph_method_state* method_state,

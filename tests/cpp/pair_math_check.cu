@@ -90,7 +90,12 @@ __global__ void constant_quotient_kernel(const int limit, unsigned long long* ba
     for (uint32_t t = 0; t < 32u; ++t) check(__uint_as_float(0x3f800000u | (mix(i * 32u + t) >> 9)));
 }
 
-// the kernels' values at n squared distances spread over the range of fast_pair
+// whether r2 is in the range of the packed arithmetic (0 is: the weight there needs no root)
+__device__ __forceinline__ bool fast_pair(const float r2, const KernelConstants& k) {
+    return r2 <= k.fast_max && (r2 >= k.fast_min || r2 == 0.0F);
+}
+
+// the kernels' values at n squared distances spread over that range
 __global__ void kernels_kernel(const float h, const uint32_t n, unsigned long long* bad, unsigned long long* tested) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;

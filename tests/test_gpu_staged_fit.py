@@ -109,3 +109,25 @@ def test_differentiable_steps_follow_too(ratio, staged):
         outs.append(out)
     for a, b in zip(*outs):
         np.testing.assert_array_equal(a.view(np.int32), b.view(np.int32))
+
+
+@pytest.mark.parametrize("count,staged", [(8000, True), (185193, False)])
+def test_radii_outside_the_packed_range_stay_per_lane(count, staged):
+    """Except with four lanes a particle, where the staged passes are faster all the same."""
+    out, launches = run(lattice(count, 2.0, h=0.0005), pbf.LaunchShape(4, 128, 128), count=2)
+    assert launches[1] == PBF_LAUNCHES[staged]
+    for a, b in zip(out, run(lattice(count, 2.0, h=0.0005), pbf.LaunchShape(0, 128, 128), count=2)[0]):
+        np.testing.assert_array_equal(a.view(np.int32), b.view(np.int32))
+
+
+def sph_launches(scene, method, scan):
+    scene.sph = scenes.sph_parameter_arrays(scene, method=method)
+    solver, state, control, params = sph.solver_for_scene(scene, sph.Method[method])
+    solver.launch_shape = pbf.LaunchShape(scan, 128, 128)
+    return steps(solver, state, control, params, 2)[1][1]
+
+
+@pytest.mark.parametrize("method", ["wcsph", "dfsph"])
+def test_sph_radii_outside_the_packed_range_stay_per_lane(method):
+    scene = lattice(8000, 2.0, h=0.0005, dt=4e-6)
+    assert sph_launches(scene, method, 4) == sph_launches(scene, method, 0)
