@@ -12,6 +12,7 @@
 // steps took 0.196, 0.713, 1.078, 1.159, 1.633, 1.037 and 3.56 ms.
 #pragma once
 
+#include <cstdint>
 #include <cuda_runtime.h>
 
 namespace pbf {
@@ -42,6 +43,17 @@ inline void launch_after(cudaStream_t stream, void (*kernel)(Parameters...), con
     config.attrs = &overlap;
     config.numAttrs = 1;
     cudaLaunchKernelEx(&config, kernel, arguments...);   // errors: cudaGetLastError()
+}
+
+// Threads of `kernel` that are resident at once on the current device, in blocks of `block`.
+template <class... Parameters>
+inline cudaError_t one_wave(void (*kernel)(Parameters...), const int block, uint32_t& threads) {
+    int device = 0, multiprocessors = 0, blocks = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&multiprocessors, cudaDevAttrMultiProcessorCount, device);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, block, 0);
+    threads = static_cast<uint32_t>(multiprocessors) * static_cast<uint32_t>(blocks) * static_cast<uint32_t>(block);
+    return e;
 }
 
 }  // namespace pbf

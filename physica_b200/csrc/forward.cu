@@ -701,6 +701,8 @@ unsigned block_of(const unsigned block) {
 }
 }  // namespace
 
+cudaError_t list_walk_wave(uint32_t& particles) { return one_wave(list_walk_kernel, kBlock, particles); }
+
 cudaError_t launch_list_scan(cudaStream_t stream, const ListScanArgs& a, const LaunchShape& shape) {
     if (a.g.count == 0) return cudaSuccess;
     const unsigned block = block_of(shape.scan_block);

@@ -178,7 +178,7 @@ enum ListScanVariant : uint32_t {
                             // shared memory (staged.cu) at the sizes where that is faster; otherwise as 3
 };
 struct LaunchShape {
-    uint32_t scan = kScanStaged16;   // fastest at every size measured (5k to 1M particles)
+    uint32_t scan = kScanStaged16;   // chooses the faster passes by size, method, radius and density
     uint32_t scan_block = 128;   // threads per block of the list scan: 32, 64, 96 or 128
     uint32_t block = 128;        // threads per block of the gather passes: 32, 64, 96 or 128
 };
@@ -194,6 +194,8 @@ bool runs_staged(const LaunchShape& shape, bool boundary, uint32_t iterations);
 cudaError_t launch_scan_density_lambda(cudaStream_t stream, const ListScanArgs& a, const DensityLambdaArgs& d,
                                        const LaunchShape& shape);
 // Device step counter and the per-step scene fields derived from it (time, grid origin, collision box).
+// Particles whose blocks of the per-lane scan are resident at once.
+cudaError_t list_walk_wave(uint32_t& particles);
 cudaError_t launch_set_step(cudaStream_t stream, unsigned long long* step, uint64_t value);
 cudaError_t launch_advance_step(cudaStream_t stream, unsigned long long* step);
 cudaError_t launch_scene_time(cudaStream_t stream, const SceneStatic* statics, SceneDesc* scenes, const unsigned long long* step,

@@ -142,6 +142,7 @@ private:
     float* packed_mass_ = nullptr;   // staged passes (no boundary particles): the sorted masses, and the
     StagedList staged_list_{};       // list of the step in progress
     StagedFit fit_;
+    uint32_t staged_wave_ = 0, list_walk_wave_ = 0;   // particles of one wave of the staged and of the per-lane scan
     bool may_run_staged(const LaunchShape& shape) const;
     uint32_t* arrival_ = nullptr;
     uint32_t* unordered_ = nullptr;
@@ -246,6 +247,8 @@ int SphEngine::init(const pbf_domain_configuration* domain, const sph_configurat
     SphSceneInput* d_input = arena_.alloc<SphSceneInput>(1, e);
     scratch_ = arena_.alloc<float4>(count_, e);
     packed_ = alloc_packed(arena_, count_, e);
+    if (int rc = check(list_walk_wave(list_walk_wave_), "occupancy of the list scan")) return rc;
+    if (int rc = check(sph::staged_sph_wave(staged_wave_), "occupancy of the staged scan")) return rc;
     if (domain->boundary_particle_count == 0 && may_run_staged(LaunchShape{})) {
         packed_mass_ = arena_.alloc<float>(static_cast<size_t>(count_) + 4u, e);
         staged_list_.windows = arena_.alloc<uint32_t>(window_words(count_), e);
@@ -430,9 +433,14 @@ int SphEngine::forward(const pbf_particle_state* state, const sph_method_state* 
     return may_run_staged(shape) ? check(fit_.measure(stream_, step_of(r).g), "staged fit") : PBF_SUCCESS;
 }
 
+// A WCSPH step uses the staged scan alone.  Between the particles of one wave of it (six blocks of 128 threads on each of
+// 148 SMs: 113,664) and of one wave of the per-lane scan (twelve: 227,328) it needs a second wave that the per-lane
+// scan does not: staged / per lane, ms a step, 60k 0.079 / 0.082, 85k 0.089 / 0.090, 110k 0.101 / 0.098, 146k 0.125 / 0.117, 179k
+// 0.143 / 0.134, 227k 0.159 / 0.157, 275k 0.193 / 0.193, 330k 0.214 / 0.230, 1M 0.576 / 0.605.  The iterative methods replay
+// staged lists and gain at every size (146k: PCISPH 0.444 / 0.454, DFSPH 0.687 / 0.714).
 bool SphEngine::may_run_staged(const LaunchShape& shape) const {
     if (!runs_staged(shape, boundary_count_ > 0, 1u) || !packed_radius(domain_.support_radius)) return false;
-    return true;
+    return config_.method != SPH_METHOD_WCSPH || count_ <= staged_wave_ || count_ > list_walk_wave_;
 }
 
 int SphEngine::launch(cudaStream_t s, const pbf_particle_state* state, const sph_method_state* method_state,

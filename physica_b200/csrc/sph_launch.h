@@ -80,6 +80,7 @@ struct SphStaged {
     PackedPositions positions;   // the sorted positions
     const float* mass;
 };
+cudaError_t staged_sph_wave(uint32_t& particles);   // particles of WCSPH's scan that are resident at once
 cudaError_t launch_staged_sph_density(cudaStream_t stream, const SphStep& st, const SphStaged& staged, uint32_t method,
                                       float* density_record, float* pressure, float* pressure_term, const float* warm);
 

@@ -220,6 +220,8 @@ cudaError_t launch(void (*kernel)(Args), cudaStream_t stream, const Args& a) {
 
 }  // namespace
 
+cudaError_t staged_sph_wave(uint32_t& particles) { return one_wave(staged_sph_density_kernel<false>, kBlockParticles, particles); }
+
 cudaError_t launch_staged_sph_density(cudaStream_t stream, const SphStep& st, const SphStaged& staged, const uint32_t method,
                                       float* density_record, float* pressure, float* pressure_term, const float* warm) {
     const DensityPassArgs a{st.g, st, staged, method, density_record, pressure, pressure_term, warm};

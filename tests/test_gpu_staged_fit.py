@@ -131,3 +131,10 @@ def sph_launches(scene, method, scan):
 def test_sph_radii_outside_the_packed_range_stay_per_lane(method):
     scene = lattice(8000, 2.0, h=0.0005, dt=4e-6)
     assert sph_launches(scene, method, 4) == sph_launches(scene, method, 0)
+
+
+@pytest.mark.parametrize("count,staged", [(91125, True), (125000, False), (216000, False), (287496, True)])
+def test_wcsph_between_the_waves_stays_per_lane(count, staged):
+    """The staged scan's second wave begins at 113,664 particles, the per-lane scan's at 227,328."""
+    scene = lattice(count, 2.0, dt=scenes.SPH_DT)
+    assert sph_launches(scene, "wcsph", 4) == sph_launches(scene, "wcsph", 0) - (1 if staged else 0)
