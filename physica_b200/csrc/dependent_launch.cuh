@@ -45,14 +45,20 @@ inline void launch_after(cudaStream_t stream, void (*kernel)(Parameters...), con
     cudaLaunchKernelEx(&config, kernel, arguments...);   // errors: cudaGetLastError()
 }
 
+// Multiprocessors of the current device (0 after an error).
+inline uint32_t multiprocessors() {
+    int device = 0, count = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+        return 0u;
+    return static_cast<uint32_t>(count);
+}
+
 // Threads of `kernel` that are resident at once on the current device, in blocks of `block`.
 template <class... Parameters>
 inline cudaError_t one_wave(void (*kernel)(Parameters...), const int block, uint32_t& threads) {
-    int device = 0, multiprocessors = 0, blocks = 0;
-    cudaError_t e = cudaGetDevice(&device);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&multiprocessors, cudaDevAttrMultiProcessorCount, device);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, block, 0);
-    threads = static_cast<uint32_t>(multiprocessors) * static_cast<uint32_t>(blocks) * static_cast<uint32_t>(block);
+    int blocks = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, block, 0);
+    threads = multiprocessors() * static_cast<uint32_t>(blocks) * static_cast<uint32_t>(block);
     return e;
 }
 

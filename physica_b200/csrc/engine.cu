@@ -148,12 +148,6 @@ constexpr uint32_t kStagedDifferentiable = 1u << 19;
 // lanes are the fastest: a forward step at 5k particles 0.164 ms against 0.240 with one lane, at 14k
 // 0.228 / 0.253.  Two lanes never were (0.176, 0.253).
 constexpr uint32_t kGroupedParticles = 20480;
-// Up to here all blocks of the per-lane passes are resident at once (nine of 128 threads on each of 148 SMs),
-// and loads they wait for overlap better than a block's staging, scan and replay, which all its blocks go
-// through at the same time, four to eight to an SM.  Above, the per-lane passes need a second wave.
-// Per lane / staged, ms a step: 22k particles 0.263 / 0.274, 64k 0.305 / 0.321, 110k 0.363 / 0.403, 169k
-// 0.488 / 0.530, 198k 0.634 / 0.548, 246k 0.715 / 0.649, 295k 0.803 / 0.725.
-constexpr uint32_t kOneWave = 9u * 148u * 128u;
 }  // namespace
 
 int Engine::init(const pbf_domain_configuration* scenes, const uint32_t scene_count, const pbf_configuration* configuration,
@@ -236,6 +230,12 @@ int Engine::init(const pbf_domain_configuration* scenes, const uint32_t scene_co
         boundary = boundary || scenes[s].boundary_particle_count > 0;
         packed_radii_ = packed_radii_ && packed_radius(scenes[s].support_radius);
     }
+    // Up to here all blocks of the per-lane passes are resident at once (nine of 128 threads on each of 148 SMs: 170,496
+    // particles), and loads they wait for overlap better than a block's staging, scan and replay, which all its
+    // blocks go through at the same time, four to eight to an SM.  Above, the per-lane passes need a second wave.
+    // Per lane / staged, ms a step: 22k particles 0.263 / 0.274, 64k 0.305 / 0.321, 110k 0.363 / 0.403, 169k
+    // 0.488 / 0.530, 198k 0.634 / 0.548, 246k 0.715 / 0.649, 295k 0.803 / 0.725.
+    if (int rc = check(fused_scan_wave(one_wave_), "occupancy of the fused scan")) return rc;
     if (!boundary && may_run_staged(LaunchShape{})) {
         packed_next_ = alloc_packed(arena_, count_, e);
         packed_velocity_ = alloc_packed(arena_, count_, e);
@@ -681,7 +681,7 @@ int Engine::record_positions_ready(cudaStream_t stream) {
 bool Engine::may_run_staged(const LaunchShape& shape) const {
     if (!runs_staged(shape, boundary_count_ > 0, iterations_)) return false;
     if (differentiable()) return count_ >= kStagedDifferentiable && packed_radii_;
-    return count_ <= kGroupedParticles || (count_ > kOneWave && packed_radii_);
+    return count_ <= kGroupedParticles || (count_ > one_wave_ && packed_radii_);
 }
 
 // The Jacobi iterations and the post-loop passes over staged windows (staged.cu, staged_group.cu): two

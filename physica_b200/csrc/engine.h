@@ -309,6 +309,7 @@ private:
     StagedFit fit_;
     bool staged_step_ = false;   // the step being launched does
     bool packed_radii_ = true;   // every support radius is in the packed arithmetic's range
+    uint32_t one_wave_ = 0;      // particles of the per-lane passes that are resident at once
     int launch_staged(cudaStream_t stream, const pbf_particle_state* state, pbf_particle_state* next_state, StepRecord& r);
     uint32_t* arrival_ = nullptr;
     uint32_t* unordered_ = nullptr;

@@ -701,6 +701,7 @@ unsigned block_of(const unsigned block) {
 }
 }  // namespace
 
+cudaError_t fused_scan_wave(uint32_t& particles) { return one_wave(scan_density_lambda_kernel, kBlock, particles); }
 cudaError_t list_walk_wave(uint32_t& particles) { return one_wave(list_walk_kernel, kBlock, particles); }
 
 cudaError_t launch_list_scan(cudaStream_t stream, const ListScanArgs& a, const LaunchShape& shape) {

@@ -381,7 +381,7 @@ cudaError_t launch_advance_step(cudaStream_t stream, unsigned long long* step) {
 cudaError_t launch_scene_time(cudaStream_t stream, const SceneStatic* statics, SceneDesc* scenes, const unsigned long long* step,
                               const uint32_t count, uint32_t* clear, const uint64_t words) {
     // four blocks an SM at most, or as many as the scenes need
-    const unsigned blocks = std::max(blocks_for(count, 128), std::min(blocks_for(words, 128), 592u));
+    const unsigned blocks = std::max(blocks_for(count, 128), std::min(blocks_for(words, 128), std::max(4u * multiprocessors(), 1u)));
     if (blocks == 0) return cudaSuccess;
     launch_after(stream, scene_time_kernel, blocks, 128, statics, scenes, step, count, clear, words);
     count_launch();

@@ -194,7 +194,8 @@ bool runs_staged(const LaunchShape& shape, bool boundary, uint32_t iterations);
 cudaError_t launch_scan_density_lambda(cudaStream_t stream, const ListScanArgs& a, const DensityLambdaArgs& d,
                                        const LaunchShape& shape);
 // Device step counter and the per-step scene fields derived from it (time, grid origin, collision box).
-// Particles whose blocks of the per-lane scan are resident at once.
+// Particles whose blocks of the fused scan, and of the per-lane scan, are resident at once.
+cudaError_t fused_scan_wave(uint32_t& particles);
 cudaError_t list_walk_wave(uint32_t& particles);
 cudaError_t launch_set_step(cudaStream_t stream, unsigned long long* step, uint64_t value);
 cudaError_t launch_advance_step(cudaStream_t stream, unsigned long long* step);
