@@ -114,9 +114,10 @@ def test_differentiable_steps_follow_too(ratio, staged):
 @pytest.mark.parametrize("count,staged", [(8000, True), (185193, False)])
 def test_radii_outside_the_packed_range_stay_per_lane(count, staged):
     """Except with four lanes a particle, where the staged passes are faster all the same."""
-    out, launches = run(lattice(count, 2.0, h=0.0005), pbf.LaunchShape(4, 128, 128), count=2)
+    scene = lattice(count, 2.0, h=0.0005, dt=1e-5)   # a step moves the particles by 0.002 h
+    out, launches = run(scene, pbf.LaunchShape(4, 128, 128), count=2)
     assert launches[1] == PBF_LAUNCHES[staged]
-    for a, b in zip(out, run(lattice(count, 2.0, h=0.0005), pbf.LaunchShape(0, 128, 128), count=2)[0]):
+    for a, b in zip(out, run(scene, pbf.LaunchShape(0, 128, 128), count=2)[0]):
         np.testing.assert_array_equal(a.view(np.int32), b.view(np.int32))
 
 
