@@ -255,7 +255,9 @@ int SphEngine::init(const pbf_domain_configuration* domain, const sph_configurat
         if (e == cudaSuccess) e = fit_.init(arena_, stream_, StagedFit::kSph);
         if (config_.method != SPH_METHOD_WCSPH) {
             const size_t padded = (static_cast<size_t>(count_) + 31u) / 32u * 32u;
-            staged_list_.list = {arena_.alloc<uint32_t>(padded * kListCapacity, e), arena_.alloc<uint32_t>(count_, e), kListCapacity};
+            // two entries a word, and no more of them than a list of slots holds
+            constexpr uint32_t words = kListCapacity / 2u;
+            staged_list_.list = {arena_.alloc<uint32_t>(padded * words, e), arena_.alloc<uint32_t>(count_, e), words};
         }
     }
     arrival_ = arena_.alloc<uint32_t>(count_, e);

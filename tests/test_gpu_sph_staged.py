@@ -119,3 +119,21 @@ def test_values_that_are_not_finite(method):
     warm = np.full(4000, 10.0, np.float32)
     warm[[2500, 3500]] = np.inf, np.nan
     check(s, method, steps=1, **({"warm": warm} if method == "dfsph" else {}))
+
+
+@pytest.mark.parametrize("method", METHODS)
+@pytest.mark.parametrize("count", [88, 95, 96, 97, 104])
+def test_lists_near_their_capacity(method, count):
+    """Balls of `count` particles within each other's support, over four stencil columns so that they fit the
+    hit records: a staged list holds up to 95 entries beside the particle itself, a longer one overflows."""
+    s = block(4 * count, method, seed=10)
+    rng = np.random.default_rng(11)
+    h = s.support_radius
+    for ball in range(4):
+        x = rng.normal(size=(3, count))
+        x *= 0.45 * h * rng.random(count) ** (1 / 3) / np.linalg.norm(x, axis=0)
+        x[0], x[1] = np.abs(x[0]) * (-1.0) ** np.arange(count), np.abs(x[1]) * (-1.0) ** (np.arange(count) // 2)
+        x[2] = np.abs(x[2])   # one cell in z
+        s.positions[:, ball * count:(ball + 1) * count] = (x + (np.array([2, 3, 2]) + ball)[:, None] * h).astype(np.float32)
+    s.box_max = (12 * h,) * 3
+    check(s, method, steps=1)
