@@ -342,9 +342,10 @@ int pbf_forward_step_preallocated(const pbf_domain_configuration* domain, const 
  *      stencil columns, 3 = as 0, and each Jacobi iteration's scan also computes density and lambda
  *      in the same kernel, replaying the list from shared memory (scenes with boundary particles run
  *      3 as 0), 4 = as 3, and every pass of a step without boundary particles (of up to 20,480 or more than 170,496
- *      particles; in differentiable mode of at least 2^19) reads its neighbours from windows of the sorted particles staged in shared memory (the default);
+ *      particles; in differentiable mode of at least 2^19) reads its neighbours from windows of the sorted particles
+ *      staged in shared memory, unless the particles turn out to be too dense for that (the default);
  *      scan_block_size and block_size: 32, 64, 96 or 128 threads (the staged passes have their own).
- *      pbf_autotune times the list-scan shapes 0, 1, 2 and 4 by their scans and gather passes, then the
+ *      pbf_autotune times the list-scan shapes by their scans and gather passes, then, unless the staged passes won, the
  *      gather block sizes, on `repeats` forward steps from `state` (writing `scratch_state` and
  *      the cache, which then hold that step); it keeps the fastest shape, returns it in `chosen`
  *      (may be NULL) and the substep time with it in `milliseconds_per_step` (may be NULL).  It

@@ -842,43 +842,51 @@ int Engine::autotune(const pbf_particle_state* state, const pbf_control* control
         timer_.enable(false);
         return rc;
     };
-    const uint32_t scans[4] = {kScanPerLane, kScanCooperative, kScanStaged, kScanStaged16};
+    const uint32_t scans[5] = {kScanPerLane, kScanCooperative, kScanStaged, kScanFusedDensity, kScanStaged16};
     const uint32_t blocks[4] = {32u, 64u, 96u, 128u};
     double ms[kPassCount];
     int rc = PBF_SUCCESS;
-    // 1. the list scan: variant x block size, by the time of the scans and the gather passes (the
-    //    variants differ in which passes they fuse).  The staged passes have a block size of their own.
+    auto gather_ms = [&ms] {
+        double sum = 0.0;
+        for (const int p : {kPassDensityLambda, kPassCorrection, kPassVorticity, kPassNormal, kPassXsph}) sum += ms[p];
+        return sum;
+    };
+    auto total_ms = [&ms] {
+        double sum = 0.0;
+        for (int p = 0; p < kPassCount; ++p) sum += ms[p];
+        return sum;
+    };
+    // Steps that cannot be staged run variant 4 as 3, staged ones have block sizes of their own.
     const bool staged = may_run_staged(LaunchShape{kScanStaged16, 128u, 128u});
+    // 1. the list scan: variant x block size, by the time of the scans and the gather passes (the
+    //    variants differ in which passes they fuse)
     LaunchShape best = previous;
     best.block = 128u;
-    double best_scan = -1.0;
-    for (int v = 0; v < 4 && !rc; ++v)
+    double best_scan = -1.0, best_gather = -1.0, best_total = 0.0;
+    for (int v = 0; v < 5 && !rc; ++v)
         for (int b = 0; b < 4 && !rc; ++b) {
+            if (!staged && scans[v] == kScanFusedDensity) continue;
             if (staged && scans[v] == kScanStaged16 && b != 3) continue;
             shape_ = best;
             shape_.scan = scans[v];
             shape_.scan_block = blocks[b];
             if ((rc = measure(ms))) break;
-            double scan_ms = ms[kPassListScan] + ms[kPassDensityLambda] + ms[kPassScanDensityLambda];
-            for (const int pass : {kPassCorrection, kPassVorticity, kPassNormal, kPassXsph}) scan_ms += ms[pass];
+            const double scan_ms = ms[kPassListScan] + ms[kPassScanDensityLambda] + gather_ms();
             if (best_scan < 0.0 || scan_ms < best_scan) {
                 best_scan = scan_ms;
                 best.scan = scans[v];
                 best.scan_block = blocks[b];
+                best_total = total_ms();
             }
         }
     // 2. the gather passes' block size, by their summed time
-    double best_gather = -1.0, best_total = 0.0;
-    for (int b = 0; b < 4 && !rc; ++b) {
+    for (int b = 0; b < 4 && !rc && !(staged && best.scan == kScanStaged16); ++b) {
         shape_ = best;
         shape_.block = blocks[b];
         if ((rc = measure(ms))) break;
-        double gather = 0.0, total = 0.0;
-        for (int p = 0; p < kPassCount; ++p) total += ms[p];
-        for (const int p : {kPassDensityLambda, kPassCorrection, kPassVorticity, kPassNormal, kPassXsph}) gather += ms[p];
-        if (best_gather < 0.0 || gather < best_gather) {
-            best_gather = gather;
-            best_total = total;
+        if (best_gather < 0.0 || gather_ms() < best_gather) {
+            best_gather = gather_ms();
+            best_total = total_ms();
             best.block = blocks[b];
         }
     }

@@ -139,3 +139,10 @@ def test_wcsph_between_the_waves_stays_per_lane(count, staged):
     """The staged scan's second wave begins at 113,664 particles, the per-lane scan's at 227,328."""
     scene = lattice(count, 2.0, dt=scenes.SPH_DT)
     assert sph_launches(scene, "wcsph", 4) == sph_launches(scene, "wcsph", 0) - (1 if staged else 0)
+
+
+def test_autotune_leaves_the_staged_passes_their_block_size():
+    """At 8,000 particles they are twice as fast as any other shape, and ignore the gather block size."""
+    solver, state, control, params = pbf.solver_for_scene(lattice(8000, 2.0))
+    shape, ms = solver.autotune(state, control, params, repeats=2)
+    assert shape == pbf.LaunchShape(4, 128, 128) and ms > 0.0
