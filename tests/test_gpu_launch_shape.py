@@ -110,10 +110,10 @@ def test_fused_density_records_the_same_iterates_for_the_adjoint():
         assert torch.equal(x, y)
 
 
-def test_hit_mask_lists_equal_index_lists_over_a_long_run_and_when_crowded():
-    """Launch-shape variant 4 stores each neighbour list as (slot base, 32-bit hit mask) pairs: 60
-    steps of a 3,375-particle dam break, and 3 steps of a clump eight times denser than the lattice
-    (its hit-mask lists overflow and walk the stencil), equal the index-list solver bit for bit."""
+def test_staged_windows_equal_lists_over_a_long_run_and_when_crowded():
+    """Launch-shape variant 4 replays windows staged in shared memory, here with four lanes a particle: 60 steps of a
+    3,375-particle dam break, and 3 steps of a clump eight times denser than the lattice (its particles fall back to
+    hit masks and stencil walks in the first), equal the per-lane solver bit for bit."""
     sc = scenes.dam_break((15, 15, 15), (0, 0, 0), (1, 2, 1), 35, 4, velocity_sigma=0.2)
     crowded = scenes.dam_break((16, 16, 16), (0, 0, 0), (1, 2, 1), 36, 3)
     crowded.positions = (crowded.positions * 0.5 + 0.1).astype(crowded.positions.dtype)
@@ -127,9 +127,9 @@ def test_hit_mask_lists_equal_index_lists_over_a_long_run_and_when_crowded():
             assert torch.equal(x, out[0][0]) and torch.equal(v, out[0][1])
 
 
-def test_hit_mask_lists_with_no_particles_and_no_iterations():
-    """An empty scene and a scene with zero Jacobi iterations (only the post-loop list) step with
-    hit-mask lists, the latter equal to index lists bit for bit."""
+def test_staged_shape_with_no_particles_and_no_iterations():
+    """With variant 4 an empty scene and a scene with zero Jacobi iterations, which has no staged passes, step as with
+    the per-lane lists, bit for bit."""
     dc = pbf.DomainConfiguration(particle_count=0, time_step=1.0 / 120.0, support_radius=0.025, particle_radius=0.005,
                                  boundary=pbf.BoxBoundary((0, 0, 0), (1, 2, 1), (0, 0, 0), True))
     solver = pbf.PBF(dc, pbf.Configuration(4, 2))

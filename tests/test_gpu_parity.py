@@ -188,15 +188,18 @@ def test_trajectory_matches_reference_after_100_steps():
     assert errs[100][2] == 0, errs   # and in fact bit for bit
 
 
-def test_hit_mask_lists_trajectory_matches_reference():
-    """The 32,768-particle dam break through hit-mask lists (launch-shape variant 4), 100 steps,
-    bit for bit against the reference."""
+@pytest.mark.parametrize("lattice,steps", [((27, 27, 27), 100), ((60, 50, 60), 10)])
+def test_staged_trajectory_matches_reference(lattice, steps):
+    """A dam break through the staged passes (launch-shape variant 4, with four lanes a particle and with one), bit for bit
+    against the reference."""
     reference = reference_or_skip()
-    sc = scenes.plain_small()
+    sc = scenes.plain_small(lattice=lattice)
     solver, state, control, params = pbf.solver_for_scene(sc)
     solver.launch_shape = pbf.LaunchShape(4, 128, 64)
-    errs = _trajectory_with(solver, state, control, params, solver.allocate_step_cache(), sc, 100, reference)
+    before = pbf.launch_count()
+    errs = _trajectory_with(solver, state, control, params, solver.allocate_step_cache(), sc, steps, reference)
     assert all(e[2] == 0 for e in errs.values()), {k: e for k, e in errs.items() if e[2]}
+    assert pbf.launch_count() - before < steps * (10 + 2 * sc.pressure_iterations)   # the per-lane passes: one launch more a step
 
 
 def test_batched_scene_layout_trajectory_matches_reference():
@@ -268,7 +271,7 @@ def test_edge_cases_match_oracle(case, list_scan):
         sc = scenes.dam_break((4, 4, 4), (0, 0, 0), (1, 2, 1), 7, 3)
         sc.positions[:, 1] = sc.positions[:, 0]    # two particles at the same point (zero distance)
     solver, state, control, params = pbf.solver_for_scene(sc)
-    solver.launch_shape = pbf.LaunchShape(list_scan, 128, 128)   # index lists, hit-mask lists
+    solver.launch_shape = pbf.LaunchShape(list_scan, 128, 128)   # per-lane lists, staged windows
     cache = solver.allocate_step_cache()
     nxt = step(solver, state, control, params, cache)
     x1, v1 = oracle.forward_step(sc, sc.positions, sc.velocities)

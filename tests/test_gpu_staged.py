@@ -51,6 +51,40 @@ def test_counts_around_the_block(count):
     check(block(count))
 
 
+@pytest.mark.parametrize("count,staged", [(20480, True), (20481, False), (170496, False), (170497, True)])
+def test_sizes_choose_the_passes(count, staged):
+    """The staged step has one kernel less: its post-loop scan is part of the vorticity pass."""
+    scene = block(count, iterations=3)
+    solver, state, control, params = pbf.solver_for_scene(scene)
+    cache, following = solver.allocate_step_cache(), solver.allocate_state()
+    for k in range(2):
+        before = pbf.launch_count()
+        solver.forward_step(state, control, params, following, cache)
+        launches = pbf.launch_count() - before
+        state, following = following, state
+    assert launches == (15 if staged else 16)
+
+
+@pytest.mark.parametrize("count,steps", [(13824, 100), (175616, 25)])
+def test_long_runs(count, steps):
+    """A falling, splashing block, with four lanes a particle and with one."""
+    scene = block(count, seed=13, iterations=4)
+    out = []
+    for shape in (PER_LANE, STAGED):
+        solver, state, control, params = pbf.solver_for_scene(scene)
+        solver.launch_shape = shape
+        cache, following = solver.allocate_step_cache(), solver.allocate_state()
+        before = pbf.launch_count()
+        for _ in range(steps):
+            solver.forward_step(state, control, params, following, cache)
+            state, following = following, state
+        out.append([state.positions.cpu().numpy(), state.velocities.cpu().numpy()])
+        launches = pbf.launch_count() - before
+    assert launches < 17.5 * steps   # 17 a staged step and 18 a per-lane one: most were staged
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a.view(np.int32), b.view(np.int32))
+
+
 @pytest.mark.parametrize("count", [8000, 180000])
 def test_spray_whose_windows_exceed_the_stage(count):
     """Thin spray beside and above a dense block: its blocks' windows cover the block's columns."""
@@ -93,7 +127,7 @@ def test_support_radii_inside_and_outside_the_packed_range(h, n):
 
 @pytest.mark.parametrize("count", [4000, 180000])
 def test_moving_box(count):
-    """The sort cells and the gather cells of a moving box round differently."""
+    """Six steps of a moving box (particles whose sort and gather cells differ: below)."""
     s = dataclasses.replace(block(count, seed=8), box_velocity=(0.37, -0.11, 0.23))
     check(s, steps=6)
 
