@@ -44,16 +44,13 @@ __device__ __forceinline__ float cubic_gradient_scale(const float distance, cons
     return __fdiv_rn(__fmul_rn(k.cubic_coefficient, derivative), __fmul_rn(k.h, distance));
 }
 
-// ---- two pairs at a time (pbf_math.cuh): the same correctly rounded values for fast_min <= r2 <= fast_max,
-// as zeros at and beyond the support.  `ns`: the negated distances of negated_lengths().
+// ---- two pairs at a time (pbf_math.cuh): the same correctly rounded values for fast_min <= r2 <
+// support_threshold, and some value beyond, up to fast_max.  `ns`: the negated distances of negated_lengths().
 __device__ __forceinline__ float2 negated_lengths(const float2 nr2, float2& approximate_inverse) {
     const float2 y = make_float2(approximate_rsqrt(-nr2.x), approximate_rsqrt(-nr2.y));
     const float2 ns0 = __fmul2_rn(nr2, y);
     approximate_inverse = y;
     return __ffma2_rn(__ffma2_rn(ns0, ns0, nr2), __fmul2_rn(y, both(0.5F)), ns0);
-}
-__device__ __forceinline__ float2 within(const float2 nr2, const float2 inside, const SphConstants& k) {
-    return make_float2(-nr2.x < k.support_threshold ? inside.x : 0.0F, -nr2.y < k.support_threshold ? inside.y : 0.0F);
 }
 __device__ __forceinline__ float2 near_or_far(const float2 negated_q, const float2 near, const float2 far) {
     return make_float2(negated_q.x >= -0.5F ? near.x : far.x, negated_q.y >= -0.5F ? near.y : far.y);
@@ -70,7 +67,7 @@ __device__ __forceinline__ float2 cubic_pair(const float2 nr2, const SphConstant
     const float2 near = __fmul2_rn(both(k.cubic_coefficient), __ffma2_rn(__ffma2_rn(t, nq, t), both(-1.0F), both(1.0F)));
     const float2 d = __fadd2_rn(both(1.0F), nq);
     const float2 far = __fmul2_rn(__fmul2_rn(__fmul2_rn(both(k.cubic_coefficient_2), d), d), d);
-    return within(nr2, near_or_far(nq, near, far), k);
+    return near_or_far(nq, near, far);
 }
 // cubic_gradient_scale of both pairs.  The reciprocal of h r starts from y / h, a relative error of at
 // most 2^-21.4 whose square 2^-42 covers, so it rounds up within 2^-18 ulp of the correctly rounded one.
@@ -85,11 +82,14 @@ __device__ __forceinline__ float2 cubic_gradient_pair(const float2 nr2, const Sp
     const float2 nb = __fmul2_rn(both(k.h), ns);
     const float2 start = __fmul2_rn(y, both(k.inverse_h));
     const float2 e = __fadd2_rn(__ffma2_rn(nb, start, both(1.0F)), both(0x1p-42F));
-    return within(nr2, quotient_pair(a, nb, __ffma2_rn(e, start, start)), k);
+    return quotient_pair(a, nb, __ffma2_rn(e, start, start));
 }
 __device__ __forceinline__ bool in_range(const float2 nr2, const SphConstants& k) {
     return -nr2.x <= k.fast_max && -nr2.x >= k.fast_min && -nr2.y <= k.fast_max && -nr2.y >= k.fast_min;
 }
+// Whether a pair is inside the support.  Lists hold pairs beyond it (their skin), whose mass or pressure may be
+// infinite: they are left out of the sums.
+__device__ __forceinline__ bool inside(const float negated_r2, const SphConstants& k) { return -negated_r2 < k.support_threshold; }
 // Any r2: the weight, 0 outside the support; the gradient scale, 0 where the pair has no gradient.
 static __device__ __noinline__ float any_cubic(const float r2, const SphConstants* k) {
     const float distance = __fsqrt_rn(r2);

@@ -5,8 +5,7 @@
 // predicted-density and pressure pass replays.  Those are most of a PCISPH, IISPH or DFSPH substep.
 // Through L1 they waited on scattered loads and spent most of their instructions on IEEE roots and
 // divisions, one pair at a time; from shared memory they take two pairs at a time with the packed
-// arithmetic of sph_math.cuh.  Lists carry a skin (sph.cu), so the packed values include the zeros
-// beyond the support; such a pair is left out of the sums, as its mass or pressure may be infinite.  Every sum keeps the reference's order and rounding.
+// arithmetic of sph_math.cuh.  Lists carry a skin (sph.cu); pairs in it are left out of the sums.  Every sum keeps the reference's order and rounding.
 //
 // A DFSPH substep at 270k particles (ten pressure iterations) went from 1.378 to 1.104 ms, a WCSPH substep at
 // 1M, which uses the scan alone, from 0.665 to 0.634.  The force and non-pressure passes stay per lane: they
@@ -66,10 +65,10 @@ __global__ void __launch_bounds__(kBlockParticles, 6) staged_sph_density_kernel(
             float2 weight = cubic_pair(nr2, k);
             if (!in_range(nr2, k)) weight = make_float2(any_cubic(-nr2.x, &k), any_cubic(-nr2.y, &k));
             if (at == hits.before) density = __fmaf_rn(o.mass, own_weight, density);
-            if (weight.x != 0.0F) density = __fmaf_rn(field[3][i0], weight.x, density);
+            if (inside(nr2.x, k)) density = __fmaf_rn(field[3][i0], weight.x, density);
             if (second) {
                 if (at + 1u == hits.before) density = __fmaf_rn(o.mass, own_weight, density);
-                if (weight.y != 0.0F) density = __fmaf_rn(field[3][i1], weight.y, density);
+                if (inside(nr2.y, k)) density = __fmaf_rn(field[3][i1], weight.y, density);
             }
         });
         if (hits.before == hits.count) density = __fmaf_rn(o.mass, own_weight, density);
@@ -131,10 +130,10 @@ __global__ void __launch_bounds__(kBlockParticles, 8) staged_predicted_density_k
             float2 weight = cubic_pair(nr2, k);
             if (!in_range(nr2, k)) weight = make_float2(any_cubic(-nr2.x, &k), any_cubic(-nr2.y, &k));
             if (at == before) density = __fmaf_rn(o.mass, own_weight, density);
-            if (weight.x != 0.0F) density = __fmaf_rn(q0.w, weight.x, density);
+            if (inside(nr2.x, k)) density = __fmaf_rn(q0.w, weight.x, density);
             if (second) {
                 if (at + 1u == before) density = __fmaf_rn(o.mass, own_weight, density);
-                if (weight.y != 0.0F) density = __fmaf_rn(q1.w, weight.y, density);
+                if (inside(nr2.y, k)) density = __fmaf_rn(q1.w, weight.y, density);
             }
             at += 2u;
         });
@@ -186,12 +185,16 @@ __global__ void __launch_bounds__(kBlockParticles, 7) staged_pressure_kernel(con
             const float4 q0 = positions[i0], q1 = positions[i1];
             const f3 d0 = sub(o.x, xyz(q0)), d1 = sub(o.x, xyz(q1));
             const float2 nr2 = negated_squares(d0, d1);
+            float f0 = __fmul_rn(-q0.w, __fadd_rn(first, term[0][i0]));
+            float f1 = __fmul_rn(-q1.w, __fadd_rn(first, term[0][i1]));
             float2 slope = cubic_gradient_pair(nr2, k);
-            if (!in_range(nr2, k)) slope = make_float2(any_cubic_gradient(-nr2.x, &k), any_cubic_gradient(-nr2.y, &k));
-            const float f0 = __fmul_rn(-q0.w, __fadd_rn(first, term[0][i0]));
-            const float f1 = __fmul_rn(-q1.w, __fadd_rn(first, term[0][i1]));
-            if (slope.x != 0.0F) acceleration = fma3(f0, scale(d0, slope.x), acceleration);
-            if (second && slope.y != 0.0F) acceleration = fma3(f1, scale(d1, slope.y), acceleration);
+            if (!in_range(nr2, k)) {
+                slope = make_float2(any_cubic_gradient(-nr2.x, &k), any_cubic_gradient(-nr2.y, &k));
+                if (nr2.x == 0.0F) f0 = 0.0F;   // coincident particles: no gradient, whatever the pressures
+                if (nr2.y == 0.0F) f1 = 0.0F;
+            }
+            if (inside(nr2.x, k)) acceleration = fma3(f0, scale(d0, slope.x), acceleration);
+            if (second && inside(nr2.y, k)) acceleration = fma3(f1, scale(d1, slope.y), acceleration);
         });
     } else {
         PressureOp<false> op;

@@ -152,9 +152,14 @@ __global__ void cubic_kernel(const float h, const uint32_t n, unsigned long long
     const float distance = __fsqrt_rn(r2);
     const float weight = distance < h ? sph::detail::cubic_inside(distance, k) : 0.0F;
     const float slope = distance < h ? sph::detail::cubic_gradient_scale(distance, k) : 0.0F;
-    count(bad, differs(sph::detail::cubic_pair(nr2, k).y, weight) || differs(sph::detail::any_cubic(r2, &k), weight));
+    count(bad, differs(sph::detail::any_cubic(r2, &k), weight) || differs(sph::detail::any_cubic_gradient(r2, &k), slope));
+    if (!sph::detail::inside(-r2, k)) {
+        count(bad, distance < h);
+        return;
+    }
+    count(bad, differs(sph::detail::cubic_pair(nr2, k).y, weight));
     const float packed = sph::detail::cubic_gradient_pair(nr2, k).y;   // a zero's sign may differ
-    count(bad, packed != slope || differs(sph::detail::any_cubic_gradient(r2, &k), slope));
+    count(bad, packed != slope);
 }
 
 unsigned long long* counter() {
