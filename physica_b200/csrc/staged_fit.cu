@@ -1,5 +1,4 @@
 // The measurement behind staged_fit.h.
-#include <algorithm>
 #include <mutex>
 #include <vector>
 
@@ -14,41 +13,49 @@ namespace {
 
 using namespace staged_detail;
 
-constexpr uint32_t kEvery = 16;            // steps
-constexpr uint32_t kSampledBlocks = 1024;  // blocks looked at, evenly spread
+// Steps from one measurement to the next: 7 us against a step of 0.09 ms (5k particles) or 0.5 ms (262k).
+constexpr uint32_t kEvery[4] = {8, 16, 8, 16};
 
-// The staged passes pay while at most `unfit` of the warps hold a particle without room, or, where the per-lane
-// passes would overflow their lists, once more than `crowded` of them hold one with more than `candidates`.
-// A sphere of the support radius holds 4 pi / 3 / 27 of its stencil's particles, so 598 candidates fill a list
-// of kListCapacity at an even density.
-// Staged / per lane, ms a step, at the shares on either side of each line:
-//   forward, 262k: unfit 0.02 0.551 / 0.612, 0.18 0.731 / 0.668; crowded 0.01 1.920 / 1.799, 0.53 1.992 / 2.211
-//   grouped, 14k: unfit 0.002 0.176 / 0.215, 0.07 0.275 / 0.232; more than 500 candidates (smaller scenes wait for
-//     the few lists that the later iterations overflow): 0.12 0.428 / 0.391, 0.59 0.459 / 0.761
-//   differentiable, 600k, which write both lists: unfit 0.02 1.089 / 1.144, 0.05 1.239 / 1.222; crowded 0.59
-//     5.744 / 3.942, 0.82 6.276 / 9.115
-//   SPH (PCISPH), 262k: unfit 0.02 0.890 / 0.931, 0.18 1.090 / 1.032; crowded ones fall back to the per-lane lists
+// The staged passes pay while few of the warps hold a particle without room: at most `columns` of them one whose
+// stencil columns outgrow its hit record, which leaves its warp waiting in every pass, and at most `unfit` one
+// of either kind (a block whose windows outgrow the stage costs its own time only).  They also pay, up to half of
+// the warps, where any particle has more than `candidates`: it overflows the per-lane passes' list, and a stencil walk
+// takes as long as its whole scene; and above, once `crowded` of the warps do.  A sphere of the support radius
+// holds 4 pi / 3 / 27 of its stencil's particles, so 598 candidates fill a list of kListCapacity at an even density.
+// Staged / per lane, ms a step (lattices by the spacings in a radius; dam breaks by the step; shares of columns, all):
+//   forward, 262k and 1M: 2.15 (0.18, 0.18) 0.731 / 0.668; step 20 (0.08, 0.12) 0.929 / 0.907; 1M step 25 (0.09, 0.12)
+//     4.65 / 5.27; 256 scenes step 40 (0.10, 0.26) 10.73 / 10.38; a few crowded ones at step 60 (0.11, 0.20) 1.302 / 1.879;
+//     crowded 0.01 at 2.7 1.920 / 1.799, 0.53 at 2.8 1.992 / 2.211
+//   grouped, 14k: 2.1 (0, 0) 0.176 / 0.215, 2.15 (0.07, 0.07) 0.275 / 0.232; step 100 (0, 0.14) 0.235 / 0.251; more than 500
+//     candidates (such scenes wait for the few lists that the later iterations overflow): 0.12 0.428 / 0.391, 0.59 0.459 / 0.761
+//   differentiable, which write both lists: 32 scenes step 20 (0.02, 0.07) 5.74 / 5.96, step 2 (0, 0.22) 5.61 / 4.93; 600k
+//     2.1 (0.05, 0.05) 1.239 / 1.222, 2.15 (0.2, 0.2) 1.634 / 1.327; crowded 0.59 5.744 / 3.942, 0.82 6.276 / 9.115
+//   SPH (PCISPH), 262k: 2.1 (0.02, 0.02) 0.890 / 0.931, 2.15 (0.18, 0.18) 1.090 / 1.032; crowded ones fall back to the
+//     per-lane lists
 struct Limits {
     uint32_t candidates;
-    float unfit, crowded;
+    float columns, unfit, crowded;
 };
-constexpr Limits kLimits[4] = {{598u, 1.0F / 16.0F, 0.5F}, {500u, 1.0F / 16.0F, 0.25F}, {598u, 1.0F / 32.0F, 0.7F},
-                               {~0u, 1.0F / 16.0F, 1.0F}};
+constexpr Limits kLimits[4] = {{598u, 0.15F, 0.2F, 0.5F}, {500u, 0.03F, 0.2F, 0.25F}, {598u, 0.1F, 0.1F, 0.7F},
+                               {~0u, 0.06F, 0.15F, 1.0F}};
+constexpr float kCrowdedUnfit = 0.5F;
+
+enum Share { kColumns, kUnfit, kCrowded, kShares };
 
 struct FitArgs {
     GatherCommon g;
-    uint32_t particles, capacity, candidates, stride, tag;
-    uint32_t* counts;   // unfit warps, crowded warps, warps, blocks done; zero before and after
-    uint64_t* result;   // the tag and both shares, in units of 1 / 65535
+    uint32_t capacity, candidates, tag;
+    uint32_t* counts;   // warps of each share, then blocks done; zero before and after
+    uint64_t* result;   // the tag and the shares, 16 bits each, in units of 1 / 65535, rounded up
 };
 
 __global__ void __launch_bounds__(kBlockParticles) staged_fit_kernel(const FitArgs a) {
     after_predecessor();
     __shared__ Windows w;
-    __shared__ uint32_t unfit_warps, crowded_warps;
-    const uint32_t first = blockIdx.x * a.stride * a.particles;
-    const uint32_t last = min(first + a.particles, a.g.count) - 1u;
-    if (threadIdx.x == 0u) unfit_warps = crowded_warps = 0u;
+    __shared__ uint32_t warps[kShares];
+    const uint32_t first = blockIdx.x * blockDim.x;
+    const uint32_t last = min(first + blockDim.x, a.g.count) - 1u;
+    if (threadIdx.x < kShares) warps[threadIdx.x] = 0u;
     find_windows(w, a.g, first, last, a.capacity);
     __syncthreads();
     const uint32_t s = first + threadIdx.x;
@@ -69,24 +76,27 @@ __global__ void __launch_bounds__(kBlockParticles) staged_fit_kernel(const FitAr
             candidates += end - begin;
         }
     }
+    const bool columns = __any_sync(kFull, longest > kColumn);
     const bool unfit = __any_sync(kFull, s <= last && (w.staged == 0u || longest > kColumn));
     const bool crowded = __any_sync(kFull, candidates > a.candidates);
     if (lane_id() == 0u) {
-        if (unfit) atomicAdd(&unfit_warps, 1u);
-        if (crowded) atomicAdd(&crowded_warps, 1u);
+        if (columns) atomicAdd(&warps[kColumns], 1u);
+        if (unfit) atomicAdd(&warps[kUnfit], 1u);
+        if (crowded) atomicAdd(&warps[kCrowded], 1u);
     }
     __syncthreads();
     if (threadIdx.x != 0u) return;
-    if (unfit_warps) atomicAdd(a.counts, unfit_warps);
-    if (crowded_warps) atomicAdd(a.counts + 1, crowded_warps);
-    atomicAdd(a.counts + 2, (last - first) / 32u + 1u);
+    for (int k = 0; k < kShares; ++k)
+        if (warps[k]) atomicAdd(a.counts + k, warps[k]);
     __threadfence();
-    if (atomicAdd(a.counts + 3, 1u) != gridDim.x - 1u) return;
+    if (atomicAdd(a.counts + kShares, 1u) != gridDim.x - 1u) return;
     __threadfence();
-    const uint32_t total_unfit = atomicExch(a.counts, 0u), total_crowded = atomicExch(a.counts + 1, 0u);
-    const uint32_t warps = atomicExch(a.counts + 2, 0u);
-    atomicExch(a.counts + 3, 0u);
-    *a.result = (static_cast<uint64_t>(a.tag) << 32) | ((total_unfit * 65535u / warps) << 16) | (total_crowded * 65535u / warps);
+    const float unit = 65535.0F / static_cast<float>((a.g.count + 31u) / 32u);
+    uint64_t result = static_cast<uint64_t>(a.tag) << 48;
+    for (int k = 0; k < kShares; ++k)
+        result |= static_cast<uint64_t>(min(__float2uint_ru(static_cast<float>(atomicExch(a.counts + k, 0u)) * unit), 65535u)) << (16 * k);
+    atomicExch(a.counts + kShares, 0u);
+    *a.result = result;
 }
 
 // Pinned words, one a solver, of one page that lives as long as the process; a solver beyond them measures
@@ -111,7 +121,7 @@ public:
         if (free_.empty()) return nullptr;
         uint64_t* word = free_.back();
         free_.pop_back();
-        if (++tag_ == 0u) ++tag_;
+        if (++tag_ == 0x10000u) tag_ = 1u;
         tag = tag_;
         return word;
     }
@@ -141,15 +151,15 @@ StagedFit::~StagedFit() {
 cudaError_t StagedFit::init(DeviceArena& arena, cudaStream_t stream, const Kind kind) {
     kind_ = kind;
     cudaError_t e = cudaSuccess;
-    counts_ = arena.alloc<uint32_t>(4, e);
-    if (e == cudaSuccess) e = cudaMemsetAsync(counts_, 0, 4 * sizeof(uint32_t), stream);
+    counts_ = arena.alloc<uint32_t>(kShares + 1, e);
+    if (e == cudaSuccess) e = cudaMemsetAsync(counts_, 0, (kShares + 1) * sizeof(uint32_t), stream);
     if (e == cudaSuccess) word_ = pinned_words().take(tag_);
     return e;
 }
 
 cudaError_t StagedFit::measure(cudaStream_t stream, const GatherCommon& g) {
     if (!word_ || g.count == 0) return cudaSuccess;
-    if (calls_ % kEvery != 0u) {
+    if (calls_ % kEvery[kind_] != 0u) {
         ++calls_;
         return cudaSuccess;
     }
@@ -160,10 +170,8 @@ cudaError_t StagedFit::measure(cudaStream_t stream, const GatherCommon& g) {
     }
     ++calls_;
     const uint32_t particles = kind_ == kGrouped ? kGroupParticles : kBlockParticles;
-    const uint32_t blocks = (g.count + particles - 1u) / particles;
-    const uint32_t stride = std::max(1u, blocks / kSampledBlocks);
-    launch_after(stream, staged_fit_kernel, (blocks + stride - 1u) / stride, particles,
-                 FitArgs{g, particles, kind_ == kGrouped ? kGroupStage : kStage, kLimits[kind_].candidates, stride, tag_, counts_, word_});
+    launch_after(stream, staged_fit_kernel, (g.count + particles - 1u) / particles, particles,
+                 FitArgs{g, kind_ == kGrouped ? kGroupStage : kStage, kLimits[kind_].candidates, tag_, counts_, word_});
     count_launch();
     return cudaGetLastError();
 }
@@ -171,10 +179,11 @@ cudaError_t StagedFit::measure(cudaStream_t stream, const GatherCommon& g) {
 bool StagedFit::pays() const {
     if (!word_) return true;
     const uint64_t word = *static_cast<const volatile uint64_t*>(word_);
-    if (static_cast<uint32_t>(word >> 32) != tag_) return true;   // not measured yet
-    const float unfit = static_cast<float>((word >> 16) & 0xffffu) / 65535.0F;
-    const float crowded = static_cast<float>(word & 0xffffu) / 65535.0F;
-    return unfit <= kLimits[kind_].unfit || crowded > kLimits[kind_].crowded;
+    if (static_cast<uint32_t>(word >> 48) != tag_) return true;   // not measured yet
+    auto share = [word](const Share k) { return static_cast<float>((word >> (16 * k)) & 0xffffu) / 65535.0F; };
+    const Limits& limits = kLimits[kind_];
+    return (share(kColumns) <= limits.columns && share(kUnfit) <= limits.unfit) ||
+           (share(kCrowded) > 0.0F && share(kUnfit) <= kCrowdedUnfit) || share(kCrowded) > limits.crowded;
 }
 
 }  // namespace pbf

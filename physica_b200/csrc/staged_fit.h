@@ -3,12 +3,12 @@
 // The windows and hit records of the staged passes have room for about 10 particles a cell, support radii of
 // 2.15 spacings.  A particle or block without room falls back inside the staged kernels, and where many do,
 // scanning in vain and warps that wait for their slowest lane cost more than the per-lane passes take
-// altogether: staged / per lane at 262k particles, ms a step of three iterations, 0.502 / 0.569 at a radius of 2 spacings, 0.551 / 0.612 at
-// 2.1, 0.731 / 0.668 at 2.15, 0.840 / 0.722 at 2.2, 1.531 / 1.031 at 2.4, 1.820 / 1.245 at 2.6.  From 2.8 spacings on the
-// per-lane lists overflow (1.992 / 2.211, and 2.445 / 4.766 at 3).  How dense the particles are is known on the device only, so every 16th step ends with a
-// small kernel that looks at its cell offsets and leaves two shares in pinned host memory, and later steps are
-// routed by them: nothing waits, and both routes give the same bits.  Until a first measurement has arrived
-// a solver takes the staged passes.
+// altogether: staged / per lane at 262k particles, ms a step of three iterations, 0.502 / 0.569 at a radius of 2
+// spacings, 0.551 / 0.612 at 2.1, 0.731 / 0.668 at 2.15, 0.840 / 0.722 at 2.2, 1.531 / 1.031 at 2.4, 1.820 / 1.245 at 2.6.
+// From 2.8 spacings on the per-lane lists overflow (1.992 / 2.211, and 2.445 / 4.766 at 3).  How dense the particles are
+// is known on the device only, so every 8th or 16th step ends with a small kernel that looks at its cell offsets and
+// leaves three shares in pinned host memory, and later steps are routed by them: nothing waits, and both routes
+// give the same bits.  Until a first measurement has arrived a solver takes the staged passes.
 #pragma once
 
 #include <cstdint>
@@ -36,7 +36,7 @@ public:
 
 private:
     uint32_t* counts_ = nullptr;        // device scratch
-    uint64_t* word_ = nullptr;          // pinned: tag, share of unfit warps, share of crowded ones
+    uint64_t* word_ = nullptr;          // pinned: a tag and the shares measured
     uint32_t tag_ = 0;                  // of this object: a word is used again after its solver is gone
     uint32_t calls_ = 0;
     Kind kind_ = kForward;
