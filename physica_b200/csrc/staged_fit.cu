@@ -1,4 +1,5 @@
 // The measurement behind staged_fit.h.
+#include <algorithm>
 #include <mutex>
 #include <vector>
 
@@ -13,8 +14,11 @@ namespace {
 
 using namespace staged_detail;
 
-// Steps from one measurement to the next: 7 us against a step of 0.09 ms (5k particles) or 0.5 ms (262k).
-constexpr uint32_t kEvery[4] = {8, 16, 8, 16};
+// Blocks of the measurement's kernel: about as many as are resident at once, since each ends with an atomic on one word.
+constexpr uint32_t kMaxBlocks = 2048;
+// Steps from one measurement to the next.  A measurement takes 8 us at 5k particles, 10 at 262k, 24 at 1M (SPH: 9), a step
+// 0.09, 0.5 and 3.4 ms, a differentiable one (2^19 particles or more) 1 ms and up.
+constexpr uint32_t kEvery[4] = {8, 16, 4, 16};
 
 // The staged passes pay while few of the warps hold a particle without room: at most `columns` of them one whose
 // stencil columns outgrow its hit record, which leaves its warp waiting in every pass, and at most `unfit` one
@@ -44,7 +48,7 @@ enum Share { kColumns, kUnfit, kCrowded, kShares };
 
 struct FitArgs {
     GatherCommon g;
-    uint32_t capacity, candidates, tag;
+    uint32_t blocks, stride, capacity, candidates, tag;   // every stride-th block
     uint32_t* counts;   // warps of each share, then blocks done; zero before and after
     uint64_t* result;   // the tag and the shares, 16 bits each, in units of 1 / 65535, rounded up
 };
@@ -53,36 +57,39 @@ __global__ void __launch_bounds__(kBlockParticles) staged_fit_kernel(const FitAr
     after_predecessor();
     __shared__ Windows w;
     __shared__ uint32_t warps[kShares];
-    const uint32_t first = blockIdx.x * blockDim.x;
-    const uint32_t last = min(first + blockDim.x, a.g.count) - 1u;
     if (threadIdx.x < kShares) warps[threadIdx.x] = 0u;
-    find_windows(w, a.g, first, last, a.capacity);
-    __syncthreads();
-    const uint32_t s = first + threadIdx.x;
-    uint32_t longest = 0u, candidates = 0u;
-    if (s <= last) {
-        const int4 c = a.g.cell[s];
-        const Grid& grid = a.g.scenes[c.w].grid;
-        const int cx = static_cast<int>(grid.cells_x), cy = static_cast<int>(grid.cells_y), cz = static_cast<int>(grid.cells_z);
-        const uint32_t z_lo = static_cast<uint32_t>(c.z > 0 ? c.z - 1 : 0);
-        const uint32_t z_hi = static_cast<uint32_t>(c.z + 1 < cz ? c.z + 1 : cz - 1);
-        for (int o = 0; o < 9; ++o) {
-            const int x = c.x + o / 3 - 1, y = c.y + o % 3 - 1;
-            if (x < 0 || x >= cx || y < 0 || y >= cy) continue;
-            const uint32_t begin = a.g.cell_offsets[cell_index(grid, x, y, z_lo)];
-            const uint32_t end = a.g.cell_offsets[cell_index(grid, x, y, z_hi) + 1u];
-            if (begin >= end) continue;
-            longest = max(longest, end - (begin & ~3u));
-            candidates += end - begin;
+    for (uint32_t block = blockIdx.x; block < a.blocks; block += gridDim.x) {
+        const uint32_t first = block * a.stride * blockDim.x;
+        const uint32_t last = min(first + blockDim.x, a.g.count) - 1u;
+        __syncthreads();
+        find_windows(w, a.g, first, last, a.capacity);
+        __syncthreads();
+        const uint32_t s = first + threadIdx.x;
+        uint32_t longest = 0u, candidates = 0u;
+        if (s <= last) {
+            const int4 c = a.g.cell[s];
+            const Grid& grid = a.g.scenes[c.w].grid;
+            const int cx = static_cast<int>(grid.cells_x), cy = static_cast<int>(grid.cells_y), cz = static_cast<int>(grid.cells_z);
+            const uint32_t z_lo = static_cast<uint32_t>(c.z > 0 ? c.z - 1 : 0);
+            const uint32_t z_hi = static_cast<uint32_t>(c.z + 1 < cz ? c.z + 1 : cz - 1);
+            for (int o = 0; o < 9; ++o) {
+                const int x = c.x + o / 3 - 1, y = c.y + o % 3 - 1;
+                if (x < 0 || x >= cx || y < 0 || y >= cy) continue;
+                const uint32_t begin = a.g.cell_offsets[cell_index(grid, x, y, z_lo)];
+                const uint32_t end = a.g.cell_offsets[cell_index(grid, x, y, z_hi) + 1u];
+                if (begin >= end) continue;
+                longest = max(longest, end - (begin & ~3u));
+                candidates += end - begin;
+            }
         }
-    }
-    const bool columns = __any_sync(kFull, longest > kColumn);
-    const bool unfit = __any_sync(kFull, s <= last && (w.staged == 0u || longest > kColumn));
-    const bool crowded = __any_sync(kFull, candidates > a.candidates);
-    if (lane_id() == 0u) {
-        if (columns) atomicAdd(&warps[kColumns], 1u);
-        if (unfit) atomicAdd(&warps[kUnfit], 1u);
-        if (crowded) atomicAdd(&warps[kCrowded], 1u);
+        const bool columns = __any_sync(kFull, longest > kColumn);
+        const bool unfit = __any_sync(kFull, s <= last && (w.staged == 0u || longest > kColumn));
+        const bool crowded = __any_sync(kFull, candidates > a.candidates);
+        if (lane_id() == 0u) {
+            if (columns) atomicAdd(&warps[kColumns], 1u);
+            if (unfit) atomicAdd(&warps[kUnfit], 1u);
+            if (crowded) atomicAdd(&warps[kCrowded], 1u);
+        }
     }
     __syncthreads();
     if (threadIdx.x != 0u) return;
@@ -91,7 +98,7 @@ __global__ void __launch_bounds__(kBlockParticles) staged_fit_kernel(const FitAr
     __threadfence();
     if (atomicAdd(a.counts + kShares, 1u) != gridDim.x - 1u) return;
     __threadfence();
-    const float unit = 65535.0F / static_cast<float>((a.g.count + 31u) / 32u);
+    const float unit = 65535.0F * static_cast<float>(a.stride) / static_cast<float>((a.g.count + 31u) / 32u);
     uint64_t result = static_cast<uint64_t>(a.tag) << 48;
     for (int k = 0; k < kShares; ++k)
         result |= static_cast<uint64_t>(min(__float2uint_ru(static_cast<float>(atomicExch(a.counts + k, 0u)) * unit), 65535u)) << (16 * k);
@@ -170,8 +177,13 @@ cudaError_t StagedFit::measure(cudaStream_t stream, const GatherCommon& g) {
     }
     ++calls_;
     const uint32_t particles = kind_ == kGrouped ? kGroupParticles : kBlockParticles;
-    launch_after(stream, staged_fit_kernel, (g.count + particles - 1u) / particles, particles,
-                 FitArgs{g, kind_ == kGrouped ? kGroupStage : kStage, kLimits[kind_].candidates, tag_, counts_, word_});
+    // Every block where one crowded particle decides; an SPH step of 1M particles is as short as 0.6 ms, and 1024 of its
+    // blocks tell its shares.
+    const uint32_t all = (g.count + particles - 1u) / particles;
+    const uint32_t stride = kind_ == kSph ? std::max(1u, all / 1024u) : 1u;
+    const uint32_t blocks = (all + stride - 1u) / stride;
+    launch_after(stream, staged_fit_kernel, std::min(blocks, kMaxBlocks), particles,
+                 FitArgs{g, blocks, stride, kind_ == kGrouped ? kGroupStage : kStage, kLimits[kind_].candidates, tag_, counts_, word_});
     count_launch();
     return cudaGetLastError();
 }

@@ -6,7 +6,7 @@
 // altogether: staged / per lane at 262k particles, ms a step of three iterations, 0.502 / 0.569 at a radius of 2
 // spacings, 0.551 / 0.612 at 2.1, 0.731 / 0.668 at 2.15, 0.840 / 0.722 at 2.2, 1.531 / 1.031 at 2.4, 1.820 / 1.245 at 2.6.
 // From 2.8 spacings on the per-lane lists overflow (1.992 / 2.211, and 2.445 / 4.766 at 3).  How dense the particles are
-// is known on the device only, so every 8th or 16th step ends with a small kernel that looks at its cell offsets and
+// is known on the device only, so every 4th to 16th step ends with a small kernel that looks at its cell offsets and
 // leaves three shares in pinned host memory, and later steps are routed by them: nothing waits, and both routes
 // give the same bits.  Until a first measurement has arrived a solver takes the staged passes.
 #pragma once
