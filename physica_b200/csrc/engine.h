@@ -17,6 +17,8 @@
 namespace pbf {
 
 void set_error(const std::string& message);
+// The process-unique ID of the current CUDA context, 0 when none is current (static_step.cu).
+int current_context_id(unsigned long long* id);
 
 // Stream-ordered device allocations released together.
 class DeviceArena {

@@ -1,7 +1,9 @@
 // The measurement behind staged_fit.h.
 #include <algorithm>
+#include <bitset>
+#include <cstdlib>
+#include <cstring>
 #include <mutex>
-#include <vector>
 
 #include "dependent_launch.cuh"
 #include "engine.h"
@@ -106,43 +108,71 @@ __global__ void __launch_bounds__(kBlockParticles) staged_fit_kernel(const FitAr
     *a.result = result;
 }
 
-// Pinned words, one a solver, of one page that lives as long as the process; a solver beyond them measures
-// nothing.
+// Pinned words, one a solver, in one page a CUDA context.  A page is host memory that is registered with its context and
+// kept, so a solver may read its word even after that context is gone (cudaDeviceReset).  A solver beyond
+// the words or pages there are measures nothing.
 class PinnedWords {
 public:
-    uint64_t* take(uint32_t& tag) {
+    struct Word {
+        uint64_t* host = nullptr;
+        uint64_t* device = nullptr;
+        uint32_t slot = 0, tag = 0;
+    };
+    Word take() {
+        unsigned long long context = 0;
+        if (current_context_id(&context) || context == 0) return {};
         const std::lock_guard<std::mutex> lock(mutex_);
-        if (!tried_) {
-            tried_ = true;
-            void* page = nullptr;
-            if (cudaHostAlloc(&page, kWords * sizeof(uint64_t), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
-                free_.reserve(kWords);
-                for (uint32_t k = 0; k < kWords; ++k) {
-                    static_cast<uint64_t*>(page)[k] = 0u;
-                    free_.push_back(static_cast<uint64_t*>(page) + k);
-                }
-            } else {
-                cudaGetLastError();
-            }
+        uint32_t p = 0;
+        while (p < used_ && pages_[p].context != context) ++p;
+        if (p == used_ && !add_page(context)) return {};
+        Page& page = pages_[p];
+        for (uint32_t k = 0; k < kWords; ++k) {
+            if (page.taken[k]) continue;
+            page.taken[k] = true;
+            if (++tag_ == 0x10000u) tag_ = 1u;
+            return {page.host + k, page.device + k, p * kWords + k, tag_};
         }
-        if (free_.empty()) return nullptr;
-        uint64_t* word = free_.back();
-        free_.pop_back();
-        if (++tag_ == 0x10000u) tag_ = 1u;
-        tag = tag_;
-        return word;
+        return {};
     }
-    void give(uint64_t* word) {
+    void give(const uint32_t slot) {
         const std::lock_guard<std::mutex> lock(mutex_);
-        free_.push_back(word);
+        pages_[slot / kWords].taken[slot % kWords] = false;
     }
 
 private:
-    static constexpr uint32_t kWords = 512;
+    static constexpr uint32_t kWords = 512, kPages = 16;
+    struct Page {
+        unsigned long long context = 0;
+        uint64_t* host = nullptr;
+        uint64_t* device = nullptr;
+        std::bitset<kWords> taken;
+    };
+    bool add_page(const unsigned long long context) {
+        if (used_ == kPages) return false;
+        void* host = std::aligned_alloc(4096, kWords * sizeof(uint64_t));
+        if (!host) return false;
+        std::memset(host, 0, kWords * sizeof(uint64_t));
+        // another thread may be capturing
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        void* device = nullptr;
+        cudaError_t e = cudaHostRegister(host, kWords * sizeof(uint64_t), cudaHostRegisterMapped);
+        if (e == cudaSuccess && (e = cudaHostGetDevicePointer(&device, host, 0)) != cudaSuccess) cudaHostUnregister(host);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            std::free(host);
+            return false;
+        }
+        pages_[used_].context = context;
+        pages_[used_].host = static_cast<uint64_t*>(host);
+        pages_[used_].device = static_cast<uint64_t*>(device);
+        ++used_;
+        return true;
+    }
     std::mutex mutex_;
-    std::vector<uint64_t*> free_;
-    uint32_t tag_ = 0;
-    bool tried_ = false;
+    Page pages_[kPages];
+    uint32_t used_ = 0, tag_ = 0;
 };
 PinnedWords& pinned_words() {
     static PinnedWords* words = new PinnedWords;   // outlives every solver
@@ -152,7 +182,7 @@ PinnedWords& pinned_words() {
 }  // namespace
 
 StagedFit::~StagedFit() {
-    if (word_) pinned_words().give(word_);
+    if (word_) pinned_words().give(slot_);
 }
 
 cudaError_t StagedFit::init(DeviceArena& arena, cudaStream_t stream, const Kind kind) {
@@ -160,8 +190,13 @@ cudaError_t StagedFit::init(DeviceArena& arena, cudaStream_t stream, const Kind 
     cudaError_t e = cudaSuccess;
     counts_ = arena.alloc<uint32_t>(kShares + 1, e);
     if (e == cudaSuccess) e = cudaMemsetAsync(counts_, 0, (kShares + 1) * sizeof(uint32_t), stream);
-    if (e == cudaSuccess) word_ = pinned_words().take(tag_);
-    return e;
+    if (e != cudaSuccess) return e;
+    const PinnedWords::Word word = pinned_words().take();
+    word_ = word.host;
+    device_word_ = word.device;
+    slot_ = word.slot;
+    tag_ = word.tag;
+    return cudaSuccess;
 }
 
 cudaError_t StagedFit::measure(cudaStream_t stream, const GatherCommon& g) {
@@ -183,7 +218,7 @@ cudaError_t StagedFit::measure(cudaStream_t stream, const GatherCommon& g) {
     const uint32_t stride = kind_ == kSph ? std::max(1u, all / 1024u) : 1u;
     const uint32_t blocks = (all + stride - 1u) / stride;
     launch_after(stream, staged_fit_kernel, std::min(blocks, kMaxBlocks), particles,
-                 FitArgs{g, blocks, stride, kind_ == kGrouped ? kGroupStage : kStage, kLimits[kind_].candidates, tag_, counts_, word_});
+                 FitArgs{g, blocks, stride, kind_ == kGrouped ? kGroupStage : kStage, kLimits[kind_].candidates, tag_, counts_, device_word_});
     count_launch();
     return cudaGetLastError();
 }

@@ -36,7 +36,9 @@ public:
 
 private:
     uint32_t* counts_ = nullptr;        // device scratch
-    uint64_t* word_ = nullptr;          // pinned: a tag and the shares measured
+    const uint64_t* word_ = nullptr;    // pinned: a tag and the shares measured
+    uint64_t* device_word_ = nullptr;   // the same for the device
+    uint32_t slot_ = 0;                 // its place among the pinned words
     uint32_t tag_ = 0;                  // of this object: a word is used again after its solver is gone
     uint32_t calls_ = 0;
     Kind kind_ = kForward;

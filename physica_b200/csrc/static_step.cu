@@ -366,6 +366,12 @@ int forward_preallocated(const pbf_domain_configuration* domain, const pbf_confi
 }
 
 }  // namespace
+
+int current_context_id(unsigned long long* id) {
+    const std::lock_guard<std::mutex> lock(g_setup_mutex);
+    return current_context(id);
+}
+
 }  // namespace pbf
 
 extern "C" {

@@ -146,3 +146,17 @@ def test_autotune_leaves_the_staged_passes_their_block_size():
     solver, state, control, params = pbf.solver_for_scene(lattice(8000, 2.0))
     shape, ms = solver.autotune(state, control, params, repeats=2)
     assert shape == pbf.LaunchShape(4, 128, 128) and ms > 0.0
+
+
+def test_a_solver_starts_unmeasured():
+    """Also where it takes the place of a solver whose particles did not fit, and among more solvers than can measure."""
+    _, launches = run(lattice(8000, 2.4), pbf.LaunchShape(4, 128, 128))
+    assert launches[1] == PBF_LAUNCHES[False]
+    made = pbf.solver_for_scene(lattice(8000, 2.0))
+    scene, others = lattice(27, 2.0), []
+    assert steps(*made, 2)[1][1] == PBF_LAUNCHES[True]
+    for _ in range(520):
+        others.append(pbf.solver_for_scene(scene))
+    for solver in (others[0], others[-1]):
+        assert steps(*solver, 3)[1][1:] == [PBF_LAUNCHES[True]] * 2
+    assert steps(*made, 2)[1][1] == PBF_LAUNCHES[True]
