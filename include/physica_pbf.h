@@ -155,7 +155,7 @@ typedef struct pbf_launch_shape {
     uint32_t list_scan;         /* 0: per-lane walk, 1: warp-cooperative scan, 2: shared-memory staged walk,
                                    3: per-lane walk with density + lambda in the same kernel,
                                    4 (the default): as 3, and steps without boundary particles run over windows
-                                   staged in shared memory at the sizes where that is faster */
+                                   staged in shared memory, or keep hit masks, where that is faster */
     uint32_t scan_block_size;   /* threads per block of the list scan: 32, 64, 96 or 128 */
     uint32_t block_size;        /* threads per block of the gather passes: 32, 64, 96 or 128 */
 } pbf_launch_shape;
@@ -343,7 +343,8 @@ int pbf_forward_step_preallocated(const pbf_domain_configuration* domain, const 
  *      in the same kernel, replaying the list from shared memory (scenes with boundary particles run
  *      3 as 0), 4 = as 3, and every pass of a step without boundary particles (of up to 20,480 or more than 170,496
  *      particles; in differentiable mode of at least 2^19) reads its neighbours from windows of the sorted particles
- *      staged in shared memory, unless the particles turn out to be too dense for that (the default);
+ *      staged in shared memory, unless the particles turn out to be too dense for that, and the other forward steps
+ *      keep hit masks in place of lists of slots where those are faster (the default);
  *      scan_block_size and block_size: 32, 64, 96 or 128 threads (the staged passes have their own).
  *      pbf_autotune times the list-scan shapes by their scans and gather passes, then, unless the staged passes won, the
  *      gather block sizes, on `repeats` forward steps from `state` (writing `scratch_state` and

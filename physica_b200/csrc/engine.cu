@@ -148,6 +148,10 @@ constexpr uint32_t kStagedDifferentiable = 1u << 19;
 // lanes are the fastest: a forward step at 5k particles 0.164 ms against 0.240 with one lane, at 14k
 // 0.228 / 0.253.  Two lanes never were (0.176, 0.253).
 constexpr uint32_t kGroupedParticles = 20480;
+// Above this many particles the per-lane passes of a forward step store hit masks rather than lists of slots, below it where some are so crowded that their lists overflow.  Hit masks / lists of slots,
+// ms a step: 32k 0.230 / 0.206, 60k 0.249 / 0.226, 110k 0.283 / 0.273, 130k 0.301 / 0.296, 149k 0.326 / 0.330, 169k 0.352 / 0.364, 262k
+// 0.561 / 0.573; at a radius of 3 spacings 60k 0.673 / 2.104, 262k 1.622 / 4.766.
+constexpr uint32_t kMaskLists = 140000;
 }  // namespace
 
 int Engine::init(const pbf_domain_configuration* scenes, const uint32_t scene_count, const pbf_configuration* configuration,
@@ -236,16 +240,18 @@ int Engine::init(const pbf_domain_configuration* scenes, const uint32_t scene_co
     // Per lane / staged, ms a step: 22k particles 0.263 / 0.274, 64k 0.305 / 0.321, 110k 0.363 / 0.403, 169k
     // 0.488 / 0.530, 198k 0.634 / 0.548, 246k 0.715 / 0.649, 295k 0.803 / 0.725.
     if (int rc = check(fused_scan_wave(one_wave_), "occupancy of the fused scan")) return rc;
+    // What a step's route depends on is measured where there is a choice.
+    if (!boundary && (may_run_staged(LaunchShape{}) || (may_store_masks(LaunchShape{}) && count_ <= kMaskLists)) && e == cudaSuccess)
+        e = fit_.init(arena_, stream_,
+                      differentiable() ? StagedFit::kDifferentiable
+                      : count_ <= kGroupedParticles ? StagedFit::kGrouped
+                      : count_ <= kMaskLists ? StagedFit::kMiddle : StagedFit::kForward);
     if (!boundary && may_run_staged(LaunchShape{})) {
         packed_next_ = alloc_packed(arena_, count_, e);
         packed_velocity_ = alloc_packed(arena_, count_, e);
         packed_mass_ = arena_.alloc<float>(static_cast<size_t>(count_) + 4u, e);
         packed_magnitude_ = arena_.alloc<float>(static_cast<size_t>(count_) + 4u, e);
         staged_list_.windows = arena_.alloc<uint32_t>(window_words(count_), e);
-        if (e == cudaSuccess)
-            e = fit_.init(arena_, stream_,
-                          mode == PBF_EXECUTION_DIFFERENTIABLE ? StagedFit::kDifferentiable
-                                                               : count_ <= kGroupedParticles ? StagedFit::kGrouped : StagedFit::kForward);
         if (mode == PBF_EXECUTION_DIFFERENTIABLE) {
             const size_t padded = (static_cast<size_t>(count_) + 31u) / 32u * 32u;
             staged_list_.list = {arena_.alloc<uint32_t>(padded * kListCapacity, e), arena_.alloc<uint32_t>(count_, e), kListCapacity};
@@ -349,7 +355,8 @@ int Engine::init(const pbf_domain_configuration* scenes, const uint32_t scene_co
 }
 
 bool Engine::GraphKey::operator==(const GraphKey& o) const {
-    if (record != o.record || positions_ready != o.positions_ready || staged != o.staged) return false;
+    if (record != o.record || positions_ready != o.positions_ready || staged != o.staged ||
+        masks != o.masks) return false;
     for (int k = 0; k < 16; ++k)
         if (p[k] != o.p[k]) return false;
     return true;
@@ -463,9 +470,11 @@ int Engine::forward(const pbf_particle_state* state, const pbf_control* control,
     host_step_ = ~0ull;   // unknown again if the step fails halfway
     int rc = PBF_SUCCESS;
     staged_step_ = may_run_staged(shape_) && fit_.pays();
+    mask_step_ = !staged_step_ && may_store_masks(shape_) && (count_ > kMaskLists || fit_.crowded());
     if (graphs_ && !timer_.enabled()) {
         GraphKey key{};
         key.staged = staged_step_;
+        key.masks = mask_step_;
         const void* ptrs[16] = {state->positions.x, state->positions.y, state->positions.z, state->velocities.x,
                                 state->velocities.y, state->velocities.z, control->external_accelerations.x,
                                 control->external_accelerations.y, control->external_accelerations.z, parameters->masses,
@@ -527,7 +536,7 @@ int Engine::forward(const pbf_particle_state* state, const pbf_control* control,
     next_state->step_index = state->step_index + 1u;
     r.valid = true;
     r.step_index = state->step_index;
-    return may_run_staged(shape_) ? check(fit_.measure(stream_, gather_common(r)), "staged fit") : PBF_SUCCESS;
+    return shape_.scan == kScanStaged16 ? check(fit_.measure(stream_, gather_common(r)), "staged fit") : PBF_SUCCESS;
 }
 
 int Engine::read_input_checks(uint32_t* flags) {
@@ -596,6 +605,7 @@ int Engine::launch_forward(cudaStream_t stream, const pbf_particle_state* state,
     timer_.end(stream, kPassGrid);
 
     if (staged_step_) return launch_staged(stream, state, next_state, r);
+    const int masks = mask_step_ ? 1 : 0;
     const GatherCommon gc = gather_common(r);
     const Field3 previous{state->positions.x, state->positions.y, state->positions.z};
     const MutField3 out_positions{next_state->positions.x, next_state->positions.y, next_state->positions.z};
@@ -604,7 +614,7 @@ int Engine::launch_forward(cudaStream_t stream, const pbf_particle_state* state,
         float4* xk1 = const_cast<float4*>(r.iterate(k + 1, K, diff));
         float* lam = keep ? r.lambda[k] : (k == 0 ? r.first_lambda : r.lambda[0]);
         const uint32_t l = keep ? k : 0u;
-        const StoredList list{r.list_entries[l], r.list_counts[l], r.list_capacity};
+        const StoredList list{r.list_entries[l], r.list_counts[l], r.list_capacity, masks};
         ListScanArgs scan{gc, xk, list, 1};
         scan.packed = packed_;
         DensityLambdaArgs d{gc, xk, lam, keep ? r.density[k] : (k == 0 ? r.first_density : nullptr),
@@ -642,7 +652,7 @@ int Engine::launch_forward(cudaStream_t stream, const pbf_particle_state* state,
     }
     if (int rc = record_positions_ready(stream)) return rc;
     const uint32_t lp = keep ? K : 0u;
-    const StoredList post{r.list_entries[lp], r.list_counts[lp], r.list_capacity};
+    const StoredList post{r.list_entries[lp], r.list_counts[lp], r.list_capacity, masks};
     timer_.begin(stream, kPassListScan);
     ListScanArgs post_scan{gc, xK, post};
     post_scan.packed = packed_;
@@ -682,6 +692,10 @@ bool Engine::may_run_staged(const LaunchShape& shape) const {
     if (!runs_staged(shape, boundary_count_ > 0, iterations_)) return false;
     if (differentiable()) return count_ >= kStagedDifferentiable && packed_radii_;
     return count_ <= kGroupedParticles || (count_ > one_wave_ && packed_radii_);
+}
+
+bool Engine::may_store_masks(const LaunchShape& shape) const {
+    return shape.scan == kScanStaged16 && !differentiable() && boundary_count_ == 0 && count_ > kGroupedParticles;
 }
 
 // The Jacobi iterations and the post-loop passes over staged windows (staged.cu, staged_group.cu): two
@@ -856,7 +870,7 @@ int Engine::autotune(const pbf_particle_state* state, const pbf_control* control
         for (int p = 0; p < kPassCount; ++p) sum += ms[p];
         return sum;
     };
-    // Steps that cannot be staged run variant 4 as 3, staged ones have block sizes of their own.
+    // staged steps have block sizes of their own
     const bool staged = may_run_staged(LaunchShape{kScanStaged16, 128u, 128u});
     // 1. the list scan: variant x block size, by the time of the scans and the gather passes (the
     //    variants differ in which passes they fuse)
@@ -865,7 +879,6 @@ int Engine::autotune(const pbf_particle_state* state, const pbf_control* control
     double best_scan = -1.0, best_gather = -1.0, best_total = 0.0;
     for (int v = 0; v < 5 && !rc; ++v)
         for (int b = 0; b < 4 && !rc; ++b) {
-            if (!staged && scans[v] == kScanFusedDensity) continue;
             if (staged && scans[v] == kScanStaged16 && b != 3) continue;
             shape_ = best;
             shape_.scan = scans[v];

@@ -242,7 +242,7 @@ private:
         const void* p[16];
         const StepRecord* record;
         cudaEvent_t positions_ready;
-        bool staged;
+        bool staged, masks;
         bool operator==(const GraphKey& o) const;
     };
     struct GraphEntry {
@@ -309,7 +309,9 @@ private:
     // also depends on how dense the particles are (staged_fit.h).
     bool may_run_staged(const LaunchShape& shape) const;
     StagedFit fit_;
-    bool staged_step_ = false;   // the step being launched does
+    // Whether per-lane steps with `shape` may store their lists as hit masks.
+    bool may_store_masks(const LaunchShape& shape) const;
+    bool staged_step_ = false, mask_step_ = false;   // the step being launched does
     bool packed_radii_ = true;   // every support radius is in the packed arithmetic's range
     uint32_t one_wave_ = 0;      // particles of the per-lane passes that are resident at once
     int launch_staged(cudaStream_t stream, const pbf_particle_state* state, pbf_particle_state* next_state, StepRecord& r);

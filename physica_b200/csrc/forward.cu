@@ -77,6 +77,7 @@ struct RangeScan {
     }
 };
 
+template <bool Masks>
 __global__ void __launch_bounds__(kBlock, 12) list_walk_kernel(const ListScanArgs a) {
     after_predecessor();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -128,6 +129,20 @@ __global__ void __launch_bounds__(kBlock, 12) list_walk_kernel(const ListScanArg
     } else if (a.packed.x) {
         // At 1M particles the packed test cut a scan from 0.233 to 0.200 ms.  A budget of 40
         // registers (12 blocks of 128 per SM) measured fastest; 45 and 52 were within 1 %.
+        if constexpr (Masks) {
+            const uint32_t pair_capacity = scan.capacity / 2u;
+            uint2* row = reinterpret_cast<uint2*>(a.list.entries) + mask_row(s, pair_capacity);
+            uint32_t pairs = 0;
+#pragma unroll 1
+            for (int o = 0; o < 9; ++o) {
+                const int x = c.x + o / 3 - 1, y = c.y + o % 3 - 1;
+                if (x < 0 || x >= cx || y < 0 || y >= cy) continue;
+                packed.run_masks(a.packed, offsets[cell_index(grid, x, y, z_lo)], offsets[cell_index(grid, x, y, z_hi) + 1u],
+                                 row, pair_capacity, pairs);
+            }
+            a.list.counts[s] = pairs <= pair_capacity ? packed.n : kOverflow;
+            return;
+        }
 #pragma unroll 1
         for (int o = 0; o < 9; ++o) {
             const int x = c.x + o / 3 - 1, y = c.y + o % 3 - 1;
@@ -373,10 +388,15 @@ __global__ void __launch_bounds__(kBlock) density_lambda_kernel(const DensityLam
 #endif
 constexpr uint32_t kStagedEntries = PBF_FUSED_STAGED_ENTRIES;   // 40: 20 KB of shared memory per 128-thread block
 
+// Masks: the list is stored as hit masks (one (base, mask) pair per block with a hit), the first
+// kStagedEntries / 2 pairs staged in the same shared memory.
+template <bool Masks>
 __global__ void __launch_bounds__(kBlock, PBF_FUSED_MIN_BLOCKS) scan_density_lambda_kernel(const ListScanArgs a,
                                                                                           const DensityLambdaArgs d) {
     after_predecessor();
-    __shared__ uint32_t staged[kStagedEntries * kBlock];
+    __shared__ __align__(8) uint32_t staged[kStagedEntries * kBlock];
+    constexpr uint32_t kStagedPairs = kStagedEntries / 2u;
+    uint2* const staged_pairs = reinterpret_cast<uint2*>(staged);
     const Particle p = locate(a.g);
     if (!p.active) return;
     const uint32_t s = p.s, lane_slot = threadIdx.x;
@@ -386,10 +406,12 @@ __global__ void __launch_bounds__(kBlock, PBF_FUSED_MIN_BLOCKS) scan_density_lam
     const uint32_t z_hi = static_cast<uint32_t>(p.c.z + 1 < cz ? p.c.z + 1 : cz - 1);
     const float4 xi = a.pos[s];
     const uint32_t capacity = a.list.capacity;
+    const uint32_t pair_capacity = capacity / 2u;
     uint32_t* __restrict__ entries = a.list.entries + list_row(s, capacity);
+    uint2* __restrict__ pairs_row = reinterpret_cast<uint2*>(a.list.entries) + mask_row(s, pair_capacity);
     const uint32_t* __restrict__ offsets = a.g.cell_offsets;
     // 1. the per-lane packed scan (PackedScan), appending to the stored list and the stage
-    uint32_t n = 0;
+    uint32_t n = 0, pairs = 0;
     {
         PackedScan scan;
         scan.nx = make_float2(-xi.x, -xi.x);
@@ -406,16 +428,26 @@ __global__ void __launch_bounds__(kBlock, PBF_FUSED_MIN_BLOCKS) scan_density_lam
             if (first >= end) continue;
             for (uint32_t base = first & ~3u; base < end; base += 32u) {
                 uint32_t mask = scan.block_mask(pk, base, first, end);
-                while (mask) {
-                    const uint32_t k = static_cast<uint32_t>(__ffs(mask)) - 1u;
-                    if (n < capacity) entries[static_cast<size_t>(n) * 32u] = base + k;
-                    if (n < kStagedEntries) staged[n * kBlock + lane_slot] = base + k;
-                    ++n;
-                    mask &= mask - 1u;
+                if constexpr (Masks) {
+                    if (mask) {
+                        const uint2 pair = make_uint2(base, mask);
+                        if (pairs < pair_capacity) pairs_row[static_cast<size_t>(pairs) * 32u] = pair;
+                        if (pairs < kStagedPairs) staged_pairs[pairs * kBlock + lane_slot] = pair;
+                        ++pairs;
+                        n += static_cast<uint32_t>(__popc(mask));
+                    }
+                } else {
+                    while (mask) {
+                        const uint32_t k = static_cast<uint32_t>(__ffs(mask)) - 1u;
+                        if (n < capacity) entries[static_cast<size_t>(n) * 32u] = base + k;
+                        if (n < kStagedEntries) staged[n * kBlock + lane_slot] = base + k;
+                        ++n;
+                        mask &= mask - 1u;
+                    }
                 }
             }
         }
-        const bool overflow = n > capacity;
+        const bool overflow = Masks ? pairs > pair_capacity : n > capacity;
         a.list.counts[s] = overflow ? kOverflow : n;
         if (overflow) n = kOverflow;
     }
@@ -436,8 +468,29 @@ __global__ void __launch_bounds__(kBlock, PBF_FUSED_MIN_BLOCKS) scan_density_lam
     if (n == kOverflow) {
         walk(op, p, a.g);
     } else if (n > 0) {
+        uint2 current{}, upcoming{};
+        uint32_t next_pair = 2u;
+        auto pair_at = [&](const uint32_t j) -> uint2 {
+            return j < kStagedPairs ? staged_pairs[j * kBlock + lane_slot] : pairs_row[static_cast<size_t>(j) * 32u];
+        };
+        if constexpr (Masks) {
+            current = pair_at(0);
+            upcoming = pairs > 1u ? pair_at(1) : make_uint2(0u, 0u);
+        }
         auto entry = [&](const uint32_t k) -> uint32_t {
-            return k < kStagedEntries ? staged[k * kBlock + lane_slot] : entries[static_cast<size_t>(k) * 32u];
+            if constexpr (Masks) {
+                (void)k;
+                if (current.y == 0u) {
+                    current = upcoming;
+                    upcoming = next_pair < pairs ? pair_at(next_pair) : make_uint2(0u, 0u);
+                    ++next_pair;
+                }
+                const uint32_t bit = static_cast<uint32_t>(__ffs(static_cast<int>(current.y))) - 1u;
+                current.y &= current.y - 1u;
+                return current.x + bit;
+            } else {
+                return k < kStagedEntries ? staged[k * kBlock + lane_slot] : entries[static_cast<size_t>(k) * 32u];
+            }
         };
         uint32_t t = entry(0);
         uint32_t tn = n > 1u ? entry(1) : 0u;
@@ -473,7 +526,7 @@ __global__ void __launch_bounds__(kBlock, PBF_FUSED_MIN_BLOCKS) scan_density_lam
 #define PBF_POST_MIN_BLOCKS 10
 #endif
 
-template <bool WithBoundary>
+template <bool WithBoundary, bool Masks>
 __global__ void __launch_bounds__(kBlock, PBF_CORRECTION_MIN_BLOCKS) correction_kernel(const CorrectionArgs a) {
     after_predecessor();
     const Particle p = locate(a.g);
@@ -496,7 +549,7 @@ __global__ void __launch_bounds__(kBlock, PBF_CORRECTION_MIN_BLOCKS) correction_
     op.artificial_full = pb.x != 0.0F;
     op.reference_weight = op.artificial_full ? poly6(mk(pb.z, 0.0F, 0.0F), p.k) : 1.0F;
     op.correction = mk(0.0F, 0.0F, 0.0F);
-    replay<2>(op, p, a.g, a.list);
+    replay_list<Masks>(op, p, a.g, a.list);
     const Box& box = p.scene->box;
     const f3 candidate = add(op.x, op.correction);
     uint32_t mask = 0u;
@@ -524,6 +577,7 @@ __global__ void __launch_bounds__(kBlock, PBF_CORRECTION_MIN_BLOCKS) correction_
 }
 
 // ---------------------------------------------------------------- vorticity
+template <bool Masks>
 __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) vorticity_kernel(const VorticityArgs a) {
     after_predecessor();
     const Particle p = locate(a.g);
@@ -536,11 +590,12 @@ __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) vorticity_kernel(
     op.x = xyz(a.pos[p.s]);
     op.v = xyz(a.velocity[p.s]);
     op.vorticity = mk(0.0F, 0.0F, 0.0F);
-    replay<2>(op, p, a.g, a.list);
+    replay_list<Masks>(op, p, a.g, a.list);
     a.vorticity[p.s] = make_float4(op.vorticity.x, op.vorticity.y, op.vorticity.z, __fsqrt_rn(sq_xfirst(op.vorticity)));
 }
 
 // ------------------------------------------------------- normal + confinement
+template <bool Masks>
 __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) normal_kernel(const NormalArgs a) {
     after_predecessor();
     const Particle p = locate(a.g);
@@ -554,7 +609,7 @@ __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) normal_kernel(con
     op.x = xyz(a.pos[p.s]);
     op.magnitude = wi.w;
     op.gradient = mk(0.0F, 0.0F, 0.0F);
-    replay<2>(op, p, a.g, a.list);
+    replay_list<Masks>(op, p, a.g, a.list);
     const float normalizer = __fsqrt_rn(sq_yfirst(op.gradient));
     const f3 normal = normalizer > 0.0F ? scale(op.gradient, __fdiv_rn(1.0F, normalizer)) : mk(0.0F, 0.0F, 0.0F);
     a.normal[p.s] = make_float4(normal.x, normal.y, normal.z, normalizer);
@@ -565,6 +620,7 @@ __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) normal_kernel(con
 }
 
 // ---------------------------------------------------------------------- XSPH
+template <bool Masks>
 __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) xsph_kernel(const XsphArgs a) {
     after_predecessor();
     const Particle p = locate(a.g);
@@ -577,7 +633,7 @@ __global__ void __launch_bounds__(kBlock, PBF_POST_MIN_BLOCKS) xsph_kernel(const
     op.x = xyz(a.pos[p.s]);
     op.v = xyz(a.confined[p.s]);
     op.smoothing = mk(0.0F, 0.0F, 0.0F);
-    replay<2>(op, p, a.g, a.list);
+    replay_list<Masks>(op, p, a.g, a.list);
     const float viscosity = a.g.params_a[p.s].z;
     const f3 out = fma3(viscosity, op.smoothing, op.v);
     const uint32_t i = a.sorted_index[p.s];
@@ -701,8 +757,8 @@ unsigned block_of(const unsigned block) {
 }
 }  // namespace
 
-cudaError_t fused_scan_wave(uint32_t& particles) { return one_wave(scan_density_lambda_kernel, kBlock, particles); }
-cudaError_t list_walk_wave(uint32_t& particles) { return one_wave(list_walk_kernel, kBlock, particles); }
+cudaError_t fused_scan_wave(uint32_t& particles) { return one_wave(scan_density_lambda_kernel<false>, kBlock, particles); }
+cudaError_t list_walk_wave(uint32_t& particles) { return one_wave(list_walk_kernel<false>, kBlock, particles); }
 
 cudaError_t launch_list_scan(cudaStream_t stream, const ListScanArgs& a, const LaunchShape& shape) {
     if (a.g.count == 0) return cudaSuccess;
@@ -710,12 +766,15 @@ cudaError_t launch_list_scan(cudaStream_t stream, const ListScanArgs& a, const L
     // the cooperative and staged scans list fluid particles only; lists with boundary particles
     // use the per-lane walk
     const bool fluid_only = !(a.boundary && a.g.boundary_offsets);
-    if (shape.scan == kScanCooperative && fluid_only)
+    if (a.list.masks) {   // the per-lane packed walk, scenes without boundary particles
+        if (!fluid_only || !a.packed.x) return cudaErrorInvalidValue;
+        launch_after(stream, list_walk_kernel<true>, grid_of(a.g.count, block), block, a);
+    } else if (shape.scan == kScanCooperative && fluid_only)
         launch_after(stream, list_scan_kernel, grid_of(a.g.count, block), block, a);
     else if (shape.scan == kScanStaged && fluid_only)
         launch_after(stream, list_staged_kernel, grid_of(a.g.count, block), block, a);
     else
-        launch_after(stream, list_walk_kernel, grid_of(a.g.count, block), block, a);
+        launch_after(stream, list_walk_kernel<false>, grid_of(a.g.count, block), block, a);
     count_launch();
     return cudaGetLastError();
 }
@@ -724,13 +783,15 @@ cudaError_t launch_scan_density_lambda(cudaStream_t stream, const ListScanArgs& 
                                        const LaunchShape& shape) {
     if (a.g.count == 0) return cudaSuccess;
     const unsigned block = block_of(shape.scan_block);
-    launch_after(stream, scan_density_lambda_kernel, grid_of(a.g.count, block), block, a, d);
+    launch_after(stream, a.list.masks ? scan_density_lambda_kernel<true> : scan_density_lambda_kernel<false>,
+                 grid_of(a.g.count, block), block, a, d);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_density_lambda(cudaStream_t stream, const DensityLambdaArgs& a, const unsigned block_size) {
     if (a.g.count == 0) return cudaSuccess;
+    if (a.list.masks) return cudaErrorInvalidValue;   // hit masks are read by the fused scan only
     const unsigned block = block_of(block_size);
     if (a.g.boundary)
         launch_after(stream, density_lambda_kernel<true>, grid_of(a.g.count, block), block, a);
@@ -744,9 +805,11 @@ cudaError_t launch_correction(cudaStream_t stream, const CorrectionArgs& a, cons
     if (a.g.count == 0) return cudaSuccess;
     const unsigned block = block_of(block_size);
     if (a.g.boundary) {
-        launch_after(stream, correction_kernel<true>, grid_of(a.g.count, block), block, a);
+        if (a.list.masks) return cudaErrorInvalidValue;
+        launch_after(stream, correction_kernel<true, false>, grid_of(a.g.count, block), block, a);
     } else {
-        launch_after(stream, correction_kernel<false>, grid_of(a.g.count, block), block, a);
+        launch_after(stream, a.list.masks ? correction_kernel<false, true> : correction_kernel<false, false>,
+                     grid_of(a.g.count, block), block, a);
     }
     count_launch();
     return cudaGetLastError();
@@ -755,7 +818,7 @@ cudaError_t launch_correction(cudaStream_t stream, const CorrectionArgs& a, cons
 cudaError_t launch_vorticity(cudaStream_t stream, const VorticityArgs& a, const unsigned block_size) {
     if (a.g.count == 0) return cudaSuccess;
     const unsigned block = block_of(block_size);
-    launch_after(stream, vorticity_kernel, grid_of(a.g.count, block), block, a);
+    launch_after(stream, a.list.masks ? vorticity_kernel<true> : vorticity_kernel<false>, grid_of(a.g.count, block), block, a);
     count_launch();
     return cudaGetLastError();
 }
@@ -763,7 +826,7 @@ cudaError_t launch_vorticity(cudaStream_t stream, const VorticityArgs& a, const 
 cudaError_t launch_normal(cudaStream_t stream, const NormalArgs& a, const unsigned block_size) {
     if (a.g.count == 0) return cudaSuccess;
     const unsigned block = block_of(block_size);
-    launch_after(stream, normal_kernel, grid_of(a.g.count, block), block, a);
+    launch_after(stream, a.list.masks ? normal_kernel<true> : normal_kernel<false>, grid_of(a.g.count, block), block, a);
     count_launch();
     return cudaGetLastError();
 }
@@ -771,7 +834,7 @@ cudaError_t launch_normal(cudaStream_t stream, const NormalArgs& a, const unsign
 cudaError_t launch_xsph(cudaStream_t stream, const XsphArgs& a, const unsigned block_size) {
     if (a.g.count == 0) return cudaSuccess;
     const unsigned block = block_of(block_size);
-    launch_after(stream, xsph_kernel, grid_of(a.g.count, block), block, a);
+    launch_after(stream, a.list.masks ? xsph_kernel<true> : xsph_kernel<false>, grid_of(a.g.count, block), block, a);
     count_launch();
     return cudaGetLastError();
 }

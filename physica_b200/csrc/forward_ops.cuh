@@ -56,6 +56,19 @@ struct PackedScan {
         if (first >= end) return;
         for (uint32_t base = first & ~3u; base < end; base += 32u) append(block_mask(p, base, first, end), base);
     }
+    // The same as hit masks: one pair per block with a hit; `pairs` counts them, n the neighbours.
+    __device__ __forceinline__ void run_masks(const PackedPositions p, const uint32_t first, const uint32_t end, uint2* row,
+                                              const uint32_t pair_capacity, uint32_t& pairs) {
+        if (first >= end) return;
+        for (uint32_t base = first & ~3u; base < end; base += 32u) {
+            const uint32_t mask = block_mask(p, base, first, end);
+            if (mask) {
+                if (pairs < pair_capacity) row[static_cast<size_t>(pairs) * 32u] = make_uint2(base, mask);
+                ++pairs;
+                n += static_cast<uint32_t>(__popc(mask));
+            }
+        }
+    }
 };
 
 // density (density/density.cu:18-40) and lambda (pbf/pbf.cu:95-127) of one particle in one walk.

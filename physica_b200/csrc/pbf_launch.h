@@ -58,13 +58,17 @@ cudaError_t launch_reference_order(cudaStream_t stream, uint32_t count, const Sc
                                    const uint32_t* sorted_index, const uint32_t* keys, const uint32_t* cell_offsets,
                                    const uint32_t* reference_offsets, uint32_t* out_index, unsigned long long* out_keys);
 
-// A stored neighbour list: `capacity` 32-bit words per particle, warp-interleaved, one sorted slot per
-// in-support neighbour, and the entries' count; kOverflow marks a particle whose list did not fit (it
-// walks its stencil instead).  The staged passes pack two entries in a word (StagedList).
+// A stored neighbour list: `capacity` 32-bit words per particle, warp-interleaved, and a count.
+// - lists of slots (masks = 0): one sorted slot per in-support neighbour, counts = entries;
+// - hit masks (masks = 1): one (slot of bit 0, 32-bit hit mask) pair per 32-slot block of a stencil column that holds a
+//   neighbour, capacity / 2 pairs per particle, counts = neighbours.
+// Either lists the same neighbours in the same order; kOverflow marks a particle whose list did not fit (it walks its
+// stencil instead).  The staged passes pack two entries in a word (StagedList).
 struct StoredList {
     uint32_t* entries = nullptr;
     uint32_t* counts = nullptr;
     uint32_t capacity = 0;
+    int masks = 0;
 };
 
 // Common inputs of every neighbour-gather pass.
@@ -175,10 +179,11 @@ enum ListScanVariant : uint32_t {
     kScanFusedDensity = 3,  // per lane, and the Jacobi iterations' scans also run density + lambda
                             // in the same kernel (scenes without boundary particles)
     kScanStaged16 = 4,      // every forward pass of scenes without boundary particles over windows staged in
-                            // shared memory (staged.cu) at the sizes where that is faster; otherwise as 3
+                            // shared memory (staged.cu) where that is faster; otherwise as 3, in forward mode
+                            // with hit masks where those are
 };
 struct LaunchShape {
-    uint32_t scan = kScanStaged16;   // chooses the faster passes by size, method, radius and density
+    uint32_t scan = kScanStaged16;   // chooses the faster passes and lists by size, method, radius and density
     uint32_t scan_block = 128;   // threads per block of the list scan: 32, 64, 96 or 128
     uint32_t block = 128;        // threads per block of the gather passes: 32, 64, 96 or 128
 };

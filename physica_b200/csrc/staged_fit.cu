@@ -18,32 +18,34 @@ using namespace staged_detail;
 
 // Blocks of the measurement's kernel: about as many as are resident at once, since each ends with an atomic on one word.
 constexpr uint32_t kMaxBlocks = 2048;
-// Steps from one measurement to the next.  A measurement takes 8 us at 5k particles, 10 at 262k, 24 at 1M (SPH: 9), a step
-// 0.09, 0.5 and 3.4 ms, a differentiable one (2^19 particles or more) 1 ms and up.
-constexpr uint32_t kEvery[4] = {8, 16, 4, 16};
+// Steps from one measurement to the next.  A measurement takes 8 us at 5k particles and 10 at 262k, a step 0.09 and 0.5 ms; a
+// differentiable one (2^19 particles or more) 24 us at 1M, a step 1 ms and up.
+constexpr uint32_t kEvery[5] = {8, 16, 4, 16, 16};
 
 // The staged passes pay while few of the warps hold a particle without room: at most `columns` of them one whose
 // stencil columns outgrow its hit record, which leaves its warp waiting in every pass, and at most `unfit` one
-// of either kind (a block whose windows outgrow the stage costs its own time only).  They also pay, up to half of
-// the warps, where any particle has more than `candidates`: it overflows the per-lane passes' list, and a stencil walk
-// takes as long as its whole scene; and above, once `crowded` of the warps do.  A sphere of the support radius
-// holds 4 pi / 3 / 27 of its stencil's particles, so 598 candidates fill a list of kListCapacity at an even density.
+// of either kind (a block whose windows outgrow the stage costs its own time only).  Where the per-lane passes keep
+// lists of slots (grouped and differentiable steps) the staged ones also pay, up to half of the warps, if any
+// particle has more than `candidates`: it overflows its list, and its stencil walk takes as long as the rest of its
+// scene; and above, once `crowded` of the warps hold one.  A sphere of the support radius holds 4 pi / 3 / 27 of its stencil's
+// particles, so 598 candidates fill a list of kListCapacity at an even density; small scenes wait for the few lists that
+// later iterations overflow, and count from 500 (480) on.
 // Staged / per lane, ms a step (lattices by the spacings in a radius; dam breaks by the step; shares of columns, all):
-//   forward, 262k and 1M: 2.15 (0.18, 0.18) 0.731 / 0.668; step 20 (0.08, 0.12) 0.929 / 0.907; 1M step 25 (0.09, 0.12)
-//     4.65 / 5.27; 256 scenes step 40 (0.10, 0.26) 10.73 / 10.38; a few crowded ones at step 60 (0.11, 0.20) 1.302 / 1.879;
-//     crowded 0.01 at 2.7 1.920 / 1.799, 0.53 at 2.8 1.992 / 2.211
-//   grouped, 14k: 2.1 (0, 0) 0.176 / 0.215, 2.15 (0.07, 0.07) 0.275 / 0.232; step 100 (0, 0.14) 0.235 / 0.251; more than 500
-//     candidates (such scenes wait for the few lists that the later iterations overflow): 0.12 0.428 / 0.391, 0.59 0.459 / 0.761
+//   forward: 262k 2.1 (0.02, 0.02) 0.547 / 0.596, 2.15 (0.18, 0.18) 0.730 / 0.651, step 20 (0.08, 0.12) 0.929 / 0.864; 1M step 30
+//     (0.11, 0.14) 4.90 / 5.04, step 100 (0.04, 0.14) 4.37 / 4.32; 256 scenes step 20 (0.01, 0.09) 8.62 / 9.91, 40 (0.10, 0.26) 10.73 / 9.88
+//   grouped, 14k: 2.1 (0, 0) 0.176 / 0.215, 2.15 (0.07, 0.07) 0.275 / 0.232; step 100 (0, 0.14) 0.235 / 0.251; crowded 0.12
+//     0.428 / 0.391, 0.59 0.459 / 0.761
 //   differentiable, which write both lists: 32 scenes step 20 (0.02, 0.07) 5.74 / 5.96, step 2 (0, 0.22) 5.61 / 4.93; 600k
 //     2.1 (0.05, 0.05) 1.239 / 1.222, 2.15 (0.2, 0.2) 1.634 / 1.327; crowded 0.59 5.744 / 3.942, 0.82 6.276 / 9.115
 //   SPH (PCISPH), 262k: 2.1 (0.02, 0.02) 0.890 / 0.931, 2.15 (0.18, 0.18) 1.090 / 1.032; crowded ones fall back to the
 //     per-lane lists
+// In between, hit masks / lists of slots: 60k 2.6 (crowded 0.2) 0.487 / 0.471, 2.7 (0.6) 0.511 / 0.696, 3 0.669 / 2.116.
 struct Limits {
     uint32_t candidates;
     float columns, unfit, crowded;
 };
-constexpr Limits kLimits[4] = {{598u, 0.15F, 0.2F, 0.5F}, {500u, 0.03F, 0.2F, 0.25F}, {598u, 0.1F, 0.1F, 0.7F},
-                               {~0u, 0.06F, 0.15F, 1.0F}};
+constexpr Limits kLimits[5] = {{~0u, 0.1F, 0.13F, 1.0F}, {500u, 0.03F, 0.2F, 0.25F}, {598u, 0.1F, 0.1F, 0.7F},
+                               {~0u, 0.06F, 0.15F, 1.0F}, {480u, 0.0F, 0.0F, 1.0F}};
 constexpr float kCrowdedUnfit = 0.5F;
 
 enum Share { kColumns, kUnfit, kCrowded, kShares };
@@ -212,10 +214,9 @@ cudaError_t StagedFit::measure(cudaStream_t stream, const GatherCommon& g) {
     }
     ++calls_;
     const uint32_t particles = kind_ == kGrouped ? kGroupParticles : kBlockParticles;
-    // Every block where one crowded particle decides; an SPH step of 1M particles is as short as 0.6 ms, and 1024 of its
-    // blocks tell its shares.
+    // every block where one crowded particle decides, a sample otherwise
     const uint32_t all = (g.count + particles - 1u) / particles;
-    const uint32_t stride = kind_ == kSph ? std::max(1u, all / 1024u) : 1u;
+    const uint32_t stride = kLimits[kind_].candidates == ~0u ? std::max(1u, all / 1024u) : 1u;
     const uint32_t blocks = (all + stride - 1u) / stride;
     launch_after(stream, staged_fit_kernel, std::min(blocks, kMaxBlocks), particles,
                  FitArgs{g, blocks, stride, kind_ == kGrouped ? kGroupStage : kStage, kLimits[kind_].candidates, tag_, counts_, device_word_});
@@ -223,14 +224,25 @@ cudaError_t StagedFit::measure(cudaStream_t stream, const GatherCommon& g) {
     return cudaGetLastError();
 }
 
-bool StagedFit::pays() const {
-    if (!word_) return true;
+uint64_t StagedFit::measured() const {
+    if (!word_) return 0u;
     const uint64_t word = *static_cast<const volatile uint64_t*>(word_);
-    if (static_cast<uint32_t>(word >> 48) != tag_) return true;   // not measured yet
-    auto share = [word](const Share k) { return static_cast<float>((word >> (16 * k)) & 0xffffu) / 65535.0F; };
-    const Limits& limits = kLimits[kind_];
-    return (share(kColumns) <= limits.columns && share(kUnfit) <= limits.unfit) ||
-           (share(kCrowded) > 0.0F && share(kUnfit) <= kCrowdedUnfit) || share(kCrowded) > limits.crowded;
+    return static_cast<uint32_t>(word >> 48) == tag_ ? word : 0u;   // otherwise another solver's
 }
+
+namespace {
+float share_of(const uint64_t word, const Share k) { return static_cast<float>((word >> (16 * k)) & 0xffffu) / 65535.0F; }
+}  // namespace
+
+bool StagedFit::pays() const {
+    const uint64_t word = measured();
+    if (word == 0u) return true;
+    const Limits& limits = kLimits[kind_];
+    const float unfit = share_of(word, kUnfit), crowded = share_of(word, kCrowded);
+    return (share_of(word, kColumns) <= limits.columns && unfit <= limits.unfit) || (crowded > 0.0F && unfit <= kCrowdedUnfit) ||
+           crowded > limits.crowded;
+}
+
+bool StagedFit::crowded() const { return share_of(measured(), kCrowded) > 0.0F; }
 
 }  // namespace pbf

@@ -21,7 +21,8 @@ class DeviceArena;
 
 class StagedFit {
 public:
-    enum Kind { kForward, kGrouped, kDifferentiable, kSph };   // kGrouped: four lanes a particle
+    // kGrouped: four lanes a particle; kMiddle: sizes that never run staged passes
+    enum Kind { kForward, kGrouped, kDifferentiable, kSph, kMiddle };
 
     StagedFit() = default;
     StagedFit(const StagedFit&) = delete;
@@ -33,8 +34,11 @@ public:
     cudaError_t measure(cudaStream_t stream, const GatherCommon& g);
     // Whether the staged passes are the faster ones.
     bool pays() const;
+    // Whether particles are so crowded that the per-lane passes' lists of slots overflow.
+    bool crowded() const;
 
 private:
+    uint64_t measured() const;          // 0: nothing yet
     uint32_t* counts_ = nullptr;        // device scratch
     const uint64_t* word_ = nullptr;    // pinned: a tag and the shares measured
     uint64_t* device_word_ = nullptr;   // the same for the device

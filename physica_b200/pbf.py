@@ -94,7 +94,7 @@ class LaunchShape:
     list_scan: 0 = per-lane walk, 1 = warp-cooperative scan, 2 = shared-memory staged walk,
     3 = per-lane walk with each Jacobi iteration's density + lambda in the same kernel,
     4 (a new solver's) = as 3, and steps without boundary particles run over windows staged in shared memory
-    at the sizes where that is faster (up to 20,480 or more than 170,496 particles; differentiable: from 2^19);
+    (up to 20,480 or more than 170,496 particles; differentiable: from 2^19) or keep hit masks, where that is faster;
     scan_block_size (list scan) and
     block_size (gather passes): 32, 64, 96 or 128."""
     list_scan: int = 0

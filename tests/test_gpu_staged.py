@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 PER_LANE, STAGED = pbf.LaunchShape(0, 128, 128), pbf.LaunchShape(4, 128, 128)
 
 
-def run(scene, shape, steps):
+def run(scene, shape, steps, fields=True):
     solver, state, control, params = pbf.solver_for_scene(scene)
     solver.launch_shape = shape
     cache, following = solver.allocate_step_cache(), solver.allocate_state()
@@ -23,15 +23,15 @@ def run(scene, shape, steps):
         out += [following.positions.clone(), following.velocities.clone()]
         for field in (pbf.CacheField.FIRST_DENSITIES, pbf.CacheField.FIRST_LAMBDAS, pbf.CacheField.NEIGHBOR_COUNTS,
                       pbf.CacheField.VORTICITY_MAGNITUDES, pbf.CacheField.VORTICITY_NORMALS, pbf.CacheField.CONFINED_VELOCITIES,
-                      pbf.CacheField.CORRECTED_POSITIONS, pbf.CacheField.RECONSTRUCTED_VELOCITIES):
+                      pbf.CacheField.CORRECTED_POSITIONS, pbf.CacheField.RECONSTRUCTED_VELOCITIES) if fields else ():
             out.append(cache.read(field))
         state, following = following, state
     solver.synchronize()
     return [t.cpu().numpy() for t in out]
 
 
-def check(scene, steps=3):
-    for a, b in zip(run(scene, PER_LANE, steps), run(scene, STAGED, steps)):
+def check(scene, steps=3, **options):
+    for a, b in zip(run(scene, PER_LANE, steps, **options), run(scene, STAGED, steps, **options)):
         np.testing.assert_array_equal(a.view(np.int32), b.view(np.int32))
 
 
@@ -63,6 +63,24 @@ def test_sizes_choose_the_passes(count, staged):
         launches = pbf.launch_count() - before
         state, following = following, state
     assert launches == (15 if staged else 16)
+
+
+@pytest.mark.parametrize("iterations", [0, 3])
+@pytest.mark.parametrize("kind", ["block", "spray", "crowded", "coincident"])
+def test_hit_mask_lists(kind, iterations):
+    """From 140,001 to 170,496 particles variant 4 runs the per-lane passes over hit masks."""
+    n = 140001 + iterations
+    s = block(n, seed=14, iterations=iterations)
+    rng = np.random.default_rng(15)
+    if kind == "spray":
+        fly = rng.permutation(n)[:n // 9]
+        s.positions[:, fly] = (rng.random((3, n // 9)) * np.asarray(s.box_max)[:, None]).astype(np.float32)
+    if kind == "crowded":   # up to 3,000 candidates: more than 48 masks
+        s.positions[:, :3000] = (0.2 + 0.06 * rng.random((3, 3000))).astype(np.float32)
+    if kind == "coincident":
+        s.positions[:, 100:200], s.velocities[:, 100:200] = s.positions[:, 200:300], s.velocities[:, 200:300]
+        s.masses[:] *= rng.choice([0.5, 1.0], n).astype(np.float32)
+    check(s, steps=2, fields=iterations > 0)
 
 
 @pytest.mark.parametrize("count,steps", [(13824, 100), (175616, 25)])

@@ -49,10 +49,11 @@ def run(scene, shape, count=3, graph=False):
 
 @pytest.mark.parametrize("graph", [False, True])
 @pytest.mark.parametrize("count,ratio,staged", [(8000, 2.0, True), (8000, 2.4, False), (8000, 3.0, True),
-                                                (64000, 2.0, False),
-                                                (185193, 2.0, True), (185193, 2.3, False), (185193, 3.2, True)])
+                                                (64000, 2.0, False), (64000, 2.9, False), (64000, 4.0, False),
+                                                (185193, 2.0, True), (185193, 2.3, False), (185193, 3.2, False)])
 def test_density_decides(count, ratio, staged, graph):
-    """Also: at a radius of three spacings and more the per-lane lists overflow, and the staged passes' hit masks are faster."""
+    """At a radius of 2.8 spacings and more lists of slots overflow: a small scene stays with the staged passes and their hit
+    masks, the others keep hit masks in the per-lane passes."""
     scene = lattice(count, ratio)
     out, launches = run(scene, pbf.LaunchShape(4, 128, 128), graph=graph)
     assert launches[1:] == [PBF_LAUNCHES[staged]] * 2, launches
