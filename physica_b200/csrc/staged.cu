@@ -11,8 +11,8 @@
 // Reading neighbours through L1 instead (lists of sorted slots or of hit masks, one pair at a time), a
 // pass waited on scattered loads and issued 70 instructions per pair, half of them for the IEEE root and
 // divisions.  At 1M particles, ms per launch before and now: scan + density/lambda 0.293 -> 0.262,
-// correction 0.155 -> 0.107, post-loop scan and vorticity 0.143 + 0.158 -> 0.305, normal 0.151 -> 0.096,
-// XSPH 0.157 -> 0.120.  What bounds them now: the scan issues 70 % of its cycles, and the replays keep
+// correction 0.155 -> 0.107, normal 0.151 -> 0.096, XSPH 0.157 -> 0.120; the post-loop scan and the vorticity,
+// 0.143 + 0.158 before and 0.305 in one kernel now, save a launch and no time.  What bounds them now: the scan issues 70 % of its cycles, and the replays keep
 // the shared-memory pipe 70-78 % busy.
 //
 // Blocks of 64 or 32 particles stage 12.4 and 15.9 slots per particle and were slower (0.264 and 0.298 ms
