@@ -320,13 +320,12 @@ __global__ void __launch_bounds__(kThreads) group_vorticity_kernel(const StagedV
         [&](const uint32_t i0, const uint32_t i1, float2 (&t0)[3], float2 (&t1)[3]) {
             const TwoPairs t = two_pairs(xi, mk(field[0][i0], field[1][i0], field[2][i0]),
                                          mk(field[0][i1], field[1][i1], field[2][i1]));
+            float2 spiky = spiky_scale_pair(t.nr2, p.k);
+            const bool rare = !in_range(t.nr2, p.k);
+            if (rare) spiky = any_spiky_scales(t.nr2, p.k);
             f3 v0 = sub(mk(field[3][i0], field[4][i0], field[5][i0]), vi);
             f3 v1 = sub(mk(field[3][i1], field[4][i1], field[5][i1]), vi);
-            float2 spiky = spiky_scale_pair(t.nr2, p.k);
-            if (!in_range(t.nr2, p.k)) {
-                spiky = any_spiky_scales(t.nr2, p.k);
-                only_inside(spiky, v0, v1);
-            }
+            if (rare) only_inside(spiky, v0, v1);
             const f3 c0 = cross_f(v0, scale(t.d0, spiky.x));
             const f3 c1 = cross_f(v1, scale(t.d1, spiky.y));
             t0[0] = make_float2(0.0F, c0.x);
@@ -379,12 +378,11 @@ __global__ void __launch_bounds__(kThreads) group_normal_kernel(const StagedNorm
         [&](const uint32_t i0, const uint32_t i1, float2 (&t0)[3], float2 (&t1)[3]) {
             const TwoPairs t = two_pairs(xi, mk(field[0][i0], field[1][i0], field[2][i0]),
                                          mk(field[0][i1], field[1][i1], field[2][i1]));
-            float f0 = __fsub_rn(field[3][i0], wi.w), f1 = __fsub_rn(field[3][i1], wi.w);
             float2 spiky = spiky_scale_pair(t.nr2, p.k);
-            if (!in_range(t.nr2, p.k)) {
-                spiky = any_spiky_scales(t.nr2, p.k);
-                only_inside(spiky, f0, f1);
-            }
+            const bool rare = !in_range(t.nr2, p.k);
+            if (rare) spiky = any_spiky_scales(t.nr2, p.k);
+            float f0 = __fsub_rn(field[3][i0], wi.w), f1 = __fsub_rn(field[3][i1], wi.w);
+            if (rare) only_inside(spiky, f0, f1);
             const f3 g0 = scale(t.d0, spiky.x), g1 = scale(t.d1, spiky.y);
             t0[0] = make_float2(f0, g0.x);
             t0[1] = make_float2(f0, g0.y);
@@ -423,13 +421,12 @@ __global__ void __launch_bounds__(kThreads) group_xsph_kernel(const StagedXsphAr
         [&](const uint32_t i0, const uint32_t i1, float2 (&t0)[3], float2 (&t1)[3]) {
             const TwoPairs t = two_pairs(xi, mk(field[0][i0], field[1][i0], field[2][i0]),
                                          mk(field[0][i1], field[1][i1], field[2][i1]));
+            float2 weight = poly6_pair(t.nr2, p.k);
+            const bool rare = !in_range(t.nr2, p.k);
+            if (rare) weight = any_poly6s(t.nr2, p.k);
             f3 v0 = sub(mk(field[3][i0], field[4][i0], field[5][i0]), vi);
             f3 v1 = sub(mk(field[3][i1], field[4][i1], field[5][i1]), vi);
-            float2 weight = poly6_pair(t.nr2, p.k);
-            if (!in_range(t.nr2, p.k)) {
-                weight = any_poly6s(t.nr2, p.k);
-                only_inside(weight, v0, v1);
-            }
+            if (rare) only_inside(weight, v0, v1);
             t0[0] = make_float2(weight.x, v0.x);
             t0[1] = make_float2(weight.x, v0.y);
             t0[2] = make_float2(weight.x, v0.z);

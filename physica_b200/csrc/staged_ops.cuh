@@ -42,6 +42,9 @@ __device__ __forceinline__ float2 any_poly6s(const float2 nr2, const KernelConst
 }
 
 // A pair whose kernel value is zero adds nothing, whatever its other factor is (it may be infinite).
+// Called in the branch that such pairs take.  With one lane a particle the factors are formed before that branch (262k
+// particles, three iterations: 0.500 against 0.504 ms a step), with four behind it, so that no call has them in flight (14k:
+// normal 18.7 against 20.1 us, XSPH 18.2 against 19.5).
 __device__ __forceinline__ void only_inside(const float2 kernel, float& f0, float& f1) {
     if (kernel.x == 0.0F) f0 = 0.0F;
     if (kernel.y == 0.0F) f1 = 0.0F;
